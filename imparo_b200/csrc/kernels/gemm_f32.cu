@@ -1,14 +1,24 @@
-// True 32-bit matrix product: out[M,N] (+)= A[M,K] * W[N,K]^T, FFMA only.
+// True 32-bit matrix product: out[M,N] (+)= A[M,K] * W[N,K]^T.
 //
-// This is the matrix product of the 32-bit path: no tensor cores, no reduced-precision
-// mode.  Every output element is one accumulator summed over k = 0..K-1 in order, so a
-// row's result does not depend on how many other rows the call carries.  Layout follows
-// the reference: W[n_out, n_in] row-major, y[t,o] = sum_i W[o,i]*x[t,i]
-// (imparo-cpu/src/ops.rs:660,688-690).
-#include "common.cuh"
+// This is the matrix product of the 32-bit path.  Layout follows the reference: W[n_out, n_in] row-major,
+// y[t,o] = sum_i W[o,i]*x[t,i] (imparo-cpu/src/ops.rs:660,688-690).  A row's result depends neither on how many other
+// rows the call carries nor on where in the call it stands.
+//
+//  (1) sgemm_split_kernel: rows of 16-byte groups.  Every 32-bit operand is cut into three bfloat16 pieces that add up
+//      to it to its last bit (8 + 8 + 8 significant bits, each piece rounded to nearest, so the remainders carry either
+//      sign), and six of the nine products of pieces run on the tensor cores: what is left out is below 2^-26 of a
+//      product, a quarter of a 32-bit rounding.  The large product of a stretch of 64 k (first piece times first piece)
+//      is summed by the tensor core into an accumulator of its own, read back and added to the others' in registers with
+//      32-bit rounding: the tensor core's accumulator truncates, and over a whole K that adds up to more than the
+//      FFMA chain's error.  The five small products, 2^-8 of it and below, share one accumulator over all of K.
+//      Nothing of this leaves the 32-bit range: a result that is not finite (an operand or a piece of it that overflowed)
+//      is computed again by the FFMA chain, which then says what it is.
+//  (2) sgemm_nt_kernel: everything else, FFMA only, one accumulator per element summed over k = 0..K-1 in order.
+#include "tcgen05.cuh"
 
 namespace imparo {
 
+// ---- (2) ----------------------------------------------------------------------------------------------------------
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
 __global__ void __launch_bounds__(256)
@@ -66,12 +76,272 @@ sgemm_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
     }
 }
 
+
+// ---- (1) ----------------------------------------------------------------------------------------------------------
+namespace sp {
+
+using namespace imparo::tc;
+
+constexpr int TM = 128;                                       // rows of A per tile (tensor-memory lanes)
+constexpr int WORKERS = 16;                                   // warps that cut operands and read accumulators out
+constexpr int THREADS = 32 * (WORKERS + 1);                   // ... and one that issues the MMAs
+constexpr int STAGES = 2;
+
+template <int TN> constexpr uint32_t a_plane() { return TM * 128; }
+template <int TN> constexpr uint32_t b_plane() { return TN * 128; }
+template <int TN> constexpr uint32_t stage_bytes() { return 3 * (a_plane<TN>() + b_plane<TN>()); }
+template <int TN> constexpr size_t smem_bytes() { return 1024 + (size_t)STAGES * stage_bytes<TN>() + 256; }
+
+struct Params {
+    const float* a; const float* w; float* c;
+    int M, N, K, lda, ldc, accumulate, kblocks;
+    int* status;
+};
+
+// two neighbours cut into three bfloat16 pieces each (h + m + l is the operand, exactly), packed in pairs
+__device__ __forceinline__ void cut(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+    auto pack = [](float u, float v) { __nv_bfloat162 t = __floats2bfloat162_rn(u, v); return *reinterpret_cast<uint32_t*>(&t); };
+    h = pack(x, y);
+    x -= __uint_as_float(h << 16); y -= __uint_as_float(h & 0xffff0000u);
+    m = pack(x, y);
+    x -= __uint_as_float(m << 16); y -= __uint_as_float(m & 0xffff0000u);
+    l = pack(x, y);
+}
+
+template <int COLS>
+__device__ __forceinline__ void tmem_add(uint32_t taddr, float (&acc)[COLS]) {
+    float v[COLS / 16][16];
+    tmem_ld_chunks<COLS / 16>(taddr, v);
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) acc[j] += v[j >> 4][j & 15];
+}
+
+// one element by the FFMA chain: what a result that is not finite is
+__device__ __noinline__ float whole_sum(const float* x, const float* w, int K) {
+    float t = 0.f;
+    for (int k = 0; k < K; ++k) t = fmaf(x[k], w[k], t);
+    return t;
+}
+
+// One CTA per tile of TM x TN outputs.  A stretch of 64 k is 3 planes of A (16 KB each) and 3 of W in shared memory, in the
+// swizzled layout of a bfloat16 K-major operand; sixteen warps read the 32-bit operands (one stretch ahead, in registers),
+// cut them and store the planes, the seventeenth issues 24 MMAs of 128 x TN x 16; meanwhile the sixteen read the large
+// accumulator of the stretch before (two of them alternate).
+// What bounds it: shared memory.  The MMAs' operand reads and the planes' writes are 288 KB per stretch at TN = 128 (2,300
+// cycles at 128 bytes a cycle; the MMAs alone 1,540), 216 KB at TN = 64; measured 4,100 and 2,900 cycles per stretch (with
+// the large product alone 3,100 and 2,000).  Sixteen workers and not eight: the loop's straight code is half as long per
+// warp, and eight waited for instructions more than for anything else (1,000 x 9,216 x 1,024: 162 against 139 us).
+// Against the FFMA kernel (B200, us): 1,000 x 9,216 x 1,024: 837 -> 139 (136 TFLOP/s); 1,000 x 1,024 x 4,608: 920 -> 114;
+// 60 x 3,072 x 1,024: 77 -> 28; error against 64 bits 5.7e-7 -> 1.1e-7 (K 1,024), 1.2e-6 -> 1.8e-7 (K 4,608).
+template <int TN>
+__global__ void __launch_bounds__(THREADS, 1)
+sgemm_split_kernel(const Params p) {
+    constexpr uint32_t A_PLANE = a_plane<TN>(), B_PLANE = b_plane<TN>(), STAGE = stage_bytes<TN>();
+    constexpr uint32_t TMEM_COLS = TN == 128 ? 512 : 256;     // two large accumulators and the small products' one
+    constexpr int ROUND = WORKERS * 4;                        // rows of a stretch per round of the workers
+    constexpr int COLS = TN * 4 / WORKERS;                    // accumulator columns of a worker thread
+    constexpr int A_IT = TM / ROUND, B_IT = TN / ROUND;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE);      // [STAGES] the stage's planes are stored
+    uint64_t* empty = full + STAGES;                                          // [STAGES] ... and read by its MMAs
+    uint64_t* acc_full = empty + STAGES;                                      // [2] a stretch's large product is summed
+    uint64_t* acc_empty = acc_full + 2;                                       // [2] ... and in the workers' registers
+    uint64_t* done = acc_empty + 2;                                           // [1] every MMA is complete
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+    pdl_trigger();
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], WORKERS); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], WORKERS); }
+        mbar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == WORKERS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot, small = tmem + 2 * TN;
+
+    if (warp == WORKERS) {
+        if (lane == 0) {
+            const uint32_t idesc = instr_desc(TM, TN);
+            bool ok = true;
+            for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+                const int s = kb % STAGES, b = kb & 1;
+                if (kb >= 2 && !mbar_wait(&acc_empty[b], ((kb >> 1) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 90, blockIdx.x, kb); ok = false; break; }
+                if (!mbar_wait(&full[s], (kb / STAGES) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 91, blockIdx.x, kb); ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t a0 = smem_desc(smem_u32(smem) + s * STAGE), b0 = smem_desc(smem_u32(smem) + s * STAGE + 3 * A_PLANE);
+                auto product = [&](uint32_t d, int pa, int pb, bool first) {
+                    const uint64_t da = a0 + (uint64_t)((pa * A_PLANE) >> 4), db = b0 + (uint64_t)((pb * B_PLANE) >> 4);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        umma(d, da + (uint64_t)((k * UMMA_K * 2) >> 4), db + (uint64_t)((k * UMMA_K * 2) >> 4), idesc, (first && k == 0) ? 0u : 1u);
+                };
+                product(tmem + (uint32_t)b * TN, 0, 0, true);
+                umma_commit(&acc_full[b]);
+                product(small, 0, 1, kb == 0);
+                product(small, 1, 0, false);
+                product(small, 0, 2, false);
+                product(small, 1, 1, false);
+                product(small, 2, 0, false);
+                umma_commit(&empty[s]);
+            }
+            // what has been issued must be complete before the CTA gives its memory back, also after a wait that ran out
+            umma_commit(done);
+            mbar_wait(done, 0);
+        }
+    } else {
+        // a thread's piece of a stretch: 8 neighbours of k (chunk `c`) of the rows r0, r0 + ROUND, ...
+        const int r0 = tid >> 3, c = tid & 7;
+        float4 ra[A_IT][2], rb[B_IT][2];                       // the stretch to be cut next
+        auto load = [&](const float* base, int ld, int row, int rows, int kb, float4 (&v)[2]) {
+            const int k = kb * 64 + c * 8;
+            const float* src = base + (size_t)row * ld + k;
+            const bool in = row < rows;
+            v[0] = (in && k < p.K) ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[1] = (in && k + 4 < p.K) ? __ldg(reinterpret_cast<const float4*>(src + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        auto load_a = [&](int kb, int i) { load(p.a, p.lda, m0 + r0 + ROUND * i, p.M, kb, ra[i]); };
+        auto load_b = [&](int kb, int i) { load(p.w, p.K, n0 + r0 + ROUND * i, p.N, kb, rb[i]); };
+        auto store = [&](uint8_t* base, uint32_t plane, int row, const float4 (&v)[2]) {
+            uint4 h, m, l;
+            cut(v[0].x, v[0].y, h.x, m.x, l.x);
+            cut(v[0].z, v[0].w, h.y, m.y, l.y);
+            cut(v[1].x, v[1].y, h.z, m.z, l.z);
+            cut(v[1].z, v[1].w, h.w, m.w, l.w);
+            uint8_t* at = base + row * 128 + ((c ^ (row & 7)) << 4);
+            *reinterpret_cast<uint4*>(at) = h;
+            *reinterpret_cast<uint4*>(at + plane) = m;
+            *reinterpret_cast<uint4*>(at + 2 * plane) = l;
+        };
+        const int quad = warp & 3, part = warp >> 2;
+        const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+        float acc[COLS];
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
+        bool ok = true;
+        auto drain = [&](int kb) {
+            const int b = kb & 1;
+            if (!mbar_wait(&acc_full[b], (kb >> 1) & 1)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 92, blockIdx.x, kb); ok = false; }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) return;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tmem_add<COLS>(tmem + lanes + (uint32_t)(b * TN + part * COLS), acc);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+        };
+#pragma unroll
+        for (int i = 0; i < B_IT; ++i) load_b(0, i);           // W is written by no kernel
+        pdl_wait();
+#pragma unroll
+        for (int i = 0; i < A_IT; ++i) load_a(0, i);
+        for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+            const int s = kb % STAGES;
+            if (kb >= STAGES) {
+                if (!mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 93, blockIdx.x, kb); ok = false; }
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+            }
+            uint8_t* base = smem + s * STAGE;
+            // a piece's registers are asked to be filled again as soon as they are stored (beyond the last stretch the
+            // loads are masked off)
+#pragma unroll
+            for (int i = 0; i < A_IT; ++i) {
+                store(base, A_PLANE, r0 + ROUND * i, ra[i]);
+                load_a(kb + 1, i);
+            }
+#pragma unroll
+            for (int i = 0; i < B_IT; ++i) {
+                store(base + 3 * A_PLANE, B_PLANE, r0 + ROUND * i, rb[i]);
+                load_b(kb + 1, i);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the planes are read by the async proxy
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[s])) : "memory");
+            if (kb > 0) drain(kb - 1);
+        }
+        if (ok) drain(p.kblocks - 1);
+        if (ok && !mbar_wait(done, 0)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 94, blockIdx.x, p.kblocks); ok = false; }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tmem_add<COLS>(small + lanes + (uint32_t)(part * COLS), acc);
+            const int row = m0 + quad * 32 + lane;
+            if (row < p.M) {
+                const int col0 = n0 + part * COLS;
+                float* out = p.c + (size_t)row * p.ldc + col0;
+                const bool vec = (p.ldc & 3) == 0 && (((uintptr_t)p.c) & 15) == 0;
+#pragma unroll
+                for (int j = 0; j < COLS; j += 4) {
+                    float v[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        v[e] = acc[j + e];
+                        if (col0 + j + e < p.N && !isfinite(v[e]))
+                            v[e] = whole_sum(p.a + (size_t)row * p.lda, p.w + (size_t)(col0 + j + e) * p.K, p.K);
+                    }
+                    if (vec && col0 + j + 4 <= p.N) {
+                        float4* dst = reinterpret_cast<float4*>(out + j);
+                        if (p.accumulate) {
+                            const float4 old = *dst;
+                            v[0] = old.x + v[0]; v[1] = old.y + v[1]; v[2] = old.z + v[2]; v[3] = old.w + v[3];
+                        }
+                        *dst = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (col0 + j + e < p.N) out[j + e] = p.accumulate ? out[j + e] + v[e] : v[e];
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == WORKERS) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+template <int TN>
+static int launch_split(const Params& p, cudaStream_t stream) {
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(sgemm_split_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<TN>());
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    launch(sgemm_split_kernel<TN>, dim3((p.M + TM - 1) / TM, (p.N + TN - 1) / TN), dim3(THREADS), smem_bytes<TN>(), stream, p);
+    IMPARO_CHECK_LAUNCH();
+    return 0;
+}
+
+}  // namespace sp
+
 }  // namespace imparo
 
+// status: where a wait that ran out is recorded.
 extern "C" int imparo_sgemm_nt(const float* A, const float* W, float* C, int M, int N, int K,
-                               int lda, int ldc, int accumulate, cudaStream_t stream) {
+                               int lda, int ldc, int accumulate, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return -1;
+    // rows of whole 16-byte groups: the tensor cores
+    if (K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && (N + 63) / 64 <= 65535) {
+        imparo::sp::Params p{A, W, C, M, N, K, lda, ldc, accumulate, (K + 63) / 64, status};
+        // tiles of 128 x 64 where tiles of 128 x 128 would leave more than half of the 148 SMs without one (1,000 x 1,024 x
+        // 4,608: 114 against 156 us); above that a wide tile costs 1.4 times a narrow one and does twice the work.  The
+        // sums are the same either way.
+        const long long tiles = (long long)((M + 127) / 128) * ((N + 127) / 128);
+        return tiles * 2 <= 148 ? imparo::sp::launch_split<64>(p, stream) : imparo::sp::launch_split<128>(p, stream);
+    }
     dim3 grid((N + imparo::BN - 1) / imparo::BN, (M + imparo::BM - 1) / imparo::BM);
     if (grid.y > 65535) return -2;
     launch(imparo::sgemm_nt_kernel, grid, dim3(256), 0, stream, A, W, C, M, N, K, lda, ldc, accumulate);

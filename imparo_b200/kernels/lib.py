@@ -73,7 +73,7 @@ def _declare_kernels(lib):
     _declare(lib, "imparo_swiglu_act", [P, P, I, I, I, S])
     _declare(lib, "imparo_add_bias", [P, I, P, I, I, S])
     _declare(lib, "imparo_gated_act", [P, P, P, I, I, I, I, c_float, S])
-    _declare(lib, "imparo_sgemm_nt", [P, P, P, I, I, I, I, I, I, S])
+    _declare(lib, "imparo_sgemm_nt", [P, P, P, I, I, I, I, I, I, P, S])
     _declare(lib, "imparo_gemm_lib_init", [P, c_size_t])
     _declare(lib, "imparo_gemm_bf16_nt", [P, P, P, I, I, I, I, I, I, I, S])
     _declare(lib, "imparo_gemm_tc_plan", [I, I, I, I, POINTER(c_int), POINTER(c_int), POINTER(c_int64), POINTER(c_int)])

@@ -500,6 +500,16 @@ def tc_usable(x: torch.Tensor, w: torch.Tensor, any_size: bool = False) -> bool:
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and w.is_contiguous())
 
 
+def _status_word(device, status: Optional[torch.Tensor]) -> torch.Tensor:
+    """`status`, or this launch state's own word where the caller brings none."""
+    if status is None:
+        key = torch.device(device).index or 0
+        status = _S.status_fallback.get(key)
+        if status is None:
+            status = _S.status_fallback[key] = new_status(device)
+    return status
+
+
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, status: Optional[torch.Tensor] = None,
             scratch: Optional[torch.Tensor] = None, act: str = "silu", limit: float = 0.0, bias: Optional[torch.Tensor] = None,
             plain: Optional[str] = None) -> None:
@@ -524,11 +534,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, 
         cnt = scratch
     else:
         scratch, cnt = _tc_buffers(x.device, floats, counters)
-    if status is None:
-        key = torch.device(x.device).index or 0
-        status = _S.status_fallback.get(key)
-        if status is None:
-            status = _S.status_fallback[key] = new_status(x.device)
+    status = _status_word(x.device, status)
     rows_alloc = (x.untyped_storage().nbytes() // x.element_size() - x.storage_offset()) // x.stride(0) if x.stride(0) else T
     rows_alloc = max(T, min(rows_alloc, 1 << 30))
     if plain is not None:
@@ -590,11 +596,7 @@ def gemm_prefill(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
     _need(tuple(out.shape) == (T, N), f"gemm_prefill: out must be [{T}, {N}]")
     want_dtype = torch.bfloat16 if epilogue in (EPI_STORE_BF16, EPI_SWIGLU) else torch.float32
     _need(out.dtype == want_dtype, f"gemm_prefill: this epilogue writes {want_dtype}")
-    if status is None:
-        key = torch.device(x.device).index or 0
-        status = _S.status_fallback.get(key)
-        if status is None:
-            status = _S.status_fallback[key] = new_status(x.device)
+    status = _status_word(x.device, status)
     rows_alloc = (x.untyped_storage().nbytes() // x.element_size() - x.storage_offset()) // x.stride(0) if x.stride(0) else T
     rows_alloc = max(T, min(rows_alloc, 1 << 30))
     if bias is not None:
@@ -674,7 +676,7 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
         if accumulate:
             settle(out)
         _check(_lib.kernels().imparo_sgemm_nt(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), N, int(accumulate),
-                                              _stream()), "sgemm_nt")
+                                              _ptr(_status_word(x.device, status)), _stream()), "sgemm_nt")
     elif x.dtype == torch.bfloat16:
         _need(not accumulate or out.dtype == torch.float32, "linear: accumulate needs a float32 output")
         if gemm_backend() == "tcgen05" and tc_usable(x, w):

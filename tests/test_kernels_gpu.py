@@ -99,6 +99,50 @@ def test_sgemm_is_true_float32(M, N, K):
     assert (out2.cpu().double() - (ref + base.double())).abs().max() <= 3e-6 * max(1.0, ref.abs().max())
 
 
+# edges of the split product's tiles (128 rows, 64 or 128 columns: the wide ones from 75 tiles on) and stretches (64 k);
+# outputs whose rows are no 16-byte groups; a row stride beyond K
+@pytest.mark.parametrize("M,N,K,ld", [(1, 1, 4, 4), (127, 63, 60, 60), (128, 64, 64, 68), (129, 65, 68, 68), (257, 130, 132, 140),
+                                      (129, 4800, 72, 72), (1, 9601, 264, 264), (300, 3201, 128, 128)])
+def test_sgemm_split_edges(M, N, K, ld):
+    o = ops()
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, ld, generator=g)[:, :K], torch.randn(N, K, generator=g)
+    a = a * torch.exp(3 * torch.randn(M, 1, generator=g))
+    x = torch.zeros(M, ld, device=DEV)[:, :K]
+    x.copy_(a)
+    ref = a.double() @ w.double().T
+    # per stretch four MMAs whose sums are cut to 32 bits, a 32-bit addition per stretch, products below 2^-25 left out
+    bound = (a.double().abs() @ w.double().abs().T) * (4 * 2.0 ** -23 + (K // 64 + 2) * 2.0 ** -24 + 2.0 ** -25)
+    out = torch.empty(M, N, device=DEV)
+    st = o.new_status(DEV)
+    o.linear(x, w.to(DEV), out, status=st)
+    o.read_status(st)
+    assert ((out.cpu().double() - ref).abs() <= bound).all()
+    base = torch.randn(M, N, generator=g)
+    out2 = base.to(DEV).clone()
+    o.linear(x, w.to(DEV), out2, accumulate=True, status=st)
+    assert torch.equal(out2, base.to(DEV) + out)                      # one 32-bit addition
+    one = torch.empty(1, N, device=DEV)
+    o.linear(x[M // 2:M // 2 + 1], w.to(DEV), one, status=st)
+    assert torch.equal(one[0], out[M // 2])                           # a row alone is the row among others
+
+
+def test_sgemm_split_infinities_and_nan():
+    o = ops()
+    g = torch.Generator().manual_seed(4)
+    a, w = torch.randn(130, 256, generator=g), torch.randn(70, 256, generator=g)
+    w[:, 1] = 0.5                                                     # a bfloat16 number: its lower pieces are zero
+    a[3, 7], a[5, 9], w[4, 2], a[7, 1], a[9] = float("inf"), float("nan"), float("-inf"), 3.4e38, 0.0
+    ref = (a.double() @ w.double().T).float()
+    out = torch.empty(130, 70, device=DEV)
+    o.linear(a.to(DEV), w.to(DEV), out)
+    out = out.cpu()
+    fin = torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(out), fin) and torch.equal(torch.isnan(out), torch.isnan(ref))
+    assert torch.equal(out[torch.isinf(ref)], ref[torch.isinf(ref)])
+    assert (out[7].double() - ref[7].double())[fin[7]].abs().max() <= 1e-6 * 3.4e38
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 96, 64), (5, 200, 136), (77, 512, 192), (300, 1000, 264)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_gemm_bf16(M, N, K, out_dtype):
