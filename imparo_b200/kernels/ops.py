@@ -2003,10 +2003,22 @@ def delta_prepare(qkv: torch.Tensor, q_off: int, k_off: int, bproj: torch.Tensor
                                                float(q_scale), _stream()), "delta_prepare")
 
 
+def delta_chunk_floats(heads: int, dim: int, vdim: int) -> int:
+    """Floats of scratch per chunk of 64 rows of delta_scan; 0: sizes that only run row by row."""
+    return int(_lib.kernels().imparo_delta_chunk_floats(int(heads), int(dim), int(vdim)))
+
+
+def delta_chunks_take(qkv: torch.Tensor, q_off: int, k_off: int, heads: int, dim: int, vdim: int) -> bool:
+    return (delta_chunk_floats(heads, dim, vdim) > 0 and q_off % 4 == 0 and k_off % 4 == 0 and qkv.stride(0) % 4 == 0
+            and qkv.data_ptr() % 16 == 0)
+
+
 def delta_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, g: torch.Tensor, beta: torch.Tensor, state: torch.Tensor,
                item_row_start, item_slot, n_items: int, out: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int,
-               status: torch.Tensor) -> None:
+               status: torch.Tensor, scratch: Optional[torch.Tensor] = None) -> None:
     """Per request and value head, rows in order: S = g * S; u = beta (v - S^T k); S += k u^T; out = S^T q.
+    scratch: float32, (T // 64 + n_items) * delta_chunk_floats(...) long: rows run in chunks of 64 side by side, where
+    delta_chunks_take(...) says so.
     qkv float32 rows (query / key heads kv_heads * dim at q_off / k_off, values heads * vdim at v_off); g float32
     [T, heads * dim]; beta float32 [T, heads]; state float32 [slots, heads, dim, vdim]; out float32 [T, heads * vdim]."""
     _cuda(g, beta, state, item_row_start, item_slot, out, status)
@@ -2021,6 +2033,17 @@ def delta_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, g: torch.T
     _need(tuple(state.shape[1:]) == (heads, dim, vdim), "delta_scan: state [slots, heads, dim, vdim]")
     _need(1 <= dim <= 256, "delta_scan: key size 1 to 256")
     _need(qkv.shape[1] >= max(q_off + kv_heads * dim, k_off + kv_heads * dim, v_off + heads * vdim), "delta_scan: column ranges")
+    if scratch is not None:
+        chunks = T // 64 + n_items
+        _cuda(scratch)
+        _need(delta_chunks_take(qkv, q_off, k_off, heads, dim, vdim), "delta_scan: rows that do not run in chunks")
+        _need(scratch.dtype == torch.float32 and scratch.numel() >= chunks * delta_chunk_floats(heads, dim, vdim), "delta_scan: chunk scratch")
+        _check(_lib.kernels().imparo_delta_chunked(_ptr(qkv), qkv.stride(0), int(q_off), int(k_off), int(v_off), _ptr(g), _ptr(beta),
+                                                   _ptr(state), _ptr(item_row_start), _ptr(item_slot), state.shape[0], n_items, chunks,
+                                                   _ptr(scratch), _ptr(out), heads, kv_heads, dim, vdim, _ptr(status), _stream()),
+               "delta_chunked")
+        COUNTS["own"] += 2
+        return
     _check(_lib.kernels().imparo_delta_scan(_ptr(qkv), qkv.stride(0), int(q_off), int(k_off), int(v_off), _ptr(g), _ptr(beta), _ptr(state),
                                             _ptr(item_row_start), _ptr(item_slot), state.shape[0], n_items, _ptr(out), heads, kv_heads,
                                             dim, vdim, _ptr(status), _stream()), "delta_scan")

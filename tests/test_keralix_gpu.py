@@ -367,6 +367,73 @@ def test_delta_rule_kernels(H, G, D, V):
         assert np.abs(state[slots[i]].cpu().numpy() - S).max() <= 3e-5 * np.abs(S).max()
 
 
+def _delta_walk_64(q, k, v, beta, g, S):
+    """The recurrence in 64 bits, heads side by side.  q, k, g [T, H, D], v [T, H, V], beta [T, H]; S [H, D, V] is moved on."""
+    import torch
+    o = torch.empty_like(v)
+    for t in range(len(q)):
+        S *= g[t][:, :, None]
+        u = beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+        S += k[t][:, :, None] * u[:, None]
+        o[t] = torch.einsum("hdv,hd->hv", S, q[t])
+    return o
+
+
+# key sizes at the edges of both builds (64 and 128 channels) and no multiple of 16, value sizes below, at and beyond a CTA's 16,
+# 64 and 128 columns; portions of 1 row, whole chunks, a chunk and a row
+@pytest.mark.parametrize("H,G,D,V", [(2, 1, 64, 128), (3, 3, 4, 4), (4, 2, 20, 36), (2, 2, 128, 132), (1, 1, 68, 16), (2, 1, 64, 260)])
+@pytest.mark.parametrize("lens", [(1, 64, 65), (200, 7), (128,)])
+def test_delta_rule_in_chunks(H, G, D, V, lens):
+    """Chunks against the recurrence in 64 bits and against the row walk, from states other than zero: outputs and states no
+    further off than the walk (twice, for sums in another order), decays of exactly zero and of exactly one among them."""
+    import torch
+    from imparo_b200.kernels import ops
+    g0 = torch.Generator().manual_seed(H * 1000 + D + V + sum(lens))
+    T, slots = sum(lens), [3, 0, 2][:len(lens)]
+    rnd = lambda *s: torch.randn(*s, generator=g0)
+    q, k = (torch.nn.functional.normalize(rnd(T, G, D), dim=-1) for _ in range(2))
+    v, beta = rnd(T, H, V), torch.sigmoid(rnd(T, H))
+    g = torch.exp(-torch.exp(2 * rnd(T, H, D) - 3))
+    g[T // 3], g[T // 2, :, ::3], g[T // 2 + 1:T // 2 + 9] = 0.0, 0.0, 1.0
+    state0 = rnd(5, H, D, V)
+    pad = 4 * G                                         # a column range ahead of q, k and v
+    qkv = torch.cat([rnd(T, pad), q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], dim=1).contiguous().cuda()
+    starts = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device="cuda")
+    args = (qkv, pad, pad + G * D, pad + 2 * G * D, g.reshape(T, -1).contiguous().cuda(), beta.cuda())
+    assert ops.delta_chunks_take(qkv, pad, pad + G * D, H, D, V)
+    got = []
+    for scratch in (None, torch.full(((T // 64 + len(lens)) * ops.delta_chunk_floats(H, D, V),), float("nan"), device="cuda")):
+        state, out, status = state0.cuda(), torch.full((T, H * V), float("nan"), device="cuda"), ops.new_status("cuda")
+        ops.delta_scan(*args, state, starts, torch.tensor(slots, dtype=torch.int32, device="cuda"), len(lens), out, H, G, D, V, status, scratch=scratch)
+        ops.read_status(status)
+        got.append((out.cpu().double().reshape(T, H, V), state.cpu().double()))
+    want_state, want = state0.double(), []
+    rep = lambda x: x.double().repeat_interleave(H // G, dim=1)
+    for i, s in enumerate(slots):
+        r = slice(int(starts[i]), int(starts[i + 1]))
+        want.append(_delta_walk_64(rep(q)[r], rep(k)[r], v.double()[r], beta.double()[r], g.double()[r], want_state[s]))
+    want = torch.cat(want)
+    (walk_o, walk_s), (o, s) = got
+    assert (o - want).norm() <= 2 * (walk_o - want).norm() + 1e-7 * want.norm()
+    assert (s - want_state).norm() <= 2 * (walk_s - want_state).norm() + 1e-7 * want_state.norm()
+    assert torch.equal(s[[1, 4]], state0[[1, 4]].double())
+
+
+def test_delta_rule_in_chunks_refuses_a_bad_slot_and_other_sizes():
+    import torch
+    from imparo_b200.kernels import ops
+    H, D, V, T = 1, 8, 8, 70
+    qkv, g, beta = torch.rand(T, 3 * 8, device="cuda"), torch.rand(T, 8, device="cuda"), torch.rand(T, 1, device="cuda")
+    state, out, status = torch.zeros(2, 1, 8, 8, device="cuda"), torch.full((T, 8), 7.0, device="cuda"), ops.new_status("cuda")
+    scratch = torch.zeros(2 * ops.delta_chunk_floats(H, D, V), device="cuda")
+    ops.delta_scan(qkv, 0, 8, 16, g, beta, state, _dev(np.array([0, T], dtype=np.int32)), _dev(np.array([5], dtype=np.int32)), 1, out, H, 1, D, V,
+                   status, scratch=scratch)
+    assert float(out.min()) == 7.0 and float(state.abs().max()) == 0.0
+    with pytest.raises(ops.KernelError, match="state slot"):
+        ops.read_status(status)
+    assert not ops.delta_chunks_take(qkv, 0, 8, 1, 6, 8) and not ops.delta_chunks_take(qkv, 0, 8, 1, 132, 8) and not ops.delta_chunks_take(qkv, 2, 8, 1, 8, 8)
+
+
 def test_delta_rule_state_carries_a_far_token():
     """A pair (k, v) written at the first token is read back hundreds of tokens later by queries along k, in a prompt and in
     single tokens, although every other key is random (tests/keralix_cases.py: far_delta_case)."""
