@@ -15,6 +15,7 @@ import sys
 import time
 from typing import Dict, List, Optional, Sequence, Union
 
+import numpy as np
 import torch
 
 from ..cache import CacheManager
@@ -152,21 +153,25 @@ class Engine:
         on the device, or None.  The result is the caller's own tensor: the step function writes
         its logits into a buffer that the next step of the same shape overwrites (a workspace view,
         or a captured graph's output), so what is handed out here is a copy of it."""
-        self._check_tokens(items)
-        out = self.step_fn(items)
+        out = self.step_fn(self._checked(items))
         return None if out is None else out.clone()
 
     def check_device_status(self) -> None:
         ops.read_status(self.status)
 
-    def _check_tokens(self, items) -> None:
+    def _checked(self, items: Sequence[StepItem]) -> List[StepItem]:
+        """The items with their tokens as arrays (made once, for the checks here and the step's description)."""
+        checked = []
         for it in items:
-            toks = it.tokens
-            if len(toks) and (min(toks) < 0 or max(toks) >= self.vocab_size):
+            toks = np.asarray(it.tokens, dtype=np.int64) if len(it.tokens) > 8 else it.tokens
+            if len(toks) and (min(toks) < 0 or max(toks) >= self.vocab_size if toks is it.tokens
+                              else toks.min() < 0 or toks.max() >= self.vocab_size):
                 raise ValueError(f"request {it.request}: token id out of range [0, {self.vocab_size})")
             if self.cache.has(it.request) and self.cache.cached(it.request) + len(toks) > self.ctx:
                 raise ValueError(f"request {it.request}: {self.cache.cached(it.request)} + {len(toks)} tokens "
                                  f"exceed the context length {self.ctx}")
+            checked.append(StepItem(it.request, toks, it.want))
+        return checked
 
     # -- generation --------------------------------------------------------------------------
     def generate(self, prompts: Sequence[Sequence[int]], max_tokens: Union[int, Sequence[int]] = 16,

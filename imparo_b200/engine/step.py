@@ -186,6 +186,14 @@ class StepFunction:
         for j_item, it in enumerate(caller_items):       # wanted rows: in the caller's order
             n = len(it.tokens)
             base = int(row_start[place[j_item]])
+            if len(it.want) > 8:                         # many: at once (a loop costs 0.12 us per place)
+                places = np.asarray(it.want, dtype=np.int64)
+                outside = (places < 0) | (places >= n)
+                if outside.any():
+                    raise ValueError(f"request {it.request}: wanted place {it.want[int(outside.argmax())]} is not among its {n} tokens")
+                want[w:w + len(places)] = base + places
+                w += len(places)
+                continue
             for j in it.want:
                 if not 0 <= j < n:
                     raise ValueError(f"request {it.request}: wanted place {j} is not among its {n} tokens")
