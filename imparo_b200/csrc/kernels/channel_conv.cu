@@ -3,12 +3,12 @@
 //
 //   y[t, c] = act( sum_j w[c, j] * u[t - taps + 1 + j, c] ),   u = product column (+ bias[c]),  zeros before the sequence
 //
-//  (1) channel_conv: a thread per (row, channel); inputs before the portion's first row come from the slot (oldest first),
+//  (1) channel_conv: a thread per (row, channel), or per four channels of several rows (conv_rows.cuh); inputs before the portion's first row come from the slot (oldest first),
 //      which is all zeros for a fresh request.  act 0: none, 1: silu.
 //  (2) channel_conv_state: moves the slot on by the portion's rows; it runs after every reader of the old state.
 // The bias belongs to the product (a projection with a bias): the slot keeps biased values, and positions before the
 // sequence count as zero, not as the bias.
-#include "common.cuh"
+#include "conv_rows.cuh"
 
 namespace imparo {
 
@@ -48,6 +48,14 @@ channel_conv_kernel(const float* __restrict__ in, size_t stride, int col0, int c
     out[(size_t)t * out_stride + c] = act == 1 ? silu(acc) : acc;
 }
 
+// 2,048 rows of 1,536 channels, four taps, silu (B200): 31 us with a thread per (row, channel), 10.9 us here.
+template <int TAPS, int R>
+__global__ void __launch_bounds__(128)
+channel_conv_rows_kernel(const ConvRows p) {
+    pdl_trigger();
+    conv_rows<TAPS, R>(p, (blockIdx.y * 128 + threadIdx.x) * 4, blockIdx.x * R);
+}
+
 __global__ void __launch_bounds__(256)
 channel_conv_state_kernel(const float* __restrict__ in, size_t stride, int col0, int channels, int taps,
                           const float* __restrict__ bias, float* __restrict__ state,
@@ -84,6 +92,20 @@ extern "C" int imparo_channel_conv(const float* in, long long stride, int col0, 
     if (n_tok <= 0) return 0;
     if (taps < 1 || taps > CC_MAX_TAPS) return -2;
     if (channels < 1 || stride < col0 + channels || out_stride < channels) return -3;
+    const ConvRows p{in, (size_t)stride, col0, channels, w, bias, nullptr, state, item_row_start, item_of_token, item_slot, n_slots, n_tok,
+                     out, (size_t)out_stride, act == 1, 72, status};
+    if (conv_rows_take(p, taps)) {
+        const int r = conv_rows_per_thread(n_tok, channels);
+        const dim3 grid((n_tok + r - 1) / r, (channels / 4 + 127) / 128);
+#define IMPARO_CC(T_) do { if (r == 4) launch(channel_conv_rows_kernel<T_, 4>, grid, dim3(128), 0, stream, p); \
+                           else launch(channel_conv_rows_kernel<T_, 1>, grid, dim3(128), 0, stream, p); } while (0)
+        if (taps == 2) IMPARO_CC(2);
+        else if (taps == 3) IMPARO_CC(3);
+        else IMPARO_CC(4);
+#undef IMPARO_CC
+        IMPARO_CHECK_LAUNCH();
+        return 0;
+    }
     launch(channel_conv_kernel, dim3(n_tok, (channels + 255) / 256), dim3(256), 0, stream, in, (size_t)stride, col0, channels, taps,
            w, bias, state, item_row_start, item_of_token, item_slot, n_slots, act, out, (size_t)out_stride, status);
     IMPARO_CHECK_LAUNCH();

@@ -538,6 +538,82 @@ def test_linear_unfolded_sums_to_the_product(T, N, K):
     assert (got - ref).abs().max() <= 8e-3 * max(1.0, ref.abs().max())
 
 
+def _ragged(lens, slots):
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    return t(starts), t([i for i, n in enumerate(lens) for _ in range(n)]), t(slots)
+
+
+def _conv64(u, taps, lens, slots, state):
+    """Causal convolution of u [T, C] per portion in 64 bits, from and into state [slots, taps - 1, C]."""
+    h, out, at = taps.shape[1] - 1, [], 0
+    for n, s in zip(lens, slots):
+        seq = torch.cat([state[s], u[at:at + n]])
+        out.append(sum(taps[:, k] * seq[k:k + n] for k in range(h + 1)))
+        state[s] = seq[n:]
+        at += n
+    return torch.cat(out)
+
+
+# portions shorter than the taps, ends inside a thread's four rows; enough rows x channels for four rows per thread, and fewer
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps,bias", [(2, False), (3, True), (4, False)])
+@pytest.mark.parametrize("lens,width", [((1, 2, 3, 5, 1, 60), 24), ((1201, 1, 2, 7, 3, 4, 90), 2048)])
+def test_gated_conv_several_rows_per_thread(dtype, taps, bias, lens, width):
+    o = ops()
+    g = torch.Generator().manual_seed(taps * 100 + width)
+    T, slots = sum(lens), [(3 * i + 1) % 8 for i in range(len(lens))]
+    bcx = torch.randn(T, 3 * width, generator=g).to(dtype)
+    w, b0, state0 = torch.randn(width, taps, generator=g), torch.randn(width, generator=g), torch.randn(8, taps - 1, width, generator=g)
+    state, st = state0.to(DEV), o.new_status(DEV)
+    y = torch.full((T, width), float("nan"), dtype=dtype, device=DEV)
+    starts, item, slot = _ragged(lens, slots)
+    o.gated_conv(bcx.to(DEV), w.to(DEV), b0.to(DEV) if bias else None, state, starts, item, slot, y, taps, st)
+    o.read_status(st)
+    x, want_state = bcx.double(), state0.double()
+    acc = _conv64(x[:, :width] * x[:, 2 * width:], w.double(), lens, slots, want_state) + (b0.double() if bias else 0.0)
+    want = x[:, width:2 * width] * acc
+    # taps + 2 roundings of 32 bits, then the stored type's
+    assert ((y.double().cpu() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6) * (want.abs() + 8.0)).all()
+    assert (state.cpu().double() - want_state).abs().max() <= 2e-6
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4, 5])
+@pytest.mark.parametrize("lens,channels", [((1, 2, 3, 5, 1, 60), 24), ((700, 1, 2, 7, 3, 90), 1536)])
+def test_channel_conv_several_rows_per_thread(taps, lens, channels):
+    o = ops()
+    g = torch.Generator().manual_seed(taps + channels)
+    T, slots = sum(lens), [(3 * i + 1) % 8 for i in range(len(lens))]
+    proj, w, b = torch.randn(T, channels + 12, generator=g), torch.randn(channels, taps, generator=g), torch.randn(channels, generator=g)
+    state0 = torch.randn(8, taps - 1, channels, generator=g)
+    starts, item, slot = _ragged(lens, slots)
+    for col0 in (4, 3):                                   # 16-byte rows, and rows that keep a thread per channel
+        for silu in (False, True):
+            state, st, out = state0.to(DEV), o.new_status(DEV), torch.full((T, channels), float("nan"), device=DEV)
+            o.channel_conv(proj.to(DEV), col0, channels, taps, w.to(DEV), b.to(DEV), state, starts, item, slot, len(lens), out, st,
+                           act="silu" if silu else None)
+            o.read_status(st)
+            want_state = state0.double()
+            want = _conv64(proj.double()[:, col0:col0 + channels] + b.double(), w.double(), lens, slots, want_state)
+            if silu:
+                want = want * torch.sigmoid(want)
+            assert (out.cpu().double() - want).abs().max() <= 1e-5 and (state.cpu().double() - want_state).abs().max() <= 1e-6
+    # the state-space mixer's: a bias on the sum, step sizes beside it
+    heads = 8
+    dt_bias, state, st = torch.randn(heads, generator=g), state0.to(DEV), o.new_status(DEV)
+    xbc, dt = torch.full((T, channels), float("nan"), device=DEV), torch.full((T, heads), float("nan"), device=DEV)
+    o.mamba2_conv(proj.to(DEV), 4, channels + 4, channels, heads, taps, w.to(DEV), b.to(DEV), dt_bias.to(DEV), state, starts, item, slot, len(lens),
+                  xbc, dt, st)
+    o.read_status(st)
+    want_state = state0.double()
+    want = _conv64(proj.double()[:, 4:4 + channels], w.double(), lens, slots, want_state) + b.double()
+    assert (xbc.cpu().double() - want * torch.sigmoid(want)).abs().max() <= 1e-5
+    want = torch.nn.functional.softplus(proj.double()[:, channels + 4:channels + 12] + dt_bias.double(), threshold=40)
+    assert (dt.cpu().double() - want).abs().max() <= 2e-6 and (state.cpu().double() - want_state).abs().max() <= 1e-6
+
+
 def test_kernels_refuse_sizes_they_do_not_take():
     o = ops()
     st = o.new_status(DEV)
