@@ -12,7 +12,7 @@
 //      every chunk's own state from zero and its total decay (as a product of weighted B rows with x rows for states up
 //      to 128, else by walking the rows); a scan over each request's chunks that leaves every
 //      chunk's starting state and the request's new state; every chunk's outputs from its starting state plus the
-//      rows inside the chunk.  32-bit on CUDA cores.
+//      rows inside the chunk.  32-bit on CUDA cores.  (Sizes that are multiples of 4 run as products: mamba2_chunk.cu.)
 //  (4) gate_group_rmsnorm: y * silu(z), then an RMS norm over each of `groups` equal stretches of the row, times a
 //      weight.
 #include "conv_rows.cuh"
@@ -444,6 +444,48 @@ mamba2_chunk_out_kernel(const float* __restrict__ xbc, const float* __restrict__
 
 // ---- (4) gate, then a norm per stretch of the row ----------------------------------------------------------------
 // grid (rows, groups): out[r, s] = (y silu(z))[r, s] / rms over the stretch * w[s]
+// Rows of up to 8,192 entries per stretch, four at a time and gated once, kept in registers between the two passes (1,999 rows of
+// 2,048: 19.5 us below, 10.3 us here).
+template <typename T, int V>
+__global__ void __launch_bounds__(256)
+gate_group_rmsnorm_wide_kernel(const float* __restrict__ y, const float* __restrict__ z, size_t z_stride, const float* __restrict__ w,
+                               float eps, T* __restrict__ out, int width, int groups) {
+    __shared__ float scratch[33];
+    pdl_trigger();
+    const int r = blockIdx.x, grp = blockIdx.y, per = width / groups;
+    const float4* wg = reinterpret_cast<const float4*>(w + (size_t)grp * per);
+    pdl_wait();
+    const float4* yr = reinterpret_cast<const float4*>(y + (size_t)r * width + (size_t)grp * per);
+    const float4* zr = reinterpret_cast<const float4*>(z + (size_t)r * z_stride + (size_t)grp * per);
+    float4 a[V], g[V];
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        const int i = threadIdx.x + 256 * u;
+        a[u] = g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (4 * i < per) { a[u] = yr[i]; g[u] = zr[i]; }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        a[u] = make_float4(a[u].x * silu(g[u].x), a[u].y * silu(g[u].y), a[u].z * silu(g[u].z), a[u].w * silu(g[u].w));
+        ss += (a[u].x * a[u].x + a[u].y * a[u].y) + (a[u].z * a[u].z + a[u].w * a[u].w);
+    }
+    ss = block_sum(ss, scratch);
+    const float scale = 1.0f / sqrtf(ss / (float)per + eps);
+    T* o = out + (size_t)r * width + (size_t)grp * per;
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        const int i = threadIdx.x + 256 * u;
+        if (4 * i < per) {
+            const float4 wv = wg[i];
+            alignas(16) T v[4] = {from_f32<T>(a[u].x * scale * wv.x), from_f32<T>(a[u].y * scale * wv.y), from_f32<T>(a[u].z * scale * wv.z),
+                                  from_f32<T>(a[u].w * scale * wv.w)};
+            if constexpr (sizeof(T) == 4) *reinterpret_cast<float4*>(o + 4 * i) = *reinterpret_cast<const float4*>(v);
+            else *reinterpret_cast<uint2*>(o + 4 * i) = *reinterpret_cast<const uint2*>(v);
+        }
+    }
+}
+
 template <typename T, typename TZ>
 __global__ void __launch_bounds__(256)
 gate_group_rmsnorm_kernel(const float* __restrict__ y, const TZ* __restrict__ z, size_t z_stride, const float* __restrict__ w,
@@ -585,6 +627,19 @@ extern "C" int imparo_gate_group_rmsnorm(const float* y, const void* z, int z_dt
     if (rows <= 0) return 0;
     if (groups < 1 || width % groups) return -2;
     dim3 grid(rows, groups);
+    const int per = width / groups;
+    if (z_dtype == IMPARO_DT_F32 && (out_dtype == IMPARO_DT_F32 || out_dtype == IMPARO_DT_BF16) && per % 4 == 0 && per <= 8192 && z_stride % 4 == 0 &&
+        (((uintptr_t)y | (uintptr_t)z | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
+#define IMPARO_GG(T_, V_) launch(gate_group_rmsnorm_wide_kernel<T_, V_>, grid, dim3(256), 0, stream, y, (const float*)z, (size_t)z_stride, w, eps, \
+                                 (T_*)out, width, groups)
+#define IMPARO_GGV(T_) do { if (per <= 1024) IMPARO_GG(T_, 1); else if (per <= 2048) IMPARO_GG(T_, 2); else if (per <= 4096) IMPARO_GG(T_, 4); \
+                            else IMPARO_GG(T_, 8); } while (0)
+        if (out_dtype == IMPARO_DT_F32) IMPARO_GGV(float); else IMPARO_GGV(__nv_bfloat16);
+#undef IMPARO_GGV
+#undef IMPARO_GG
+        IMPARO_CHECK_LAUNCH();
+        return 0;
+    }
     if (z_dtype == IMPARO_DT_F32 && out_dtype == IMPARO_DT_F32)
         launch(gate_group_rmsnorm_kernel<float, float>, grid, dim3(256), 0, stream, y, (const float*)z, (size_t)z_stride, w, eps,
                (float*)out, width, groups);

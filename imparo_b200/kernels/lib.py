@@ -135,6 +135,8 @@ def _declare_kernels(lib):
     _declare(lib, "imparo_scale_rows", [P, c_int64, c_float, S])
     _declare(lib, "imparo_mamba2_conv", [P, I, c_int64, I, I, I, I, I, P, P, P, P, P, P, P, I, I, I, P, P, P, S])
     _declare(lib, "imparo_mamba2_scan", [P, P, P, P, P, P, P, I, I, P, I, I, I, I, P, S])
+    _declare(lib, "imparo_mamba2_products_take", [I, I, I, I])
+    _declare(lib, "imparo_mamba2_products", [P, P, P, P, P, P, P, I, I, P, I, I, I, I, I, P, P, P, S])
     _declare(lib, "imparo_mamba2_scan_chunked", [P, P, P, P, P, P, P, I, I, P, I, I, I, I, I, I, P, P, P, P, S])
     _declare(lib, "imparo_gate_group_rmsnorm", [P, P, I, c_int64, P, c_float, P, I, I, I, I, S])
     _declare(lib, "imparo_moe_route", [P, I, P, I, I, I, I, I, I, I, I, I, P, c_float, c_float, I, P, P, P, P, S])

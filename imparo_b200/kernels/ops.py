@@ -1631,7 +1631,8 @@ def mamba2_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: tor
     S = exp(-exp(A_log) dt) S + dt B x^T;  y = S^T C + D x.  xbc float32 [T, heads*vdim + 2*groups*N] = [x | B | C].
     chunk > 0 (steps with long portions): the rows of a request are cut into chunks of that many rows that run side by
     side; scratch = (int32 [3*max_chunks + n_items + 1], float32 [max_chunks*heads*N*vdim], float32 [max_chunks*heads])
-    with max_chunks = T // chunk + n_items.  The result differs from the row-by-row walk by 32-bit rounding only."""
+    with max_chunks = T // chunk + n_items.  The result differs from the row-by-row walk by 32-bit rounding only.  Chunks of 64
+    rows whose state and value sizes are multiples of 4 (state up to 128) run as products (the int32 scratch is then not used)."""
     _cuda(xbc, dt, A_log, D, state, item_row_start, item_slot, y, status)
     T = xbc.shape[0]
     inner = heads * vdim
@@ -1649,6 +1650,14 @@ def mamba2_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: tor
         _need(si.dtype == torch.int32 and si.numel() >= 3 * max_chunks + n_items + 1 and cs.dtype == torch.float32
               and cs.numel() >= max_chunks * heads * n_state * vdim and cd.dtype == torch.float32 and cd.numel() >= max_chunks * heads,
               "mamba2_scan: chunk scratch too small")
+        if (chunk == 64 and _lib.kernels().imparo_mamba2_products_take(heads, vdim, n_state, groups)
+                and all(t.data_ptr() % 16 == 0 for t in (xbc, state, y, cs))):
+            _check(_lib.kernels().imparo_mamba2_products(_ptr(xbc), _ptr(dt), _ptr(A_log), _ptr(D), _ptr(state), _ptr(item_row_start),
+                                                         _ptr(item_slot), int(n_items), state.shape[0], _ptr(y), heads, vdim, n_state,
+                                                         groups, int(max_chunks), _ptr(cs), _ptr(cd), _ptr(status), _stream()),
+                   "mamba2_products")
+            COUNTS["own"] += 2
+            return
         _check(_lib.kernels().imparo_mamba2_scan_chunked(_ptr(xbc), _ptr(dt), _ptr(A_log), _ptr(D), _ptr(state), _ptr(item_row_start),
                                                          _ptr(item_slot), int(n_items), state.shape[0], _ptr(y), heads, vdim, n_state,
                                                          groups, int(chunk), int(max_chunks), _ptr(si), _ptr(cs), _ptr(cd), _ptr(status),

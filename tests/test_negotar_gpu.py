@@ -420,6 +420,59 @@ def test_state_space_kernels(dtype, heads, vdim, N, groups, taps, norm_groups):
         assert np.abs(g - w).max() <= (3e-5 if dtype == "float32" else 1e-2) * np.abs(w).max()
 
 
+def _scan_64(x, B, C, dt, A_log, D, S, per):
+    """The recurrence in 64 bits, heads side by side: x [T, H, V], B, C [T, groups, N], dt [T, H]; S [H, N, V] is moved on."""
+    import torch
+    y, a = torch.empty_like(x), -torch.exp(A_log)
+    for t in range(len(x)):
+        b, c = B[t].repeat_interleave(per, 0), C[t].repeat_interleave(per, 0)
+        S *= torch.exp(a * dt[t])[:, None, None]
+        S += dt[t][:, None, None] * b[:, :, None] * x[t][:, None]
+        y[t] = torch.einsum("hnv,hn->hv", S, c) + D[:, None] * x[t]
+    return y
+
+
+# state sizes at the edges of both builds, value sizes around a CTA's 64 columns, one, two and four heads per CTA, two groups;
+# portions of one row, whole chunks, a chunk and a row
+@pytest.mark.parametrize("heads,groups,N,vdim", [(3, 3, 4, 4), (2, 1, 64, 64), (2, 2, 68, 20), (4, 1, 128, 132), (8, 2, 60, 64)])
+@pytest.mark.parametrize("lens", [(1, 64, 65), (200, 7), (4800, 128)])
+def test_state_space_products(heads, groups, N, vdim, lens):
+    """Chunks as products against the recurrence in 64 bits and against the row walk, from states other than zero: outputs and
+    states no further off than the walk (twice, for sums in another order); decays that reach zero among them."""
+    import torch
+    from imparo_b200.kernels import ops
+    g = torch.Generator().manual_seed(heads * 1000 + N + vdim + sum(lens))
+    T, slots, inner = sum(lens), [3, 0, 2][:len(lens)], heads * vdim
+    if T > 1000 and heads * vdim > 300:
+        pytest.skip("the oracle's loop is long; the sizes are covered by the others")
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    xbc, dt = rnd(T, inner + 2 * groups * N), torch.nn.functional.softplus(rnd(T, heads) - 2)
+    dt[T // 2] = 200.0
+    A_log, D, state0 = rnd(heads), rnd(heads), rnd(5, heads, N, vdim)
+    starts = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device="cuda")
+    most = T // 64 + len(lens)
+    got = []
+    for chunk, scratch in ((0, None), (64, (torch.empty(3 * most + len(lens) + 1, dtype=torch.int32, device="cuda"),
+                                            torch.full((most * heads * N * vdim,), float("nan"), device="cuda"),
+                                            torch.full((most * heads,), float("nan"), device="cuda")))):
+        state, y, status = state0.cuda(), torch.full((T, inner), float("nan"), device="cuda"), ops.new_status("cuda")
+        ops.mamba2_scan(xbc.cuda(), dt.cuda(), A_log.cuda(), D.cuda(), state, starts, torch.tensor(slots, dtype=torch.int32, device="cuda"),
+                        len(lens), y, heads, vdim, N, groups, status, chunk=chunk, scratch=scratch)
+        ops.read_status(status)
+        got.append((y.cpu().double().reshape(T, heads, vdim), state.cpu().double()))
+    want_state, want, x64 = state0.double(), [], xbc.double()
+    for i, s in enumerate(slots):
+        r = slice(int(starts[i]), int(starts[i + 1]))
+        want.append(_scan_64(x64[r, :inner].reshape(-1, heads, vdim), x64[r, inner:inner + groups * N].reshape(-1, groups, N),
+                             x64[r, inner + groups * N:].reshape(-1, groups, N), dt.double()[r], A_log.double(), D.double(), want_state[s],
+                             heads // groups))
+    want = torch.cat(want)
+    (walk_y, walk_s), (y, s) = got
+    assert (y - want).norm() <= 2 * (walk_y - want).norm() + 1e-7 * want.norm()
+    assert (s - want_state).norm() <= 2 * (walk_s - want_state).norm() + 1e-7 * want_state.norm()
+    assert torch.equal(s[[1, 4]], state0[[1, 4]].double())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width,ff,experts,top,rows", [(64, 40, 6, 2, 5), (96, 64, 5, 1, 90), (100, 30, 3, 3, 33), (128, 64, 8, 2, 300),
                                                        (72, 50, 7, 2, 1), (256, 200, 5, 3, 700), (64, 328, 40, 4, 130)])
