@@ -155,6 +155,7 @@ def _declare_kernels(lib):
     _declare(lib, "imparo_channel_conv_state", [P, c_int64, I, I, I, P, P, P, P, I, I, S])
     _declare(lib, "imparo_delta_prepare", [P, c_int64, I, I, P, c_int64, I, P, P, P, P, I, I, I, I, c_float, c_float, S])
     _declare(lib, "imparo_delta_scan", [P, c_int64, I, I, I, P, P, P, P, P, I, I, P, I, I, I, I, P, S])
+    _declare(lib, "imparo_attention_prefill_f32", [P, P, P, P, P, I, P, I, I, I, I, c_float, P, I, I, I, I, P, S])
     _declare(lib, "imparo_delta_chunk_floats", [I, I, I], c_int64)
     _declare(lib, "imparo_delta_chunked", [P, c_int64, I, I, I, P, P, P, P, P, I, I, I, P, P, I, I, I, I, P, S])
     _declare(lib, "imparo_head_norm_gate", [P, P, c_float, P, I, I, c_int64, P, I, I, I, I, I, S])

@@ -1147,6 +1147,25 @@ def attention_prefill(q, k_cache, v_cache, item_row_start, item_start_pos, n_ite
     return True
 
 
+def attention_prefill_f32(q, k_cache, v_cache, item_row_start, item_start_pos, n_items, table, page_size, n_pages, window, scale, out, nh,
+                          nkv, hd, status) -> bool:
+    """Attention for prompt portions in 32-bit, tiles of 64 queries against tiles of 64 keys (csrc/kernels/attention_f32.cu).
+    Returns False, having launched nothing, unless q is float32 and the head size a multiple of 4 up to 128."""
+    if q.dtype != torch.float32 or hd % 4 or hd > 128 or any(t.data_ptr() % 16 for t in (q, k_cache, v_cache, out)):
+        return False
+    _cuda(q, k_cache, v_cache, item_row_start, item_start_pos, table, out, status)
+    T = q.shape[0]
+    _need(q.shape == (T, nh * hd) and out.shape == (T, nh * hd) and out.dtype == q.dtype, "attention_prefill_f32: q/out shapes")
+    _need(k_cache.dtype == q.dtype and v_cache.dtype == q.dtype, "cache dtype must match q")
+    _need(k_cache.numel() >= n_pages * page_size * nkv * hd, "cache arena smaller than n_pages")
+    _need(table.dtype == torch.int32 and table.dim() == 2 and table.shape[0] >= n_items, "block table must be int32 [items, blocks]")
+    _need(item_row_start.numel() >= n_items + 1 and item_start_pos.numel() >= n_items, "attention_prefill_f32: item arrays")
+    _check(_lib.kernels().imparo_attention_prefill_f32(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(item_row_start), _ptr(item_start_pos), n_items,
+                                                       _ptr(table), table.shape[1], page_size, n_pages, int(window or 0), float(scale),
+                                                       _ptr(out), T, nh, nkv, hd, _ptr(status), _stream()), "attention_prefill_f32")
+    return True
+
+
 # ---- attention with sigmoid weights (csrc/kernels/attention_sigmoid.cu) -----------------------------------------
 def _sigmoid_takes(q, k_cache, v_cache, nh, nkv, hd, vd) -> bool:
     return (q.dtype == torch.bfloat16 and k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and hd % 16 == 0 and vd % 16 == 0

@@ -454,6 +454,11 @@ class AttentionMixer(Part):
         ops.qk_norm_rope_store(qkv, batch.positions, batch.item_of_token, self.q_norm, self.k_norm, inv_freq, n_rot,
                                self.eps, q, kv.k, kv.v, table, kv.page_size, kv.n_pages, nh, nkv, hd, rt.status)
         done = False
+        # the prompt kernels: tensor cores for bfloat16, tiles of 32-bit products else
+        if rt.act_dtype == torch.float32:
+            prefill, beside = ops.attention_prefill_f32, {}
+        else:
+            prefill, beside = ops.attention_prefill, {"dependents_after_wait": ops.switches().attn_side_by_side}
         n1 = getattr(batch, "n_single", 0)             # decode rows come first when the step also holds portions
         if batch.max_tokens_per_item >= 8 and 0 < n1 < batch.n_items and nh // self.nkv <= 8:
             # Portions beside decode rows: the prompt kernel walks a request's keys tile by tile in one
@@ -461,9 +466,8 @@ class AttentionMixer(Part):
             # context.  So the portions (requests n1 onward) go to the prompt kernel and the decode rows
             # (the first n1 tokens, one per request) to the split-key kernel, which cuts their keys
             # over many CTAs.
-            done = ops.attention_prefill(q, kv.k, kv.v, batch.item_row_start[n1:], batch.item_start_pos[n1:],
-                                         batch.n_items - n1, table[n1:], kv.page_size, kv.n_pages, self.window, self.scale,
-                                         out, nh, self.nkv, hd, rt.status, dependents_after_wait=ops.switches().attn_side_by_side)
+            done = prefill(q, kv.k, kv.v, batch.item_row_start[n1:], batch.item_start_pos[n1:], batch.n_items - n1, table[n1:],
+                           kv.page_size, kv.n_pages, self.window, self.scale, out, nh, self.nkv, hd, rt.status, **beside)
             if done:
                 chunk, n_splits = ops.split_plan(n1, self.nkv, table.shape[1] * kv.page_size)
                 room = self._partials_room(table.shape[1] * kv.page_size)
@@ -473,9 +477,14 @@ class AttentionMixer(Part):
                                           kv.page_size, kv.n_pages, self.window, self.scale, out[:n1], part_acc, part_ml,
                                           chunk, n_splits, nh, self.nkv, hd, rt.status, fresh=1, overlap_prev=done == 2)
         elif batch.max_tokens_per_item >= 8:
-            # prompt portions: the tensor-core kernel (bfloat16, head size 64 or 128), tiles of one request each
-            done = ops.attention_prefill(q, kv.k, kv.v, batch.item_row_start, batch.item_start_pos, batch.n_items, table,
-                                         kv.page_size, kv.n_pages, self.window, self.scale, out, nh, self.nkv, hd, rt.status)
+            # prompt portions, tiles of one request each
+            done = prefill(q, kv.k, kv.v, batch.item_row_start, batch.item_start_pos, batch.n_items, table, kv.page_size, kv.n_pages,
+                           self.window, self.scale, out, nh, self.nkv, hd, rt.status)
+            if done and rt.act_dtype == torch.float32:
+                # the decode rows' scratch as the split-key kernel would have made it here, so that a step of decode rows finds it
+                room = self._partials_room(table.shape[1] * kv.page_size)
+                rt.workspace.get("attn_part_acc", (1,), torch.float32, reserve=room * hd)
+                rt.workspace.get("attn_part_ml", (1,), torch.float32, reserve=room * 2)
         if not done and nh // self.nkv <= 8 and T <= 65535:
             # keys cut into chunks; the cut depends on the launch's shape (tokens, table width) only
             chunk, n_splits = ops.split_plan(T, self.nkv, table.shape[1] * kv.page_size)

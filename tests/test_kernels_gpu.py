@@ -758,6 +758,45 @@ def test_attention_prefill_tensor_cores(nh, nkv, hd, page, window, kernel):
             t += 1
 
 
+# head sizes around both builds (64 and 128 channels), windows shorter than a tile and across tiles, pages below and above a tile
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 64), (3, 1, 12), (2, 2, 68), (9, 1, 128)])
+@pytest.mark.parametrize("page,window", [(4, None), (16, 50), (96, 7), (128, 200)])
+def test_attention_prefill_f32(nh, nkv, hd, page, window):
+    o = ops()
+    rng = np.random.default_rng(nh * 100 + hd + page)
+    portions = [(37, 130), (0, 1), (0, 64), (200, 9), (115, 129)]            # (start position, tokens)
+    table, kc, vc, ks, vs, n_pages = make_paged(rng, [s + n for s, n in portions], page, nkv, hd, torch.float32)
+    T, lead = sum(n for _, n in portions), 3                                 # rows of other requests ahead of the portions
+    q = torch.from_numpy(rng.standard_normal((lead + T, nh * hd)).astype(np.float32))
+    dev = lambda a: torch.from_numpy(np.asarray(a, dtype=np.int32)).to(DEV)
+    out, status, scale = torch.full((lead + T, nh * hd), float("nan"), device=DEV), o.new_status(DEV), 1 / math.sqrt(hd)
+    assert o.attention_prefill_f32(q.to(DEV), kc.to(DEV), vc.to(DEV), dev(lead + np.concatenate([[0], np.cumsum([n for _, n in portions])])),
+                                   dev([s for s, _ in portions]), len(portions), dev(table), page, n_pages, window, scale, out, nh, nkv, hd, status)
+    o.read_status(status)
+    got = out.cpu().double().numpy()
+    assert np.isnan(got[:lead]).all()
+    t = lead
+    for r, (s, n) in enumerate(portions):
+        for i in range(n):
+            if i % 7 in (0, 3) or i > n - 3:
+                ref = attention_reference(q[t].double().numpy(), ks[r].double().numpy(), vs[r].double().numpy(), s + i, nh, nkv, hd, scale, window)
+                assert np.abs(got[t] - ref).max() <= 3e-6 * max(1.0, np.abs(ref).max()), (r, s + i)
+            t += 1
+
+
+def test_attention_prefill_f32_refuses_bad_pages_and_other_shapes():
+    o = ops()
+    z, status = torch.zeros(70, 64, device=DEV), o.new_status(DEV)
+    kv = torch.zeros(2 * 64, 64, device=DEV)
+    one = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    assert o.attention_prefill_f32(z, kv, kv, one(0, 70), one(0), 1, one(1, 2).view(1, 2), 64, 2, None, 1.0, torch.empty_like(z), 1, 1, 64, status)
+    with pytest.raises(o.KernelError, match="page"):
+        o.read_status(status)
+    assert not o.attention_prefill_f32(z, kv, kv, None, None, 1, None, 64, 2, None, 1.0, z, 1, 1, 66, None)
+    zb = z.bfloat16()
+    assert not o.attention_prefill_f32(zb, zb, zb, None, None, 1, None, 64, 2, None, 1.0, zb, 1, 1, 64, None)
+
+
 @pytest.mark.parametrize("nh,nkv", [(6, 2), (8, 2), (5, 1)])
 @pytest.mark.parametrize("start,n", [(3180, 488), (2017, 130), (1, 260)])
 def test_attention_prefill_portion_far_into_its_request(nh, nkv, start, n):
