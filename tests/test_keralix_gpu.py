@@ -280,6 +280,13 @@ def test_stream_copies_kernels(n, width, dtype):
         assert np.abs(e.cpu().numpy()[:, s * width:(s + 1) * width] - want_e).max() <= 1e-6 * np.abs(want_e).max()
 
 
+# two and four copies have builds of their own, widths that are no multiples of four another; rows longer than a block's first round
+@pytest.mark.parametrize("n,width", [(2, 64), (2, 33), (4, 1030), (4, 2052), (5, 516)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_stream_copies_kernels_by_copies_and_width(n, width, dtype):
+    test_stream_copies_kernels(n, width, dtype)
+
+
 @pytest.mark.parametrize("channels,taps,act,biased", [(96, 3, None, True), (40, 1, "silu", False), (300, 5, "silu", False), (17, 2, None, True)])
 def test_channel_conv_kernel(channels, taps, act, biased):
     """Three requests of unequal length in one launch, then their next portions and single tokens from the inputs the
