@@ -10,7 +10,7 @@
 //      product, a quarter of a 32-bit rounding.  The large product of a stretch of 64 k (first piece times first piece)
 //      is summed by the tensor core into an accumulator of its own, read back and added to the others' in registers with
 //      32-bit rounding: the tensor core's accumulator truncates, and over a whole K that adds up to more than the
-//      FFMA chain's error.  The five small products, 2^-8 of it and below, share one accumulator over all of K.
+//      FFMA chain's error.  The small products, 2^-8 and 2^-16 of it, keep two accumulators over all of K.
 //      Nothing of this leaves the 32-bit range: a result that is not finite (an operand or a piece of it that overflowed)
 //      is computed again by the FFMA chain, which then says what it is.
 //  (2) sgemm_nt_kernel: everything else, FFMA only, one accumulator per element summed over k = 0..K-1 in order.
@@ -87,10 +87,12 @@ constexpr int WORKERS = 16;                                   // warps that cut 
 constexpr int THREADS = 32 * (WORKERS + 1);                   // ... and one that issues the MMAs
 constexpr int STAGES = 2;
 
-template <int TN> constexpr uint32_t a_plane() { return TM * 128; }
+constexpr uint32_t A_PLANE = TM * 128;
 template <int TN> constexpr uint32_t b_plane() { return TN * 128; }
-template <int TN> constexpr uint32_t stage_bytes() { return 3 * (a_plane<TN>() + b_plane<TN>()); }
+template <int TN> constexpr uint32_t stage_bytes() { return 3 * (A_PLANE + b_plane<TN>()); }
 template <int TN> constexpr size_t smem_bytes() { return 1024 + (size_t)STAGES * stage_bytes<TN>() + 256; }
+// Accumulators, TN columns each: [large, even stretches | small | small | large, odd stretches]
+template <int TN> constexpr uint32_t tmem_cols() { return 4 * TN; }
 
 struct Params {
     const float* a; const float* w; float* c;
@@ -123,21 +125,30 @@ __device__ __noinline__ float whole_sum(const float* x, const float* w, int K) {
     return t;
 }
 
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(0u) : "memory");
+}
+
 // One CTA per tile of TM x TN outputs.  A stretch of 64 k is 3 planes of A (16 KB each) and 3 of W in shared memory, in the
-// swizzled layout of a bfloat16 K-major operand; sixteen warps read the 32-bit operands (one stretch ahead, in registers),
-// cut them and store the planes, the seventeenth issues 24 MMAs of 128 x TN x 16; meanwhile the sixteen read the large
-// accumulator of the stretch before (two of them alternate).
-// What bounds it: shared memory.  The MMAs' operand reads and the planes' writes are 288 KB per stretch at TN = 128 (2,300
-// cycles at 128 bytes a cycle; the MMAs alone 1,540), 216 KB at TN = 64; measured 4,100 and 2,900 cycles per stretch (with
-// the large product alone 3,100 and 2,000).  Sixteen workers and not eight: the loop's straight code is half as long per
-// warp, and eight waited for instructions more than for anything else (1,000 x 9,216 x 1,024: 162 against 139 us).
-// Against the FFMA kernel (B200, us): 1,000 x 9,216 x 1,024: 837 -> 139 (136 TFLOP/s); 1,000 x 1,024 x 4,608: 920 -> 114;
-// 60 x 3,072 x 1,024: 77 -> 28; error against 64 bits 5.7e-7 -> 1.1e-7 (K 1,024), 1.2e-6 -> 1.8e-7 (K 4,608).
+// swizzled layout of a bfloat16 K-major operand; sixteen warps read the 32-bit operands (one stretch ahead, in registers), cut
+// them and store the planes, the seventeenth issues the MMAs; before a stage is filled again the sixteen read the large
+// accumulator of the stretch that had it (two alternate) and clear it.
+// The planes of W lie one after the other, so that one MMA takes two of them as its N operand where the two accumulators are
+// neighbours: (first piece x first, x second) and (second x first, x second) are one MMA each per 16 k, 16 per stretch instead
+// of 24, and A's planes are read for four instead of six.  For that the odd stretches swap W's first two planes, and which of
+// the two small accumulators takes which of the small products alternates.  The order of the sums is the same for both widths.
+// What bounds it: the workers' share of a stretch (loads, cutting, stores, reading out, one after the other in a warp), 3,000
+// cycles at TN = 128 and 2,250 at TN = 64, which is what the large product alone takes (3,100 and 2,000).  Sixteen workers and
+// not eight: the loop's straight code is half as long per warp, and eight waited for instructions more than for anything else.
+// At TN = 64 one MMA could take all three planes (12 per stretch, 93 -> 86 us at K 4,608); the sums would not be those of the
+// wide tile.
+// FFMA kernel -> 24 MMAs -> this (B200, us): 1,000 x 9,216 x 1,024: 837 -> 139 -> 132 (143 TFLOP/s); 1,000 x 1,024 x 4,608:
+// 920 -> 112 -> 93; 60 x 3,072 x 1,024: 77 -> 27.6 -> 23.6; 2,048 x 1,024 x 8,192: 230 -> 215 (the last two).  Error against
+// 64 bits: 5.7e-7 -> 1.05e-7 -> 1.04e-7 (K 1,024), 1.2e-6 -> 1.8e-7 -> 1.7e-7 (K 4,608).
 template <int TN>
 __global__ void __launch_bounds__(THREADS, 1)
 sgemm_split_kernel(const Params p) {
-    constexpr uint32_t A_PLANE = a_plane<TN>(), B_PLANE = b_plane<TN>(), STAGE = stage_bytes<TN>();
-    constexpr uint32_t TMEM_COLS = TN == 128 ? 512 : 256;     // two large accumulators and the small products' one
+    constexpr uint32_t B_PLANE = b_plane<TN>(), STAGE = stage_bytes<TN>();
     constexpr int ROUND = WORKERS * 4;                        // rows of a stretch per round of the workers
     constexpr int COLS = TN * 4 / WORKERS;                    // accumulator columns of a worker thread
     constexpr int A_IT = TM / ROUND, B_IT = TN / ROUND;
@@ -145,52 +156,51 @@ sgemm_split_kernel(const Params p) {
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE);      // [STAGES] the stage's planes are stored
     uint64_t* empty = full + STAGES;                                          // [STAGES] ... and read by its MMAs
-    uint64_t* acc_full = empty + STAGES;                                      // [2] a stretch's large product is summed
-    uint64_t* acc_empty = acc_full + 2;                                       // [2] ... and in the workers' registers
+    uint64_t* acc_empty = empty + STAGES;                                     // [2] a stretch's large products are in the workers' registers
     uint64_t* done = acc_empty + 2;                                           // [1] every MMA is complete
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
-    pdl_trigger();
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], WORKERS); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], WORKERS); }
+        for (int b = 0; b < 2; ++b) mbar_init(&acc_empty[b], WORKERS);
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == WORKERS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols<TN>()) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot, small = tmem + 2 * TN;
+    const uint32_t tmem = *tmem_slot;
+    pdl_trigger();                                            // (after the allocation: a follower's cannot come before it)
 
     if (warp == WORKERS) {
         if (lane == 0) {
-            const uint32_t idesc = instr_desc(TM, TN);
-            bool ok = true;
-            for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+            const uint32_t one = instr_desc(TM, TN), two = instr_desc(TM, 2 * TN);
+            for (int kb = 0; kb < p.kblocks; ++kb) {
                 const int s = kb % STAGES, b = kb & 1;
-                if (kb >= 2 && !mbar_wait(&acc_empty[b], ((kb >> 1) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 90, blockIdx.x, kb); ok = false; break; }
-                if (!mbar_wait(&full[s], (kb / STAGES) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 91, blockIdx.x, kb); ok = false; break; }
+                if (kb >= 2 && !mbar_wait(&acc_empty[b], ((kb >> 1) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 90, blockIdx.x, kb); break; }
+                if (!mbar_wait(&full[s], (kb / STAGES) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 91, blockIdx.x, kb); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t a0 = smem_desc(smem_u32(smem) + s * STAGE), b0 = smem_desc(smem_u32(smem) + s * STAGE + 3 * A_PLANE);
-                auto product = [&](uint32_t d, int pa, int pb, bool first) {
-                    const uint64_t da = a0 + (uint64_t)((pa * A_PLANE) >> 4), db = b0 + (uint64_t)((pb * B_PLANE) >> 4);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma(d, da + (uint64_t)((k * UMMA_K * 2) >> 4), db + (uint64_t)((k * UMMA_K * 2) >> 4), idesc, (first && k == 0) ? 0u : 1u);
+                // (every accumulator is zero before it is first used: the workers clear them)
+                auto mma = [&](uint32_t d, int pa, int pb, int k, uint32_t idesc) {
+                    umma(tmem + d, a0 + (uint64_t)((pa * A_PLANE + k * UMMA_K * 2) >> 4), b0 + (uint64_t)((pb * B_PLANE + k * UMMA_K * 2) >> 4), idesc, 1u);
                 };
-                product(tmem + (uint32_t)b * TN, 0, 0, true);
-                umma_commit(&acc_full[b]);
-                product(small, 0, 1, kb == 0);
-                product(small, 1, 0, false);
-                product(small, 0, 2, false);
-                product(small, 1, 1, false);
-                product(small, 2, 0, false);
+                // planes of W: first, second, third; in odd stretches second, first, third
+                const uint32_t small = b ? TN : 2 * TN;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma(b ? 2 * TN : 0, 0, 0, k, two);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma(TN, 1, 0, k, two);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma(small, 0, 2, k, one);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma(small, 2, b, k, one);
                 umma_commit(&empty[s]);
             }
             // what has been issued must be complete before the CTA gives its memory back, also after a wait that ran out
@@ -210,16 +220,17 @@ sgemm_split_kernel(const Params p) {
         };
         auto load_a = [&](int kb, int i) { load(p.a, p.lda, m0 + r0 + ROUND * i, p.M, kb, ra[i]); };
         auto load_b = [&](int kb, int i) { load(p.w, p.K, n0 + r0 + ROUND * i, p.N, kb, rb[i]); };
-        auto store = [&](uint8_t* base, uint32_t plane, int row, const float4 (&v)[2]) {
+        // first, second, third: offsets of the pieces' planes
+        auto store = [&](uint8_t* base, uint32_t first, uint32_t second, uint32_t third, int row, const float4 (&v)[2]) {
             uint4 h, m, l;
             cut(v[0].x, v[0].y, h.x, m.x, l.x);
             cut(v[0].z, v[0].w, h.y, m.y, l.y);
             cut(v[1].x, v[1].y, h.z, m.z, l.z);
             cut(v[1].z, v[1].w, h.w, m.w, l.w);
             uint8_t* at = base + row * 128 + ((c ^ (row & 7)) << 4);
-            *reinterpret_cast<uint4*>(at) = h;
-            *reinterpret_cast<uint4*>(at + plane) = m;
-            *reinterpret_cast<uint4*>(at + 2 * plane) = l;
+            *reinterpret_cast<uint4*>(at + first) = h;
+            *reinterpret_cast<uint4*>(at + second) = m;
+            *reinterpret_cast<uint4*>(at + third) = l;
         };
         const int quad = warp & 3, part = warp >> 2;
         const uint32_t lanes = (uint32_t)(quad * 32) << 16;
@@ -227,13 +238,18 @@ sgemm_split_kernel(const Params p) {
 #pragma unroll
         for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
         bool ok = true;
+        // the large products of stretch kb, whose MMAs are complete (`empty` of its stage: what says so)
         auto drain = [&](int kb) {
             const int b = kb & 1;
-            if (!mbar_wait(&acc_full[b], (kb >> 1) & 1)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 92, blockIdx.x, kb); ok = false; }
+            if (!mbar_wait(&empty[kb % STAGES], (kb / STAGES) & 1)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 92, blockIdx.x, kb); ok = false; }
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) return;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tmem_add<COLS>(tmem + lanes + (uint32_t)(b * TN + part * COLS), acc);
+            const uint32_t at = tmem + lanes + (uint32_t)((b ? 3 * TN : 0) + part * COLS);
+            tmem_add<COLS>(at, acc);
+#pragma unroll
+            for (int j = 0; j < COLS; j += 16) tmem_zero16(at + j);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
@@ -243,37 +259,47 @@ sgemm_split_kernel(const Params p) {
         pdl_wait();
 #pragma unroll
         for (int i = 0; i < A_IT; ++i) load_a(0, i);
+#pragma unroll
+        for (int j = 0; j < (int)tmem_cols<TN>() / 4; j += 16) tmem_zero16(tmem + lanes + (uint32_t)(part * (tmem_cols<TN>() / 4) + j));
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");       // (the first stretch's arrival tells the MMAs)
         for (int kb = 0; kb < p.kblocks && ok; ++kb) {
             const int s = kb % STAGES;
-            if (kb >= STAGES) {
-                if (!mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 93, blockIdx.x, kb); ok = false; }
-                ok = __all_sync(0xffffffffu, ok);
+            if (kb >= STAGES) {                                // the stage is free, and its stretch's accumulator can be read
+                drain(kb - STAGES);
                 if (!ok) break;
             }
             uint8_t* base = smem + s * STAGE;
+            const bool swapped = kb & 1;
             // a piece's registers are asked to be filled again as soon as they are stored (beyond the last stretch the
             // loads are masked off)
 #pragma unroll
             for (int i = 0; i < A_IT; ++i) {
-                store(base, A_PLANE, r0 + ROUND * i, ra[i]);
+                store(base, 0, A_PLANE, 2 * A_PLANE, r0 + ROUND * i, ra[i]);
                 load_a(kb + 1, i);
             }
 #pragma unroll
             for (int i = 0; i < B_IT; ++i) {
-                store(base + 3 * A_PLANE, B_PLANE, r0 + ROUND * i, rb[i]);
+                store(base + 3 * A_PLANE, swapped ? B_PLANE : 0, swapped ? 0 : B_PLANE, 2 * B_PLANE, r0 + ROUND * i, rb[i]);
                 load_b(kb + 1, i);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the planes are read by the async proxy
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[s])) : "memory");
-            if (kb > 0) drain(kb - 1);
         }
-        if (ok) drain(p.kblocks - 1);
+        for (int kb = max(0, p.kblocks - STAGES); kb < p.kblocks && ok; ++kb) drain(kb);
         if (ok && !mbar_wait(done, 0)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 94, blockIdx.x, p.kblocks); ok = false; }
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tmem_add<COLS>(small + lanes + (uint32_t)(part * COLS), acc);
+            float small[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) small[j] = 0.f;
+            const uint32_t at = tmem + lanes + (uint32_t)(part * COLS);
+            tmem_add<COLS>(at + TN, small);
+            tmem_add<COLS>(at + 2 * TN, small);
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) acc[j] += small[j];
             const int row = m0 + quad * 32 + lane;
             if (row < p.M) {
                 const int col0 = n0 + part * COLS;
@@ -307,7 +333,7 @@ sgemm_split_kernel(const Params p) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == WORKERS) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols<TN>()) : "memory");
     }
 }
 
@@ -337,8 +363,8 @@ extern "C" int imparo_sgemm_nt(const float* A, const float* W, float* C, int M, 
     if (K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && (N + 63) / 64 <= 65535) {
         imparo::sp::Params p{A, W, C, M, N, K, lda, ldc, accumulate, (K + 63) / 64, status};
         // tiles of 128 x 64 where tiles of 128 x 128 would leave more than half of the 148 SMs without one (1,000 x 1,024 x
-        // 4,608: 114 against 156 us); above that a wide tile costs 1.4 times a narrow one and does twice the work.  The
-        // sums are the same either way.
+        // 4,608: 93 against 121 us); above that the wide tile is the faster one (500 x 3,072 x 1,024, 96 wide tiles: 34 against
+        // 49 us; 1,000 x 9,216 x 1,024: 132 against 194).  The sums are the same either way.
         const long long tiles = (long long)((M + 127) / 128) * ((N + 127) / 128);
         return tiles * 2 <= 148 ? imparo::sp::launch_split<64>(p, stream) : imparo::sp::launch_split<128>(p, stream);
     }
