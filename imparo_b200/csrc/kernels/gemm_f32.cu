@@ -4,15 +4,17 @@
 // y[t,o] = sum_i W[o,i]*x[t,i] (imparo-cpu/src/ops.rs:660,688-690).  A row's result depends neither on how many other
 // rows the call carries nor on where in the call it stands.
 //
-//  (1) sgemm_split_kernel: rows of 16-byte groups.  Every 32-bit operand is cut into three bfloat16 pieces that add up
-//      to it to its last bit (8 + 8 + 8 significant bits, each piece rounded to nearest, so the remainders carry either
-//      sign), and six of the nine products of pieces run on the tensor cores: what is left out is below 2^-26 of a
-//      product, a quarter of a 32-bit rounding.  The large product of a stretch of 64 k (first piece times first piece)
-//      is summed by the tensor core into an accumulator of its own, read back and added to the others' in registers with
-//      32-bit rounding: the tensor core's accumulator truncates, and over a whole K that adds up to more than the
-//      FFMA chain's error.  The small products, 2^-8 and 2^-16 of it, keep two accumulators over all of K.
-//      Nothing of this leaves the 32-bit range: a result that is not finite (an operand or a piece of it that overflowed)
-//      is computed again by the FFMA chain, which then says what it is.
+//  (1) sgemm_split_kernel: rows of 16-byte groups.  Every 32-bit operand is cut into three bfloat16 pieces, h + m / 2^8 +
+//      l / 2^16, that add up to it to its last bit (8 + 8 + 8 significant bits, each piece rounded to nearest, so the
+//      remainders carry either sign; held at their own scales, the lower pieces keep all their bits however small the operand
+//      is), and six of the nine products of pieces run on the tensor cores: what is left out is below 2^-26 of a product, a
+//      quarter of a 32-bit rounding, or, where an operand is subnormal, below 2^-151 of the other operand, a quarter of half
+//      its last place.  The large product of a stretch of 64 k (h times h) is summed by the tensor core into an accumulator
+//      of its own, read back and added to the others' in registers with 32-bit rounding: the tensor core's accumulator
+//      truncates, and over a whole K that adds up to more than the FFMA chain's error.  The small products, 2^-8 and 2^-16
+//      of it, have an accumulator each over all of K, at their scales, so that what they add to a small result is not lost
+//      below the smallest 32-bit number.  At the upper end a result that is not finite (an operand whose first piece
+//      rounds to infinity, a sum that overflows) is computed again by the FFMA chain, which then says what it is.
 //  (2) sgemm_nt_kernel: everything else, FFMA only, one accumulator per element summed over k = 0..K-1 in order.
 #include "tcgen05.cuh"
 
@@ -91,7 +93,7 @@ constexpr uint32_t A_PLANE = TM * 128;
 template <int TN> constexpr uint32_t b_plane() { return TN * 128; }
 template <int TN> constexpr uint32_t stage_bytes() { return 3 * (A_PLANE + b_plane<TN>()); }
 template <int TN> constexpr size_t smem_bytes() { return 1024 + (size_t)STAGES * stage_bytes<TN>() + 256; }
-// Accumulators, TN columns each: [large, even stretches | small | small | large, odd stretches]
+// Accumulators, TN columns each: [large, even stretches | small x 2^8 | small x 2^16 | large, odd stretches]
 template <int TN> constexpr uint32_t tmem_cols() { return 4 * TN; }
 
 struct Params {
@@ -100,14 +102,19 @@ struct Params {
     int* status;
 };
 
-// two neighbours cut into three bfloat16 pieces each (h + m + l is the operand, exactly), packed in pairs
+// two neighbours cut into three bfloat16 pieces each (h + m / 2^8 + l / 2^16 is the operand, exactly), packed in pairs
 __device__ __forceinline__ void cut(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
     auto pack = [](float u, float v) { __nv_bfloat162 t = __floats2bfloat162_rn(u, v); return *reinterpret_cast<uint32_t*>(&t); };
-    h = pack(x, y);
-    x -= __uint_as_float(h << 16); y -= __uint_as_float(h & 0xffff0000u);
-    m = pack(x, y);
-    x -= __uint_as_float(m << 16); y -= __uint_as_float(m & 0xffff0000u);
-    l = pack(x, y);
+    auto rest = [](float2 v, uint32_t piece) {       // (both steps are exact: the subtraction, and times a power of two)
+        v = __ffma2_rn(make_float2(__uint_as_float(piece << 16), __uint_as_float(piece & 0xffff0000u)), make_float2(-1.f, -1.f), v);
+        return __fmul2_rn(v, make_float2(256.f, 256.f));
+    };
+    float2 v = make_float2(x, y);
+    h = pack(v.x, v.y);
+    v = rest(v, h);
+    m = pack(v.x, v.y);
+    v = rest(v, m);
+    l = pack(v.x, v.y);
 }
 
 template <int COLS>
@@ -134,9 +141,8 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
 // them and store the planes, the seventeenth issues the MMAs; before a stage is filled again the sixteen read the large
 // accumulator of the stretch that had it (two alternate) and clear it.
 // The planes of W lie one after the other, so that one MMA takes two of them as its N operand where the two accumulators are
-// neighbours: (first piece x first, x second) and (second x first, x second) are one MMA each per 16 k, 16 per stretch instead
-// of 24, and A's planes are read for four instead of six.  For that the odd stretches swap W's first two planes, and which of
-// the two small accumulators takes which of the small products alternates.  The order of the sums is the same for both widths.
+// neighbours: (h x m, h x l) and (m x h, m x m) are one MMA each per 16 k into the two small accumulators, 16 per stretch
+// instead of 24, and A's planes are read for four instead of six.  The order of the sums is the same for both widths.
 // What bounds it: the workers' share of a stretch (loads, cutting, stores, reading out, one after the other in a warp), 3,000
 // cycles at TN = 128 and 2,250 at TN = 64, which is what the large product alone takes (3,100 and 2,000).  Sixteen workers and
 // not eight: the loop's straight code is half as long per warp, and eight waited for instructions more than for anything else.
@@ -191,16 +197,14 @@ sgemm_split_kernel(const Params p) {
                 auto mma = [&](uint32_t d, int pa, int pb, int k, uint32_t idesc) {
                     umma(tmem + d, a0 + (uint64_t)((pa * A_PLANE + k * UMMA_K * 2) >> 4), b0 + (uint64_t)((pb * B_PLANE + k * UMMA_K * 2) >> 4), idesc, 1u);
                 };
-                // planes of W: first, second, third; in odd stretches second, first, third
-                const uint32_t small = b ? TN : 2 * TN;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma(b ? 2 * TN : 0, 0, 0, k, two);
+                for (int k = 0; k < 4; ++k) mma(b ? 3 * TN : 0, 0, 0, k, one);         // h x h
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma(TN, 1, 0, k, two);
+                for (int k = 0; k < 4; ++k) mma(TN, 0, 1, k, two);                     // h x m, h x l
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma(small, 0, 2, k, one);
+                for (int k = 0; k < 4; ++k) mma(TN, 1, 0, k, two);                     // m x h, m x m
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma(small, 2, b, k, one);
+                for (int k = 0; k < 4; ++k) mma(2 * TN, 2, 0, k, one);                 // l x h
                 umma_commit(&empty[s]);
             }
             // what has been issued must be complete before the CTA gives its memory back, also after a wait that ran out
@@ -220,17 +224,16 @@ sgemm_split_kernel(const Params p) {
         };
         auto load_a = [&](int kb, int i) { load(p.a, p.lda, m0 + r0 + ROUND * i, p.M, kb, ra[i]); };
         auto load_b = [&](int kb, int i) { load(p.w, p.K, n0 + r0 + ROUND * i, p.N, kb, rb[i]); };
-        // first, second, third: offsets of the pieces' planes
-        auto store = [&](uint8_t* base, uint32_t first, uint32_t second, uint32_t third, int row, const float4 (&v)[2]) {
+        auto store = [&](uint8_t* base, uint32_t plane, int row, const float4 (&v)[2]) {
             uint4 h, m, l;
             cut(v[0].x, v[0].y, h.x, m.x, l.x);
             cut(v[0].z, v[0].w, h.y, m.y, l.y);
             cut(v[1].x, v[1].y, h.z, m.z, l.z);
             cut(v[1].z, v[1].w, h.w, m.w, l.w);
             uint8_t* at = base + row * 128 + ((c ^ (row & 7)) << 4);
-            *reinterpret_cast<uint4*>(at + first) = h;
-            *reinterpret_cast<uint4*>(at + second) = m;
-            *reinterpret_cast<uint4*>(at + third) = l;
+            *reinterpret_cast<uint4*>(at) = h;
+            *reinterpret_cast<uint4*>(at + plane) = m;
+            *reinterpret_cast<uint4*>(at + 2 * plane) = l;
         };
         const int quad = warp & 3, part = warp >> 2;
         const uint32_t lanes = (uint32_t)(quad * 32) << 16;
@@ -270,17 +273,16 @@ sgemm_split_kernel(const Params p) {
                 if (!ok) break;
             }
             uint8_t* base = smem + s * STAGE;
-            const bool swapped = kb & 1;
             // a piece's registers are asked to be filled again as soon as they are stored (beyond the last stretch the
             // loads are masked off)
 #pragma unroll
             for (int i = 0; i < A_IT; ++i) {
-                store(base, 0, A_PLANE, 2 * A_PLANE, r0 + ROUND * i, ra[i]);
+                store(base, A_PLANE, r0 + ROUND * i, ra[i]);
                 load_a(kb + 1, i);
             }
 #pragma unroll
             for (int i = 0; i < B_IT; ++i) {
-                store(base + 3 * A_PLANE, swapped ? B_PLANE : 0, swapped ? 0 : B_PLANE, 2 * B_PLANE, r0 + ROUND * i, rb[i]);
+                store(base + 3 * A_PLANE, B_PLANE, r0 + ROUND * i, rb[i]);
                 load_b(kb + 1, i);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the planes are read by the async proxy
@@ -292,14 +294,16 @@ sgemm_split_kernel(const Params p) {
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float small[COLS];
+            const uint32_t at = tmem + lanes + (uint32_t)(part * COLS);
+            float small[COLS];                                 // (m m + h l + l h) / 2^8 + h m + m h, then / 2^8
 #pragma unroll
             for (int j = 0; j < COLS; ++j) small[j] = 0.f;
-            const uint32_t at = tmem + lanes + (uint32_t)(part * COLS);
-            tmem_add<COLS>(at + TN, small);
             tmem_add<COLS>(at + 2 * TN, small);
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) acc[j] += small[j];
+            for (int j = 0; j < COLS; ++j) small[j] *= 0.00390625f;
+            tmem_add<COLS>(at + TN, small);
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) acc[j] = fmaf(small[j], 0.00390625f, acc[j]);
             const int row = m0 + quad * 32 + lane;
             if (row < p.M) {
                 const int col0 = n0 + part * COLS;

@@ -127,6 +127,27 @@ def test_sgemm_split_edges(M, N, K, ld):
     assert torch.equal(one[0], out[M // 2])                           # a row alone is the row among others
 
 
+# operands and results at the lower end of the range, where bfloat16 pieces of the operands' own scale would lose bits
+@pytest.mark.parametrize("ea,ew", [(-100, 60), (-112, 80), (-124, 110), (-135, 120), (-148, 120), (100, -124), (120, -140), (-60, -66), (-70, -68)])
+@pytest.mark.parametrize("M,N,K", [(130, 70, 200), (129, 4800, 72)])
+def test_sgemm_split_small_operands(M, N, K, ea, ew):
+    o = ops()
+    g = torch.Generator().manual_seed(1000 + ea)
+    draw = lambda rows, e: (torch.randn(rows, K, generator=g, dtype=torch.float64) * 2.0 ** e).float()
+    a, w = draw(M, ea), draw(N, ew)
+    a[M // 2:, 1::3] = torch.randn(M - M // 2, len(range(1, K, 3)), generator=g)          # small operands beside ordinary ones ...
+    w[:, 1::3] *= 2.0 ** -max(0, ew)                                                      # ... whose products are small
+    ref = a.double() @ w.double().T
+    total = a.double().abs() @ w.double().abs().T
+    ends = a.double().abs().sum(1)[:, None] + w.double().abs().sum(1)[None]
+    # the bound of test_sgemm_split_edges; what is left out beside a subnormal operand; roundings of subnormal sums
+    bound = total * (4 * 2.0 ** -23 + (K // 64 + 2) * 2.0 ** -24 + 2.0 ** -25) + ends * 2.0 ** -151 + K * 2.0 ** -149
+    out, st = torch.empty(M, N, device=DEV), o.new_status(DEV)
+    o.linear(a.to(DEV), w.to(DEV), out, status=st)
+    o.read_status(st)
+    assert ((out.cpu().double() - ref).abs() <= bound).all()
+
+
 def test_sgemm_split_infinities_and_nan():
     o = ops()
     g = torch.Generator().manual_seed(4)
