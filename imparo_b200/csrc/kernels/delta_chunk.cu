@@ -440,7 +440,22 @@ delta_out_kernel(const Rows p, const float* __restrict__ scratch, float* __restr
         }
     };
     terms(acc, 0, dim);
-    terms(inner, dim, dim + (rq & ~15) + 16);               // rows of u up to the warp's last row
+    // rows of u before the thread's first, then its own, each row with the ones up to itself: a term beyond a row is left out and
+    // not multiplied by zero, so that a row that is not finite reaches no earlier one
+    terms(inner, dim, dim + rq);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const float4 a = *reinterpret_cast<const float4*>(left + (dim + rq + u) * C + rq), a1 = *reinterpret_cast<const float4*>(left + (dim + rq + u) * C + rq + 4);
+        const float4 b = *reinterpret_cast<const float4*>(right + (dim + rq + u) * 64 + vq);
+        const float2 b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
+        const float av[8] = {a.x, a.y, a.z, a.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int i = u; i < 8; ++i) {
+            const float2 a2 = make_float2(av[i], av[i]);
+            inner[i][0] = __ffma2_rn(a2, b0, inner[i][0]);
+            inner[i][1] = __ffma2_rn(a2, b1, inner[i][1]);
+        }
+    }
     if (v0 + vq >= vdim) return;
 #pragma unroll
     for (int i = 0; i < 8; ++i)

@@ -426,6 +426,43 @@ def test_delta_rule_in_chunks(H, G, D, V, lens):
     assert torch.equal(s[[1, 4]], state0[[1, 4]].double())
 
 
+# (head size 64 and 68: both builds; rows in the middle of a thread's eight and at the end of a chunk)
+@pytest.mark.parametrize("H,G,D,V", [(2, 1, 64, 128), (1, 1, 68, 16)])
+@pytest.mark.parametrize("what", ["v", "k", "q", "g"])
+def test_delta_rule_in_chunks_keeps_what_is_not_finite_where_it_is(H, G, D, V, what):
+    """A row that is not finite changes no earlier row, no other request and (values) no other column, and the outputs that are not
+    finite are those of the row walk."""
+    import torch
+    from imparo_b200.kernels import ops
+    g0 = torch.Generator().manual_seed(D + V)
+    lens = [150, 70]
+    T, rnd = sum(lens), lambda *s: torch.randn(*s, generator=g0)
+    base = {"q": torch.nn.functional.normalize(rnd(T, G, D), dim=-1), "k": torch.nn.functional.normalize(rnd(T, G, D), dim=-1),
+            "v": rnd(T, H, V), "g": torch.exp(-torch.exp(rnd(T, H, D) - 3))}
+    beta, state0 = torch.sigmoid(rnd(T, H)), rnd(2, H, D, V)
+    starts, slots = _dev(np.array([0, 150, 220], dtype=np.int32)), _dev(np.array([0, 1], dtype=np.int32))
+
+    def run(x, chunks):
+        qkv = torch.cat([x["q"].reshape(T, -1), x["k"].reshape(T, -1), x["v"].reshape(T, -1)], dim=1).contiguous().cuda()
+        state, out, status = state0.cuda(), torch.empty(T, H * V, device="cuda"), ops.new_status("cuda")
+        scratch = torch.zeros((T // 64 + 2) * ops.delta_chunk_floats(H, D, V), device="cuda") if chunks else None
+        ops.delta_scan(qkv, 0, G * D, 2 * G * D, x["g"].reshape(T, -1).contiguous().cuda(), beta.cuda(), state, starts, slots, 2, out, H, G, D, V,
+                       status, scratch=scratch)
+        ops.read_status(status)
+        return out.cpu().reshape(T, H, V), state.cpu()
+    clean, clean_state = run(base, True)
+    for row, value in ((37, float("inf")), (63, float("nan")), (72, float("-inf")), (211, float("nan"))):
+        x = dict(base)
+        x[what] = base[what].clone()
+        x[what][row, 0, 3] = value
+        (out, state), (walk, walk_state) = run(x, True), run(x, False)
+        assert not torch.isfinite(out).all()
+        assert torch.equal(torch.isfinite(out), torch.isfinite(walk)) and torch.equal(torch.isfinite(state), torch.isfinite(walk_state))
+        untouched = torch.isfinite(walk)
+        assert untouched[:row].all() and torch.equal(out[untouched], clean[untouched])
+        assert torch.equal(state[torch.isfinite(walk_state)], clean_state[torch.isfinite(walk_state)])
+
+
 def test_delta_rule_in_chunks_refuses_a_bad_slot_and_other_sizes():
     import torch
     from imparo_b200.kernels import ops
