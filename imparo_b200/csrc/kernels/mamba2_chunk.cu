@@ -49,14 +49,16 @@ __device__ __forceinline__ void cp16(float* dst, const float* src) {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// acc[8][4] += left[k][l0 ..] x right[k][r0 ..] over k in [from, to): three 16-byte reads of shared memory per 32 operations.
+// acc[8][4] += left[k][l0 ..] x right[k][r0 ..] over k in [0, to): three 16-byte reads of shared memory per 32 operations.
 // Every 32 terms are summed by themselves: a third less rounding than one chain of 64 (3% more operations).
-template <int LD>
-__device__ __forceinline__ void product(float2 (&acc)[8][2], const float* left, int l0, const float* right, int r0, int from, int to) {
+// CAUSAL (to = l0 + 8): row l0 + i has the terms up to its own.  Those beyond are left out and not multiplied by zero, so that a
+// row that is not finite reaches no earlier one.
+template <int LD, bool CAUSAL = false>
+__device__ __forceinline__ void product(float2 (&acc)[8][2], const float* left, int l0, const float* right, int r0, int to) {
 #pragma unroll 1
-    for (int k0 = from; k0 < to; k0 += 32) {
+    for (int k0 = 0; k0 < to; k0 += 32) {
         float2 part[8][2] = {};
-        const int end = min(k0 + 32, to);
+        const int end = min(k0 + 32, CAUSAL ? l0 : to);
 #pragma unroll 4
         for (int k = k0; k < end; ++k) {
             const float4 a = *reinterpret_cast<const float4*>(left + k * LD + l0), b = *reinterpret_cast<const float4*>(left + k * LD + l0 + 4);
@@ -68,6 +70,21 @@ __device__ __forceinline__ void product(float2 (&acc)[8][2], const float* left, 
                 const float2 a2 = make_float2(av[i], av[i]);
                 part[i][0] = __ffma2_rn(a2, r01, part[i][0]);
                 part[i][1] = __ffma2_rn(a2, r23, part[i][1]);
+            }
+        }
+        if (CAUSAL && k0 + 32 > l0) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float4 a = *reinterpret_cast<const float4*>(left + (l0 + u) * LD + l0), b = *reinterpret_cast<const float4*>(left + (l0 + u) * LD + l0 + 4);
+                const float4 r = *reinterpret_cast<const float4*>(right + (l0 + u) * VB + r0);
+                const float2 r01 = make_float2(r.x, r.y), r23 = make_float2(r.z, r.w);
+                const float av[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int i = u; i < 8; ++i) {
+                    const float2 a2 = make_float2(av[i], av[i]);
+                    part[i][0] = __ffma2_rn(a2, r01, part[i][0]);
+                    part[i][1] = __ffma2_rn(a2, r23, part[i][1]);
+                }
             }
         }
 #pragma unroll
@@ -153,7 +170,7 @@ state_kernel(const Rows p, float* __restrict__ chunk_state, float* __restrict__ 
 #pragma unroll
         for (int nb = 0; nb < NM; nb += 64) {
             float2 acc[8][2] = {};
-            product<NM>(acc, bs, nb + nq, x, vq, 0, n);
+            product<NM>(acc, bs, nb + nq, x, vq, n);
             if (vq < cols) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -269,7 +286,7 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
     const int lq = (tid >> 4) * 8, rq = (tid & 15) * 4;
     {
         float2 acc[8][2] = {};                             // rows j, columns i
-        product<C>(acc, bt, lq, ct, rq, 0, NM);
+        product<C>(acc, bt, lq, ct, rq, NM);
         __syncthreads();                                   // bt is written over from here on
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -297,8 +314,8 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
         const float* s = right;
         const float* x = s + NM * VB;
         float2 acc[8][2] = {}, inside[8][2] = {};
-        product<C>(acc, ct, lq, s, rq, 0, NM);
-        product<C>(inside, bt, lq, x, rq, 0, (lq & ~15) + 16);          // rows up to the warp's last one
+        product<C>(acc, ct, lq, s, rq, NM);
+        product<C, true>(inside, bt, lq, x, rq, lq + 8);
         const float skip = p.D[h0 + hh];
         float c = 1.f;
         for (int r = 0; r < lq; ++r) c *= es[hh * C + r];

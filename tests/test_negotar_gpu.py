@@ -473,6 +473,45 @@ def test_state_space_products(heads, groups, N, vdim, lens):
     assert torch.equal(s[[1, 4]], state0[[1, 4]].double())
 
 
+# (both builds of the state size; rows in the middle of a thread's eight and at the end of a chunk)
+@pytest.mark.parametrize("heads,groups,N,vdim", [(4, 2, 64, 20), (2, 1, 68, 64)])
+@pytest.mark.parametrize("what", ["x", "B", "C", "dt"])
+def test_state_space_products_keep_what_is_not_finite_where_it_is(heads, groups, N, vdim, what):
+    """A row that is not finite changes no earlier row, no other request, group or (values) column, and the outputs that are not
+    finite are those of the row walk."""
+    import torch
+    from imparo_b200.kernels import ops
+    g = torch.Generator().manual_seed(N + vdim)
+    lens, inner = [150, 70], heads * vdim
+    T, rnd = sum(lens), lambda *s: torch.randn(*s, generator=g)
+    xbc0, dt0 = rnd(T, inner + 2 * groups * N), torch.nn.functional.softplus(rnd(T, heads) - 2)
+    A_log, D, state0 = rnd(heads).cuda(), rnd(heads).cuda(), rnd(2, heads, N, vdim)
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    most = T // 64 + 2
+
+    def run(xbc, dt, chunk):
+        scratch = (torch.empty(3 * most + 3, dtype=torch.int32, device="cuda"), torch.zeros(most * heads * N * vdim, device="cuda"),
+                   torch.zeros(most * heads, device="cuda")) if chunk else None
+        state, y, status = state0.cuda(), torch.empty(T, inner, device="cuda"), ops.new_status("cuda")
+        ops.mamba2_scan(xbc.cuda(), dt.cuda(), A_log, D, state, dev([0, 150, 220]), dev([0, 1]), 2, y, heads, vdim, N, groups, status, chunk=chunk,
+                        scratch=scratch)
+        ops.read_status(status)
+        return y.cpu(), state.cpu()
+    clean, clean_state = run(xbc0, dt0, 64)
+    for row, value in ((37, float("inf")), (63, float("nan")), (72, float("-inf")), (211, float("nan"))):
+        xbc, dt = xbc0.clone(), dt0.clone()
+        if what == "dt":
+            dt[row, 1] = float("nan")
+        else:
+            xbc[row, {"x": 3, "B": inner + 2, "C": inner + groups * N + 2}[what]] = value
+        (y, state), (walk, walk_state) = run(xbc, dt, 64), run(xbc, dt, 0)
+        assert not torch.isfinite(y).all()
+        assert torch.equal(torch.isfinite(y), torch.isfinite(walk)) and torch.equal(torch.isfinite(state), torch.isfinite(walk_state))
+        untouched = torch.isfinite(walk)
+        assert untouched[:row].all() and torch.equal(y[untouched], clean[untouched])
+        assert torch.equal(state[torch.isfinite(walk_state)], clean_state[torch.isfinite(walk_state)])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width,ff,experts,top,rows", [(64, 40, 6, 2, 5), (96, 64, 5, 1, 90), (100, 30, 3, 3, 33), (128, 64, 8, 2, 300),
                                                        (72, 50, 7, 2, 1), (256, 200, 5, 3, 700), (64, 328, 40, 4, 130)])
