@@ -135,7 +135,7 @@ state_kernel(const Rows p, float* __restrict__ chunk_state, float* __restrict__ 
     for (int e = tid; e < HG * C; e += THREADS) {
         const int hh = e / C, r = e % C;
         const float step = r < n ? p.dt[(size_t)(first + r) * p.heads + h0 + hh] : 0.f;
-        es[e] = -expf(p.A_log[h0 + hh]) * step;
+        es[e] = r < n ? -expf(p.A_log[h0 + hh]) * step : 0.f;           // (not -infinity times zero beyond the rows)
         ws[e] = step;
     }
     __syncthreads();
@@ -280,7 +280,7 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
         const int hh = e / C, r = e % C;
         const float step = r < n ? p.dt[(size_t)(first + r) * p.heads + h0 + hh] : 0.f;
         ds[e] = step;
-        es[e] = expf(-expf(p.A_log[h0 + hh]) * step);
+        es[e] = r < n ? expf(-expf(p.A_log[h0 + hh]) * step) : 1.f;
     }
     __syncthreads();
     const int lq = (tid >> 4) * 8, rq = (tid & 15) * 4;

@@ -512,6 +512,27 @@ def test_state_space_products_keep_what_is_not_finite_where_it_is(heads, groups,
         assert torch.equal(state[torch.isfinite(walk_state)], clean_state[torch.isfinite(walk_state)])
 
 
+def test_state_space_products_of_a_decay_rate_beyond_the_range():
+    """exp(A_log) overflows: a state keeps its last row only; the rows that fill up a request's last chunk add nothing."""
+    import torch
+    from imparo_b200.kernels import ops
+    heads, N, vdim, T = 2, 8, 8, 70
+    g = torch.Generator().manual_seed(3)
+    xbc, dt = torch.randn(T, heads * vdim + 2 * N, generator=g).cuda(), torch.rand(T, heads, generator=g).cuda() + 0.1
+    A_log, D = torch.tensor([100.0, 0.5], device="cuda"), torch.ones(heads, device="cuda")
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    got = []
+    for chunk in (0, 64):
+        state, y, status = torch.ones(1, heads, N, vdim, device="cuda"), torch.empty(T, heads * vdim, device="cuda"), ops.new_status("cuda")
+        scratch = (torch.empty(8, dtype=torch.int32, device="cuda"), torch.empty(2 * heads * N * vdim, device="cuda"), torch.empty(2 * heads, device="cuda"))
+        ops.mamba2_scan(xbc, dt, A_log, D, state, dev([0, T]), dev([0]), 1, y, heads, vdim, N, 1, status, chunk=chunk, scratch=scratch if chunk else None)
+        ops.read_status(status)
+        got.append((y, state))
+    assert torch.isfinite(got[0][0]).all() and torch.isfinite(got[0][1]).all()
+    for a, b in zip(*got):
+        assert float((a - b).abs().max()) <= 1e-5 * float(a.abs().max())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width,ff,experts,top,rows", [(64, 40, 6, 2, 5), (96, 64, 5, 1, 90), (100, 30, 3, 3, 33), (128, 64, 8, 2, 300),
                                                        (72, 50, 7, 2, 1), (256, 200, 5, 3, 700), (64, 328, 40, 4, 130)])
