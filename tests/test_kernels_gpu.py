@@ -805,6 +805,38 @@ def test_attention_prefill_f32(nh, nkv, hd, page, window):
             t += 1
 
 
+# (both builds of the head size; a key in the middle of a tile, at a tile's end, in the first tile of a window)
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [None, 50, 9])
+def test_attention_prefill_f32_keeps_what_is_not_finite_where_it_is(hd, window):
+    """A value or key row that is not finite reaches the queries that see it and leaves every other as it is."""
+    o = ops()
+    rng = np.random.default_rng(hd)
+    portions, page, nh, nkv = [(37, 150), (0, 90)], 16, 2, 1
+    table, kc, vc, _, _, n_pages = make_paged(rng, [s + n for s, n in portions], page, nkv, hd, torch.float32)
+    T = sum(n for _, n in portions)
+    q = torch.from_numpy(rng.standard_normal((T, nh * hd)).astype(np.float32)).to(DEV)
+    dev = lambda a: torch.from_numpy(np.asarray(a, dtype=np.int32)).to(DEV)
+
+    def run(k, v):
+        out, status = torch.empty(T, nh * hd, device=DEV), o.new_status(DEV)
+        assert o.attention_prefill_f32(q, k.to(DEV), v.to(DEV), dev([0, 150, 240]), dev([37, 0]), 2, dev(table), page, n_pages, window, 1 / math.sqrt(hd),
+                                       out, nh, nkv, hd, status)
+        o.read_status(status)
+        return out.cpu()
+    clean = run(kc, vc)
+    for pos in (36, 63, 64, 100, 141):                                  # of the first portion's request
+        for which, value in (("k", float("nan")), ("v", float("inf")), ("v", float("nan"))):
+            k, v = kc.clone(), vc.clone()
+            (k if which == "k" else v).view(-1, nkv * hd)[int(table[0][pos // page]) * page + pos % page, 5] = value
+            out = run(k, v)
+            seen = [t for t in range(150) if 37 + t >= pos and (window is None or 37 + t - pos < window)]
+            rest = sorted(set(range(T)) - set(seen))
+            assert torch.equal(out[rest], clean[rest])
+            if seen:
+                assert not torch.isfinite(out[seen]).all(dim=1).any()
+
+
 def test_attention_prefill_f32_refuses_bad_pages_and_other_shapes():
     o = ops()
     z, status = torch.zeros(70, 64, device=DEV), o.new_status(DEV)
