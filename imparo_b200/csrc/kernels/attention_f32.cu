@@ -144,7 +144,7 @@ attn_prefill_f32_kernel(const Params p) {
             float sum = 0.f;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                pr[i][c] = seen[c] ? expf(pr[i][c] - m_new) : 0.f;
+                pr[i][c] = seen[c] && m_new != -INFINITY ? expf(pr[i][c] - m_new) : 0.f;
                 sum += pr[i][c];
             }
             l[i] = l[i] * alpha[i] + sum;

@@ -837,6 +837,26 @@ def test_attention_prefill_f32_keeps_what_is_not_finite_where_it_is(hd, window):
                 assert not torch.isfinite(out[seen]).all(dim=1).any()
 
 
+def test_attention_prefill_f32_scores_of_minus_infinity():
+    """Keys whose scores overflow to minus infinity weigh nothing, a whole first tile of them included; a query all of whose keys are
+    such gets zeros, as from the split-key kernel."""
+    o = ops()
+    T, hd, n_low = 140, 64, 70
+    v = torch.randn(T, hd, generator=torch.Generator().manual_seed(1)).to(DEV)
+    k = torch.zeros(192, hd, device=DEV)
+    k[:n_low] = -1e20
+    q, out, status = torch.full((T, hd), 1e20, device=DEV), torch.empty(T, hd, device=DEV), o.new_status(DEV)
+    vc = torch.zeros(192, hd, device=DEV)
+    vc[:T] = v
+    one = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    assert o.attention_prefill_f32(q, k, vc, one(0, T), one(0), 1, one(0, 1, 2).view(1, 3), 64, 3, None, 0.125, out, 1, 1, hd, status)
+    o.read_status(status)
+    want = torch.zeros(T, hd, dtype=torch.float64)
+    for t in range(n_low, T):
+        want[t] = v[n_low:t + 1].double().cpu().mean(0)
+    assert float((out.cpu().double() - want).abs().max()) <= 1e-6
+
+
 def test_attention_prefill_f32_refuses_bad_pages_and_other_shapes():
     o = ops()
     z, status = torch.zeros(70, 64, device=DEV), o.new_status(DEV)
