@@ -150,7 +150,7 @@ state_kernel(const Rows p, float* __restrict__ chunk_state, float* __restrict__ 
     for (int e = tid; e < HG * C; e += THREADS) {
         const int hh = e / C, r = e % C;
         float w = ws[e];
-        for (int i = C - 1; i > r; --i) w *= es[hh * C + i];          // (rows beyond the chunk's decay by one)
+        for (int i = n - 1; i > r; --i) w *= es[hh * C + i];
         ws[e] = w;
     }
     const int nq = (tid >> 4) * 8, vq = (tid & 15) * 4;
@@ -284,9 +284,10 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
     }
     __syncthreads();
     const int lq = (tid >> 4) * 8, rq = (tid & 15) * 4;
+    const bool busy = (lq & ~15) < n;                      // the warp's 16 rows: a short chunk's products are its own warps' only
     {
         float2 acc[8][2] = {};                             // rows j, columns i
-        product<C>(acc, bt, lq, ct, rq, NM);
+        if (busy) product<C>(acc, bt, lq, ct, rq, NM);
         __syncthreads();                                   // bt is written over from here on
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -296,9 +297,9 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
         fetch(hh);
         cp_commit();
         __syncthreads();                                   // gt is whole
-        {
+        const int i = tid & (C - 1), j_lo = (tid >> 6) * 32, j_hi = j_lo + 31;
+        if (i < n) {
             // row i, columns j of one half, from the diagonal down: the decay grows by one row at a time
-            const int i = tid & (C - 1), j_lo = (tid >> 6) * 32, j_hi = j_lo + 31;
             const float* e = es + hh * C;
             const float* d = ds + hh * C;
             float w = 1.f;
@@ -314,8 +315,10 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
         const float* s = right;
         const float* x = s + NM * VB;
         float2 acc[8][2] = {}, inside[8][2] = {};
-        product<C>(acc, ct, lq, s, rq, NM);
-        product<C, true>(inside, bt, lq, x, rq, lq + 8);
+        if (busy) {
+            product<C>(acc, ct, lq, s, rq, NM);
+            product<C, true>(inside, bt, lq, x, rq, lq + 8);
+        }
         const float skip = p.D[h0 + hh];
         float c = 1.f;
         for (int r = 0; r < lq; ++r) c *= es[hh * C + r];

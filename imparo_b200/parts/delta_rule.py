@@ -28,10 +28,6 @@ class GatedDeltaRule(Part):
 
     forward(..., accumulate=False) overwrites `residual` (then any float32 [tokens, hidden] buffer)."""
     adds_with_linear = True
-    # Portions from this many tokens on (rounded up to a power of two: 257 and more) run in chunks of 64 rows side by side.  Key
-    # size 64, value size 128, 8 heads, walk against chunks: 300 rows 64 / 65 us, 2,048 rows 421 / 142 us; 16 heads of key size
-    # 128: 2,048 rows 677 / 380 us.
-    CHUNK_FROM = 512
     CHUNK = 64
 
     NAMES = {"q": "q", "k": "k", "v": "v", "q_conv": "q.conv", "k_conv": "k.conv", "v_conv": "v.conv", "b": "b", "A_log": "A_log",
@@ -94,6 +90,16 @@ class GatedDeltaRule(Part):
     def cache_specs(self):
         return (SlotState((self.heads, self.dim, self.vdim)), SlotState((max(self.taps - 1, 1), self.channels)))
 
+    def _in_chunks(self, longest: int, tokens: int, portions: int) -> bool:
+        """Whether a step's portions (tokens rows of that many requests) run in chunks of 64 rows side by side and not row by row
+        (the longest one's length comes rounded up to a power of two).  The walk takes as long as the longest portion, the chunks
+        a whole chunk for every short portion, which many wide heads pay in full.  Walk against chunks in us (B200): key size 64,
+        value size 128, 8 heads: 257 rows 56 / 64, 300 rows 64 / 65, 2,048 rows 421 / 142; 300 rows beside 8 portions of 16: 98 /
+        79, beside 31 portions of 8: 94 / 133.  16 heads of key size 128: 300 rows 105 / 82, 2,048 rows 677 / 380; 300 rows beside 8
+        portions of 16: 167 / 194, 512 beside 8 of 64: 323 / 226; 32 such heads: 257 rows 136 / 153, 300 rows 157 / 154."""
+        least = 32 if self.heads * self.dim <= 512 else 64
+        return longest >= 512 and tokens >= max(300, least * portions)
+
     def forward(self, x, batch, caches, residual, accumulate=True):
         st, conv = caches
         rt, T = self.rt, x.shape[0]
@@ -115,11 +121,18 @@ class GatedDeltaRule(Part):
         ops.delta_prepare(qkv, 0, self.qk, proj, self.channels, a, self.A_log, self.dt_bias, beta, H, self.kv_heads, D,
                           self.unit_eps, float(D) ** -0.5)
         o = ws.get("delta_o", (T, self.vv), torch.float32, first="tokens")
-        scratch = None
-        if batch.max_tokens_per_item >= self.CHUNK_FROM and ops.delta_chunks_take(qkv, 0, self.qk, H, D, V):
-            scratch = ws.get("delta_chunks", ((T // self.CHUNK + batch.n_items) * ops.delta_chunk_floats(H, D, V),), torch.float32)
-        ops.delta_scan(qkv, 0, self.qk, 2 * self.qk, a, beta, st.state, batch.item_row_start, batch.item_slot, batch.n_items, o,
-                       H, self.kv_heads, D, V, rt.status, scratch=scratch)
+        def scan(first, n, scratch=None):                      # requests [first, first + n)
+            ops.delta_scan(qkv, 0, self.qk, 2 * self.qk, a, beta, st.state, batch.item_row_start[first:], batch.item_slot[first:], n, o,
+                           H, self.kv_heads, D, V, rt.status, scratch=scratch)
+        n1 = getattr(batch, "n_single", 0)                     # decode rows come first when the step also holds portions
+        portions = batch.n_items - n1
+        if self._in_chunks(batch.max_tokens_per_item, T - n1, portions) and ops.delta_chunks_take(qkv, 0, self.qk, H, D, V):
+            if n1:
+                scan(0, n1)
+            per = ops.delta_chunk_floats(H, D, V)
+            scan(n1, portions, ws.get("delta_chunks", ((T // self.CHUNK + portions) * per,), torch.float32))
+        else:
+            scan(0, batch.n_items)
         y = ws.get("delta_y", (T, self.vv), rt.act_dtype, first="tokens")
         ops.head_norm_gate(o, self.w_norm, self.eps, gate, y, H, V)
         ops.linear(y, self.w_o, residual, accumulate=accumulate, status=rt.status)

@@ -23,7 +23,6 @@ class Mamba2Mixer(Part):
 
     forward(..., accumulate=False) overwrites `residual` (then any float32 [tokens, hidden] buffer)."""
     adds_with_linear = True
-    CHUNK_FROM = 128          # portions from this many tokens on (rounded up to a power of two) run in chunks
     CHUNK = 64
 
     NAMES = {"in": "in", "conv": "conv", "conv_bias": "conv.b", "dt_bias": "dt_bias", "A_log": "A_log", "D": "D",
@@ -74,6 +73,14 @@ class Mamba2Mixer(Part):
     def cache_specs(self):
         return (SlotState((self.heads, self.n_state, self.vdim)), SlotState((max(self.taps - 1, 1), self.channels)))
 
+    @staticmethod
+    def _in_chunks(longest: int, tokens: int, portions: int) -> bool:
+        """Whether a step's portions (tokens rows of that many requests) run in chunks of 64 rows side by side and not row by row
+        (the longest one's length comes rounded up to a power of two).  The walk takes as long as the longest portion, the chunks
+        a whole chunk for every short portion.  Walk against chunks in us (B200, 32 heads of 64, state size 64): 66 rows 22 / 26,
+        100 rows 32 / 26, 512 rows 154 / 32; 100 rows beside 31 portions of 8: 44 / 77; 400 beside 16 of 16: 132 / 68."""
+        return longest >= 128 and (longest > 256 or tokens >= 16 * portions)
+
     def forward(self, x, batch, caches, residual, accumulate=True):
         ssm, conv = caches
         rt, T = self.rt, x.shape[0]
@@ -88,16 +95,22 @@ class Mamba2Mixer(Part):
                         self.dt_bias, conv.state, batch.item_row_start, batch.item_of_token, batch.item_slot, batch.n_items,
                         xbc, dt, rt.status)
         y = ws.get("mamba_y", (T, inner), torch.float32, first="tokens")
-        chunk, scratch = 0, None
-        if batch.max_tokens_per_item >= self.CHUNK_FROM:
+        def scan(first, n, chunk=0, scratch=None):             # requests [first, first + n)
+            ops.mamba2_scan(xbc, dt, self.A_log, self.D, ssm.state, batch.item_row_start[first:], batch.item_slot[first:], n, y,
+                            self.heads, self.vdim, self.n_state, self.groups, rt.status, chunk=chunk, scratch=scratch)
+        n1 = getattr(batch, "n_single", 0)                     # decode rows come first when the step also holds portions
+        portions = batch.n_items - n1
+        if self._in_chunks(batch.max_tokens_per_item, T - n1, portions):
             # long portions: chunks of rows side by side; the chunk length is fixed, so the cut depends on the rows alone
-            chunk = self.CHUNK
-            most = T // chunk + batch.n_items
-            scratch = (ws.get("mamba_chunk_i", (3 * most + batch.n_items + 1,), torch.int32),
-                       ws.get("mamba_chunk_state", (most * self.heads * self.n_state * self.vdim,), torch.float32),
-                       ws.get("mamba_chunk_decay", (most * self.heads,), torch.float32))
-        ops.mamba2_scan(xbc, dt, self.A_log, self.D, ssm.state, batch.item_row_start, batch.item_slot, batch.n_items, y,
-                        self.heads, self.vdim, self.n_state, self.groups, rt.status, chunk=chunk, scratch=scratch)
+            if n1:
+                scan(0, n1)
+            per = self.heads * self.n_state * self.vdim
+            most = T // self.CHUNK + portions
+            scan(n1, portions, self.CHUNK, (ws.get("mamba_chunk_i", (3 * most + portions + 1,), torch.int32),
+                                            ws.get("mamba_chunk_state", (most * per,), torch.float32),
+                                            ws.get("mamba_chunk_decay", (most * self.heads,), torch.float32)))
+        else:
+            scan(0, batch.n_items)
         g = ws.get("mamba_gated", (T, inner), rt.act_dtype, first="tokens")
         ops.gate_group_rmsnorm(y, proj[:, :inner], self.w_norm, self.eps, self.norm_groups, g)
         ops.linear(g, self.w_o, residual, accumulate=accumulate, status=rt.status)

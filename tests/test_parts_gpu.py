@@ -270,3 +270,78 @@ def test_two_engines_in_one_process_do_not_share_launch_state():
         eng.check_device_status()
         eng.end_request(1)
         assert eng.step_fn.graph_replays >= 1
+
+
+RECURRENCES = {"gated_delta_rule": ({"hidden": 64, "heads": 4, "kv_heads": 2, "dim": 64, "vdim": 32, "conv": 3, "decay_rank": 8, "gate_rank": 8, "eps": 1e-6},
+                                    "delta_scan"),
+               "mamba2": ({"hidden": 64, "heads": 4, "vdim": 32, "state": 16, "groups": 2, "conv": 4, "norm_groups": 2, "eps": 1e-6}, "mamba2_scan")}
+
+
+def _steps_of_a_recurrence(kind, steps, monkeypatch, rows=40):
+    """Each step: {request: tokens}.  -> ([step's output rows by request], [(requests of a scan, in chunks?) per step], the runtime)"""
+    from imparo_b200.engine.step import StepItem
+    from imparo_b200.kernels import ops
+    from imparo_b200.parts.spec import PartSpec
+    params, scan = RECURRENCES[kind]
+    rt = runtime("float32")
+    rt.workspace.expect(tokens=2048, rows=rows)
+    part, _ = build("mixer", PartSpec(kind, dict(params)), "L.", rt)
+    cache, fn = batch_for(part, rt, None, slots=rows)
+    calls, real = [], getattr(ops, scan)
+
+    def spy(*args, **kw):
+        calls[-1].append((args[7 if scan == "mamba2_scan" else 9], kw.get("scratch") is not None))
+        real(*args, **kw)
+    monkeypatch.setattr(ops, scan, spy)
+    outs, gen = [], torch.Generator().manual_seed(1)
+    for step in steps:
+        items, x = [], {}
+        for r, n in step.items():
+            if not cache.has(r):
+                cache.add(r)
+            cache.reserve(r, n)
+            items.append(StepItem(r, [0] * n))
+            x[r] = torch.randn(n, params["hidden"], generator=gen)
+        batch = fn.build_batch(items, singles_first=True)
+        order = sorted(step, key=lambda r: step[r] != 1) if 1 in step.values() else list(step)
+        xin = torch.cat([x[r] for r in order]).to(DEV)
+        out = torch.zeros(xin.shape[0], params["hidden"], device=DEV)
+        calls.append([])
+        part.forward(xin, batch, cache.views(0), out)
+        outs.append(dict(zip(order, out.split([step[r] for r in order]))))
+        for r, n in step.items():
+            cache.commit(r, n)
+    ops.read_status(rt.status)
+    return outs, calls, rt
+
+
+def _part_class(kind):
+    from imparo_b200.parts.delta_rule import GatedDeltaRule
+    from imparo_b200.parts.mamba2 import Mamba2Mixer
+    return GatedDeltaRule if kind == "gated_delta_rule" else Mamba2Mixer
+
+
+@pytest.mark.parametrize("kind", sorted(RECURRENCES))
+def test_decode_rows_beside_a_long_portion_run_row_by_row(kind, monkeypatch):
+    """Rows of one token are walked, to the bit as in a step of their own kind; the portions beside them run in chunks."""
+    steps = [{1: 9, 2: 30, 3: 5}, {1: 1, 2: 1, 9: 600, 3: 1}, {1: 1, 9: 1}]
+    outs, calls, _ = _steps_of_a_recurrence(kind, steps, monkeypatch)
+    assert calls == [[(3, False)], [(3, False), (1, True)], [(2, False)]]
+    monkeypatch.undo()
+    monkeypatch.setattr(_part_class(kind), "_in_chunks", staticmethod(lambda *a: False))
+    walked, calls, _ = _steps_of_a_recurrence(kind, steps, monkeypatch)
+    assert calls[1] == [(4, False)]
+    for r in (1, 2, 3):
+        assert torch.equal(outs[1][r], walked[1][r])
+    for step in (1, 2):
+        scale = float(walked[step][9].abs().max())
+        assert float((outs[step][9] - walked[step][9]).abs().max()) <= 1e-5 * scale
+
+
+@pytest.mark.parametrize("kind,steps,want", [
+    ("gated_delta_rule", [{1: 299}, {2: 300}, {3: 256}, {**{4: 300}, **{10 + i: 2 for i in range(30)}}, {**{5: 600}, **{50 + i: 2 for i in range(8)}}],
+     [[(1, False)], [(1, True)], [(1, False)], [(31, False)], [(9, True)]]),
+    ("mamba2", [{1: 64}, {2: 65}, {**{4: 200}, **{10 + i: 2 for i in range(30)}}, {**{5: 300}, **{50 + i: 2 for i in range(8)}}],
+     [[(1, False)], [(1, True)], [(31, False)], [(9, True)]])])
+def test_few_tokens_per_portion_run_row_by_row(kind, steps, want, monkeypatch):
+    assert _steps_of_a_recurrence(kind, steps, monkeypatch, rows=60)[1] == want
