@@ -130,7 +130,10 @@ class GatedDeltaRule(Part):
             if n1:
                 scan(0, n1)
             per = ops.delta_chunk_floats(H, D, V)
-            scan(n1, portions, ws.get("delta_chunks", ((T // self.CHUNK + portions) * per,), torch.float32))
+            most = ws.most["tokens"]
+            scratch = ws.get("delta_chunks", ((T // self.CHUNK + portions) * per,), torch.float32,
+                             reserve=(most // self.CHUNK + min(ws.most["rows"], most // 32)) * per)
+            scan(n1, portions, scratch)
         else:
             scan(0, batch.n_items)
         y = ws.get("delta_y", (T, self.vv), rt.act_dtype, first="tokens")

@@ -106,9 +106,11 @@ class Mamba2Mixer(Part):
                 scan(0, n1)
             per = self.heads * self.n_state * self.vdim
             most = T // self.CHUNK + portions
-            scan(n1, portions, self.CHUNK, (ws.get("mamba_chunk_i", (3 * most + portions + 1,), torch.int32),
-                                            ws.get("mamba_chunk_state", (most * per,), torch.float32),
-                                            ws.get("mamba_chunk_decay", (most * self.heads,), torch.float32)))
+            room = ws.most["tokens"] // self.CHUNK + ws.most["rows"]
+            scan(n1, portions, self.CHUNK,
+                 (ws.get("mamba_chunk_i", (3 * most + portions + 1,), torch.int32, reserve=4 * room + 1),
+                  ws.get("mamba_chunk_state", (most * per,), torch.float32, reserve=room * per),
+                  ws.get("mamba_chunk_decay", (most * self.heads,), torch.float32, reserve=room * self.heads)))
         else:
             scan(0, batch.n_items)
         g = ws.get("mamba_gated", (T, inner), rt.act_dtype, first="tokens")

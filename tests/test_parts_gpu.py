@@ -345,3 +345,10 @@ def test_decode_rows_beside_a_long_portion_run_row_by_row(kind, monkeypatch):
      [[(1, False)], [(1, True)], [(31, False)], [(9, True)]])])
 def test_few_tokens_per_portion_run_row_by_row(kind, steps, want, monkeypatch):
     assert _steps_of_a_recurrence(kind, steps, monkeypatch, rows=60)[1] == want
+
+
+@pytest.mark.parametrize("kind", sorted(RECURRENCES))
+def test_chunk_scratch_stays_where_it_is(kind, monkeypatch):
+    """Made once for the largest step: longer portions neither move it nor make recorded steps stale."""
+    _, calls, rt = _steps_of_a_recurrence(kind, [{1: 320}, {1: 640}, {2: 1000, 3: 1000}], monkeypatch)
+    assert all(in_chunks for step in calls for _, in_chunks in step) and rt.workspace.generation == 0
