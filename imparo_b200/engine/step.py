@@ -35,7 +35,7 @@ class StepBatch:
     """The step's batch on the device.  All index arrays are int32."""
     __slots__ = ("n_tokens", "n_items", "token_ids", "positions", "item_of_token", "item_row_start",
                  "item_slot", "item_start_pos", "tables", "want_rows", "n_want", "max_tokens_per_item",
-                 "max_context", "decode_only", "host", "token_src", "n_single", "fresh_slots", "notes")
+                 "max_context", "decode_only", "host", "token_src", "n_single", "fresh_slots", "notes", "portions_from_start")
 
 
 def _round_up(x: int, m: int) -> int:
@@ -247,8 +247,13 @@ class StepFunction:
         b.max_tokens_per_item = 1 if longest <= 1 else 1 << (longest - 1).bit_length()
         b.max_context = int(max(start_pos[i] + (row_start[i + 1] - row_start[i]) for i in range(R)))
         b.decode_only = b.max_tokens_per_item == 1
+        # 32-bit: whether every portion of more than one token starts its request.  The attention's choice of kernel depends on it,
+        # so it is part of the step's shape
+        b.portions_from_start = (self.rt.precision == "float32" and bool(fresh)
+                                 and not start_pos[:R][np.diff(row_start[:R + 1]) > 1].any())
         b.host = {"start_pos": start_pos[:R].copy(), "slots": slot[:R].copy(), "row_start": row_start[:R + 1].copy(),
-                  "key": (T, R, W, tuple(strides), b.max_tokens_per_item, n_single, bool(fresh)), "h2d_bytes": n_ints * 4,
+                  "key": (T, R, W, tuple(strides), b.max_tokens_per_item, n_single,
+                          bool(fresh) + b.portions_from_start), "h2d_bytes": n_ints * 4,
                   "n_want_real": W_real, "padding_rows": pad}
         return b
 

@@ -1166,6 +1166,22 @@ def attention_prefill_f32(q, k_cache, v_cache, item_row_start, item_start_pos, n
     return True
 
 
+def attention_f32_tiles_pay(n_tok: int, n_items: int, nh: int, nkv: int, from_start: bool) -> bool:
+    """Whether 32-bit portions (n_tok rows of n_items requests) go to the tiles (attention_prefill_f32) and not to the split-key
+    kernel.  The tiles walk a request's keys in one CTA per 64 rows and head, at 0.12 us per key (head size 64) however few rows the
+    tile holds, as long as every SM has at most 1.5 CTAs or so; the split-key kernel spreads the keys over the chip and takes
+    (56 + 24 nh / nkv) ps per key, row and kv head.  Where the two meet, both sides in us (B200, 16 heads of 64, 8 kv heads):
+    8,000 keys before the portion: 64 rows 417 split / 964 tiles, 128 rows 816 / 971, 256 rows 1,656 / 1,144; 8 rows at 30,000 keys:
+    259 / 3,771.  Head size 128 shifts both sides alike.  Portions that start at position 0 (from_start) have few keys, and the
+    split-key launch is made for as many as the tables can hold: there the line lies at half the rows (64 rows: 14.2 / 13.7;
+    32 heads, 8 kv heads: 22.1 / 13.8).  Groups of more than 8 heads: the split-key kernel does not take them."""
+    group = nh // nkv
+    if group > 8:
+        return True
+    rounds = max(1.0, nh * (n_tok // 64 + n_items) / 220)
+    return n_tok * nkv * (7 + 3 * group) >= (6500 if from_start else 13000) * rounds
+
+
 # ---- attention with sigmoid weights (csrc/kernels/attention_sigmoid.cu) -----------------------------------------
 def _sigmoid_takes(q, k_cache, v_cache, nh, nkv, hd, vd) -> bool:
     return (q.dtype == torch.bfloat16 and k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and hd % 16 == 0 and vd % 16 == 0

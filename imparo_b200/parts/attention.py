@@ -455,12 +455,17 @@ class AttentionMixer(Part):
                                self.eps, q, kv.k, kv.v, table, kv.page_size, kv.n_pages, nh, nkv, hd, rt.status)
         done = False
         # the prompt kernels: tensor cores for bfloat16, tiles of 32-bit products else
+        n1 = getattr(batch, "n_single", 0)             # decode rows come first when the step also holds portions
+        portions = batch.max_tokens_per_item >= 8
+        beside_rows = 0 < n1 < batch.n_items and nh // self.nkv <= 8
         if rt.act_dtype == torch.float32:
             prefill, beside = ops.attention_prefill_f32, {}
+            lead = n1 if beside_rows else 0
+            portions = portions and ops.attention_f32_tiles_pay(T - lead, batch.n_items - lead, nh, self.nkv,
+                                                                getattr(batch, "portions_from_start", False))
         else:
             prefill, beside = ops.attention_prefill, {"dependents_after_wait": ops.switches().attn_side_by_side}
-        n1 = getattr(batch, "n_single", 0)             # decode rows come first when the step also holds portions
-        if batch.max_tokens_per_item >= 8 and 0 < n1 < batch.n_items and nh // self.nkv <= 8:
+        if portions and beside_rows:
             # Portions beside decode rows: the prompt kernel walks a request's keys tile by tile in one
             # CTA per 128 query rows, which for a single query token is one CTA crawling over the whole
             # context.  So the portions (requests n1 onward) go to the prompt kernel and the decode rows
@@ -476,7 +481,7 @@ class AttentionMixer(Part):
                 ops.paged_attention_split(q[:n1], kv.k, kv.v, batch.positions[:n1], batch.item_of_token[:n1], table,
                                           kv.page_size, kv.n_pages, self.window, self.scale, out[:n1], part_acc, part_ml,
                                           chunk, n_splits, nh, self.nkv, hd, rt.status, fresh=1, overlap_prev=done == 2)
-        elif batch.max_tokens_per_item >= 8:
+        elif portions:
             # prompt portions, tiles of one request each
             done = prefill(q, kv.k, kv.v, batch.item_row_start, batch.item_start_pos, batch.n_items, table, kv.page_size, kv.n_pages,
                            self.window, self.scale, out, nh, self.nkv, hd, rt.status)

@@ -352,3 +352,51 @@ def test_chunk_scratch_stays_where_it_is(kind, monkeypatch):
     """Made once for the largest step: longer portions neither move it nor make recorded steps stale."""
     _, calls, rt = _steps_of_a_recurrence(kind, [{1: 320}, {1: 640}, {2: 1000, 3: 1000}], monkeypatch)
     assert all(in_chunks for step in calls for _, in_chunks in step) and rt.workspace.generation == 0
+
+
+def test_short_portions_over_many_keys_take_the_split_key_kernel(monkeypatch):
+    """32-bit: the tiles walk a request's keys in one CTA per 64 rows, so portions of few rows leave them to the split-key kernel."""
+    from imparo_b200.engine.step import StepItem
+    from imparo_b200.kernels import ops
+    from imparo_b200.parts.spec import PartSpec
+    rt, H = runtime("float32"), 64
+    rt.workspace.expect(tokens=1024, rows=8)
+    part, _ = build("mixer", PartSpec("attention", {"hidden": H, "n_heads": 4, "n_kv_heads": 2, "head_dim": 64, "eps": 1e-6,
+                                                    "position": PartSpec("rope_neox", {"head_dim": 64, "theta": 1e4})}), "L.", rt)
+    took = []
+    for name in ("attention_prefill_f32", "paged_attention_split"):
+        def spy(q, *args, _real=getattr(ops, name), _name=name, **kw):
+            took[-1].append((_name, len(q) if _name == "paged_attention_split" else args[4]))        # rows | requests
+            return _real(q, *args, **kw)
+        monkeypatch.setattr(ops, name, spy)
+    x = torch.randn(1100, H, generator=torch.Generator().manual_seed(2)).to(DEV)
+
+    def run(steps, rule=None):
+        if rule is not None:
+            monkeypatch.setattr(ops, "attention_f32_tiles_pay", rule)
+        cache, fn = batch_for(part, rt, None, page=16, pages=200)
+        outs, at = [], 0
+        del took[:]
+        for step in steps:
+            for r, n in step.items():
+                if not cache.has(r):
+                    cache.add(r)
+                cache.reserve(r, n)
+            batch = fn.build_batch([StepItem(r, [0] * n) for r, n in step.items()], singles_first=True)
+            took.append([])
+            out = torch.zeros(batch.n_tokens, H, device=DEV)
+            part.forward(x[at:at + batch.n_tokens], batch, cache.views(0), out)
+            outs.append(out)
+            at += batch.n_tokens
+            for r, n in step.items():
+                cache.commit(r, n)
+        ops.read_status(rt.status)
+        return outs, list(took)
+    steps = [{1: 300}, {1: 9}, {1: 300}, {1: 1, 2: 260}, {1: 1, 2: 30}]
+    outs, took_ = run(steps)
+    tiles, split = "attention_prefill_f32", "paged_attention_split"
+    assert took_ == [[(tiles, 1)], [(split, 9)], [(split, 300)], [(tiles, 1), (split, 1)], [(split, 31)]]
+    want, took_ = run(steps, lambda *a: True)
+    assert [t[0][0] for t in took_] == [tiles] * 5
+    for a, b in zip(outs, want):
+        assert float((a - b).abs().max()) <= 3e-6 * max(1.0, float(b.abs().max()))
