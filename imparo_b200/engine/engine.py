@@ -158,6 +158,8 @@ class Engine:
 
     def check_device_status(self) -> None:
         ops.read_status(self.status)
+        for word in self.rt.launch_state.status_fallback.values():       # launches that were given no word of their own
+            ops.read_status(word)
 
     def _checked(self, items: Sequence[StepItem]) -> List[StepItem]:
         """The items with their tokens as arrays (made once, for the checks here and the step's description)."""

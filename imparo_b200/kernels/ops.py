@@ -625,7 +625,7 @@ def linear_swiglu(x, w_gu: torch.Tensor, out: torch.Tensor, status: Optional[tor
     if callable(tmp):
         tmp = tmp()
     _need(tmp is not None and tmp.shape == (x.shape[0], w_gu.shape[0]), "linear_swiglu: tmp [T, 2F] needed on this path")
-    linear(x, w_gu, tmp)
+    linear(x, w_gu, tmp, status=status)
     swiglu_act(tmp, out)
 
 

@@ -246,7 +246,7 @@ class RoutedExperts(Part):
 
         def dense():
             if rt.act_dtype == torch.float32:
-                ops.linear(x, self.w_shared_gu, mid)
+                ops.linear(x, self.w_shared_gu, mid, status=rt.status)
                 ops.activation(mid, mid, self.act)
             else:
                 ops.linear_act(x, self.w_shared_gu, mid, self.act, status=rt.status)

@@ -99,6 +99,17 @@ def test_sgemm_is_true_float32(M, N, K):
     assert (out2.cpu().double() - (ref + base.double())).abs().max() <= 3e-6 * max(1.0, ref.abs().max())
 
 
+def test_32_bit_gate_and_up_product_reports_to_the_word_it_is_given():
+    o = ops()
+    previous = o.use_state(o.LaunchState())
+    try:
+        x, w, st = torch.ones(20, 64, device=DEV), torch.ones(96, 64, device=DEV), o.new_status(DEV)
+        o.linear_swiglu(x, w, torch.empty(20, 48, device=DEV), status=st, tmp=torch.empty(20, 96, device=DEV))
+        assert not o._S.status_fallback
+    finally:
+        o.use_state(previous)
+
+
 # edges of the split product's tiles (128 rows, 64 or 128 columns: the wide ones from 75 tiles on) and stretches (64 k);
 # outputs whose rows are no 16-byte groups; a row stride beyond K
 @pytest.mark.parametrize("M,N,K,ld", [(1, 1, 4, 4), (127, 63, 60, 60), (128, 64, 64, 68), (129, 65, 68, 68), (257, 130, 132, 140),

@@ -682,3 +682,21 @@ def test_command_line_and_trace_runner(tmp_path):
     errs = [e for e in all_errors(steps, got, want) if (e[1], e[2]) not in skip]
     assert max(e[3] for e in errs) <= WORST["bfloat16"] * scale
     assert sum(e[3] > TOL["bfloat16"] * scale for e in errs) <= 0.1 * len(errs)
+
+
+def test_32_bit_products_report_to_the_engine():
+    """A shared expert without a gate in a step of many rows: no product is left without the engine's status word; and a word of
+    launches that were given none is read by the engine's check too."""
+    import torch
+    from imparo_b200.kernels import ops
+    from imparo_b200.engine import StepItem
+    steps = traces.whole(make_requests("B", [300]))
+    engine = engine_for("B", "float32", steps, use_graphs=False)
+    engine.add_request(1)
+    engine.step([StepItem(1, steps[0]["entries"][0]["tokens"], (0,))])
+    engine.check_device_status()
+    assert not engine.rt.launch_state.status_fallback
+    engine.rt.launch_state.status_fallback[0] = torch.tensor([4, 91, 0, 0], dtype=torch.int32, device="cuda")
+    with pytest.raises(ops.KernelError, match="kernel 91"):
+        engine.check_device_status()
+    engine.check_device_status()
