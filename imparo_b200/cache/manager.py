@@ -53,9 +53,11 @@ class SlotStateView:
 
 class CacheManager:
     def __init__(self, requirements: Sequence[Tuple[int, Tuple]], page_size: int, num_pages: int, num_slots: int,
-                 kv_dtype: torch.dtype = torch.bfloat16, device=None, num_pages_by_group: Optional[Dict] = None):
+                 kv_dtype: torch.dtype = torch.bfloat16, device=None, num_pages_by_group: Optional[Dict] = None,
+                 status: Optional[torch.Tensor] = None):
         """requirements: (schedule entry, cache specs) for every entry that owns a cache.
-        device None: bookkeeping only (no arenas), for host-side use and tests.
+        device None: bookkeeping only (no arenas), for host-side use and tests.  status: the status word that the clearing of
+        slots reports to (an engine's; one of its own otherwise).
 
         Every arena holds one page and one state slot more than the bookkeeping hands out (spare_page(group),
         spare_slot): rows of a step that belong to no request (the step function's padding rows) write there."""
@@ -96,7 +98,6 @@ class CacheManager:
         if not self._cm:
             raise CacheError("cache manager: bad sizes")
         # device arenas
-        self._slot_numbers = self._zero_status = None              # made at the first clearing of a slot
         self.k_arena: List[Optional[torch.Tensor]] = []
         self.v_arena: List[Optional[torch.Tensor]] = []
         self.state: Dict[Tuple[int, int], torch.Tensor] = {}
@@ -129,6 +130,9 @@ class CacheManager:
             self.state_segments = torch.tensor(segs if segs else [(0, 0)], dtype=torch.int64, device=device)
             self.n_state_segments = len(segs)
             self.state_max_per_slot = max((per for _, per in segs), default=0)     # sizes the clearing kernel's grid
+            # what the clearing kernel reads before it waits for the kernel ahead of it: there before any launch
+            self._slot_numbers = torch.tensor(range(slots), dtype=torch.int32, device=device)
+            self.status = status if status is not None else torch.zeros(4, dtype=torch.int32, device=device)
 
     def __del__(self):
         try:
@@ -179,11 +183,10 @@ class CacheManager:
             return
         # one launch for all state tensors (one fill each: 4 us of a step's stream per tensor)
         from ..kernels import ops
-        if self._slot_numbers is None:
-            self._slot_numbers = torch.arange(self.arena_slots, dtype=torch.int32, device=self.state_arena.device)
-            self._zero_status = ops.new_status(self.state_arena.device)
-        ops.zero_state_slots(self.state_arena, self.state_segments, self.n_state_segments, self._slot_numbers[slot:slot + 1],
-                             self.arena_slots, self._zero_status, max_per_slot=self.state_max_per_slot)
+        slot = range(self.arena_slots)[slot]                       # (an index: IndexError beyond the slots there are)
+        with torch.cuda.device(self.state_arena.device):
+            ops.zero_state_slots(self.state_arena, self.state_segments, self.n_state_segments, self._slot_numbers[slot:slot + 1],
+                                 self.arena_slots, self.status, max_per_slot=self.state_max_per_slot)
 
     def has(self, req: int) -> bool:
         return self._h.imparo_cm_slot(self._cm, req) >= 0

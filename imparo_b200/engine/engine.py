@@ -112,7 +112,7 @@ class Engine:
         if num_pages is None:
             num_pages = self.parallel * ((self.ctx + self.page_size - 1) // self.page_size)
         self.cache = CacheManager(self.model.cache_requirements(), self.page_size, int(num_pages), self.parallel,
-                                  kv_dtype=self.rt.act_dtype, device=self.device)
+                                  kv_dtype=self.rt.act_dtype, device=self.device, status=self.status)
         self.max_step_tokens = int(max_step_tokens)
         self.step_fn = StepFunction(self.model, self.cache, self.max_step_tokens, self.parallel, use_graphs=cfg.use_graphs,
                                     pad_rows=cfg.pad_rows, capture_first=cfg.capture_first)

@@ -400,3 +400,22 @@ def test_short_portions_over_many_keys_take_the_split_key_kernel(monkeypatch):
     assert [t[0][0] for t in took_] == [tiles] * 5
     for a, b in zip(outs, want):
         assert float((a - b).abs().max()) <= 3e-6 * max(1.0, float(b.abs().max()))
+
+
+def test_clearing_a_slot_reports_like_indexing_it():
+    """Slots count as indices do, one that is not there is refused, and a kernel's report goes to the word the manager was given."""
+    from imparo_b200.cache import CacheManager
+    from imparo_b200.kernels import ops
+    from imparo_b200.parts.spec import SlotState
+    status = ops.new_status(DEV)
+    cm = CacheManager([(0, (SlotState((5, 3)), SlotState((7,))))], 4, 4, 3, device=torch.device(DEV), status=status)
+    assert cm.status is status
+    for slot, zeroed in ((1, 1), (-1, 3), (0, 0)):
+        cm.state_arena.fill_(1.0)
+        cm.zero_slot(slot)
+        for t in cm.state.values():
+            assert t.flatten(1).sum(1).eq(0).tolist() == [i == zeroed for i in range(4)]
+    for slot in (4, -5):
+        with pytest.raises(IndexError):
+            cm.zero_slot(slot)
+    ops.read_status(status)
