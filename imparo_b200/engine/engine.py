@@ -15,7 +15,6 @@ import sys
 import time
 from typing import Dict, List, Optional, Sequence, Union
 
-import numpy as np
 import torch
 
 from ..cache import CacheManager
@@ -29,7 +28,7 @@ from ..sampling import Sampler
 from ..weights.loader import load_weights, target_dtype
 from ..weights.random_init import draw_random_tensors
 from .scheduler import Scheduler, padded_rows
-from .step import StepFunction, StepItem
+from .step import StepFunction, StepItem, int_array
 
 _PRECISIONS = {"bfloat16": "bfloat16", "bf16": "bfloat16", "float32": "float32", "fp32": "float32", "f32": "float32"}
 
@@ -162,12 +161,17 @@ class Engine:
             ops.read_status(word)
 
     def _checked(self, items: Sequence[StepItem]) -> List[StepItem]:
-        """The items with their tokens as arrays (made once, for the checks here and the step's description)."""
+        """The items with their tokens as arrays where they are many (made once, for the checks here and the step's description)."""
         checked = []
         for it in items:
-            toks = np.asarray(it.tokens, dtype=np.int64) if len(it.tokens) > 8 else it.tokens
-            if len(toks) and (min(toks) < 0 or max(toks) >= self.vocab_size if toks is it.tokens
-                              else toks.min() < 0 or toks.max() >= self.vocab_size):
+            toks = it.tokens
+            array = int_array(toks) if len(toks) > 8 else None
+            if array is not None:
+                toks = array
+                outside = array.min() < 0 or array.max() >= self.vocab_size
+            else:
+                outside = len(toks) and (min(toks) < 0 or max(toks) >= self.vocab_size)
+            if outside:
                 raise ValueError(f"request {it.request}: token id out of range [0, {self.vocab_size})")
             if self.cache.has(it.request) and self.cache.cached(it.request) + len(toks) > self.ctx:
                 raise ValueError(f"request {it.request}: {self.cache.cached(it.request)} + {len(toks)} tokens "

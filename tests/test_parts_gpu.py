@@ -419,3 +419,22 @@ def test_clearing_a_slot_reports_like_indexing_it():
         with pytest.raises(IndexError):
             cm.zero_slot(slot)
     ops.read_status(status)
+
+
+@pytest.mark.parametrize("make", [list, tuple, set, lambda w: np.array(w, dtype=np.int8), lambda w: {i: None for i in w}, torch.tensor])
+def test_wanted_places_of_any_kind(make):
+    """Many wanted places, given as anything that holds whole numbers; one outside the request's tokens is refused."""
+    from imparo_b200.engine.step import StepItem
+    from imparo_b200.parts.spec import PartSpec
+    rt = runtime("float32")
+    part, _ = build("mixer", PartSpec("short_conv", {"hidden": 16, "taps": 3, "bias": False}), "L.", rt)
+    cache, fn = batch_for(part, rt, None)
+    for r in (1, 2):
+        cache.add(r)
+    want = list(range(2, 40, 3))
+    made = make(want)
+    batch = fn.build_batch([StepItem(1, [0] * 300), StepItem(2, [0] * 40, made)])
+    assert batch.n_want == len(want) and batch.want_rows.tolist() == [300 + int(w) for w in made]
+    for wrong in (40, -1):
+        with pytest.raises(ValueError, match=f"wanted place {wrong} is not among its 40 tokens"):
+            fn.build_batch([StepItem(1, [0] * 300), StepItem(2, [0] * 40, make(want + [wrong]))])

@@ -1,5 +1,56 @@
-"""What a step's shape decides on the host (no GPU): which kernel takes 32-bit portions."""
+"""A step's items on the host (no GPU): tokens and wanted places as arrays, their checks, and the rule that chooses the 32-bit
+attention's kernel from a step's shape."""
+from types import SimpleNamespace
+
+import numpy as np
 import pytest
+import torch
+
+from imparo_b200.engine import Engine, StepItem
+from imparo_b200.engine import engine as engine_module
+from imparo_b200.engine.step import int_array
+
+
+def test_whole_numbers_as_an_array():
+    for values in ([5, 0, 7], (5, 0, 7), range(3), np.arange(3), np.arange(3, dtype=np.int8), np.arange(3, dtype=np.uint32), [np.int64(4), True],
+                   [torch.tensor(3)]):
+        got = int_array(values)
+        assert got.dtype == np.int64 and got.tolist() == [int(v) for v in values]
+    exact = np.arange(4)
+    assert int_array(exact) is exact
+    for values in ({1, 2}, [0.5, 1], [2 ** 70], np.array([0.5]), np.array([[1, 2]]), torch.arange(3), {1: 2}, [], "12"):
+        assert int_array(values) is None
+
+
+def _checked(items):
+    return Engine._checked(SimpleNamespace(vocab_size=100, ctx=64, cache=SimpleNamespace(has=lambda r: r == 7, cached=lambda r: 50)), items)
+
+
+@pytest.mark.parametrize("n", [3, 20])
+def test_tokens_out_of_the_vocabulary_are_refused(n):
+    good = list(range(n))
+    for make in (list, tuple, np.array, lambda t: np.array(t, dtype=np.int16), torch.tensor):
+        (item,) = _checked([StepItem(1, make(good), (0,))])
+        assert [int(t) for t in item.tokens] == good and item.want == (0,) and item.request == 1
+        for wrong in (100, -1):
+            with pytest.raises(ValueError, match="request 1: token id out of range"):
+                _checked([StepItem(1, make(good[:-1] + [wrong]))])
+    for wrong in (2 ** 70, -2 ** 70, -0.5, 100.0):
+        with pytest.raises(ValueError, match="token id out of range"):
+            _checked([StepItem(1, good[:-1] + [wrong])])
+    if n > 14:
+        with pytest.raises(ValueError, match="exceed the context length"):
+            _checked([StepItem(7, good)])
+
+
+def test_arrays_are_not_walked_entry_by_entry(monkeypatch):
+    def walked(values):
+        raise AssertionError("walked in Python")
+    for name in ("min", "max"):
+        monkeypatch.setattr(engine_module, name, walked, raising=False)
+    for dtype in (np.int64, np.int32):
+        tokens = np.arange(60, dtype=dtype)
+        assert np.array_equal(_checked([StepItem(1, tokens)])[0].tokens, tokens)
 
 
 # both sides of the line where they were measured (16 and 32 heads of 64 on 8, 8 of 128 on 2, 4 of 64 on 4): portions of one or several
