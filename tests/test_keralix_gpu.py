@@ -386,8 +386,8 @@ def _delta_walk_64(q, k, v, beta, g, S):
     return o
 
 
-# key sizes at the edges of both builds (64 and 128 channels) and no multiple of 16, value sizes below, at and beyond a CTA's 16,
-# 64 and 128 columns; portions of 1 row, whole chunks, a chunk and a row
+# key sizes at the edges of both builds (64 and 128 channels) and no multiple of 16, value sizes below and beyond a CTA's 8
+# columns (scan), 64 (outputs) and 128 (solves); portions of 1 row, whole chunks, a chunk and a row
 @pytest.mark.parametrize("H,G,D,V", [(2, 1, 64, 128), (3, 3, 4, 4), (4, 2, 20, 36), (2, 2, 128, 132), (1, 1, 68, 16), (2, 1, 64, 260)])
 @pytest.mark.parametrize("lens", [(1, 64, 65), (200, 7), (128,)])
 def test_delta_rule_in_chunks(H, G, D, V, lens):

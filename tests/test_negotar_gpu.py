@@ -432,7 +432,7 @@ def _scan_64(x, B, C, dt, A_log, D, S, per):
     return y
 
 
-# state sizes at the edges of both builds, value sizes around a CTA's 64 columns, one, two and four heads per CTA, two groups;
+# state sizes at the edges of both builds, value sizes around a CTA's 64 columns, one head per CTA, two groups;
 # portions of one row, whole chunks, a chunk and a row
 @pytest.mark.parametrize("heads,groups,N,vdim", [(3, 3, 4, 4), (2, 1, 64, 64), (2, 2, 68, 20), (4, 1, 128, 132), (8, 2, 60, 64)])
 @pytest.mark.parametrize("lens", [(1, 64, 65), (200, 7), (4800, 128)])
@@ -471,6 +471,31 @@ def test_state_space_products(heads, groups, N, vdim, lens):
     assert (y - want).norm() <= 2 * (walk_y - want).norm() + 1e-7 * want.norm()
     assert (s - want_state).norm() <= 2 * (walk_s - want_state).norm() + 1e-7 * want_state.norm()
     assert torch.equal(s[[1, 4]], state0[[1, 4]].double())
+
+
+# enough CTAs (heads x chunks x value columns / 64) for two and for four heads per CTA: the builds a prompt of many heads takes.  Two:
+# 494 with heads per group no multiple of four; four: 832 and, over two and three blocks of value columns, 624 and 936
+@pytest.mark.parametrize("heads,groups,N,vdim", [(38, 1, 8, 4), (38, 1, 72, 4), (64, 1, 8, 4), (64, 2, 72, 4), (24, 3, 8, 68), (24, 3, 72, 132)])
+def test_state_space_products_several_heads_per_cta(heads, groups, N, vdim):
+    test_state_space_products(heads, groups, N, vdim, (700, 65))
+
+
+# one, two, four and eight 16-byte groups per thread, and beyond them the kernel without registers
+@pytest.mark.parametrize("out_dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("per,groups", [(4, 3), (1024, 2), (1028, 2), (2048, 1), (2052, 2), (4096, 1), (4100, 1), (8192, 1), (8196, 1), (1030, 1)])
+def test_gated_norm_of_wide_stretches(per, groups, out_dtype):
+    import torch
+    from imparo_b200.kernels import ops
+    g = torch.Generator().manual_seed(per)
+    rows, width = 5, per * groups
+    y, proj, w = torch.randn(rows, width, generator=g), torch.randn(rows, width + 8, generator=g) * 3, torch.randn(width, generator=g)
+    out = torch.full((rows, width), float("nan"), dtype=getattr(torch, out_dtype), device="cuda")
+    ops.gate_group_rmsnorm(y.cuda(), proj.cuda()[:, :width], w.cuda(), 1e-5, groups, out)
+    z = proj[:, :width].double()
+    v = (y.double() * z * torch.sigmoid(z)).view(rows, groups, per)
+    want = (v / torch.sqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5)).view(rows, width) * w.double()
+    # silu, three products and the root, each a few units of 2^-24; then the stored type's rounding
+    assert ((out.cpu().double() - want).abs() <= (2e-6 if out_dtype == "float32" else 2.0 ** -8 + 2e-6) * want.abs()).all()
 
 
 # (both builds of the state size; rows in the middle of a thread's eight and at the end of a chunk)
