@@ -460,7 +460,7 @@ gate_group_rmsnorm_wide_kernel(const float* __restrict__ y, const float* __restr
     float4 a[V], g[V];
 #pragma unroll
     for (int u = 0; u < V; ++u) {
-        const int i = threadIdx.x + 256 * u;
+        const int i = threadIdx.x + blockDim.x * u;
         a[u] = g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (4 * i < per) { a[u] = yr[i]; g[u] = zr[i]; }
     }
@@ -475,7 +475,7 @@ gate_group_rmsnorm_wide_kernel(const float* __restrict__ y, const float* __restr
     T* o = out + (size_t)r * width + (size_t)grp * per;
 #pragma unroll
     for (int u = 0; u < V; ++u) {
-        const int i = threadIdx.x + 256 * u;
+        const int i = threadIdx.x + blockDim.x * u;
         if (4 * i < per) {
             const float4 wv = wg[i];
             alignas(16) T v[4] = {from_f32<T>(a[u].x * scale * wv.x), from_f32<T>(a[u].y * scale * wv.y), from_f32<T>(a[u].z * scale * wv.z),
@@ -630,7 +630,9 @@ extern "C" int imparo_gate_group_rmsnorm(const float* y, const void* z, int z_dt
     const int per = width / groups;
     if (z_dtype == IMPARO_DT_F32 && (out_dtype == IMPARO_DT_F32 || out_dtype == IMPARO_DT_BF16) && per % 4 == 0 && per <= 8192 && z_stride % 4 == 0 &&
         (((uintptr_t)y | (uintptr_t)z | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
-#define IMPARO_GG(T_, V_) launch(gate_group_rmsnorm_wide_kernel<T_, V_>, grid, dim3(256), 0, stream, y, (const float*)z, (size_t)z_stride, w, eps, \
+        // as many warps as a short stretch fills: 256 threads for 64 groups of four cost 1,000 rows of 8 x 256 20 us
+        const dim3 threads(per < 1024 ? (per / 4 + 31) / 32 * 32 : 256);
+#define IMPARO_GG(T_, V_) launch(gate_group_rmsnorm_wide_kernel<T_, V_>, grid, threads, 0, stream, y, (const float*)z, (size_t)z_stride, w, eps, \
                                  (T_*)out, width, groups)
 #define IMPARO_GGV(T_) do { if (per <= 1024) IMPARO_GG(T_, 1); else if (per <= 2048) IMPARO_GG(T_, 2); else if (per <= 4096) IMPARO_GG(T_, 4); \
                             else IMPARO_GG(T_, 8); } while (0)
