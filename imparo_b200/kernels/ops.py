@@ -1166,20 +1166,24 @@ def attention_prefill_f32(q, k_cache, v_cache, item_row_start, item_start_pos, n
     return True
 
 
-def attention_f32_tiles_pay(n_tok: int, n_items: int, nh: int, nkv: int, from_start: bool) -> bool:
+def attention_f32_tiles_pay(n_tok: int, n_items: int, nh: int, nkv: int, hd: int, from_start: bool) -> bool:
     """Whether 32-bit portions (n_tok rows of n_items requests) go to the tiles (attention_prefill_f32) and not to the split-key
-    kernel.  The tiles walk a request's keys in one CTA per 64 rows and head, at 0.12 us per key (head size 64) however few rows the
-    tile holds, as long as every SM has at most 1.5 CTAs or so; the split-key kernel spreads the keys over the chip and takes
-    (56 + 24 nh / nkv) ps per key, row and kv head.  Where the two meet, both sides in us (B200, 16 heads of 64, 8 kv heads):
-    8,000 keys before the portion: 64 rows 417 split / 964 tiles, 128 rows 816 / 971, 256 rows 1,656 / 1,144; 8 rows at 30,000 keys:
-    259 / 3,771.  Head size 128 shifts both sides alike.  Portions that start at position 0 (from_start) have few keys, and the
-    split-key launch is made for as many as the tables can hold: there the line lies at half the rows (64 rows: 14.2 / 13.7;
-    32 heads, 8 kv heads: 22.1 / 13.8).  Groups of more than 8 heads: the split-key kernel does not take them."""
+    kernel.  Both take so many ns per key of the context (B200): the tiles walk a request's keys in one CTA per 64 rows and head, 119
+    (186 beyond head size 64) however few rows a tile holds, more from some 50 CTAs on, as more of them share SMs; the split-key
+    kernel spreads the keys over the chip and takes time for each row: per kv head 0.087, 0.098, 0.121, 0.145, 0.165 with groups of 1
+    to 5 heads of 64, 0.455, 0.525, 0.62 with 6 to 8 (spilled registers), and 0.40, 0.58, 0.97, 1.45, 1.8 times that at head sizes 16,
+    32, 48, 96, 128.  The line lies at 0.85 of equal times, as measured (us, split-key against tiles, 16 heads of 64 on 8 after 8,000
+    positions: 64 rows 417 / 964, 128 rows 816 / 971, 256 rows 1,656 / 1,144; 48 heads of
+    64 on 8 after 2,000: 32 rows 280 / 246, 64 rows 532 / 295).  Portions that start at position 0 (from_start) have few keys, while the split-key launch is made for all the
+    tables can hold: their line lies at 0.3 (64 rows: 14.2 / 13.7; 32 heads on 8: 22.1 / 13.8; 4 heads on 4, 128 rows: 15 / 21).
+    Groups of more than 8 heads: the split-key kernel does not take them."""
     group = nh // nkv
     if group > 8:
         return True
-    rounds = max(1.0, nh * (n_tok // 64 + n_items) / 220)
-    return n_tok * nkv * (7 + 3 * group) >= (6500 if from_start else 13000) * rounds
+    ctas = nh * (n_tok // 64 + n_items)
+    tiles = (119 if hd <= 64 else 186) * max(1 + min(ctas, 128) / 300, ctas / 220)
+    split = n_tok * nkv * (0.064 + 0.020 * group if group <= 5 else 0.075 * group) * (hd + 8) / 72
+    return split >= (0.3 if from_start else 0.85) * tiles
 
 
 # ---- attention with sigmoid weights (csrc/kernels/attention_sigmoid.cu) -----------------------------------------

@@ -461,7 +461,7 @@ class AttentionMixer(Part):
         if rt.act_dtype == torch.float32:
             prefill, beside = ops.attention_prefill_f32, {}
             lead = n1 if beside_rows else 0
-            portions = portions and ops.attention_f32_tiles_pay(T - lead, batch.n_items - lead, nh, self.nkv,
+            portions = portions and ops.attention_f32_tiles_pay(T - lead, batch.n_items - lead, nh, self.nkv, hd,
                                                                 getattr(batch, "portions_from_start", False))
         else:
             prefill, beside = ops.attention_prefill, {"dependents_after_wait": ops.switches().attn_side_by_side}

@@ -1,5 +1,5 @@
-"""A step's items on the host (no GPU): tokens and wanted places as arrays, their checks, and the rule that chooses the 32-bit
-attention's kernel from a step's shape."""
+"""A step's items on the host (no GPU): tokens and wanted places as arrays, their checks, and the rules that choose a kernel from a
+step's shape."""
 from types import SimpleNamespace
 
 import numpy as np
@@ -53,14 +53,15 @@ def test_arrays_are_not_walked_entry_by_entry(monkeypatch):
         assert np.array_equal(_checked([StepItem(1, tokens)])[0].tokens, tokens)
 
 
-# both sides of the line where they were measured (16 and 32 heads of 64 on 8, 8 of 128 on 2, 4 of 64 on 4): portions of one or several
-# requests after thousands of positions, or from position 0
-@pytest.mark.parametrize("nh,nkv,rows,requests,from_start,tiles", [
-    (16, 8, 8, 1, False, False), (16, 8, 64, 1, False, False), (16, 8, 256, 1, False, True), (32, 8, 64, 1, False, False), (32, 8, 256, 1, False, True),
-    (8, 2, 256, 1, False, False), (8, 2, 512, 1, False, True), (4, 4, 256, 1, False, False), (4, 4, 512, 1, False, True),
-    (16, 8, 256, 32, False, False), (32, 8, 256, 32, False, False), (16, 8, 400, 4, False, True), (16, 8, 80, 16, False, False),
-    (16, 8, 16, 1, True, False), (16, 8, 128, 1, True, True), (32, 8, 64, 1, True, True), (16, 8, 1000, 3, True, True), (8, 2, 128, 1, True, False),
-    (18, 2, 8, 1, False, True)])
-def test_where_32_bit_portions_go_to_the_tiles(nh, nkv, rows, requests, from_start, tiles):
+# both sides of the line where they were measured: portions of one or several requests after thousands of positions, or from position 0
+@pytest.mark.parametrize("nh,nkv,hd,rows,requests,from_start,tiles", [
+    (16, 8, 64, 8, 1, False, False), (16, 8, 64, 64, 1, False, False), (16, 8, 64, 256, 1, False, True), (32, 8, 64, 64, 1, False, False),
+    (32, 8, 64, 256, 1, False, True), (8, 2, 128, 256, 1, False, False), (8, 2, 128, 512, 1, False, True), (4, 4, 64, 256, 1, False, False),
+    (4, 4, 64, 512, 1, False, True), (16, 8, 64, 256, 32, False, False), (32, 8, 64, 256, 32, False, False), (16, 8, 64, 400, 4, False, True),
+    (16, 8, 64, 80, 16, False, False), (32, 4, 64, 64, 1, False, True), (48, 8, 64, 64, 1, False, True), (16, 2, 64, 16, 1, False, False),
+    (16, 8, 16, 256, 1, False, False), (16, 8, 16, 1000, 1, False, True), (16, 8, 32, 128, 1, False, False), (16, 8, 48, 256, 1, False, True),
+    (16, 8, 64, 16, 1, True, False), (16, 8, 64, 128, 1, True, True), (32, 8, 64, 64, 1, True, True), (16, 8, 64, 1000, 3, True, True),
+    (8, 2, 128, 64, 1, True, False), (4, 4, 64, 64, 1, True, False), (18, 2, 64, 8, 1, False, True)])
+def test_where_32_bit_portions_go_to_the_tiles(nh, nkv, hd, rows, requests, from_start, tiles):
     from imparo_b200.kernels import ops
-    assert ops.attention_f32_tiles_pay(rows, requests, nh, nkv, from_start) is tiles
+    assert ops.attention_f32_tiles_pay(rows, requests, nh, nkv, hd, from_start) is tiles
