@@ -1663,6 +1663,14 @@ def mamba2_conv(proj: torch.Tensor, x_off: int, dt_off: int, channels: int, head
         COUNTS["own"] += 1
 
 
+def mamba2_products_pay(heads: int, vdim: int, chunks: int) -> bool:
+    """Whether chunks of the state-space recurrence run as products and not as row walks side by side.  A CTA of the products has room
+    for 64 value columns, a warp of the walks for 32: with up to 32 the walks do less, and are the faster ones once there are more than
+    four CTAs per SM.  Products against walks in us (B200): 64 heads of 32, state 16, 512 rows 43 / 46, 2,000 rows 117 / 84; state 128,
+    256 rows 52 / 72, 2,000 rows 243 / 161; 64 heads of 36, state 16, 2,000 rows 118 / 135; of 64, state 128, 262 / 321."""
+    return vdim > 32 or heads * chunks <= 592
+
+
 def mamba2_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: torch.Tensor, state: torch.Tensor, item_row_start,
                 item_slot, n_items: int, y: torch.Tensor, heads: int, vdim: int, n_state: int, groups: int, status: torch.Tensor,
                 chunk: int = 0, scratch=None) -> None:
@@ -1671,7 +1679,8 @@ def mamba2_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: tor
     chunk > 0 (steps with long portions): the rows of a request are cut into chunks of that many rows that run side by
     side; scratch = (int32 [3*max_chunks + n_items + 1], float32 [max_chunks*heads*N*vdim], float32 [max_chunks*heads])
     with max_chunks = T // chunk + n_items.  The result differs from the row-by-row walk by 32-bit rounding only.  Chunks of 64
-    rows whose state and value sizes are multiples of 4 (state up to 128) run as products (the int32 scratch is then not used)."""
+    rows whose state and value sizes are multiples of 4 (state up to 128) run as products where that pays (mamba2_products_pay; the
+    int32 scratch is then not used)."""
     _cuda(xbc, dt, A_log, D, state, item_row_start, item_slot, y, status)
     T = xbc.shape[0]
     inner = heads * vdim
@@ -1689,7 +1698,7 @@ def mamba2_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: tor
         _need(si.dtype == torch.int32 and si.numel() >= 3 * max_chunks + n_items + 1 and cs.dtype == torch.float32
               and cs.numel() >= max_chunks * heads * n_state * vdim and cd.dtype == torch.float32 and cd.numel() >= max_chunks * heads,
               "mamba2_scan: chunk scratch too small")
-        if (chunk == 64 and _lib.kernels().imparo_mamba2_products_take(heads, vdim, n_state, groups)
+        if (chunk == 64 and mamba2_products_pay(heads, vdim, max_chunks) and _lib.kernels().imparo_mamba2_products_take(heads, vdim, n_state, groups)
                 and all(t.data_ptr() % 16 == 0 for t in (xbc, state, y, cs))):
             _check(_lib.kernels().imparo_mamba2_products(_ptr(xbc), _ptr(dt), _ptr(A_log), _ptr(D), _ptr(state), _ptr(item_row_start),
                                                          _ptr(item_slot), int(n_items), state.shape[0], _ptr(y), heads, vdim, n_state,

@@ -65,3 +65,10 @@ def test_arrays_are_not_walked_entry_by_entry(monkeypatch):
 def test_where_32_bit_portions_go_to_the_tiles(nh, nkv, hd, rows, requests, from_start, tiles):
     from imparo_b200.kernels import ops
     assert ops.attention_f32_tiles_pay(rows, requests, nh, nkv, hd, from_start) is tiles
+
+
+@pytest.mark.parametrize("heads,vdim,rows,products", [(64, 32, 512, True), (64, 32, 2000, False), (64, 16, 2000, False), (32, 16, 512, True),
+                                                      (64, 36, 2000, True), (64, 64, 2000, True), (8, 8, 2000, True)])
+def test_where_state_space_chunks_run_as_products(heads, vdim, rows, products):
+    from imparo_b200.kernels import ops
+    assert ops.mamba2_products_pay(heads, vdim, rows // 64 + 1) is products
