@@ -91,14 +91,28 @@ class GatedDeltaRule(Part):
         return (SlotState((self.heads, self.dim, self.vdim)), SlotState((max(self.taps - 1, 1), self.channels)))
 
     def _in_chunks(self, longest: int, tokens: int, portions: int) -> bool:
-        """Whether a step's portions (tokens rows of that many requests) run in chunks of 64 rows side by side and not row by row
-        (the longest one's length comes rounded up to a power of two).  The walk takes as long as the longest portion, the chunks
-        a whole chunk for every short portion, which many wide heads pay in full.  Walk against chunks in us (B200): key size 64,
-        value size 128, 8 heads: 257 rows 56 / 64, 300 rows 64 / 65, 2,048 rows 421 / 142; 300 rows beside 8 portions of 16: 98 /
-        79, beside 31 portions of 8: 94 / 133.  16 heads of key size 128: 300 rows 105 / 82, 2,048 rows 677 / 380; 300 rows beside 8
-        portions of 16: 167 / 194, 512 beside 8 of 64: 323 / 226; 32 such heads: 257 rows 136 / 153, 300 rows 157 / 154."""
-        least = 32 if self.heads * self.dim <= 512 else 64
-        return longest >= 512 and tokens >= max(300, least * portions)
+        """Whether a step's portions (tokens rows of that many requests, the longest one's length rounded up to a power of two) run
+        in chunks of 64 rows side by side and not row by row: the smaller of two estimates in us (B200), from 257 rows on.  The walk
+        takes its time per row of the longest portion (more as the value columns fill the chip) or per row and value column of all;
+        the chunks a start, then time per chunk and head, or per chunk of the longest portion.  Walk / chunks as measured: key size
+        64, value size 128, 8 heads: 257 rows 56 / 64, 300 rows 64 / 65, 2,048 rows 421 / 141, 300 rows beside 31 portions of 8:
+        94 / 133; 64 heads of 64 / 64: 400 rows 124 / 137, 512 rows 158 / 143, four portions of 257: 239 / 331; 128 heads of 32 /
+        32: two of 1,000: 477 / 736; 16 heads of 128 / 128: 300 rows 105 / 82, beside 8 portions of 16: 167 / 194.  Over 135 such
+        shapes what is chosen takes 0.2% longer than the better one, at most 12%."""
+        if longest < 512:
+            return False
+        longest = tokens if portions == 1 else min(longest, tokens)
+        columns = self.heads * self.vdim
+        filled = min(max(columns - 1024, 0) / 3072, 1.0)
+        if self.dim > 64:
+            start, per_head, per_chunk = 42.0, 0.40 + 0.0024 * self.vdim, 3.2
+            per_row, per_column = 0.255 + 0.34 * filled, 1.57e-4
+        else:
+            start, per_head, per_chunk = 48.0, 0.16 + 0.0013 * self.vdim, 1.8
+            per_row, per_column = (0.207 if self.dim > 32 else 0.32) + 0.16 * filled, 6.3e-5
+        chunks = start + max(self.heads * (tokens / 64 + portions / 2) * per_head, longest / 64 * per_chunk)
+        walk = 4.0 + max(longest * per_row, tokens * columns * per_column)
+        return chunks < walk
 
     def forward(self, x, batch, caches, residual, accumulate=True):
         st, conv = caches

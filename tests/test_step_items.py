@@ -72,3 +72,17 @@ def test_where_32_bit_portions_go_to_the_tiles(nh, nkv, hd, rows, requests, from
 def test_where_state_space_chunks_run_as_products(heads, vdim, rows, products):
     from imparo_b200.kernels import ops
     assert ops.mamba2_products_pay(heads, vdim, rows // 64 + 1) is products
+
+
+# walk / chunks in us where both were measured: the portions' lengths, whose longest the rule sees rounded up to a power of two
+@pytest.mark.parametrize("heads,dim,vdim,portions,chunks", [
+    (8, 64, 128, [256], False), (8, 64, 128, [257], False), (8, 64, 128, [512], True), (8, 64, 128, [8] * 31 + [300], False),
+    (8, 64, 128, [16] * 8 + [300], True), (8, 64, 128, [64] * 8 + [512], True), (64, 64, 64, [400], False), (64, 64, 64, [512], True),
+    (64, 64, 64, [257] * 4, False), (128, 64, 64, [512], False), (128, 32, 32, [1000, 1000], False), (32, 64, 128, [100] * 10 + [600], True),
+    (16, 128, 128, [257], True), (16, 128, 128, [16] * 8 + [300], False), (16, 128, 128, [64] * 8 + [512], True), (32, 128, 128, [512], True),
+    (32, 128, 128, [8] * 31 + [300], False), (2, 64, 64, [16] * 16 + [400], True), (32, 16, 16, [300], True), (4, 128, 256, [2048], True)])
+def test_where_the_delta_rule_runs_in_chunks(heads, dim, vdim, portions, chunks):
+    from imparo_b200.parts.delta_rule import GatedDeltaRule
+    part = GatedDeltaRule({"hidden": 64, "heads": heads, "kv_heads": heads, "dim": dim, "vdim": vdim, "conv": 4, "decay_rank": 8, "gate_rank": 8,
+                           "eps": 1e-6}, "L.", None)
+    assert part._in_chunks(1 << (max(portions) - 1).bit_length(), sum(portions), len(portions)) is chunks
