@@ -67,11 +67,13 @@ def test_where_32_bit_portions_go_to_the_tiles(nh, nkv, hd, rows, requests, from
     assert ops.attention_f32_tiles_pay(rows, requests, nh, nkv, hd, from_start) is tiles
 
 
-@pytest.mark.parametrize("heads,vdim,rows,products", [(64, 32, 512, True), (64, 32, 2000, False), (64, 16, 2000, False), (32, 16, 512, True),
-                                                      (64, 36, 2000, True), (64, 64, 2000, True), (8, 8, 2000, True)])
-def test_where_state_space_chunks_run_as_products(heads, vdim, rows, products):
+@pytest.mark.parametrize("heads,vdim,state,rows,products", [
+    (64, 32, 16, 511, True), (64, 32, 16, 1999, False), (64, 32, 128, 256, True), (64, 32, 128, 511, False), (64, 16, 16, 256, False),
+    (64, 16, 16, 100, True), (32, 16, 64, 511, True), (32, 16, 128, 1999, False), (64, 36, 16, 1999, True), (64, 64, 128, 1999, True),
+    (8, 8, 8, 1999, True)])
+def test_where_state_space_chunks_run_as_products(heads, vdim, state, rows, products):
     from imparo_b200.kernels import ops
-    assert ops.mamba2_products_pay(heads, vdim, rows // 64 + 1) is products
+    assert ops.mamba2_products_pay(heads, vdim, state, rows // 64 + 1) is products
 
 
 # walk / chunks in us where both were measured: the portions' lengths, whose longest the rule sees rounded up to a power of two
