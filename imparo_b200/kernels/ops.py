@@ -662,150 +662,6 @@ def _partials_scratch(device, floats: int) -> torch.Tensor:
 
 def linear(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
            status: Optional[torch.Tensor] = None) -> None:
-    _need(x.is_cuda and w.is_cuda and out.is_cuda, "kernels run on CUDA tensors only (there is no CPU path)")
-    _need(tc_usable(x, w, any_size=True), "gemm_tc: bfloat16 operands, K a multiple of 8, 16-byte aligned rows")
-    T, K = x.shape
-    N = w.shape[0] // 2 if epilogue == EPI_SWIGLU else w.shape[0]
-    _need(w.shape[1] == K and (epilogue != EPI_SWIGLU or w.shape[0] % 2 == 0), "gemm_tc: weight shape")
-    if not (out.shape == (T, N) and out.stride(1) == 1):
-        raise KernelError(f"gemm_tc: out must be [{T}, {N}]")
-    want_dtype = torch.bfloat16 if epilogue in (EPI_STORE_BF16, EPI_SWIGLU) else torch.float32
-    if not (epilogue == EPI_PARTIAL or out.dtype == want_dtype):
-        raise KernelError(f"gemm_tc: this epilogue writes {want_dtype}")
-    nt, splits, floats, counters = _tc_plan(T, N, K, epilogue)
-    if epilogue == EPI_PARTIAL:
-        _need(scratch is not None and scratch.dtype == torch.float32 and scratch.numel() >= floats, "gemm_tc: partials scratch")
-        cnt = scratch
-    else:
-        scratch, cnt = _tc_buffers(x.device, floats, counters)
-    status = _status_word(x.device, status)
-    rows_alloc = (x.untyped_storage().nbytes() // x.element_size() - x.storage_offset()) // x.stride(0) if x.stride(0) else T
-    rows_alloc = max(T, min(rows_alloc, 1 << 30))
-    if plain is not None:
-        if bias is not None:
-            _cuda(bias)
-        _need(epilogue == EPI_STORE_BF16 and (bias is None or (bias.dtype == torch.float32 and bias.numel() == N)), "gemm_tc: plain activation")
-        _check(_lib.kernels().imparo_gemm_tc_act(_ptr(x), x.stride(0), rows_alloc, _ptr(w), _ptr(out), out.stride(0), T, N, K,
-                                                 ACTIVATIONS[plain], _ptr(bias), _ptr(scratch), _ptr(cnt), _ptr(status), _stream()),
-               "gemm_tc_act")
-        return
-    if epilogue == EPI_SWIGLU and (act != "silu" or bias is not None):
-        if bias is not None:
-            _cuda(bias)
-            _need(bias.dtype == torch.float32 and bias.numel() == 2 * N and bias.is_contiguous(), "gemm_tc: bias float32 [2N]")
-        _check(_lib.kernels().imparo_gemm_tc_gated(_ptr(x), x.stride(0), rows_alloc, _ptr(w), _ptr(out), out.stride(0), T, N, K,
-                                                   GATED_ACTIVATIONS[act], float(limit), _ptr(bias), _ptr(scratch), _ptr(cnt),
-                                                   _ptr(status), _stream()), "gemm_tc_gated")
-        return
-    _check(_lib.kernels().imparo_gemm_tc(_ptr(x), x.stride(0), rows_alloc, _ptr(w), _ptr(out), out.stride(0), T, N, K, epilogue,
-                                         _ptr(scratch), _ptr(cnt), _ptr(status), _stream()), "gemm_tc")
-
-
-# ---- tcgen05 product for prompt-sized batches (csrc/kernels/gemm_prefill.cu) ---------------------
-# From this many tokens on the persistent 128 x 256-tile kernel takes the product (below it, down to
-# TC_MAX_TOKENS, the library does): a tile holds 128 tokens, and its SwiGLU epilogue saves the
-# [T, 2F] intermediate only where the kernel also keeps up with the library on the product itself.
-
-
-def prefill_tc_min_tokens() -> int:
-    return _S.switches.prefill_tc_min_tokens
-
-
-def prefill_tc_usable(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False) -> bool:
-    """Whether gemm_prefill takes out (+)= x w^T: bfloat16 operands with 16-byte rows, an output whose rows
-    are 16-byte aligned groups, enough tokens, and the own product not switched off."""
-    if gemm_backend() != "tcgen05" or _S.switches.prefill_gemm != "tcgen05":
-        return False
-    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.shape[0] < prefill_tc_min_tokens():
-        return False
-    K = x.shape[1]
-    N = w.shape[0] // 2 if swiglu else w.shape[0]
-    group = 4 if out.dtype == torch.float32 else 8
-    return (K % 8 == 0 and x.stride(0) % 8 == 0 and x.stride(1) == 1 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and w.is_contiguous() and out.stride(1) == 1 and N % group == 0 and out.stride(0) % group == 0
-            and out.data_ptr() % 16 == 0 and out.dtype in (torch.float32, torch.bfloat16))
-
-
-def gemm_prefill(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, status: Optional[torch.Tensor] = None,
-                 act: str = "silu", limit: float = 0.0, bias: Optional[torch.Tensor] = None, plain: Optional[str] = None) -> None:
-    """The persistent tensor-core product for many tokens.  plain: with EPI_STORE_BF16, one of ACTIVATIONS applied to the product.
-    epilogue: EPI_STORE_BF16 | EPI_STORE_F32 |
-    EPI_ADD_F32 (out += x w^T) | EPI_SWIGLU (w = [gate rows; up rows], out = act(x gate^T + b_g, x up^T + b_u) with act one of
-    gated_act's kinds, "silu" by default, and bias float32 [2N] or None)."""
-    _need(x.is_cuda and w.is_cuda and out.is_cuda, "kernels run on CUDA tensors only (there is no CPU path)")
-    _need(epilogue in (EPI_STORE_BF16, EPI_STORE_F32, EPI_ADD_F32, EPI_SWIGLU), "gemm_prefill: unknown epilogue")
-    T, K = x.shape
-    N = w.shape[0] // 2 if epilogue == EPI_SWIGLU else w.shape[0]
-    _need(w.shape[1] == K and (epilogue != EPI_SWIGLU or w.shape[0] % 2 == 0), "gemm_prefill: weight shape")
-    _need(tuple(out.shape) == (T, N), f"gemm_prefill: out must be [{T}, {N}]")
-    want_dtype = torch.bfloat16 if epilogue in (EPI_STORE_BF16, EPI_SWIGLU) else torch.float32
-    _need(out.dtype == want_dtype, f"gemm_prefill: this epilogue writes {want_dtype}")
-    status = _status_word(x.device, status)
-    rows_alloc = (x.untyped_storage().nbytes() // x.element_size() - x.storage_offset()) // x.stride(0) if x.stride(0) else T
-    rows_alloc = max(T, min(rows_alloc, 1 << 30))
-    if bias is not None:
-        _cuda(bias)
-        _need(epilogue == EPI_SWIGLU and bias.dtype == torch.float32 and bias.numel() == 2 * N and bias.is_contiguous(),
-              "gemm_prefill: bias float32 [2N] with the gated epilogue")
-    _need(plain is None or epilogue == EPI_STORE_BF16, "gemm_prefill: a plain activation goes with the bfloat16 store")
-    kind = GATED_ACTIVATIONS[act] if plain is None else ACTIVATIONS[plain]
-    _check(_lib.kernels().imparo_gemm_prefill(_ptr(x), x.stride(0), rows_alloc, _ptr(w), _ptr(out), out.stride(0), T, N, K,
-                                              epilogue if plain is None else EPI_ACT_BF16, kind, float(limit), _ptr(bias), _ptr(status),
-                                              _stream()), "gemm_prefill")
-
-
-def linear_swiglu(x, w_gu: torch.Tensor, out: torch.Tensor, status: Optional[torch.Tensor] = None,
-                  tmp: Optional[torch.Tensor] = None) -> None:
-    """out[T, F] = silu(x gate^T) * (x up^T) with w_gu = [gate; up] of shape [2F, K].
-    bfloat16 on the tensor-core kernels (the weight streamer for few tokens, the persistent tile kernel for
-    many): one launch, the activation in the epilogue.  Otherwise: the product into tmp [T, 2F] (a tensor,
-    or a function that makes it, called only on this path), then the activation kernel."""
-    if x.dtype == torch.bfloat16 and gemm_backend() == "tcgen05" and tc_usable(x, w_gu):
-        gemm_tc(x, w_gu, out, EPI_SWIGLU, status)
-        return
-    if prefill_tc_usable(x, w_gu, out, swiglu=True):
-        gemm_prefill(x, w_gu, out, EPI_SWIGLU, status)
-        return
-    if callable(tmp):
-        tmp = tmp()
-    _need(tmp is not None and tmp.shape == (x.shape[0], w_gu.shape[0]), "linear_swiglu: tmp [T, 2F] needed on this path")
-    linear(x, w_gu, tmp, status=status)
-    swiglu_act(tmp, out)
-
-
-def linear_gated(x, w_gu: torch.Tensor, out: torch.Tensor, kind: str, limit: float = 0.0, bias: Optional[torch.Tensor] = None,
-                 status: Optional[torch.Tensor] = None, tmp=None) -> None:
-    """out[T, F] = act(x gate^T + b_g, x up^T + b_u) with w_gu = [gate; up] ([2F, K]), bias float32 [2F] or None, for the
-    gated activations of gated_act: the product into tmp [T, 2F] (a tensor, or a function that makes it), then one kernel
-    that adds the biases and applies the activation.  For many bfloat16 tokens: the persistent tensor-core product with the
-    biases and the activation in its epilogue (one launch, no [T, 2F] tensor); for few: the weight-streaming tensor-core
-    product with the same epilogue."""
-    if x.dtype == torch.bfloat16 and gemm_backend() == "tcgen05" and tc_usable(x, w_gu):
-        gemm_tc(x, w_gu, out, EPI_SWIGLU, status, act=kind, limit=limit, bias=bias)
-        return
-    if prefill_tc_usable(x, w_gu, out, swiglu=True):
-        gemm_prefill(x, w_gu, out, EPI_SWIGLU, status, act=kind, limit=limit, bias=bias)
-        return
-    if callable(tmp):
-        tmp = tmp()
-    _need(tmp is not None and tmp.shape == (x.shape[0], w_gu.shape[0]), "linear_gated: tmp [T, 2F] needed")
-    linear(x, w_gu, tmp, status=status)
-    gated_act(tmp, out, kind, limit, bias)
-
-
-def _partials_scratch(device, floats: int) -> torch.Tensor:
-    """Scratch for the split partials of a product whose reader folds them (one set at a time), at least `floats` long."""
-    key = torch.device(device).index or 0
-    buf = _S.partials.get(key)
-    if buf is None or buf.numel() < floats:
-        _need(not torch.cuda.is_current_stream_capturing(), "partials scratch would grow during graph capture")
-        _S.generation += 0 if buf is None else 1              # a buffer that did not exist is in no captured graph
-        buf = _S.partials[key] = torch.empty(_grown(floats, buf), dtype=torch.float32, device=device)
-    return buf
-
-
-def linear(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
-           status: Optional[torch.Tensor] = None) -> None:
     """out[M,N] (+)= x[M,K] @ w[N,K]^T.  float32 x/w -> true 32-bit (csrc/kernels/gemm_f32.cu: products of bfloat16 pieces that
     add up to the operands, FFMA where rows are no 16-byte groups); bfloat16 x/w -> tensor cores with 32-bit accumulation, out
     float32 or bfloat16.  w is a weight: its first tiles are read before the kernel ahead in the stream has ended.
