@@ -475,7 +475,7 @@ def test_state_space_products(heads, groups, N, vdim, lens):
 
 # enough CTAs (heads x chunks x value columns / 64) for two and for four heads per CTA: the builds a prompt of many heads takes.  Two:
 # 494 with heads per group no multiple of four; four: 832 and, over two and three blocks of value columns, 624 and 936
-@pytest.mark.parametrize("heads,groups,N,vdim", [(38, 1, 8, 4), (38, 1, 72, 4), (64, 1, 8, 4), (64, 2, 72, 4), (24, 3, 8, 68), (24, 3, 72, 132)])
+@pytest.mark.parametrize("heads,groups,N,vdim", [(38, 1, 8, 36), (38, 1, 72, 36), (64, 1, 8, 36), (64, 2, 72, 36), (24, 3, 8, 68), (24, 3, 72, 132)])
 def test_state_space_products_several_heads_per_cta(heads, groups, N, vdim):
     test_state_space_products(heads, groups, N, vdim, (700, 65))
 
