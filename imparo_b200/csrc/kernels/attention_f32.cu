@@ -1,9 +1,11 @@
 // Causal attention of prompt portions over the paged cache in 32-bit: tiles of 64 queries of one head against tiles of 64 keys.
 //
-// The split-key kernel (attention_split.cu) that took these rows reads every key for every query: 1,000 tokens in three portions
-// of 16 heads of 64 took 241 us with its combine.  Here a key is read once per 64 queries and both products run on patches of 8 x 4
-// in registers, so it is bound by the issue of 32-bit operations and, for few tiles, by the longest portion's last tile:
-// 96 us (B200; a warp per scheduler and CTA, so mostly latency).  Scores, softmax (expf, running maximum per row) and sums are 32-bit; keys are added tile by tile in order.
+// The split-key kernel (attention_split.cu) reads every key for every query: 1,000 tokens in three portions of 16 heads of 64 took
+// 241 us with its combine.  Here a key is read once per 64 queries and both products run on patches of 8 x 4 in registers, so it is
+// bound by the issue of 32-bit operations and, for few tiles, by the longest portion's last tile, whose CTA walks all of the
+// request's keys: 94 us (B200; a warp per scheduler and CTA, so mostly latency).  Few rows over many keys are the split-key kernel's
+// therefore (kernels/ops.py, attention_f32_tiles_pay).  Scores, softmax (expf, running maximum per row) and sums are 32-bit; keys are
+// added tile by tile in order.
 #include "common.cuh"
 #include <type_traits>
 

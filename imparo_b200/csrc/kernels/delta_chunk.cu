@@ -14,8 +14,8 @@
 // row (never a quotient, nor the exponential of a difference of long sums): a decay of zero needs no care, and the error is
 // the row walk's (tests compare both with 64 bits).
 //
-// B200, 8 heads of key size 64 and value size 128, 2,048 rows: 421 us for the row walk, 142 us for the three launches (local 45,
-// scan 60, out 22); error against 64 bits 1.1e-7 and 1.4e-7.
+// B200, 8 heads of key size 64 and value size 128, 2,048 rows: 421 us for the row walk, 141 us for the three launches (local 43,
+// scan 82, out 16); error against 64 bits 1.1e-7 and 1.4e-7.  Which portions come here: parts/delta_rule.py.
 //
 // A request's rows are cut into chunks from its portion's first row on, so the cut depends on the portion alone.
 #include "common.cuh"

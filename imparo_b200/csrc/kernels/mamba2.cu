@@ -12,7 +12,8 @@
 //      every chunk's own state from zero and its total decay (as a product of weighted B rows with x rows for states up
 //      to 128, else by walking the rows); a scan over each request's chunks that leaves every
 //      chunk's starting state and the request's new state; every chunk's outputs from its starting state plus the
-//      rows inside the chunk.  32-bit on CUDA cores.  (Sizes that are multiples of 4 run as products: mamba2_chunk.cu.)
+//      rows inside the chunk.  32-bit on CUDA cores.  (Sizes that are multiples of 4 run as products where
+//      these do less: mamba2_chunk.cu.)
 //  (4) gate_group_rmsnorm: y * silu(z), then an RMS norm over each of `groups` equal stretches of the row, times a
 //      weight.
 #include "conv_rows.cuh"

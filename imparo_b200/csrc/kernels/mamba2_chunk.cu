@@ -11,9 +11,10 @@
 //             state terms per entry.
 // Everything is 32-bit; a decay between two rows is the product of the rows' decays between them.
 //
-// Two launches walked the rows before (a state column per thread, 3 operations per row and state entry): with 32 heads of 64
+// Two launches walk the rows in mamba2.cu (a state column per thread, 3 operations per row and state entry): with 32 heads of 64
 // values, state size 64 and 1,999 rows 47 + 20 + 68 us (state, scan, out), here 18 + 7 + 42 (B200; bound by the latency of the
-// products' reads at 8 warps per SM).  Error against 64 bits 1.4e-7 and 1.7e-7.
+// products' reads at 8 warps per SM).  Error against 64 bits 1.4e-7 and 1.7e-7.  Which portions come here: parts/mamba2.py and
+// mamba2_products_pay in kernels/ops.py.
 #include "common.cuh"
 
 namespace imparo {
