@@ -480,9 +480,9 @@ def test_state_space_products_several_heads_per_cta(heads, groups, N, vdim):
     test_state_space_products(heads, groups, N, vdim, (700, 65))
 
 
-# one, two, four and eight 16-byte groups per thread, and beyond them the kernel without registers
+# one warp, two, eight; one, two, four and eight 16-byte groups per thread, and beyond them the kernel without registers
 @pytest.mark.parametrize("out_dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("per,groups", [(4, 3), (1024, 2), (1028, 2), (2048, 1), (2052, 2), (4096, 1), (4100, 1), (8192, 1), (8196, 1), (1030, 1)])
+@pytest.mark.parametrize("per,groups", [(4, 3), (128, 5), (132, 4), (1020, 1), (1024, 2), (1028, 2), (2048, 1), (2052, 2), (4096, 1), (4100, 1), (8192, 1), (8196, 1), (1030, 1)])
 def test_gated_norm_of_wide_stretches(per, groups, out_dtype):
     import torch
     from imparo_b200.kernels import ops
