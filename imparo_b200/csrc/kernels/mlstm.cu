@@ -29,7 +29,7 @@
 //               m' = max(b + m_in, m_loc), S' = exp(b + m_in - m') S_in + exp(m_loc - m') S_loc; the slot's S and n at the end
 //        out:   every chunk alone from its starting state: the outputs of its rows (the row walk of (1))
 //      The chunk walk is the same arithmetic as the row walk; results differ by the order of additions only.
-#include "common.cuh"
+#include "mlstm_chunk.cuh"
 
 namespace imparo {
 
@@ -402,6 +402,20 @@ extern "C" int imparo_mlstm_scan(const float* proj, long long stride, int q_off,
     c.proj = proj; c.stride = (size_t)stride;
     c.q_off = q_off; c.k_off = k_off; c.v_off = v_off; c.i_off = i_off; c.f_off = f_off;
     c.i_bias = i_bias; c.f_bias = f_bias; c.cap = cap; c.q_scale = q_scale;
+    if (chunk == MLSTM_PRODUCTS_CHUNK) {
+        const int vblocks = (vdim + 31) / 32, most = n_tok / chunk + n_items;
+        const MlstmProducts x{proj, (size_t)stride, q_off, k_off, v_off, i_off, f_off, i_bias, f_bias, cap, q_scale, item_row_start, item_slot,
+                              n_items, n_slots, heads, dim, vdim, vblocks, chunk_S, chunk_n, chunk_mb, state_m, out};
+        if (mlstm_products_take(x)) {
+            int rc = mlstm_products_local(x, most, stream);
+            if (rc) return rc;
+            const int entries = dim * vdim + vblocks * dim;
+            launch(mlstm_chunk_scan_kernel, dim3(n_items, heads, (entries + 255) / 256), dim3(256), 0, stream, chunk_S, chunk_n, chunk_mb, state_S,
+                   state_n, (const float*)state_m, item_row_start, item_slot, n_slots, chunk, heads, dim, vdim, vblocks, status);
+            IMPARO_CHECK_LAUNCH();
+            return mlstm_products_out(x, most, stream);
+        }
+    }
     if (dim <= 32)
         return mlstm_launch<32>(c, state_S, state_n, state_m, item_row_start, item_slot, n_slots, n_items, n_tok, out, heads, dim, vdim,
                                 chunk, chunk_S, chunk_n, chunk_mb, status, stream);

@@ -2245,6 +2245,11 @@ def mlstm_value_blocks(vdim: int) -> int:
     return (int(vdim) + 31) // 32
 
 
+def mlstm_products_take(proj: torch.Tensor, dim: int, vdim: int) -> bool:
+    """Whether chunks of 64 rows run as products (csrc/kernels/mlstm_chunk.cu; q, k and v at multiples of 4 columns of proj)."""
+    return dim % 4 == 0 and dim <= 128 and vdim % 4 == 0 and proj.stride(0) % 4 == 0 and proj.data_ptr() % 16 == 0
+
+
 def mlstm_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, i_off: int, f_off: int, i_bias: torch.Tensor,
                f_bias: torch.Tensor, cap: float, q_scale: float, state_S: torch.Tensor, state_n: torch.Tensor, state_m: torch.Tensor,
                item_row_start, item_slot, n_items: int, out: torch.Tensor, heads: int, dim: int, vdim: int, status: torch.Tensor,

@@ -81,7 +81,7 @@ class MatrixMemory(Part):
         self.w_in = view
 
     def forward(self, x, batch, caches, residual, accumulate=True, projected=None):
-        S, n, m = caches
+        S, n_, m = caches
         rt, T = self.rt, x.shape[0]
         ws = rt.workspace
         H = self.heads
@@ -93,24 +93,32 @@ class MatrixMemory(Part):
             proj = ws.get("mlstm_in", (T, self.w_in.shape[0]), torch.float32, first="tokens")
             ops.linear(x, self.w_in, proj, status=rt.status)
         o = ws.get("mlstm_o", (T, vv), torch.float32, first="tokens")
-        chunk, scratch = 0, None
+        def scan(first, n, chunk=0, scratch=None):             # requests [first, first + n)
+            ops.mlstm_scan(proj, 0, qk, 2 * qk, 2 * qk + 2 * vv, 2 * qk + 2 * vv + H, self.b_i, self.b_f, self.cap, self.dim ** -0.5,
+                           S.state, n_.state, m.state, batch.item_row_start[first:], batch.item_slot[first:], n, o, H, self.dim, self.vdim,
+                           rt.status, chunk=chunk, scratch=scratch)
         if batch.max_tokens_per_item >= self.CHUNK_FROM:
-            # long portions: chunks of rows side by side.  A chunk's CTA walks its rows one after the other, so the chunks are
+            # long portions: chunks of rows side by side.  As products where the sizes allow (the decode rows beside them walk);
+            # else a chunk's CTA walks its rows one after the other, and the chunks are
             # halved while they would leave SMs without a CTA (with several CTAs on an SM the walks share its issue slots
             # and shorter chunks only add to the scan: 123 against 134 us per layer at 2,048 tokens, 8 heads); the length
             # follows the step's totals alone (tokens, requests), which are part of its shape
             vb = ops.mlstm_value_blocks(self.vdim)
             chunk = self.CHUNK
+            products = ops.mlstm_products_take(proj, self.dim, self.vdim)
             per_cta = 128 if self.dim <= 64 else 64          # value columns a CTA of the recurrence covers
-            if (T // chunk + batch.n_items) * H * -(-self.vdim // per_cta) < ops.sm_count():
+            if not products and (T // chunk + batch.n_items) * H * -(-self.vdim // per_cta) < ops.sm_count():
                 chunk //= 2
             most = T // chunk + batch.n_items
             scratch = (ws.get("mlstm_chunk_S", (most * H * self.dim * self.vdim,), torch.float32),
                        ws.get("mlstm_chunk_n", (most * H * vb * self.dim,), torch.float32),
                        ws.get("mlstm_chunk_mb", (most * H * vb * 3,), torch.float32))
-        ops.mlstm_scan(proj, 0, qk, 2 * qk, 2 * qk + 2 * vv, 2 * qk + 2 * vv + H, self.b_i, self.b_f, self.cap, self.dim ** -0.5,
-                       S.state, n.state, m.state, batch.item_row_start, batch.item_slot, batch.n_items, o, H, self.dim, self.vdim,
-                       rt.status, chunk=chunk, scratch=scratch)
+            n1 = getattr(batch, "n_single", 0) if products else 0          # decode rows come first when the step also holds portions
+            if n1:
+                scan(0, n1)
+            scan(n1, batch.n_items - n1, chunk, scratch)
+        else:
+            scan(0, batch.n_items)
         y = ws.get("mlstm_y", (T, vv), rt.act_dtype, first="tokens")
         ops.head_norm_gate(o, self.w_norm, self.eps, proj[:, 2 * qk + vv:2 * qk + 2 * vv], y, H, self.vdim)
         ops.linear(y, self.w_o, residual, accumulate=accumulate, status=rt.status)
