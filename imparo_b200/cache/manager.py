@@ -13,6 +13,7 @@ Arena layout per group: K [entries, pages, page_size, kv_heads*head_dim] and V t
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
@@ -184,7 +185,8 @@ class CacheManager:
         # one launch for all state tensors (one fill each: 4 us of a step's stream per tensor)
         from ..kernels import ops
         slot = range(self.arena_slots)[slot]                       # (an index: IndexError beyond the slots there are)
-        with torch.cuda.device(self.state_arena.device):
+        device = self.state_arena.device
+        with torch.cuda.device(device) if torch.cuda.current_device() != device.index else contextlib.nullcontext():
             ops.zero_state_slots(self.state_arena, self.state_segments, self.n_state_segments, self._slot_numbers[slot:slot + 1],
                                  self.arena_slots, self.status, max_per_slot=self.state_max_per_slot)
 

@@ -10,7 +10,6 @@ state (lib.rs:1141-1145); the cache advances only after the step succeeded
 """
 from __future__ import annotations
 
-import array
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -18,6 +17,7 @@ import numpy as np
 import torch
 
 from ..cache import CacheFull, CacheManager
+from ..kernels import lib as _lib
 from ..kernels import ops
 from ..parts.model import Model
 from .scheduler import padded_rows
@@ -33,23 +33,45 @@ class StepItem:
 
 
 class StepBatch:
-    """The step's batch on the device.  All index arrays are int32."""
+    """The step's batch on the device.  All index arrays are int32.  The arrays are views into the step's one upload, made when the
+    first of them is asked for: a step that replays its captured graph asks for none (a view costs the host 1 to 2 us)."""
     __slots__ = ("n_tokens", "n_items", "token_ids", "positions", "item_of_token", "item_row_start",
                  "item_slot", "item_start_pos", "tables", "want_rows", "n_want", "max_tokens_per_item",
-                 "max_context", "decode_only", "host", "token_src", "n_single", "fresh_slots", "notes", "portions_from_start")
+                 "max_context", "decode_only", "host", "token_src", "n_single", "fresh_slots", "notes", "portions_from_start", "_layout")
+    _VIEWS = frozenset(("token_ids", "positions", "item_of_token", "item_row_start", "item_slot", "item_start_pos", "want_rows", "tables",
+                        "token_src", "fresh_slots"))
+
+    def __getattr__(self, name):                 # (only where the slot is empty)
+        if name not in self._VIEWS:
+            raise AttributeError(name)
+        d, offs, strides, fresh = self._layout
+        T, R, W, ng = self.n_tokens, self.n_items, self.n_want, len(strides)
+        self.token_ids, self.positions, self.item_of_token = (d[offs[i]:offs[i] + T] for i in range(3))
+        self.item_row_start = d[offs[3]:offs[3] + R + 1]
+        self.item_slot = d[offs[4]:offs[4] + R]
+        self.item_start_pos = d[offs[5]:offs[5] + R]
+        self.want_rows = d[offs[6]:offs[6] + max(W, 1)]
+        self.tables = [d[offs[7 + g]:offs[7 + g] + R * strides[g]].view(R, strides[g]) for g in range(ng)]
+        self.token_src = d[offs[7 + ng]:offs[7 + ng] + T]
+        self.fresh_slots = d[offs[8 + ng]:offs[8 + ng] + R] if fresh else None
+        return getattr(self, name)
 
 
 def int_array(values) -> Optional[np.ndarray]:
-    """Whole numbers as a 64-bit array: integer arrays, and lists, tuples and ranges of integers (2,000 of them in 33 us, where
-    numpy's own conversion takes 56).  None for anything else, also for numbers beyond 64 bits, floats and sets: a caller then goes
-    through them one by one."""
+    """Whole numbers as a 64-bit array: integer arrays, and lists, tuples and ranges of integers (a list of 2,000 in 15 us by the
+    native reader, where an array.array takes 34 and numpy's own conversion about 60).  None for anything else, also for numbers beyond 64
+    bits, floats and sets: a caller then goes through them one by one."""
     if isinstance(values, np.ndarray):
         return values.astype(np.int64, copy=False) if values.ndim == 1 and values.dtype.kind in "iu" else None
-    if isinstance(values, (list, tuple, range)) and values:
+    if isinstance(values, range) and values:
         try:
-            return np.frombuffer(array.array("q", values), dtype=np.int64)
-        except (TypeError, OverflowError):
-            pass
+            return np.arange(values.start, values.stop, values.step, dtype=np.int64)
+        except OverflowError:
+            return None
+    if isinstance(values, (list, tuple)) and values:
+        out = np.empty(len(values), dtype=np.int64)
+        if _lib.host_objects().imparo_int_sequence(values, isinstance(values, tuple), len(values), out.ctypes.data) == 0:
+            return out
     return None
 
 
@@ -96,13 +118,16 @@ class StepFunction:
         self._cap = 0
 
     # -- the batch descriptor -------------------------------------------------------------
-    def _host_buffer(self, n_ints: int) -> torch.Tensor:
-        """A pinned host buffer no copy is still reading: a ring of four, each guarded by
+    def _host_buffer(self, n_ints: int):
+        """A pinned host buffer no copy is still reading, and the same as an array: a ring of four, each guarded by
         the event recorded after its last upload."""
         if n_ints > self._cap:
             cap = max(n_ints, 2 * self._cap, 4096)
             torch.cuda.current_stream().synchronize()
-            self._ring = [[torch.empty(cap, dtype=torch.int32, pin_memory=True), None] for _ in range(4)]
+            self._ring = []
+            for _ in range(4):                       # the buffer, the event of its last copy, the same memory as an array
+                buf = torch.empty(cap, dtype=torch.int32, pin_memory=True)
+                self._ring.append([buf, None, buf.numpy()])
             self._dev = torch.empty(cap, dtype=torch.int32, device=self.device)
             self._cap = cap
             self._graphs.clear()     # captured graphs hold the old buffer's address
@@ -110,7 +135,7 @@ class StepFunction:
         slot = self._ring[self._turn]
         if slot[1] is not None:
             slot[1].synchronize()
-        return slot[0]
+        return slot[0], slot[2]
 
     def reserve(self, tokens: int, rows: int, pages_per_request: int) -> None:
         """Make the descriptor buffers for the largest step now (they move, and captured graphs with them, whenever
@@ -172,9 +197,10 @@ class StepFunction:
         # the last array (one source index per token, -1 = the id the host wrote) is there in every
         # step, so that the layout depends on the step's totals only
         sizes = [T, T, T, R + 1, R, R, max(W, 1)] + [R * s for s in strides] + [T, R]
-        offs = np.concatenate([[0], np.cumsum([_round_up(s, 4) for s in sizes])])
-        host = self._host_buffer(int(offs[-1]))
-        h = host.numpy()
+        offs = [0]
+        for s in sizes:
+            offs.append(offs[-1] + _round_up(s, 4))
+        host, h = self._host_buffer(offs[-1])
         tok, pos, iot = (h[offs[i]:offs[i] + T] for i in range(3))
         row_start = h[offs[3]:offs[3] + R + 1]
         slot = h[offs[4]:offs[4] + R]
@@ -189,7 +215,8 @@ class StepFunction:
                 continue
             n = len(it.tokens)
             start = cache.cached(it.request)
-            tok[t:t + n] = np.asarray(it.tokens, dtype=np.int64)
+            ids = int_array(it.tokens) if n > 8 else None
+            tok[t:t + n] = np.asarray(it.tokens, dtype=np.int64) if ids is None else ids
             pos[t:t + n] = np.arange(start, start + n, dtype=np.int32)
             iot[t:t + n] = i
             row_start[i] = t
@@ -203,10 +230,10 @@ class StepFunction:
             base = int(row_start[place[j_item]])
             places = int_array(it.want) if len(it.want) > 8 else None
             if places is not None:                       # many: at once (a loop costs 0.12 us per place)
-                outside = (places < 0) | (places >= n)
-                if outside.any():
+                if places.min() < 0 or places.max() >= n:
+                    outside = (places < 0) | (places >= n)
                     raise ValueError(f"request {it.request}: wanted place {places[outside.argmax()]} is not among its {n} tokens")
-                want[w:w + len(places)] = base + places
+                np.add(places, base, out=want[w:w + len(places)], casting="unsafe")
                 w += len(places)
                 continue
             for j in it.want:
@@ -235,25 +262,18 @@ class StepFunction:
         fresh = [int(slot[i]) for i in range(R) if start_pos[i] == 0 and items[i] is not None]
         fresh_at = offs[8 + ng]
         h[fresh_at:fresh_at + R] = (fresh + [-1] * (R - len(fresh))) if fresh else -1
-        n_ints = int(offs[-1])
+        n_ints = offs[-1]
         self.last_h2d_bytes = n_ints * 4
         self._dev[:n_ints].copy_(host[:n_ints], non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-        self._ring[self._turn][1] = ev
-        d = self._dev
+        used = self._ring[self._turn]
+        if used[1] is None:
+            used[1] = torch.cuda.Event()
+        used[1].record()                         # (its last use has been waited for: _host_buffer)
         b = StepBatch()
         b.notes = {}            # what one part leaves for a later part of the same step (tensors of this step's rows)
         b.n_tokens, b.n_items, b.n_want = T, R, W
-        b.token_ids, b.positions, b.item_of_token = (d[offs[i]:offs[i] + T] for i in range(3))
-        b.item_row_start = d[offs[3]:offs[3] + R + 1]
-        b.item_slot = d[offs[4]:offs[4] + R]
-        b.item_start_pos = d[offs[5]:offs[5] + R]
-        b.want_rows = d[offs[6]:offs[6] + max(W, 1)]
-        b.tables = [d[offs[7 + g]:offs[7 + g] + R * strides[g]].view(R, strides[g]) for g in range(ng)]
-        b.token_src = d[offs[7 + ng]:offs[7 + ng] + T]
+        b._layout = (self._dev, offs, strides, bool(fresh))
         b.n_single = n_single
-        b.fresh_slots = d[fresh_at:fresh_at + R] if fresh else None
         # The longest portion, rounded up to a power of two: launches may depend on it (which attention kernel takes
         # the step; how far back a request's cache rows are surely older than this step), and as an upper bound it
         # serves every step whose longest portion is no longer, so that steps of a continuous batch, whose longest

@@ -14,6 +14,7 @@ from . import build
 _lock = threading.Lock()
 _kernels = None
 _host = None
+_host_objects = None
 
 P = c_void_p
 I = c_int
@@ -44,6 +45,19 @@ def kernels():
                 _declare_kernels(lib)
                 _kernels = lib
     return _kernels
+
+
+def host_objects():
+    """The host library's functions that take Python objects (called with the interpreter's lock held)."""
+    global _host_objects
+    if _host_objects is None:
+        host()
+        with _lock:
+            if _host_objects is None:
+                lib = ctypes.PyDLL(build.build_host())
+                _declare(lib, "imparo_int_sequence", [ctypes.py_object, c_int, c_int64, c_void_p])
+                _host_objects = lib
+    return _host_objects
 
 
 def host():
