@@ -79,6 +79,7 @@ class LaunchState:
         self.pending_mean = {}       # data_ptr -> arguments of a norm_mean_add the next reader of the stream carries out
         self.pending_mix = {}        # data_ptr -> arguments of a streams_mix_add the next reader of the stream carries out
         self.pending_gnorm = {}      # data_ptr -> arguments of a group_norm_add the next reader of the stream carries out
+        self.waiting_norms = {}      # data_ptr of a norm's output -> (stream, weight, eps): not made, the products that read it norm themselves
         self.unfinished = {}         # data_ptr of an output buffer whose reader finishes it -> [partials or None, bias or None]
         self.partials = {}           # device index -> scratch of products into the stream
         self.consumer_parts = {}     # device index -> scratch of products a consumer kernel folds
@@ -176,6 +177,7 @@ def embed_gather(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, stat
     _S.pending_mix.pop(out.data_ptr(), None)
     _S.pending_gnorm.pop(out.data_ptr(), None)
     _S.unfinished.clear()
+    _S.waiting_norms.clear()
     n, width = out.shape
     _need(ids.dtype == torch.int32 and ids.numel() >= n, "ids must be int32, one per output row")
     _need(out.dtype == torch.float32 and table.shape[1] == width, "embedding output is float32 [tokens, width]")
@@ -209,7 +211,8 @@ def prepare(device, rows: int = 8) -> None:
         # shared-memory attributes and the cluster plan's occupancy table (a query the runtime refuses under capture)
         with torch.cuda.device(device):
             _check(_lib.kernels().imparo_gemm_tc_configure(), "gemm_tc_configure")
-        COUNTS["own"] -= 1           # nothing was launched
+            _check(_lib.kernels().imparo_gemm_rows_configure(), "gemm_rows_configure")
+        COUNTS["own"] -= 2           # nothing was launched
         _tc_configured = True
     if key not in _S.partials:
         _S.partials[key] = torch.empty(_grown(0, None), dtype=torch.float32, device=device)
@@ -344,8 +347,18 @@ def _group_norm_add(x, args, nw=None, neps=0.0, out=None) -> None:
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor,
-            rows: Optional[torch.Tensor] = None) -> None:
+            rows: Optional[torch.Tensor] = None, may_wait: bool = False) -> None:
+    """out = x (or its rows `rows`) over its root mean square, times w.  may_wait: the caller promises that out is read by ops.linear,
+    linear_unfolded, linear_swiglu, linear_gated and linear_conv_rows only, before x changes: with few rows nothing is launched
+    then, and those products norm the stream themselves."""
     _cuda(x, w, out, rows)
+    _S.waiting_norms.pop(out.data_ptr(), None)
+    if (may_wait and rows is None and x.data_ptr() not in _S.pending and x.data_ptr() not in _S.pending_mean
+            and x.data_ptr() not in _S.pending_gnorm and x.data_ptr() not in _S.pending_mix and out.dtype == torch.bfloat16
+            and x.dtype == torch.float32 and w.dtype == torch.float32 and out.shape == x.shape and w.numel() == x.shape[1]
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and _few_rows(x.shape[0], x.shape[1], True)):
+        _S.waiting_norms[out.data_ptr()] = (x, w, float(eps), out)          # (out: its address stays its own while the entry is there)
+        return
     pm = _S.pending_mean.get(x.data_ptr())
     if pm is not None:
         if rows is None and out.shape == x.shape and w.numel() == x.shape[1] and w.dtype == torch.float32:
@@ -610,12 +623,97 @@ def gemm_prefill(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
                                               _stream()), "gemm_prefill")
 
 
+# ---- products of at most eight rows (csrc/kernels/gemm_rows.cu) -----------------------------------
+ROWS_BF16, ROWS_F32, ROWS_ADD, ROWS_GATED = 0, 1, 2, 3
+_rows_plans = {}
+
+
+def _few_rows(T: int, K: int, norm: bool) -> bool:
+    """Whether the few-rows product takes rows of K entries (of the stream, if norm) from T tokens."""
+    return T <= 8 and K % 64 == 0 and (not norm or K <= 2048) and _S.switches.few_rows and gemm_backend() == "tcgen05" and tc_max_tokens() >= T
+
+
+def _rows_take(x: torch.Tensor, w: torch.Tensor, parts: int = 1) -> bool:
+    """Whether the few-rows product takes x w^T, w [parts * F, K]: a question of shape and alignment only."""
+    T, K = x.shape
+    wait = x.data_ptr() in _S.waiting_norms
+    if not (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and _few_rows(T, K, wait) and w.is_contiguous()
+            and w.data_ptr() % 16 == 0 and (wait or (x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and x.stride(1) == 1))):
+        return False
+    key = (T, w.shape[0], K, parts, wait)
+    takes = _rows_plans.get(key)
+    if takes is None:
+        takes = _rows_plans[key] = bool(_lib.kernels().imparo_gemm_rows_takes(T, w.shape[0] // parts, K, parts, int(wait), sm_count()))
+    return takes
+
+
+def _rows_input(x: torch.Tensor):
+    """(tensor, row stride, norm weight or None, eps): what the product reads for its input x, the stream where x is a norm that waits."""
+    waiting = _S.waiting_norms.get(x.data_ptr())
+    if waiting is None:
+        return x, x.stride(0), None, 0.0
+    return waiting[0], waiting[0].shape[1], waiting[1], waiting[2]
+
+
+def combine_apart(T: int, w_out: torch.Tensor) -> bool:
+    """Whether the attention's output product of T decode rows is faster with the combine of the key chunks as a kernel of its own:
+    where the few-rows product takes it, which leaves the stream whole, so that the norm behind it need not be a kernel."""
+    return w_out.dtype == torch.bfloat16 and _few_rows(T, w_out.shape[1], False)
+
+
+def forget_waiting(x: torch.Tensor) -> None:
+    """x's readers are done: a norm that waited for them is not made any more."""
+    _S.waiting_norms.pop(x.data_ptr(), None)
+
+
+def make_waiting(x: torch.Tensor) -> None:
+    """Make the norm whose output x is, if it was left to the products that read it."""
+    waiting = _S.waiting_norms.pop(x.data_ptr(), None)
+    if waiting is not None:
+        rmsnorm(waiting[0], waiting[1], waiting[2], x)
+
+
+def _gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: int, parts: int = 1, act: str = "silu", limit: float = 0.0,
+               bias: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None) -> None:
+    src, ld, norm, eps = _rows_input(x)
+    T, K = x.shape
+    _check(_lib.kernels().imparo_gemm_rows(_ptr(src), ld, _ptr(norm), eps, _ptr(w), _ptr(out), out.stride(0), T, w.shape[0] // parts, K,
+                                           kind, GATED_ACTIVATIONS[act], float(limit), _ptr(bias), _ptr(_status_word(x.device, status)), _stream()),
+           "gemm_rows")
+
+
+def linear_conv_rows(x: torch.Tensor, w: torch.Tensor, taps_w: torch.Tensor, bias: Optional[torch.Tensor], state: torch.Tensor,
+                     item_of_token: torch.Tensor, item_slot: torch.Tensor, y: torch.Tensor, taps: int, status: torch.Tensor) -> bool:
+    """linear_unfolded and gated_conv in one kernel for a step of one-token rows (every token its request's only one): y [T, F] from
+    x [T, K] and w [3F, K].  False, having launched nothing, when the kernel does not take the case."""
+    F = w.shape[0] // 3
+    if not (2 <= taps <= 4 and y.dtype == torch.bfloat16 and _rows_take(x, w, parts=3)):
+        return False
+    _cuda(w, taps_w, bias, state, item_of_token, item_slot, y, status)
+    T = x.shape[0]
+    _need(w.shape == (3 * F, x.shape[1]) and y.shape == (T, F), "linear_conv_rows: w [3F, K], y [tokens, F]")
+    _need(taps_w.dtype == torch.float32 and taps_w.shape == (F, taps), "linear_conv_rows: taps must be float32 [F, taps]")
+    _need(state.dtype == torch.float32 and state.dim() == 3 and state.shape[1:] == (taps - 1, F),
+          "linear_conv_rows: state must be float32 [slots, taps-1, F]")
+    _need(bias is None or (bias.dtype == torch.float32 and bias.numel() == F), "linear_conv_rows: bias must be float32 [F]")
+    src, ld, norm, eps = _rows_input(x)
+    _check(_lib.kernels().imparo_gemm_rows_conv(_ptr(src), ld, _ptr(norm), eps, _ptr(w), _ptr(taps_w), _ptr(bias), _ptr(state),
+                                                _ptr(item_of_token), _ptr(item_slot), _ptr(y), T, F, x.shape[1], taps, state.shape[0],
+                                                _ptr(status), _stream()), "gemm_rows_conv")
+    return True
+
+
 def linear_swiglu(x, w_gu: torch.Tensor, out: torch.Tensor, status: Optional[torch.Tensor] = None,
                   tmp: Optional[torch.Tensor] = None) -> None:
     """out[T, F] = silu(x gate^T) * (x up^T) with w_gu = [gate; up] of shape [2F, K].
     bfloat16 on the tensor-core kernels (the weight streamer for few tokens, the persistent tile kernel for
     many): one launch, the activation in the epilogue.  Otherwise: the product into tmp [T, 2F] (a tensor,
     or a function that makes it, called only on this path), then the activation kernel."""
+    if out.dtype == torch.bfloat16 and _rows_take(x, w_gu, parts=2):
+        _need(out.shape == (x.shape[0], w_gu.shape[0] // 2) and w_gu.shape[1] == x.shape[1] and out.stride(1) == 1, "linear_swiglu: shapes")
+        _gemm_rows(x, w_gu, out, ROWS_GATED, parts=2, status=status)
+        return
+    make_waiting(x)
     if x.dtype == torch.bfloat16 and gemm_backend() == "tcgen05" and tc_usable(x, w_gu):
         gemm_tc(x, w_gu, out, EPI_SWIGLU, status)
         return
@@ -636,6 +734,14 @@ def linear_gated(x, w_gu: torch.Tensor, out: torch.Tensor, kind: str, limit: flo
     that adds the biases and applies the activation.  For many bfloat16 tokens: the persistent tensor-core product with the
     biases and the activation in its epilogue (one launch, no [T, 2F] tensor); for few: the weight-streaming tensor-core
     product with the same epilogue."""
+    if out.dtype == torch.bfloat16 and _rows_take(x, w_gu, parts=2):
+        _need(out.shape == (x.shape[0], w_gu.shape[0] // 2) and w_gu.shape[1] == x.shape[1] and out.stride(1) == 1, "linear_gated: shapes")
+        if bias is not None:
+            _cuda(bias)
+            _need(bias.dtype == torch.float32 and bias.numel() == w_gu.shape[0], "linear_gated: bias float32 [2F]")
+        _gemm_rows(x, w_gu, out, ROWS_GATED, parts=2, act=kind, limit=limit, bias=bias, status=status)
+        return
+    make_waiting(x)
     if x.dtype == torch.bfloat16 and gemm_backend() == "tcgen05" and tc_usable(x, w_gu):
         gemm_tc(x, w_gu, out, EPI_SWIGLU, status, act=kind, limit=limit, bias=bias)
         return
@@ -681,6 +787,12 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
                                               _ptr(_status_word(x.device, status)), _stream()), "sgemm_nt")
     elif x.dtype == torch.bfloat16:
         _need(not accumulate or out.dtype == torch.float32, "linear: accumulate needs a float32 output")
+        if out.dtype in _DT and _rows_take(x, w):
+            if accumulate:
+                settle(out)
+            _gemm_rows(x, w, out, ROWS_ADD if accumulate else ROWS_F32 if out.dtype == torch.float32 else ROWS_BF16, status=status)
+            return
+        make_waiting(x)
         if gemm_backend() == "tcgen05" and tc_usable(x, w):
             epi = EPI_ADD_F32 if accumulate else (EPI_STORE_F32 if out.dtype == torch.float32 else EPI_STORE_BF16)
             u = _S.unfinished.get(out.data_ptr()) if not accumulate else None
@@ -759,18 +871,24 @@ def linear_unfolded(x, w: torch.Tensor, out: torch.Tensor, status: Optional[torc
     PartialProduct: each split's CTAs store their tile and are done, with no fold across CTAs inside
     the product, and the consumer adds the splits while it reads."""
     if unfolded_products() and x.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32) and out.is_contiguous() \
-            and gemm_backend() == "tcgen05" and tc_usable(x, w):
+            and gemm_backend() == "tcgen05" and (tc_usable(x, w) or x.data_ptr() in _S.waiting_norms):
         M, K = x.shape
         N = w.shape[0]
-        nt, splits, floats, _ = _tc_plan(M, N, K, EPI_PARTIAL)
-        if splits > 1:
+        whole = x.data_ptr() in _S.waiting_norms and w.shape[1] == K and _rows_take(x, w)    # K is not cut: one part, the product
+        splits, floats = (1, M * N) if whole else _tc_plan(M, N, K, EPI_PARTIAL)[1:3]
+        if splits > 1 or whole:
             key = torch.device(x.device).index or 0
             buf = _S.consumer_parts.get(key)
             if buf is None or buf.numel() < floats:
                 _need(not torch.cuda.is_current_stream_capturing(), "partials scratch would grow during graph capture")
                 _S.generation += 0 if buf is None else 1
                 buf = _S.consumer_parts[key] = torch.empty(_grown(floats, buf), dtype=torch.float32, device=x.device)
-            gemm_tc(x, w, out, EPI_PARTIAL, status, scratch=buf)
+            if whole:
+                _need(out.shape == (M, N), "linear_unfolded: out must be [tokens, N]")
+                _gemm_rows(x, w, buf[:M * N].view(M, N), ROWS_F32, status=status)
+            else:
+                make_waiting(x)
+                gemm_tc(x, w, out, EPI_PARTIAL, status, scratch=buf)
             return PartialProduct(buf, splits, (M, N), out)
     linear(x, w, out, status=status)
     return out

@@ -47,6 +47,7 @@ class AttentionMixer(Part):
     forward(..., accumulate=False) overwrites `residual` (then any float32 [tokens, hidden] buffer) instead of adding
     into it: a mixer that runs beside others hands its output to whoever combines them."""
     adds_with_linear = True
+    input_by_products = True
 
 
     NAMES = {"q": "self_attn.q_proj.weight", "k": "self_attn.k_proj.weight", "v": "self_attn.v_proj.weight",
@@ -318,7 +319,7 @@ class AttentionMixer(Part):
                 # decode rows: the output product combines the partial results while it makes its operand, unless a fixed sink,
                 # a gate or a bias comes between
                 in_product = (batch.decode_only and n_splits <= 64 and ops.fuse_producers() and self.b_o is None and not self.gate
-                              and (not self.sink or self.sinks is not None))
+                              and not (accumulate and ops.combine_apart(T, self.w_o)) and (not self.sink or self.sinks is not None))
                 done = ops.paged_attention_split(q[:n], kv.k, kv.v, batch.positions[:n], batch.item_of_token[:n], table,
                                                  kv.page_size, kv.n_pages, self.window, self.scale, None if in_product else out[:n],
                                                  part_acc, part_ml, chunk, n_splits, nh, self.nkv, hd, rt.status,
@@ -357,7 +358,7 @@ class AttentionMixer(Part):
         room = self._partials_room(table.shape[1] * kv.page_size)
         part_acc = rt.workspace.get("attn_part_acc", (T * nh * n_splits * hd,), torch.float32, reserve=room * hd)
         part_ml = rt.workspace.get("attn_part_ml", (T * nh * n_splits * 2,), torch.float32, reserve=room * 2)
-        in_product = ops.fuse_producers() and self.b_o is None
+        in_product = ops.fuse_producers() and self.b_o is None and not (accumulate and ops.combine_apart(T, self.w_o))
         out = rt.workspace.get("attn_out", (T, nh * hd), rt.act_dtype, first="tokens")
         if not ops.attention_decode_from_qkv(qkv, batch.positions, batch.item_of_token, None, None, inv_freq, n_rot, 0.0, kv.k, kv.v, table,
                                              kv.page_size, kv.n_pages, self.window, self.scale, None if in_product else out, part_acc,
@@ -394,7 +395,8 @@ class AttentionMixer(Part):
         room = rows * nh * n_splits if len(spans) > 1 else self._partials_room(spans[0])
         part_acc = rt.workspace.get("attn_part_acc", (n * nh * n_splits * vd,), torch.float32, reserve=room * vd)
         part_ml = rt.workspace.get("attn_part_ml", (n * nh * n_splits * 2,), torch.float32, reserve=room * 2)
-        in_product = batch.decode_only and n == T and n_splits <= 64 and ops.fuse_producers() and self.b_o is None and not self.gate
+        in_product = (batch.decode_only and n == T and n_splits <= 64 and ops.fuse_producers() and self.b_o is None and not self.gate
+                      and not (accumulate and ops.combine_apart(T, self.w_o)))
         if not ops.attention_sigmoid_split(q[:n], kv.k, kv.v, batch.positions[:n], batch.item_of_token[:n], table, kv.page_size,
                                            kv.n_pages, self.window, self.chunk, self.scale, self.score_bias,
                                            None if in_product else out[:n], part_acc, part_ml, range_, n_splits, nh, self.nkv, hd, vd,
@@ -436,7 +438,8 @@ class AttentionMixer(Part):
             room = self._partials_room(table.shape[1] * kv.page_size)
             part_acc = rt.workspace.get("attn_part_acc", (T * nh * n_splits * hd,), torch.float32, reserve=room * hd)
             part_ml = rt.workspace.get("attn_part_ml", (T * nh * n_splits * 2,), torch.float32, reserve=room * 2)
-            in_product = n_splits <= 64 and ops.fuse_producers()          # the output product combines the partials while it makes its operand
+            # the output product combines the partials while it makes its operand
+            in_product = n_splits <= 64 and ops.fuse_producers() and not ops.combine_apart(T, self.w_o)
             # every key chunk's CTA makes the group's queries again: worth the q/k kernel it saves up to 16 chunks or so
             # (batch 8: 0.846 against 0.851 ms per step at 2,560 positions, equal at 16 k, 1.44-1.52 against 1.34-1.36 at 32 k)
             if n_splits <= 16 and ops.attention_decode_from_qkv(qkv, batch.positions, batch.item_of_token, self.q_norm, self.k_norm, inv_freq,
@@ -496,7 +499,8 @@ class AttentionMixer(Part):
             room = self._partials_room(table.shape[1] * kv.page_size)
             part_acc = rt.workspace.get("attn_part_acc", (T * nh * n_splits * hd,), torch.float32, reserve=room * hd)
             part_ml = rt.workspace.get("attn_part_ml", (T * nh * n_splits * 2,), torch.float32, reserve=room * 2)
-            if batch.decode_only and rt.act_dtype == torch.bfloat16 and n_splits <= 64 and ops.fuse_producers():
+            if (batch.decode_only and rt.act_dtype == torch.bfloat16 and n_splits <= 64 and ops.fuse_producers()
+                    and not ops.combine_apart(T, self.w_o)):
                 # decode rows: the partial results stay as they are and the output product combines them while it
                 # makes its token operand; no combine kernel and no tensor between the two
                 ops.paged_attention_split(q, kv.k, kv.v, batch.positions, batch.item_of_token, table, kv.page_size,

@@ -127,6 +127,9 @@ class Part:
     # (ops.add_bias after it is fine): that add may then stay split partials that the next norm folds in
     # (ops.allow_deferred_add).  A part that writes the residual any other way keeps False.
     adds_with_linear = False
+    # Its input is read by products of ops (linear, linear_unfolded, linear_swiglu, linear_gated, linear_conv_rows) and nothing else:
+    # the norm before it may then be left to them (ops.rmsnorm(may_wait=True)).
+    input_by_products = False
 
     def __init__(self, params: dict, prefix: str, rt: Runtime):
         self.params = dict(params)

@@ -49,8 +49,9 @@ class PreNormResidualBlock(Block):
         from ..kernels import ops
         if self.rt.probe_now:
             return self._forward_probed(x, batch, caches, only_rows)
-        h = self.mixer_norm.forward(x, tag="normed_mixer")
+        h = self.mixer_norm.forward(x, tag="normed_mixer", **({"may_wait": True} if self.mixer.input_by_products else {}))
         self._run(self.mixer, x, lambda: self.mixer.forward(h, batch, caches, x))
+        ops.forget_waiting(h)
         if only_rows is not None:
             rows, n = only_rows
             if n == 0:
@@ -68,7 +69,7 @@ class PreNormResidualBlock(Block):
         from ..kernels import ops
         copy = None
         if self.ff is not None:
-            ff_in = self.ff_norm.forward(x, tag="normed_ff")
+            ff_in = self.ff_norm.forward(x, tag="normed_ff", **({"may_wait": True} if self.ff.input_by_products and not probe else {}))
             if probe:
                 probe("ff_norm", ff_in)
             kw = {"accumulate": True} if self._ff_accumulates else {}
@@ -80,6 +81,7 @@ class PreNormResidualBlock(Block):
                 ops.settle(x)
             else:
                 self._run(self.ff, x, lambda: self.ff.forward(ff_in, batch, x, **kw))
+                ops.forget_waiting(ff_in)
         if self.after is not None:
             self.after.forward(x, batch, rows=rows, **({"copy": copy} if copy is not None else {}))
 

@@ -17,6 +17,7 @@ class SwiGLU(Part):
     product).  forward(..., accumulate=False) overwrites `residual` (then any float32 [tokens, hidden] buffer) instead of
     adding into it."""
     adds_with_linear = True
+    input_by_products = True
 
 
     NAMES = {"gate": "feed_forward.w1.weight", "up": "feed_forward.w3.weight", "down": "feed_forward.w2.weight",

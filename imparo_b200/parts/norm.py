@@ -51,9 +51,10 @@ class RMSNorm(Part):
             self.coef = tensors[self.coef_name]
 
     def forward(self, x: torch.Tensor, rows: Optional[torch.Tensor] = None, n_rows: Optional[int] = None,
-                tag: str = "normed") -> torch.Tensor:
+                tag: str = "normed", may_wait: bool = False) -> torch.Tensor:
         """x: 32-bit [tokens, width].  rows (int32, device) picks input rows; n_rows is how
-        many of them.  Returns activations in the path's dtype."""
+        many of them.  Returns activations in the path's dtype.  may_wait: their reader takes them through products only
+        (Part.input_by_products), which may then make the norm themselves."""
         n = x.shape[0] if rows is None else int(n_rows if n_rows is not None else rows.numel())
         out = self.rt.workspace.get(tag, (n, self.width), self.rt.act_dtype, first="tokens" if rows is None else "rows")
         if self.by_copies:
@@ -61,5 +62,5 @@ class RMSNorm(Part):
         elif self.groups:
             ops.group_rmsnorm(x, self.weight, self.eps, self.groups, out, rows)
         else:
-            ops.rmsnorm(x, self.weight, self.eps, out, rows)
+            ops.rmsnorm(x, self.weight, self.eps, out, rows, may_wait=may_wait)
         return out

@@ -13,6 +13,7 @@ from .spec import SlotState, WeightSpec
 class ShortConvMixer(Part):
     """params: hidden, taps, bias (bool), names (optional)."""
     adds_with_linear = True
+    input_by_products = True
 
 
     NAMES = {"in": "conv.in_proj.weight", "conv": "conv.conv.weight", "out": "conv.out_proj.weight",
@@ -54,13 +55,19 @@ class ShortConvMixer(Part):
     def forward(self, x, batch, caches, residual):
         st = caches[0]
         rt, T, H = self.rt, x.shape[0], self.hidden
+        y = rt.workspace.get("conv_y", (T, H), rt.act_dtype, first="tokens")
+        if batch.decode_only and self.b_in is None and ops.linear_conv_rows(x, self.w_in, self.w_conv, self.b_conv, st.state, batch.item_of_token,
+                                                                            batch.item_slot, y, self.taps, rt.status):
+            ops.linear(y, self.w_out, residual, accumulate=True, status=rt.status)
+            if self.b_out is not None:
+                ops.add_bias(residual, self.b_out)
+            return
         bcx = rt.workspace.get("conv_bcx", (T, 3 * H), rt.act_dtype, first="tokens")
         if self.b_in is None:
             bcx = ops.linear_unfolded(x, self.w_in, bcx, status=rt.status)     # the conv kernel can add split partials itself
         else:
             ops.linear(x, self.w_in, bcx, status=rt.status)
             ops.add_bias(bcx, self.b_in)
-        y = rt.workspace.get("conv_y", (T, H), rt.act_dtype, first="tokens")
         ops.gated_conv(bcx, self.w_conv, self.b_conv, st.state, batch.item_row_start, batch.item_of_token,
                        batch.item_slot, y, self.taps, rt.status)
         ops.linear(y, self.w_out, residual, accumulate=True, status=rt.status)
