@@ -86,13 +86,14 @@ using namespace imparo::tc;
 
 constexpr int TM = 128;                                       // rows of A per tile (tensor-memory lanes)
 constexpr int WORKERS = 16;                                   // warps that cut operands and read accumulators out
-constexpr int THREADS = 32 * (WORKERS + 1);                   // ... and one that issues the MMAs
-constexpr int STAGES = 2;
+// ... one that issues the MMAs and, where the operands are cut beforehand, one that loads them
+template <bool CUT> constexpr int threads() { return 32 * (WORKERS + (CUT ? 2 : 1)); }
+template <int TN, bool CUT> constexpr int stages() { return CUT && TN == 64 ? 3 : 2; }
 
 constexpr uint32_t A_PLANE = TM * 128;
 template <int TN> constexpr uint32_t b_plane() { return TN * 128; }
 template <int TN> constexpr uint32_t stage_bytes() { return 3 * (A_PLANE + b_plane<TN>()); }
-template <int TN> constexpr size_t smem_bytes() { return 1024 + (size_t)STAGES * stage_bytes<TN>() + 256; }
+template <int TN, bool CUT> constexpr size_t smem_bytes() { return 1024 + (size_t)stages<TN, CUT>() * stage_bytes<TN>() + 256; }
 // Accumulators, TN columns each: [large, even stretches | small x 2^8 | small x 2^16 | large, odd stretches]
 template <int TN> constexpr uint32_t tmem_cols() { return 4 * TN; }
 
@@ -151,10 +152,18 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
 // FFMA kernel -> 24 MMAs -> this (B200, us): 1,000 x 9,216 x 1,024: 837 -> 139 -> 132 (143 TFLOP/s); 1,000 x 1,024 x 4,608:
 // 920 -> 112 -> 93; 60 x 3,072 x 1,024: 77 -> 27.6 -> 23.6; 2,048 x 1,024 x 8,192: 230 -> 215 (the last two).  Error against
 // 64 bits: 5.7e-7 -> 1.05e-7 -> 1.04e-7 (K 1,024), 1.2e-6 -> 1.8e-7 -> 1.7e-7 (K 4,608).
-template <int TN>
-__global__ void __launch_bounds__(THREADS, 1)
-sgemm_split_kernel(const Params p) {
+//
+// CUT: the operands have been cut beforehand (cut_planes_kernel): map_a and map_w are their planes, three times M and three times N
+// rows one below the other, and a loading warp brings a stretch's six tiles by TMA; the workers only read the accumulators out.  In
+// the kernel alone every tile of W is cut once per 128 rows of A and every tile of A once per 64 or 128 columns, which with some
+// hundred rows or more is most of the workers' time.  The sums are the same, bit for bit.  What bounds it then: shared memory, 160 KB of
+// operands read and 96 KB written per stretch of a wide tile.  1,000 x 9,216 x 1,024 (B200, with the cutting): 131 -> 116 us; 1,000 x
+// 1,024 x 4,608: 94 -> 82; 2,048 x 16,384 x 2,048: 900 -> 747.  Where it pays: _cut_pays in kernels/ops.py.
+template <int TN, bool CUT>
+__global__ void __launch_bounds__(threads<CUT>(), 1)
+sgemm_split_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w) {
     constexpr uint32_t B_PLANE = b_plane<TN>(), STAGE = stage_bytes<TN>();
+    constexpr int STAGES = stages<TN, CUT>();
     constexpr int ROUND = WORKERS * 4;                        // rows of a stretch per round of the workers
     constexpr int COLS = TN * 4 / WORKERS;                    // accumulator columns of a worker thread
     constexpr int A_IT = TM / ROUND, B_IT = TN / ROUND;
@@ -169,7 +178,7 @@ sgemm_split_kernel(const Params p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
     if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], WORKERS); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], CUT ? 1 : WORKERS); mbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; ++b) mbar_init(&acc_empty[b], WORKERS);
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -189,7 +198,8 @@ sgemm_split_kernel(const Params p) {
             const uint32_t one = instr_desc(TM, TN), two = instr_desc(TM, 2 * TN);
             for (int kb = 0; kb < p.kblocks; ++kb) {
                 const int s = kb % STAGES, b = kb & 1;
-                if (kb >= 2 && !mbar_wait(&acc_empty[b], ((kb >> 1) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 90, blockIdx.x, kb); break; }
+                // CUT: the workers arrive once more, when they have cleared all accumulators
+                if ((CUT || kb >= 2) && !mbar_wait(&acc_empty[b], ((kb >> 1) - (CUT ? 0 : 1)) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 90, blockIdx.x, kb); break; }
                 if (!mbar_wait(&full[s], (kb / STAGES) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 91, blockIdx.x, kb); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t a0 = smem_desc(smem_u32(smem) + s * STAGE), b0 = smem_desc(smem_u32(smem) + s * STAGE + 3 * A_PLANE);
@@ -210,6 +220,25 @@ sgemm_split_kernel(const Params p) {
             // what has been issued must be complete before the CTA gives its memory back, also after a wait that ran out
             umma_commit(done);
             mbar_wait(done, 0);
+        }
+    } else if (CUT && warp == WORKERS + 1) {
+        if (lane == 0) {
+            pdl_wait();                                       // the planes were written by the kernel before
+            int kb = 0;
+            bool ok = true;
+            // (the first stretch's MMAs also wait for the workers to have cleared the accumulators: acc_empty, below)
+            for (; kb < p.kblocks; ++kb) {
+                const int s = kb % STAGES;
+                if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 93, blockIdx.x, kb); ok = false; break; }
+                uint8_t* base = smem + s * STAGE;
+                mbar_expect_tx(&full[s], STAGE);
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    tma_load_2d(base + u * A_PLANE, &map_a, &full[s], kb * 64, u * p.M + m0);
+                    tma_load_2d(base + 3 * A_PLANE + u * B_PLANE, &map_w, &full[s], kb * 64, u * p.N + n0);
+                }
+            }
+            if (!ok) for (int u = max(0, kb - STAGES); u < kb; ++u) mbar_wait(&full[u % STAGES], (u / STAGES) & 1);      // the copies land
         }
     } else {
         // a thread's piece of a stretch: 8 neighbours of k (chunk `c`) of the rows r0, r0 + ROUND, ...
@@ -257,16 +286,24 @@ sgemm_split_kernel(const Params p) {
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
         };
+        if constexpr (!CUT) {
 #pragma unroll
-        for (int i = 0; i < B_IT; ++i) load_b(0, i);           // W is written by no kernel
-        pdl_wait();
+            for (int i = 0; i < B_IT; ++i) load_b(0, i);       // W is written by no kernel
+            pdl_wait();
 #pragma unroll
-        for (int i = 0; i < A_IT; ++i) load_a(0, i);
+            for (int i = 0; i < A_IT; ++i) load_a(0, i);
+        }
 #pragma unroll
         for (int j = 0; j < (int)tmem_cols<TN>() / 4; j += 16) tmem_zero16(tmem + lanes + (uint32_t)(part * (tmem_cols<TN>() / 4) + j));
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");       // (the first stretch's arrival tells the MMAs)
-        for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+        if constexpr (CUT) {
+            __syncwarp();
+            if (lane < 2) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[lane])) : "memory");
+            pdl_wait();                                       // before any result is written, or added to what the kernel before wrote
+            for (int kb = 0; kb < p.kblocks && ok; ++kb) drain(kb);
+        }
+        for (int kb = 0; !CUT && kb < p.kblocks && ok; ++kb) {
             const int s = kb % STAGES;
             if (kb >= STAGES) {                                // the stage is free, and its stretch's accumulator can be read
                 drain(kb - STAGES);
@@ -289,7 +326,7 @@ sgemm_split_kernel(const Params p) {
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[s])) : "memory");
         }
-        for (int kb = max(0, p.kblocks - STAGES); kb < p.kblocks && ok; ++kb) drain(kb);
+        for (int kb = max(0, p.kblocks - STAGES); !CUT && kb < p.kblocks && ok; ++kb) drain(kb);
         if (ok && !mbar_wait(done, 0)) { if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 94, blockIdx.x, p.kblocks); ok = false; }
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
@@ -341,18 +378,55 @@ sgemm_split_kernel(const Params p) {
     }
 }
 
-template <int TN>
-static int launch_split(const Params& p, cudaStream_t stream) {
+// The planes of a matrix of `rows` rows of K (row stride ld): [3][rows][Kp] bfloat16, Kp = K rounded up to 8, zeros beyond K.  A thread
+// cuts eight neighbours.  Bound by memory: 4 bytes in, 6 out.  Both operands in one launch: the first a_rows rows are A's.
+__global__ void __launch_bounds__(256)
+cut_planes_kernel(const float* __restrict__ a, int lda, int a_rows, const float* __restrict__ w, int w_rows, int K, uint4* __restrict__ pa, uint4* __restrict__ pw) {
+    pdl_trigger();
+    const int per_row = (K + 7) / 8;
+    const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long r = idx / per_row;
+    const int c = (int)(idx - r * per_row);
+    const bool mine = r < (long long)a_rows + w_rows, of_a = r < a_rows;
+    const float* src = of_a ? a + (size_t)r * lda + c * 8 : w + (size_t)(r - a_rows) * K + c * 8;
+    float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
+    auto load = [&]() {
+        v0 = __ldg(reinterpret_cast<const float4*>(src));
+        if (c * 8 + 4 < K) v1 = __ldg(reinterpret_cast<const float4*>(src) + 1);
+    };
+    if (mine && !of_a) load();                                // W is written by no kernel
+    pdl_wait();
+    if (!mine) return;
+    if (of_a) load();
+    uint4 h, m, l;
+    cut(v0.x, v0.y, h.x, m.x, l.x);
+    cut(v0.z, v0.w, h.y, m.y, l.y);
+    cut(v1.x, v1.y, h.z, m.z, l.z);
+    cut(v1.z, v1.w, h.w, m.w, l.w);
+    uint4* dst = of_a ? pa + (size_t)r * per_row + c : pw + (size_t)(r - a_rows) * per_row + c;
+    const size_t plane = (size_t)(of_a ? a_rows : w_rows) * per_row;
+    dst[0] = h;
+    dst[plane] = m;
+    dst[2 * plane] = l;
+}
+
+template <int TN, bool CUT>
+static int launch_split(const Params& p, const CUtensorMap& ma, const CUtensorMap& mw, cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(sgemm_split_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<TN>());
+        const cudaError_t e = cudaFuncSetAttribute(sgemm_split_kernel<TN, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<TN, CUT>());
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    launch(sgemm_split_kernel<TN>, dim3((p.M + TM - 1) / TM, (p.N + TN - 1) / TN), dim3(THREADS), smem_bytes<TN>(), stream, p);
+    launch(sgemm_split_kernel<TN, CUT>, dim3((p.M + TM - 1) / TM, (p.N + TN - 1) / TN), dim3(threads<CUT>()), smem_bytes<TN, CUT>(), stream, p, ma, mw);
     IMPARO_CHECK_LAUNCH();
     return 0;
 }
+
+// tiles of 128 x 64 where tiles of 128 x 128 would leave more than half of the 148 SMs without one (1,000 x 1,024 x
+// 4,608: 93 against 121 us); above that the wide tile is the faster one (500 x 3,072 x 1,024, 96 wide tiles: 34 against
+// 49 us; 1,000 x 9,216 x 1,024: 132 against 194).  The sums are the same either way.
+static bool narrow(int M, int N) { return (long long)((M + 127) / 128) * ((N + 127) / 128) * 2 <= 148; }
 
 }  // namespace sp
 
@@ -366,15 +440,41 @@ extern "C" int imparo_sgemm_nt(const float* A, const float* W, float* C, int M, 
     // rows of whole 16-byte groups: the tensor cores
     if (K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && (N + 63) / 64 <= 65535) {
         imparo::sp::Params p{A, W, C, M, N, K, lda, ldc, accumulate, (K + 63) / 64, status};
-        // tiles of 128 x 64 where tiles of 128 x 128 would leave more than half of the 148 SMs without one (1,000 x 1,024 x
-        // 4,608: 93 against 121 us); above that the wide tile is the faster one (500 x 3,072 x 1,024, 96 wide tiles: 34 against
-        // 49 us; 1,000 x 9,216 x 1,024: 132 against 194).  The sums are the same either way.
-        const long long tiles = (long long)((M + 127) / 128) * ((N + 127) / 128);
-        return tiles * 2 <= 148 ? imparo::sp::launch_split<64>(p, stream) : imparo::sp::launch_split<128>(p, stream);
+        const CUtensorMap none = {};
+        return imparo::sp::narrow(M, N) ? imparo::sp::launch_split<64, false>(p, none, none, stream)
+                                        : imparo::sp::launch_split<128, false>(p, none, none, stream);
     }
     dim3 grid((N + imparo::BN - 1) / imparo::BN, (M + imparo::BM - 1) / imparo::BM);
     if (grid.y > 65535) return -2;
     launch(imparo::sgemm_nt_kernel, grid, dim3(256), 0, stream, A, W, C, M, N, K, lda, ldc, accumulate);
     IMPARO_CHECK_LAUNCH();
     return 0;
+}
+
+// Scratch that imparo_sgemm_cut needs, in bytes; 0 where it does not take the product (rows of no 16-byte groups).
+extern "C" long long imparo_sgemm_cut_bytes(int M, int N, int K) {
+    if (M <= 0 || N <= 0 || K <= 0 || K % 4 != 0 || (N + 63) / 64 > 65535) return 0;
+    return 6LL * ((K + 7) / 8 * 8) * ((long long)M + N);
+}
+
+// imparo_sgemm_nt with the operands cut into their planes first, by a launch of its own, into scratch (16-byte aligned,
+// imparo_sgemm_cut_bytes).  -25: not taken, nothing launched.
+extern "C" int imparo_sgemm_cut(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldc, int accumulate,
+                                void* scratch, int* status, cudaStream_t stream) {
+    using namespace imparo;
+    if (imparo_sgemm_cut_bytes(M, N, K) == 0 || lda % 4 != 0 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)scratch) & 15)) return -25;
+    const uint64_t Kp = (uint64_t)(K + 7) / 8 * 8;
+    uint16_t* pa = reinterpret_cast<uint16_t*>(scratch);
+    uint16_t* pw = pa + 3 * (size_t)M * Kp;
+    const long long threads = ((long long)M + N) * (long long)(Kp / 8), blocks = (threads + 255) / 256;
+    if (blocks > 0x7fffffffLL) return -25;
+    CUtensorMap ma, mw;
+    const bool thin = sp::narrow(M, N);
+    int rc = tc::get_map(pa, 3 * (uint64_t)M, Kp, Kp, 128u, &ma);
+    if (!rc) rc = tc::get_map(pw, 3 * (uint64_t)N, Kp, Kp, thin ? 64u : 128u, &mw);
+    if (rc) return rc;
+    launch(sp::cut_planes_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, A, lda, M, W, N, K, reinterpret_cast<uint4*>(pa), reinterpret_cast<uint4*>(pw));
+    IMPARO_CHECK_LAUNCH();
+    const sp::Params p{A, W, C, M, N, K, lda, ldc, accumulate, (K + 63) / 64, status};
+    return thin ? sp::launch_split<64, true>(p, ma, mw, stream) : sp::launch_split<128, true>(p, ma, mw, stream);
 }

@@ -131,6 +131,8 @@ def _declare_kernels(lib):
     _declare(lib, "imparo_gemm_rows_conv", [P, I, P, c_float, P, P, P, P, P, P, P, I, I, I, I, I, P, S])
     _declare(lib, "imparo_gemm_rows_takes", [I, I, I, I, I, I])
     _declare(lib, "imparo_gemm_rows_configure", [])
+    _declare(lib, "imparo_sgemm_cut_bytes", [I, I, I], c_int64)
+    _declare(lib, "imparo_sgemm_cut", [P, P, P, I, I, I, I, I, I, P, P, S])
     _declare(lib, "imparo_sample_rows_parts", [P, P, P, P, P, P, I, I, I, S])
     _declare(lib, "imparo_take_sampled_tokens", [P, P, P, I, I, S])
     _declare(lib, "imparo_selftest_wait_limit", [P, I, P, S])

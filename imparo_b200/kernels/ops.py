@@ -87,6 +87,7 @@ class LaunchState:
         self.argmax_scratch = {}
         self.sample_scratch = {}
         self.status_fallback = {}
+        self.planes = {}             # device index -> scratch of cut operands (prepare_cut), or none
         self.generation = 0          # bumped when a scratch buffer moves: captured graphs that used it are stale
 
 
@@ -228,6 +229,45 @@ def prepare(device, rows: int = 8) -> None:
     if key not in _S.sample_scratch:
         _S.sample_scratch[key] = (torch.empty(n * 64, dtype=torch.float32, device=device),
                                   torch.empty(n * 32, dtype=torch.int32, device=device))
+
+
+CUT_MOST_BYTES = 512 << 20       # of scratch for cut operands
+
+
+def prepare_cut(device, most_rows: int, matrices) -> None:
+    """Scratch for 32-bit products whose operands are cut beforehand (csrc/kernels/gemm_f32.cu), for the launch state that is current:
+    made once, for the largest of the (N, K) in `matrices` that fits CUT_MOST_BYTES beside most_rows rows.  Without it, or where a
+    product needs more, linear() cuts inside the product."""
+    device = torch.device(device)
+    need = [_lib.kernels().imparo_sgemm_cut_bytes(int(most_rows), int(n), int(k)) for n, k in matrices]
+    need = max((b for b in need if b <= CUT_MOST_BYTES), default=0)
+    key = device.index or 0
+    if need and (key not in _S.planes or _S.planes[key].numel() < need):
+        _S.generation += 1 if key in _S.planes else 0
+        _S.planes[key] = torch.empty(need, dtype=torch.uint8, device=device)
+
+
+def _cut_scratch(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """The scratch to cut x's and w's operands into, where that is the faster way and there is room.  In the product every stretch of
+    64 k takes about 0.42 us longer per round of tiles; beforehand the operands are read once and written once and a half, 6 TB/s
+    together, in a launch of its own.  In the product / beforehand, as measured in us (rows x N x K): 65 x 3,072 x 1,024 23.5 / 22.2,
+    65 x 9,216 x 1,024 24.4 / 30.7, 130 x 9,216 x 1,024 34.9 / 36.9, 1,000 x 9,216 x 1,024 131 / 116, 65 x 1,024 x 4,608 89 / 71, 1,000 x
+    1,024 x 4,608 94 / 82, 257 x 6,144 x 2,048 61.3 / 62.1, 400 x 6,144 x 2,048 115 / 103, 257 x 16,384 x 2,048 176 / 183, 2,048 x 16,384 x
+    2,048 900 / 747.  (Fewer than 65 rows were not measured.)"""
+    M, K = x.shape
+    if not _cut_pays(M, w.shape[0], K):
+        return None
+    buf = _S.planes.get(x.device.index or 0)
+    if buf is None or x.stride(0) % 4 != 0 or (x.data_ptr() | w.data_ptr()) % 16 != 0:
+        return None
+    need = _lib.kernels().imparo_sgemm_cut_bytes(M, w.shape[0], K)
+    return buf if 0 < need <= buf.numel() else None
+
+
+def _cut_pays(M: int, N: int, K: int) -> bool:
+    rows, wide = -(-M // 128), -(-N // 128)
+    tiles = rows * wide if rows * wide * 2 > 148 else rows * -(-N // 64)          # (the product's own choice of tile)
+    return M >= 65 and 0.42 * -(-tiles // 148) * -(-K // 64) > 1.5 + 1.6e-6 * (M + N) * K
 
 
 def defer_adds() -> bool:
@@ -783,6 +823,12 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
         _need(out.dtype == torch.float32, "linear: float32 product writes float32")
         if accumulate:
             settle(out)
+        planes = _cut_scratch(x, w)
+        if planes is not None:
+            _check(_lib.kernels().imparo_sgemm_cut(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), N, int(accumulate), _ptr(planes),
+                                                   _ptr(_status_word(x.device, status)), _stream()), "sgemm_cut")
+            COUNTS["own"] += 1           # two launches
+            return
         _check(_lib.kernels().imparo_sgemm_nt(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), N, int(accumulate),
                                               _ptr(_status_word(x.device, status)), _stream()), "sgemm_nt")
     elif x.dtype == torch.bfloat16:
