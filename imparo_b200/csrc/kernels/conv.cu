@@ -243,6 +243,12 @@ gated_conv_rows_kernel(const T* __restrict__ bcx, const float* __restrict__ w, c
         for (int i = 0; i < V; ++i) v[i] = bf[i] * xf[i];
     };
     auto at = [&](int t, int part) { return *reinterpret_cast<const W*>(bcx + (size_t)t * stride + (size_t)part * width + ch); };
+    // whose rows these are: from the batch description, so before the wait, and for all rows at once
+    int item_r[R], start_r[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) item_r[r] = item_of_token[min(t0 + r, n_tok - 1)];
+#pragma unroll
+    for (int r = 0; r < R; ++r) start_r[r] = item_row_start[item_r[r]];
     pdl_wait();
     W b[H + R], x[H + R], c[R];
 #pragma unroll
@@ -254,8 +260,7 @@ gated_conv_rows_kernel(const T* __restrict__ bcx, const float* __restrict__ w, c
     for (int r = 0; r < R; ++r) {
         const int t = t0 + r;
         if (t >= n_tok) break;
-        const int item = item_of_token[t];
-        const int start = item_row_start[item];
+        const int item = item_r[r], start = start_r[r];
         const int rel = t - start;
         if (rel >= H) {
             float v[TAPS][V];

@@ -44,6 +44,15 @@ __device__ __forceinline__ void conv_rows(const ConvRows& p, int c, int t0) {
         if (p.in_bias) ib = *reinterpret_cast<const float4*>(p.in_bias + c);
         if (p.out_bias) ob = *reinterpret_cast<const float4*>(p.out_bias + c);
     }
+    // whose rows these are: from the batch description, so before the wait, and for all rows at once
+    int slot_r[R], j_r[R];
+    if (on) {
+        int item_r[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) item_r[r] = p.item_of_token[min(t0 + r, p.n_tok - 1)];
+#pragma unroll
+        for (int r = 0; r < R; ++r) { j_r[r] = t0 + r - p.item_row_start[item_r[r]]; slot_r[r] = p.item_slot[item_r[r]]; }
+    }
     pdl_wait();
     if (!on) return;
     float4 u[H + R];
@@ -60,7 +69,7 @@ __device__ __forceinline__ void conv_rows(const ConvRows& p, int c, int t0) {
     for (int r = 0; r < R; ++r) {
         const int t = t0 + r;
         if (t >= p.n_tok) break;
-        const int item = p.item_of_token[t], j = t - p.item_row_start[item], slot = p.item_slot[item];
+        const int j = j_r[r], slot = slot_r[r];
         if (slot < 0 || slot >= p.n_slots) {
             if (c == 0) report(p.status, IMPARO_ST_SLOT_RANGE, p.kernel, t, slot);
             continue;
