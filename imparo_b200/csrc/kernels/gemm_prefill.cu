@@ -3,12 +3,12 @@
 //
 // Where gemm_tcgen05.cu streams weights for a handful of tokens, this kernel is bound by the
 // tensor cores: hundreds to thousands of tokens, every weight tile reused by many token tiles.
-//   * The tokens are the MMA's M operand (128 per tile, tensor-memory lanes = tokens), the rows
-//     of W its N operand (256 per tile): one tcgen05.mma is 128 x 256 x 16.
+//   * The tokens are the MMA's M operand (128, tensor-memory lanes = tokens), the rows of W its N operand (256 or 192): one
+//     tcgen05.mma is 128 x 256 x 16.  A tile is 128 or 256 tokens (see Tile and plan).
 //   * Persistent CTAs, one per SM, walk the output tiles in an order that keeps CTAs that run
 //     together on the same rows of W (W is read from HBM once, X stays in the L2).
-//   * Warp 0 feeds a 4-stage ring of (X tile 16 KB | W tile 32 KB) by TMA (128-byte swizzle, no
-//     multicast); warp 1 issues the MMAs; the accumulator lives in tensor memory, twice: while
+//   * Warp 0 feeds a ring of three or four stages (X 16 KB or twice that | W 24 or 32 KB) by TMA (128-byte swizzle, no
+//     multicast); warp 1 issues the MMAs; with 128 tokens the accumulator lives in tensor memory twice: while
 //     warps 2-5 read one accumulator out (tcgen05.ld) and run the epilogue, the MMAs of the next
 //     tile already fill the other.
 //   * Epilogues, all on the accumulator in registers, a token row per thread:
@@ -30,13 +30,22 @@ namespace tcp {
 
 using namespace imparo::tc;
 
-constexpr int TM = 128;            // tokens per tile (MMA M)
-constexpr int TN = 256;            // rows of W per tile (MMA N); SwiGLU: 128 gate + 128 up
-constexpr int STAGES = 4;
-constexpr int THREADS = 192;       // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue
-constexpr uint32_t A_BYTES = TM * BK * 2, B_BYTES = TN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr uint32_t TMEM_COLS = 2 * TN;
-constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + 256;
+constexpr int TM = 128;            // tokens per MMA (M)
+constexpr uint32_t A_BYTES = TM * BK * 2;
+constexpr uint32_t ACC = 256;      // tensor-memory columns from one accumulator to the next
+constexpr uint32_t TMEM_COLS = 2 * ACC;
+
+// A tile is MT * 128 tokens by TN rows of W (MMA N; SwiGLU: TN / 2 gate and as many up rows).  MT 1: the two accumulators hold two tiles in
+// turn.  MT 2: they are the tile's two halves of tokens, which share each stage's W; the operands of a tile cross from the L2 for
+// twice the products, and what they lose is the overlap of one tile's epilogue with the next tile's products.
+// Warp 0: TMA, warp 1: MMA + tensor memory, then four epilogue warps per half.
+template <int MT, int TN> struct Tile {
+    static constexpr uint32_t B_BYTES = TN * BK * 2, STAGE_BYTES = MT * A_BYTES + B_BYTES;
+    static constexpr int STAGES = MT == 2 && TN == 256 ? 3 : 4;
+    static constexpr int THREADS = 64 + 128 * MT;
+    static constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + 256;
+    static_assert(SMEM_BYTES <= 227 * 1024, "stage ring exceeds shared memory");
+};
 
 enum Epilogue { STORE_BF16 = 0, STORE_F32 = 1, ADD_F32 = 2, SWIGLU_BF16 = 3, ACT_BF16 = 4 };
 
@@ -85,9 +94,12 @@ __device__ __forceinline__ void tile_of(int idx, const Params& p, int& tm, int& 
     tm = idx - tn * p.m_tiles;
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int EPI, int MT, int TN>
+__global__ void __launch_bounds__((Tile<MT, TN>::THREADS), 1)
 gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
+    using L = Tile<MT, TN>;
+    constexpr int STAGES = L::STAGES, H = TN / 2;
+    constexpr uint32_t B_BYTES = L::B_BYTES, STAGE_BYTES = L::STAGE_BYTES;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* aux = smem + STAGES * STAGE_BYTES;
@@ -102,7 +114,7 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4 * MT); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -119,20 +131,22 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             // W is written by no kernel: the first ring of W tiles is requested before the wait on
             // the previous kernel.  g counts k-blocks over all of this CTA's tiles.
             int w_row0 = 0;                                  // first row of the tile's group in the stacked W
+            uint32_t halves = 1;                             // of the tile's tokens that there are
             auto load_w = [&](int g, int tn, int kb) {
                 const int s = g % STAGES;
-                uint8_t* b = smem + s * STAGE_BYTES + A_BYTES;
-                mbar_expect_tx(&full[s], STAGE_BYTES);
+                uint8_t* b = smem + s * STAGE_BYTES + MT * A_BYTES;
+                mbar_expect_tx(&full[s], B_BYTES + halves * A_BYTES);
                 if (EPI == SWIGLU_BF16) {
-                    tma_load_2d(b, &map_w, &full[s], kb * BK, w_row0 + tn * 128);                      // 128 gate rows
-                    tma_load_2d(b + B_BYTES / 2, &map_w, &full[s], kb * BK, w_row0 + p.N + tn * 128);  // their 128 up rows
+                    tma_load_2d(b, &map_w, &full[s], kb * BK, w_row0 + tn * H);                        // the gate rows
+                    tma_load_2d(b + B_BYTES / 2, &map_w, &full[s], kb * BK, w_row0 + p.N + tn * H);    // their up rows
                 } else {
                     tma_load_2d(b, &map_w, &full[s], kb * BK, w_row0 + tn * TN);
                 }
             };
             auto load_x = [&](int g, int tm, int kb) {
                 const int s = g % STAGES;
-                tma_load_2d(smem + s * STAGE_BYTES, &map_x, &full[s], kb * BK, tm * TM);
+                tma_load_2d(smem + s * STAGE_BYTES, &map_x, &full[s], kb * BK, tm * (MT * TM));
+                if (MT == 2 && halves == 2) tma_load_2d(smem + s * STAGE_BYTES + A_BYTES, &map_x, &full[s], kb * BK, tm * (MT * TM) + TM);
             };
             pdl_trigger();
             int g = 0;
@@ -146,6 +160,7 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     if (grp < 0) continue;
                     w_row0 = grp * p.group_rows;
                 }
+                if (MT == 2) halves = tm * (MT * TM) + TM < p.T ? 2 : 1;
                 int kb = 0;
                 if (first) {
                     const int early = p.kblocks < STAGES ? p.kblocks : STAGES;
@@ -171,24 +186,23 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = instr_desc(TM, TN);
-            const uint64_t desc_a0 = smem_desc(smem_u32(smem)), desc_b0 = smem_desc(smem_u32(smem) + A_BYTES);
+            const uint64_t desc_a0 = smem_desc(smem_u32(smem)), desc_b0 = smem_desc(smem_u32(smem) + MT * A_BYTES);
             int g = 0, it = -1;
             bool ok = true;
             if (p.tile_group) pdl_wait();
             for (int idx = blockIdx.x; idx < n_tiles_total && ok; idx += gridDim.x) {
-                if (p.tile_group) {
-                    int tm, tn;
-                    tile_of(idx, p, tm, tn);
-                    if (p.tile_group[tm] < 0) continue;
-                }
+                int tm, tn;
+                tile_of(idx, p, tm, tn);
+                if (p.tile_group && p.tile_group[tm] < 0) continue;
                 ++it;
-                const int b = it & 1, use = it >> 1;
+                const int b = MT == 2 ? 0 : it & 1, use = MT == 2 ? it : it >> 1;
+                const bool two = MT == 2 && tm * (MT * TM) + TM < p.T;
                 if (use > 0 && !mbar_wait(&acc_empty[b], (use - 1) & 1)) {       // the epilogue has read this accumulator out
                     report(p.status, IMPARO_ST_WAIT_LIMIT, 21, idx, b);
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d_tmem = tmem_base + (uint32_t)b * TN;
+                const uint32_t d_tmem = tmem_base + (uint32_t)b * ACC;
                 for (int kb = 0; kb < p.kblocks; ++kb, ++g) {
                     const int s = g % STAGES;
                     if (!mbar_wait(&full[s], (g / STAGES) & 1)) {
@@ -205,6 +219,12 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
                     for (int k = 1; k < BK / UMMA_K; ++k)
                         umma(d_tmem, da + (uint64_t)((k * UMMA_K * 2) >> 4), db + (uint64_t)((k * UMMA_K * 2) >> 4), idesc, 1u);
+                    if (two) {
+#pragma unroll
+                        for (int k = 0; k < BK / UMMA_K; ++k)
+                            umma(d_tmem + ACC, da + (uint64_t)((A_BYTES + k * UMMA_K * 2) >> 4), db + (uint64_t)((k * UMMA_K * 2) >> 4), idesc,
+                                 (kb > 0 || k > 0) ? 1u : 0u);
+                    }
                     umma_commit(&empty[s]);
                 }
                 if (ok) umma_commit(&acc_full[b]);
@@ -212,7 +232,7 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
     } else {
         // ---- epilogue: warps 2..5 own tensor-memory lanes 32*(warp%4) .. +32; a lane is a token ----
-        const int quad = warp & 3;
+        const int quad = warp & 3, half = (warp - 2) >> 2;
         pdl_wait();                                             // before any global write or residual read
         int it = -1;
         for (int idx = blockIdx.x; idx < n_tiles_total; idx += gridDim.x) {
@@ -220,27 +240,31 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             tile_of(idx, p, tm, tn);
             if (p.tile_group && p.tile_group[tm] < 0) continue;
             ++it;
-            const int b = it & 1, use = it >> 1;
+            const int b = MT == 2 ? 0 : it & 1, use = MT == 2 ? it : it >> 1;
             const bool ok = p.kblocks == 0 || mbar_wait(&acc_full[b], use & 1);
             if (!ok) {
                 if (lane == 0) report(p.status, IMPARO_ST_WAIT_LIMIT, 23, idx, b);
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)b * TN;
-            const int t = tm * TM + quad * 32 + lane;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b + half) * ACC;
+            const int t = (tm * MT + half) * TM + quad * 32 + lane;
+            if (MT == 2 && (tm * MT + half) * TM >= p.T) {               // a half without tokens
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+                continue;
+            }
             const bool live = t < p.T;
             if (EPI == SWIGLU_BF16) {
                 __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)t * p.ldo;
-                const int f0 = tn * 128;
+                const int f0 = tn * H;
 #pragma unroll 1
-                for (int c = 0; c < 128; c += 32) {
+                for (int c = 0; c < H; c += 32) {
                     uint32_t gr[32], ur[32];
                     tmem_ld32(taddr + c, gr);
-                    tmem_ld32(taddr + 128 + c, ur);
+                    tmem_ld32(taddr + H + c, ur);
                     tmem_ld_wait();
                     pin32(gr); pin32(ur);
-                    if (c + 32 >= 128) {
+                    if (c + 32 >= H) {
                         // everything of this accumulator is in registers: hand it back to the MMAs
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
@@ -343,13 +367,13 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
 }
 
-template <int EPI>
-static int launch_prefill(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int ctas, cudaStream_t stream) {
-    auto kern = gemm_prefill_kernel<EPI>;
+template <int EPI, int MT, int TN>
+static int launch_tiles(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int ctas, cudaStream_t stream) {
+    auto kern = gemm_prefill_kernel<EPI, MT, TN>;
     static bool configured = false;
     cudaError_t e;
     if (!configured) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<MT, TN>::SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -357,8 +381,8 @@ static int launch_prefill(const CUtensorMap& mw, const CUtensorMap& mx, const Pa
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.blockDim = dim3(Tile<MT, TN>::THREADS);
+    cfg.dynamicSmemBytes = Tile<MT, TN>::SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -367,6 +391,11 @@ static int launch_prefill(const CUtensorMap& mw, const CUtensorMap& mx, const Pa
     cfg.numAttrs = imparo_pdl_enabled() ? 1 : 0;
     e = cudaLaunchKernelEx(&cfg, kern, mw, mx, p);
     return e == cudaSuccess ? 0 : (int)e;
+}
+template <int EPI>
+static int launch_prefill(int mt, int tn, const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int ctas, cudaStream_t stream) {
+    if (mt == 2) return tn == 192 ? launch_tiles<EPI, 2, 192>(mw, mx, p, ctas, stream) : launch_tiles<EPI, 2, 256>(mw, mx, p, ctas, stream);
+    return launch_tiles<EPI, 1, 256>(mw, mx, p, ctas, stream);
 }
 
 static int sm_count() {
@@ -377,6 +406,22 @@ static int sm_count() {
             n = 1;
     }
     return n;
+}
+
+// The tile for T tokens and `rows` rows of W (SwiGLU: both of a feature): the least estimate in units of 10 ns, a start plus the rounds of
+// tiles that the device walks.  A round takes 0.385 us per 64 k for 128 x 256; 0.55 for 256 x 192 and 0.70 for 256 x 256, no more per
+// product, but their epilogues come on top.  So they are for counts of tiles whose last round leaves the chip idle: 512 tokens, 13,824
+// rows, K 1,536: 216 tiles of 128 x 256 in two rounds 25.0 us, 144 of 256 x 192 in one 20.2, 108 of 256 x 256 in one 24.3; 512 x 16,384 x
+// 2,048: 31.2 / 40.4 / 29.2; 700 x 9,216 x 1,024: 19.8 / 15.9 / 18.7; 1,300 x 16,384 x 2,048: 69 / 78 / 76 (B200).
+static void plan(int T, long long rows, int kblocks, int sms, int* mt, int* tn) {
+    struct Kind { int mt, tn, start, per_round, per_k; };
+    const Kind kinds[3] = {{1, 256, 900, 0, 385}, {2, 192, 400, 200, 550}, {2, 256, 500, 150, 700}};
+    long long best = -1;
+    for (const Kind& k : kinds) {
+        const long long tiles = (long long)((T + k.mt * TM - 1) / (k.mt * TM)) * ((rows + k.tn - 1) / k.tn);
+        const long long cost = k.start + (tiles + sms - 1) / sms * (k.per_round + (long long)k.per_k * kblocks / 10);
+        if (best < 0 || cost < best) { best = cost; *mt = k.mt; *tn = k.tn; }
+    }
 }
 
 }  // namespace tcp
@@ -402,26 +447,29 @@ extern "C" int imparo_gemm_prefill(const void* x, int ldx, int x_rows_alloc, con
     if (N % (f32_out ? 4 : 8) != 0 || ldo % (f32_out ? 4 : 8) != 0) return -23;
     if (epilogue < 0 || epilogue > 4) return -22;
     const int w_rows = epilogue == SWIGLU_BF16 ? 2 * N : N;
+    int mt = 1, tn = 256;
+    plan(T, w_rows, (K + BK - 1) / BK, sm_count(), &mt, &tn);
     CUtensorMap mw, mx;
-    int rc = get_map(w, (uint64_t)w_rows, (uint64_t)K, (uint64_t)K, epilogue == SWIGLU_BF16 ? 128u : (uint32_t)TN, &mw);
+    int rc = get_map(w, (uint64_t)w_rows, (uint64_t)K, (uint64_t)K, (uint32_t)(epilogue == SWIGLU_BF16 ? tn / 2 : tn), &mw);
     if (rc) return rc;
     rc = get_map(x, (uint64_t)(x_rows_alloc > T ? x_rows_alloc : T), (uint64_t)K, (uint64_t)ldx, (uint32_t)TM, &mx);
     if (rc) return rc;
     Params p = {};
     p.out = out; p.status = status;
     p.T = T; p.N = N; p.K = K; p.ldo = ldo; p.kblocks = (K + BK - 1) / BK;
-    p.m_tiles = (T + TM - 1) / TM;
-    p.n_tiles = epilogue == SWIGLU_BF16 ? (N + 127) / 128 : (N + TN - 1) / TN;
+    p.m_tiles = (T + mt * TM - 1) / (mt * TM);
+    const int cols = epilogue == SWIGLU_BF16 ? tn / 2 : tn;
+    p.n_tiles = (N + cols - 1) / cols;
     p.act = act; p.limit = limit; p.bias = bias;
     const long long tiles = (long long)p.m_tiles * p.n_tiles;
     if (tiles > (1 << 30)) return -2;
     const int ctas = (int)(tiles < sm_count() ? tiles : sm_count());
     switch (epilogue) {
-        case STORE_BF16: return launch_prefill<STORE_BF16>(mw, mx, p, ctas, stream);
-        case STORE_F32: return launch_prefill<STORE_F32>(mw, mx, p, ctas, stream);
-        case ACT_BF16: return launch_prefill<ACT_BF16>(mw, mx, p, ctas, stream);
-        case ADD_F32: return launch_prefill<ADD_F32>(mw, mx, p, ctas, stream);
-        default: return launch_prefill<SWIGLU_BF16>(mw, mx, p, ctas, stream);
+        case STORE_BF16: return launch_prefill<STORE_BF16>(mt, tn, mw, mx, p, ctas, stream);
+        case STORE_F32: return launch_prefill<STORE_F32>(mt, tn, mw, mx, p, ctas, stream);
+        case ACT_BF16: return launch_prefill<ACT_BF16>(mt, tn, mw, mx, p, ctas, stream);
+        case ADD_F32: return launch_prefill<ADD_F32>(mt, tn, mw, mx, p, ctas, stream);
+        default: return launch_prefill<SWIGLU_BF16>(mt, tn, mw, mx, p, ctas, stream);
     }
 }
 
@@ -443,7 +491,7 @@ extern "C" int imparo_gemm_prefill_grouped(const void* x, int ldx, const void* w
     const int group_rows = epilogue == SWIGLU_BF16 ? 2 * N : N;
     const int T = m_tiles * TM;
     CUtensorMap mw, mx;
-    int rc = get_map(w, (uint64_t)n_groups * group_rows, (uint64_t)K, (uint64_t)K, epilogue == SWIGLU_BF16 ? 128u : (uint32_t)TN, &mw);
+    int rc = get_map(w, (uint64_t)n_groups * group_rows, (uint64_t)K, (uint64_t)K, epilogue == SWIGLU_BF16 ? 128u : 256u, &mw);
     if (rc) return rc;
     rc = get_map(x, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, (uint32_t)TM, &mx);
     if (rc) return rc;
@@ -451,7 +499,7 @@ extern "C" int imparo_gemm_prefill_grouped(const void* x, int ldx, const void* w
     p.out = out; p.status = status;
     p.T = T; p.N = N; p.K = K; p.ldo = ldo; p.kblocks = (K + BK - 1) / BK;
     p.m_tiles = m_tiles;
-    p.n_tiles = epilogue == SWIGLU_BF16 ? (N + 127) / 128 : (N + TN - 1) / TN;
+    p.n_tiles = epilogue == SWIGLU_BF16 ? (N + 127) / 128 : (N + 255) / 256;
     p.tile_group = tile_group;
     p.group_rows = group_rows;
     p.act = act; p.limit = limit;
@@ -459,9 +507,9 @@ extern "C" int imparo_gemm_prefill_grouped(const void* x, int ldx, const void* w
     if (tiles > (1 << 30)) return -2;
     const int ctas = (int)(tiles < sm_count() ? tiles : sm_count());
     switch (epilogue) {
-        case STORE_BF16: return launch_prefill<STORE_BF16>(mw, mx, p, ctas, stream);
-        case STORE_F32: return launch_prefill<STORE_F32>(mw, mx, p, ctas, stream);
-        case ACT_BF16: return launch_prefill<ACT_BF16>(mw, mx, p, ctas, stream);
-        default: return launch_prefill<SWIGLU_BF16>(mw, mx, p, ctas, stream);
+        case STORE_BF16: return launch_prefill<STORE_BF16>(1, 256, mw, mx, p, ctas, stream);
+        case STORE_F32: return launch_prefill<STORE_F32>(1, 256, mw, mx, p, ctas, stream);
+        case ACT_BF16: return launch_prefill<ACT_BF16>(1, 256, mw, mx, p, ctas, stream);
+        default: return launch_prefill<SWIGLU_BF16>(1, 256, mw, mx, p, ctas, stream);
     }
 }
