@@ -126,22 +126,38 @@ moe_pick_kernel(const float* __restrict__ logits, int n_rows, int experts, int c
                 float weight_scale, int out_stride, int* __restrict__ ids, float* __restrict__ wts, float* __restrict__ extra_out) {
     extern __shared__ __align__(16) float pick_smem[];   // [4][experts] scores, then [4][groups] scores of the groups
     pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r = blockIdx.x * 4 + warp;
+    // For the few rows of a decode step this is one warp's chain (5.0 -> 3.5 us for eight rows).  So it has one trip to memory: a logit's pieces together, the first
+    // experts' corrections before the wait (no kernel writes them), and nothing that was written is read back.
+    const float early = correction && lane < experts ? correction[lane] : 0.f;
+    pdl_wait();
     if (r >= n_rows) return;
     float* s = pick_smem + (size_t)warp * experts;
     auto logit = [&](int e) {
         const float* l = logits + (size_t)r * parts * columns + e;
-        float v = l[0];
-        for (int k = 1; k < parts; ++k) v += l[(size_t)k * columns];
+        float piece[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) piece[k] = k < parts ? __ldcg(l + (size_t)k * columns) : 0.f;
+        float v = piece[0];
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+            if (k < parts) v += piece[k];
         return v;
     };
+    const float last = extra_out && lane == 0 ? logit(experts) : 0.f;
+    float score0 = 0.f;                                    // with a correction: expert `lane`'s score without it
     for (int e = lane; e < experts; e += 32) {
         const float v = logit(e);
-        s[e] = correction ? 1.0f / (1.0f + expf(-v)) + correction[e] : v;
+        if (correction) {
+            const float score = 1.0f / (1.0f + expf(-v));
+            if (e == lane) score0 = score;
+            s[e] = score + (e == lane ? early : correction[e]);
+        } else {
+            s[e] = v;
+        }
     }
-    if (extra_out && lane == 0) extra_out[r] = 1.0f / (1.0f + expf(-logit(experts)));
+    if (extra_out && lane == 0) extra_out[r] = 1.0f / (1.0f + expf(-last));
     __syncwarp();
     // Without a correction the choice goes by the logits: scores are monotone in them, and a sigmoid that has reached 1 in
     // 32-bit would tie.
@@ -183,7 +199,7 @@ moe_pick_kernel(const float* __restrict__ logits, int n_rows, int experts, int c
         }
         __syncwarp();
     }
-    float total = 0.f;
+    float total = 0.f, mine = 0.f;                         // lane k: the k-th choice's score
     for (int k = 0; k < top; ++k) {
         float best = -INFINITY;
         int arg = 0x7fffffff;
@@ -197,17 +213,22 @@ moe_pick_kernel(const float* __restrict__ logits, int n_rows, int experts, int c
             const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
             if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
         }
-        const float score = softmax_scores ? expf(best - m) / l : 1.0f / (1.0f + expf(-(correction ? logit(arg) : best)));
+        float score;
+        if (softmax_scores) score = expf(best - m) / l;
+        else if (!correction) score = 1.0f / (1.0f + expf(-best));
+        else if (arg < 32) score = __shfl_sync(0xffffffffu, score0, arg);
+        else score = arg < experts ? 1.0f / (1.0f + expf(-logit(arg))) : best;      // (no candidate is a number: there is no choice)
         if (lane == 0) {
             ids[(size_t)r * out_stride + k] = arg;
-            wts[(size_t)r * out_stride + k] = score;
-            s[arg] = -INFINITY;
+            if (arg < experts) s[arg] = -INFINITY;
         }
+        if (lane == k) mine = score;
         total += score;
         __syncwarp();
     }
-    if (renormalise && lane < top) wts[(size_t)r * out_stride + lane] = wts[(size_t)r * out_stride + lane] / (total + renorm_eps) * weight_scale;
-    else if (weight_scale != 1.0f && lane < top) wts[(size_t)r * out_stride + lane] *= weight_scale;
+    if (renormalise) mine = mine / (total + renorm_eps) * weight_scale;
+    else if (weight_scale != 1.0f) mine *= weight_scale;
+    if (lane < top) wts[(size_t)r * out_stride + lane] = mine;
     // choices beyond `top` (out_stride > top) are experts every row uses with weight 1: numbers experts, experts + 1, ...
     for (int k = top + lane; k < out_stride; k += 32) {
         ids[(size_t)r * out_stride + k] = experts + (k - top);
@@ -294,7 +315,7 @@ __device__ __forceinline__ int few_pairs_of(const int* __restrict__ ids, int n_p
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     if (n_pairs <= 32) {
-        int id = lane < n_pairs ? ids[lane] : -1;
+        int id = lane < n_pairs ? __ldcg(ids + lane) : -1;
         if (id >= experts) id = -1;
         const unsigned same = __match_any_sync(0xffffffffu, id);
         const bool first = id >= 0 && (same & below) == 0;
@@ -313,7 +334,7 @@ __device__ __forceinline__ int few_pairs_of(const int* __restrict__ ids, int n_p
     for (int i = threadIdx.x; i < FEW_EXPERTS / 32; i += blockDim.x) named[i] = 0u;
     __syncthreads();
     for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-        const int id = ids[p];
+        const int id = __ldcg(ids + p);
         if (id >= 0 && id < experts) atomicOr(&named[id >> 5], 1u << (id & 31));
     }
     __syncthreads();
@@ -360,8 +381,9 @@ moe_few_kernel(const T* __restrict__ in, const T* __restrict__ w, const int* __r
                SharedRows sh) {
     extern __shared__ __align__(16) uint8_t few_smem[];
     __shared__ int list[FEW_PAIRS];
-    pdl_trigger();
+    if (!UP) pdl_trigger();
     pdl_wait();
+    if (UP) pdl_trigger();                                 // (moe_few_mma_kernel says why)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T* xs = reinterpret_cast<T*>(few_smem);
     // the shared expert's blocks come first: they have the most to do
@@ -432,7 +454,7 @@ moe_few_kernel(const T* __restrict__ in, const T* __restrict__ w, const int* __r
 }
 
 // ---- few rows in bfloat16 on tensor cores ----------------------------------------------------------------------------
-constexpr int MM_WARPS = 8, MM_ROUND = 4;              // warps of a block; 32-entry stretches a warp has in flight
+constexpr int MM_WARPS = 8;                            // warps of a block
 
 __device__ __forceinline__ uint4 ld_stream(const void* p) {
     uint4 v;
@@ -445,38 +467,71 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
 }
 
 // As moe_few_kernel, with 16 matrix rows per block (gated: the gate and up rows of eight features) and NB tiles of eight rows at
-// once.  A warp takes every MM_WARPS-th round of 32-entry stretches of the row length.  In a stretch lane (g, t) of the warp holds
+// once; grid (feature stretches, shared row tiles + experts at most).  A warp takes every MM_WARPS-th round of ROUND 32-entry
+// stretches of the row length, a round's loads all in flight at once.  In a stretch lane (g, t) of the warp holds
 // entries 8 t .. 8 t + 7 of matrix rows g and g + 8 and of row g of the operand, 16 bytes each: a dot product does not mind in which
 // order its terms are taken, so the four entries that an mma calls k = 2t, 2t + 1, 2t + 8, 2t + 9 are the lane's own neighbours, in
 // both operands.  The warps' partial sums are added in warp order.  n a multiple of 8, 16-byte aligned pointers.
-template <bool UP, int NB>
-__global__ void __launch_bounds__(MM_WARPS * 32, NB == 1 ? 4 : 2)
+//
+// What bounds it: the matrices of the experts that are named, read once; and the chain of a block, choice -> matrix rows -> sums, of
+// which an SM runs three or four beside each other.  So a block asks for its first round of matrix rows before the wait on the kernel
+// ahead wherever it can know them: a shared expert's always, and all of the down launch's.  That launch's choices were made two
+// kernels ahead, and the up launch lets it start only once its own wait is over (pdl_trigger after pdl_wait, in every block), so
+// when a block of it runs, the kernel that chose is complete.  The blocks without an expert come last in the grid.
+// B200, eight rows, ten experts of 1,536 x 1,024 named and a shared one (36 MB a launch): up 11.4 -> 10.3 us, down 13.4 -> 10.7 (with
+// rounds of six).  Blocks that stay and walk over units, the next unit's rows asked for while the sums meet, took as long together
+// (up 12.0, down 9.0): what one launch no longer waits for, the other does.
+template <bool UP, int NB, int ROUND>
+__global__ void __launch_bounds__(MM_WARPS * 32, NB == 1 ? (ROUND > 4 ? 3 : 4) : 2)
 moe_few_mma_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w, const int* __restrict__ ids,
                    const float* __restrict__ wts, int n_rows, int n, int n_feat, int top, int experts, int weight_input, int gated, int act,
                    float limit, void* __restrict__ out, SharedRows sh) {
     using T = __nv_bfloat16;
     __shared__ int list[FEW_PAIRS];
     __shared__ __align__(16) float part[MM_WARPS][NB][128];
-    pdl_trigger();
-    pdl_wait();
+    if (!UP) pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int shared_tiles = sh.w ? (n_rows + 8 * NB - 1) / (8 * NB) : 0;
-    const bool shared = (int)blockIdx.x < shared_tiles;
+    const bool shared = (int)blockIdx.y < shared_tiles;
     if (shared) { n = sh.n; n_feat = sh.n_feat; gated = 0; }
-    const int f0 = blockIdx.y * (gated ? 8 : 16);
+    const int f0 = blockIdx.x * (gated ? 8 : 16);
+    const bool early = !UP || shared;                      // the matrix rows are known before the wait
+    if (!early || f0 >= n_feat) {
+        pdl_wait();
+        if (UP) pdl_trigger();
+    }
     if (f0 >= n_feat) return;
     int e = 0, count = n_rows;
     if (!shared) {
-        e = few_pairs_of(ids, n_rows * top, experts, blockIdx.x - shared_tiles, list, count);
-        if (e < 0) return;
+        e = few_pairs_of(ids, n_rows * top, experts, blockIdx.y - shared_tiles, list, count);
+        if (e < 0) {
+            if (early) pdl_wait();
+            return;
+        }
     }
     const T* src = shared ? (const T*)sh.in : in;
     const T* mat = shared ? (const T*)sh.w : w + (size_t)e * (gated ? 2 : 1) * n_feat * n;
     const int fa = f0 + g, fb = gated ? f0 + g : f0 + g + 8;
     const T* ra = fa < n_feat ? mat + (size_t)fa * n + 8 * t : nullptr;
     const T* rb = fb < n_feat ? mat + (size_t)(gated ? n_feat + fb : fb) * n + 8 * t : nullptr;
-    const int lo = shared ? blockIdx.x * 8 * NB : 0, hi = shared ? min(n_rows, lo + 8 * NB) : count;
+    const int lo = shared ? blockIdx.y * 8 * NB : 0, hi = shared ? min(n_rows, lo + 8 * NB) : count;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    uint4 a[ROUND], c[ROUND];
+    auto load_rows = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < ROUND; ++u) {
+            const int k = k0 + 32 * u;
+            const bool live = k + 8 * t < n;
+            a[u] = live && ra ? ld_stream(ra + k) : zero;
+            c[u] = live && rb ? ld_stream(rb + k) : zero;
+        }
+    };
+    const int first = warp * ROUND * 32;
+    load_rows(first);
+    if (early) {
+        pdl_wait();
+        if (UP) pdl_trigger();
+    }
     for (int r0 = lo; r0 < hi; r0 += 8 * NB) {
         const T* xr[NB];
         float xw[NB];
@@ -493,38 +548,37 @@ moe_few_mma_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __
                 if (UP && weight_input && !shared) xw[b] = wts[item];
             }
         }
-        for (int k0 = warp * MM_ROUND * 32; k0 < n; k0 += MM_WARPS * MM_ROUND * 32) {
-            uint4 a[MM_ROUND], c[MM_ROUND], x[MM_ROUND][NB];             // all loads of a round are in flight at once
+        for (int k0 = first; k0 < n; k0 += MM_WARPS * ROUND * 32) {
+            if (k0 != first || r0 != lo) load_rows(k0);
+            constexpr int HALF = ROUND > 4 ? ROUND / 2 : ROUND;    // (registers)
 #pragma unroll
-            for (int u = 0; u < MM_ROUND; ++u) {
-                const int k = k0 + 32 * u;
-                const bool live = k + 8 * t < n;
-                a[u] = live && ra ? ld_stream(ra + k) : zero;
-                c[u] = live && rb ? ld_stream(rb + k) : zero;
-            }
+            for (int u0 = 0; u0 < ROUND; u0 += HALF) {
+                uint4 x[HALF][NB];
 #pragma unroll
-            for (int u = 0; u < MM_ROUND; ++u)
+                for (int u = 0; u < HALF; ++u)
 #pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    const int k = k0 + 32 * u;
-                    x[u][b] = k + 8 * t < n && xr[b] ? *reinterpret_cast<const uint4*>(xr[b] + k) : zero;
-                }
-#pragma unroll
-            for (int u = 0; u < MM_ROUND; ++u) {
-                if (k0 + 32 * u >= n) break;
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    uint4 xv = x[u][b];
-                    if (UP && weight_input && !shared) {
-                        __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&xv);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float2 f = __bfloat1622float2(v[i]);
-                            v[i] = __floats2bfloat162_rn(xw[b] * f.x, xw[b] * f.y);
-                        }
+                    for (int b = 0; b < NB; ++b) {
+                        const int k = k0 + 32 * (u0 + u);
+                        x[u][b] = k + 8 * t < n && xr[b] ? __ldcg(reinterpret_cast<const uint4*>(xr[b] + k)) : zero;   // (not before the wait)
                     }
-                    mma_16x8x16(acc[b], a[u].x, c[u].x, a[u].y, c[u].y, xv.x, xv.y);
-                    mma_16x8x16(acc[b], a[u].z, c[u].z, a[u].w, c[u].w, xv.z, xv.w);
+#pragma unroll
+                for (int u = 0; u < HALF; ++u) {
+                    if (k0 + 32 * (u0 + u) >= n) break;
+                    const uint4 wa = a[u0 + u], wc = c[u0 + u];
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        uint4 xv = x[u][b];
+                        if (UP && weight_input && !shared) {
+                            __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&xv);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const float2 f = __bfloat1622float2(v[i]);
+                                v[i] = __floats2bfloat162_rn(xw[b] * f.x, xw[b] * f.y);
+                            }
+                        }
+                        mma_16x8x16(acc[b], wa.x, wc.x, wa.y, wc.y, xv.x, xv.y);
+                        mma_16x8x16(acc[b], wa.z, wc.z, wa.w, wc.w, xv.z, xv.w);
+                    }
                 }
             }
         }
@@ -1012,12 +1066,20 @@ static int few_launch(const void* in, const void* w, const int* ids, const float
                 st = st > (sh.n_feat + 15) / 16 ? st : (sh.n_feat + 15) / 16;
                 tl = (n_rows + 8 * nb - 1) / (8 * nb);
             }
-            const dim3 grid(tl + (pairs < experts ? pairs : experts), st), block(MM_WARPS * 32);
+            const dim3 grid(st, tl + (pairs < experts ? pairs : experts)), block(MM_WARPS * 32);
             if (st > 65535) return -2;
-            if (nb == 1) launch(moe_few_mma_kernel<UP, 1>, grid, block, 0, stream, (const T*)in, (const T*)w, ids, wts, n_rows, n, n_feat, top,
-                                experts, weight_input, gated, act, limit, out, sh);
-            else launch(moe_few_mma_kernel<UP, 2>, grid, block, 0, stream, (const T*)in, (const T*)w, ids, wts, n_rows, n, n_feat, top, experts,
-                        weight_input, gated, act, limit, out, sh);
+            // Rounds of six stretches where that saves a block a turn of its warps (1,536 entries: one turn instead of two, of
+            // which the second had half the warps idle), else of four, which leave room for a fourth block.
+            auto turns = [&](int round) { return ((n + 31) / 32 + round * MM_WARPS - 1) / (round * MM_WARPS); };
+            auto go = [&](auto kern) {
+                launch(kern, grid, block, 0, stream, (const T*)in, (const T*)w, ids, wts, n_rows, n, n_feat, top, experts, weight_input, gated,
+                       act, limit, out, sh);
+            };
+            if (turns(6) < turns(4)) {
+                if (nb == 1) go(moe_few_mma_kernel<UP, 1, 6>);
+                else go(moe_few_mma_kernel<UP, 2, 6>);
+            } else if (nb == 1) go(moe_few_mma_kernel<UP, 1, 4>);
+            else go(moe_few_mma_kernel<UP, 2, 4>);
             IMPARO_CHECK_LAUNCH();
             return 0;
         }
