@@ -235,7 +235,7 @@ attn_split_partial_kernel(const T* __restrict__ q, const T* __restrict__ k_cache
     }
 }
 
-// One block per (token, head): fold the splits in order.  The splits' (max, sum) pairs go
+// One block per (token, head): fold the splits in order.  Beyond 32 splits their (max, sum) pairs go
 // through shared memory and the first sixteen splits' accumulators are requested at the same
 // time, so the usual launch costs one round trip to memory.
 constexpr int COMBINE_MAX_SPLITS = 2048;
@@ -253,6 +253,33 @@ __global__ void attn_split_combine_kernel(const float* __restrict__ part_acc, co
     const float* ml = part_ml + th * n_splits * 2;
     const float* acc = part_acc + th * n_splits * hd;
     const int d0 = threadIdx.x;
+    if (n_splits <= 32) {
+        // a lane a split, each warp by itself: one trip to memory and no barrier (a decode step's usual launch is bound by the
+        // chain of one block: 128 heads of 128 in 17 splits 4.1 -> 3.5 us)
+        const int lane = threadIdx.x & 31;
+        const float2 v = lane < n_splits ? __ldcg(reinterpret_cast<const float2*>(ml) + lane) : make_float2(0.f, 0.f);
+        for (int d = d0; d - lane < hd; d += blockDim.x) {                             // (whole warps)
+            float p[32];
+#pragma unroll
+            for (int u = 0; u < 32; ++u) p[u] = u < n_splits && d < hd ? __ldcg(acc + (size_t)u * hd + d) : 0.f;
+            const unsigned live = __ballot_sync(0xffffffffu, v.y > 0.f);
+            float M = warp_max(v.y > 0.f ? v.x : -INFINITY);
+            if (sink) M = fmaxf(M, sink_at);
+            const float f = v.y > 0.f ? expf(v.x - M) : 0.f;
+            float a = 0.f, L = sink ? expf(sink_at - M) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 32; ++u) {
+                if (u % 8 == 0 && u >= n_splits) break;
+                const float fs = __shfl_sync(0xffffffffu, f, u), ls = __shfl_sync(0xffffffffu, v.y, u);
+                if ((live >> u) & 1u) {
+                    a += p[u] * fs;
+                    L += ls * fs;
+                }
+            }
+            if (d < hd) out[th * hd + d] = from_f32<T>(L > 0.f ? a / L : 0.f);
+        }
+        return;
+    }
     float pa[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) pa[u] = (u < n_splits && d0 < hd) ? __ldcg(acc + (size_t)u * hd + d0) : 0.f;

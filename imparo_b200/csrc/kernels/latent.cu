@@ -161,7 +161,7 @@ latent_rot_store_kernel(const float* __restrict__ proj, size_t stride, int heads
     for (int d = threadIdx.x * N; d < tail; d += blockDim.x * N) turn_to(c + rank, d, dst + rank + d);
 }
 
-constexpr int HL_ROWS = 8;
+constexpr int HL_ROWS = 8, HL_EARLY = 4;
 
 // A warp per (head, output feature) and tile of HL_ROWS rows: the lanes stride over the head's inputs (the matrix row is
 // read once, coalesced), every row's sum is finished by a warp sum in a fixed order.
@@ -171,32 +171,43 @@ heads_linear_kernel(const T* __restrict__ x, size_t x_stride, const T* __restric
                     size_t gate_stride, T* __restrict__ out, size_t out_stride, int n_tok, int n_in, int n_out,
                     int x_head, int out_head, int gate_per_head) {
     pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int h = blockIdx.y;
     const int o = blockIdx.x * 4 + warp;
     const int t0 = blockIdx.z * HL_ROWS;
+    const T* wr = w + ((size_t)h * n_out + o) * n_in;
+    // A step of few rows waits for each trip to memory and for little else: the matrix row's first entries are read before the wait
+    // (no kernel writes them), all rows' inputs of a turn together, and a row's gate by the lane that will write the row (eight rows, 16 heads of 64: 3.9 -> 3.5 us).
+    T w0[HL_EARLY];
+#pragma unroll
+    for (int k = 0; k < HL_EARLY; ++k) w0[k] = o < n_out && lane + 32 * k < n_in ? wr[lane + 32 * k] : from_f32<T>(0.f);
+    pdl_wait();
     if (o >= n_out) return;
     const int rows = min(HL_ROWS, n_tok - t0);
-    const T* wr = w + ((size_t)h * n_out + o) * n_in;
     const T* xh = x + (size_t)t0 * x_stride + (size_t)h * x_head;
+    float gated = 0.f;
+    if (gate && lane < rows) gated = gate[(size_t)(t0 + lane) * gate_stride + (gate_per_head ? (size_t)h : (size_t)h * n_out + o)];
     float acc[HL_ROWS];
 #pragma unroll
     for (int r = 0; r < HL_ROWS; ++r) acc[r] = 0.f;
-    for (int i = lane; i < n_in; i += 32) {
-        const float wv = to_f32(wr[i]);
+    auto turn = [&](int i, float wv) {
 #pragma unroll
         for (int r = 0; r < HL_ROWS; ++r)
             if (r < rows) acc[r] += wv * to_f32(xh[(size_t)r * x_stride + i]);
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < HL_EARLY; ++k)
+        if (lane + 32 * k < n_in) turn(lane + 32 * k, to_f32(w0[k]));
+    for (int i = lane + 32 * HL_EARLY; i < n_in; i += 32) turn(i, to_f32(wr[i]));
+    float mine = 0.f;
 #pragma unroll
     for (int r = 0; r < HL_ROWS; ++r) {
         const float v = warp_sum(acc[r]);
-        if (lane == 0 && r < rows) {
-            float res = v;
-            if (gate) res *= 1.0f / (1.0f + expf(-gate[(size_t)(t0 + r) * gate_stride + (gate_per_head ? (size_t)h : (size_t)h * n_out + o)]));
-            out[(size_t)(t0 + r) * out_stride + (size_t)h * out_head + o] = from_f32<T>(res);
-        }
+        if (lane == r) mine = v;
+    }
+    if (lane < rows) {
+        if (gate) mine *= 1.0f / (1.0f + expf(-gated));
+        out[(size_t)(t0 + lane) * out_stride + (size_t)h * out_head + o] = from_f32<T>(mine);
     }
 }
 
