@@ -559,6 +559,10 @@ constexpr int stages_for(int nt) { return nt <= 64 ? 4 : nt == 128 ? 5 : 4; }
 // fit with an exchange buffer of its own; the buffer lies over the ring instead.  Batch 8: 5 stages 0.769-0.773 ms per
 // step, 6 stages 0.763-0.765, 7 stages 0.781-0.784 (the next product's CTA no longer fits beside it).  Batch 64:
 // 4 stages 1.272-1.284 ms, 5 stages 1.236-1.242, 6 stages 1.233-1.236.
+// More CTAs than SMs, 32 or 64 tokens: rings of which two fit an SM, so that there is no second round of CTAs that begins when the
+// first is through (21,504 x 2,048 with its gate, B200: 32 tokens 26.5 -> 17.2 us, 64
+// tokens 28.8 -> 19.0).
+constexpr int swiglu_paired_stages_for(int nt) { return nt <= 32 ? 5 : 4; }
 constexpr int swiglu_stages_for(int nt) { return nt <= 64 ? 6 : nt == 128 ? 5 : 4; }
 
 template <int EPI>
@@ -567,8 +571,10 @@ static int launch_nt(int nt, const CUtensorMap& mw, const CUtensorMap& mx, const
     if (EPI == SWIGLU_BF16) {
         switch (nt) {
             case 16: return launch<16, swiglu_stages_for(16), EPI>(mw, mx, mo, p, grid, stream);
-            case 32: return launch<32, swiglu_stages_for(32), EPI>(mw, mx, mo, p, grid, stream);
-            case 64: return launch<64, swiglu_stages_for(64), EPI>(mw, mx, mo, p, grid, stream);
+            case 32: return deep ? launch<32, swiglu_stages_for(32), EPI>(mw, mx, mo, p, grid, stream)
+                                 : launch<32, swiglu_paired_stages_for(32), EPI>(mw, mx, mo, p, grid, stream);
+            case 64: return deep ? launch<64, swiglu_stages_for(64), EPI>(mw, mx, mo, p, grid, stream)
+                                 : launch<64, swiglu_paired_stages_for(64), EPI>(mw, mx, mo, p, grid, stream);
             case 128: return launch<128, swiglu_stages_for(128), EPI>(mw, mx, mo, p, grid, stream);
             case 256: return launch<256, swiglu_stages_for(256), EPI>(mw, mx, mo, p, grid, stream);
         }
