@@ -270,30 +270,31 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         __syncwarp();
                         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
                     }
+                    // (one question for all 32 results which activation it is: asked pair by pair, they ran one after the other)
+                    uint32_t w[16];
+                    if (p.act == 0 && p.bias == nullptr) {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            w[e] = pack_bf16(silu_bf16(__uint_as_float(gr[2 * e])) * __uint_as_float(ur[2 * e]),
+                                             silu_bf16(__uint_as_float(gr[2 * e + 1])) * __uint_as_float(ur[2 * e + 1]));
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            const int f = f0 + c + 2 * e;
+                            float b0 = 0.f, b1 = 0.f, c0 = 0.f, c1 = 0.f;
+                            if (p.bias && f < p.N) {
+                                b0 = p.bias[f]; b1 = p.bias[f + 1];
+                                c0 = p.bias[p.N + f]; c1 = p.bias[p.N + f + 1];
+                            }
+                            w[e] = pack_bf16(gated_act_bf16(p.act, p.limit, __uint_as_float(gr[2 * e]) + b0, __uint_as_float(ur[2 * e]) + c0),
+                                             gated_act_bf16(p.act, p.limit, __uint_as_float(gr[2 * e + 1]) + b1, __uint_as_float(ur[2 * e + 1]) + c1));
+                        }
+                    }
                     if (live) {
 #pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            const int f = f0 + c + j;
-                            if (f < p.N) {                      // N is a multiple of 8: whole 16-byte groups
-                                uint32_t w[4];
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const float g0 = __uint_as_float(gr[j + 2 * e]), g1 = __uint_as_float(gr[j + 2 * e + 1]);
-                                    const float u0 = __uint_as_float(ur[j + 2 * e]), u1 = __uint_as_float(ur[j + 2 * e + 1]);
-                                    if (p.act == 0 && p.bias == nullptr) {
-                                        w[e] = pack_bf16(silu_bf16(g0) * u0, silu_bf16(g1) * u1);
-                                    } else {
-                                        float b0 = 0.f, b1 = 0.f, c0 = 0.f, c1 = 0.f;
-                                        if (p.bias) {
-                                            b0 = p.bias[f + 2 * e]; b1 = p.bias[f + 2 * e + 1];
-                                            c0 = p.bias[p.N + f + 2 * e]; c1 = p.bias[p.N + f + 2 * e + 1];
-                                        }
-                                        w[e] = pack_bf16(gated_act_bf16(p.act, p.limit, g0 + b0, u0 + c0),
-                                                         gated_act_bf16(p.act, p.limit, g1 + b1, u1 + c1));
-                                    }
-                                }
-                                *reinterpret_cast<uint4*>(out + f) = make_uint4(w[0], w[1], w[2], w[3]);
-                            }
+                        for (int j = 0; j < 4; ++j) {
+                            const int f = f0 + c + 8 * j;       // N is a multiple of 8: whole 16-byte groups
+                            if (f < p.N) *reinterpret_cast<uint4*>(out + f) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
                         }
                     }
                 }
