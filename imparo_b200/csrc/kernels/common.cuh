@@ -154,7 +154,8 @@ __device__ __forceinline__ float plain_act_bf16(int kind, float z) {
 // their weight tiles (which no kernel writes).  Without the launch attribute both are no-ops.
 // Before its wait a kernel may read only what no kernel of the chain writes: weights, and the
 // batch description of the step (positions, request of a token, portion starts, state slots,
-// block tables), which the host copies to the device before the step's first kernel.
+// block tables), which the host copies to the device before the step's first kernel.  (One exception: the routed experts' down
+// launch reads the choices of a kernel two launches back; moe.cu says what makes that safe.)
 #ifndef IMPARO_TIMELINE
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

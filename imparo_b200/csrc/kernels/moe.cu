@@ -454,7 +454,7 @@ moe_few_kernel(const T* __restrict__ in, const T* __restrict__ w, const int* __r
 }
 
 // ---- few rows in bfloat16 on tensor cores ----------------------------------------------------------------------------
-constexpr int MM_WARPS = 8;                            // warps of a block
+constexpr int MM_WARPS = 8, ROUND = 4;                 // warps of a block; 32-entry stretches a warp has in flight
 
 __device__ __forceinline__ uint4 ld_stream(const void* p) {
     uint4 v;
@@ -474,15 +474,17 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
 // both operands.  The warps' partial sums are added in warp order.  n a multiple of 8, 16-byte aligned pointers.
 //
 // What bounds it: the matrices of the experts that are named, read once; and the chain of a block, choice -> matrix rows -> sums, of
-// which an SM runs three or four beside each other.  So a block asks for its first round of matrix rows before the wait on the kernel
+// which an SM runs four beside each other.  So a block asks for its first round of matrix rows before the wait on the kernel
 // ahead wherever it can know them: a shared expert's always, and all of the down launch's.  That launch's choices were made two
 // kernels ahead, and the up launch lets it start only once its own wait is over (pdl_trigger after pdl_wait, in every block), so
 // when a block of it runs, the kernel that chose is complete.  The blocks without an expert come last in the grid.
-// B200, eight rows, ten experts of 1,536 x 1,024 named and a shared one (36 MB a launch): up 11.4 -> 10.3 us, down 13.4 -> 10.7 (with
-// rounds of six).  Blocks that stay and walk over units, the next unit's rows asked for while the sums meet, took as long together
-// (up 12.0, down 9.0): what one launch no longer waits for, the other does.
-template <bool UP, int NB, int ROUND>
-__global__ void __launch_bounds__(MM_WARPS * 32, NB == 1 ? (ROUND > 4 ? 3 : 4) : 2)
+// B200, eight rows, ten experts of 1,536 x 1,024 named (36 MB a launch): up 11.4 -> 10.3 us, down 13.4 -> 11.5.  Blocks that stay and
+// walk over units, the next unit's rows asked for while the sums meet, took as long together (up 12.0, down 9.0): what one launch no
+// longer waits for, the other does.
+// Rounds of six for rows of 1,536 (one turn of the warps, not one and a half) gained 0.8 us of the down launch, but another order of
+// the sums for it.
+template <bool UP, int NB>
+__global__ void __launch_bounds__(MM_WARPS * 32, NB == 1 ? 4 : 2)
 moe_few_mma_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w, const int* __restrict__ ids,
                    const float* __restrict__ wts, int n_rows, int n, int n_feat, int top, int experts, int weight_input, int gated, int act,
                    float limit, void* __restrict__ out, SharedRows sh) {
@@ -550,35 +552,30 @@ moe_few_mma_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __
         }
         for (int k0 = first; k0 < n; k0 += MM_WARPS * ROUND * 32) {
             if (k0 != first || r0 != lo) load_rows(k0);
-            constexpr int HALF = ROUND > 4 ? ROUND / 2 : ROUND;    // (registers)
+            uint4 x[ROUND][NB];
 #pragma unroll
-            for (int u0 = 0; u0 < ROUND; u0 += HALF) {
-                uint4 x[HALF][NB];
+            for (int u = 0; u < ROUND; ++u)
 #pragma unroll
-                for (int u = 0; u < HALF; ++u)
+                for (int b = 0; b < NB; ++b) {
+                    const int k = k0 + 32 * u;
+                    x[u][b] = k + 8 * t < n && xr[b] ? __ldcg(reinterpret_cast<const uint4*>(xr[b] + k)) : zero;   // (not before the wait)
+                }
 #pragma unroll
-                    for (int b = 0; b < NB; ++b) {
-                        const int k = k0 + 32 * (u0 + u);
-                        x[u][b] = k + 8 * t < n && xr[b] ? __ldcg(reinterpret_cast<const uint4*>(xr[b] + k)) : zero;   // (not before the wait)
-                    }
+            for (int u = 0; u < ROUND; ++u) {
+                if (k0 + 32 * u >= n) break;
 #pragma unroll
-                for (int u = 0; u < HALF; ++u) {
-                    if (k0 + 32 * (u0 + u) >= n) break;
-                    const uint4 wa = a[u0 + u], wc = c[u0 + u];
+                for (int b = 0; b < NB; ++b) {
+                    uint4 xv = x[u][b];
+                    if (UP && weight_input && !shared) {
+                        __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&xv);
 #pragma unroll
-                    for (int b = 0; b < NB; ++b) {
-                        uint4 xv = x[u][b];
-                        if (UP && weight_input && !shared) {
-                            __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&xv);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float2 f = __bfloat1622float2(v[i]);
-                                v[i] = __floats2bfloat162_rn(xw[b] * f.x, xw[b] * f.y);
-                            }
+                        for (int i = 0; i < 4; ++i) {
+                            const float2 f = __bfloat1622float2(v[i]);
+                            v[i] = __floats2bfloat162_rn(xw[b] * f.x, xw[b] * f.y);
                         }
-                        mma_16x8x16(acc[b], wa.x, wc.x, wa.y, wc.y, xv.x, xv.y);
-                        mma_16x8x16(acc[b], wa.z, wc.z, wa.w, wc.w, xv.z, xv.w);
                     }
+                    mma_16x8x16(acc[b], a[u].x, c[u].x, a[u].y, c[u].y, xv.x, xv.y);
+                    mma_16x8x16(acc[b], a[u].z, c[u].z, a[u].w, c[u].w, xv.z, xv.w);
                 }
             }
         }
@@ -1068,18 +1065,12 @@ static int few_launch(const void* in, const void* w, const int* ids, const float
             }
             const dim3 grid(st, tl + (pairs < experts ? pairs : experts)), block(MM_WARPS * 32);
             if (st > 65535) return -2;
-            // Rounds of six stretches where that saves a block a turn of its warps (1,536 entries: one turn instead of two, of
-            // which the second had half the warps idle), else of four, which leave room for a fourth block.
-            auto turns = [&](int round) { return ((n + 31) / 32 + round * MM_WARPS - 1) / (round * MM_WARPS); };
             auto go = [&](auto kern) {
                 launch(kern, grid, block, 0, stream, (const T*)in, (const T*)w, ids, wts, n_rows, n, n_feat, top, experts, weight_input, gated,
                        act, limit, out, sh);
             };
-            if (turns(6) < turns(4)) {
-                if (nb == 1) go(moe_few_mma_kernel<UP, 1, 6>);
-                else go(moe_few_mma_kernel<UP, 2, 6>);
-            } else if (nb == 1) go(moe_few_mma_kernel<UP, 1, 4>);
-            else go(moe_few_mma_kernel<UP, 2, 4>);
+            if (nb == 1) go(moe_few_mma_kernel<UP, 1>);
+            else go(moe_few_mma_kernel<UP, 2>);
             IMPARO_CHECK_LAUNCH();
             return 0;
         }
