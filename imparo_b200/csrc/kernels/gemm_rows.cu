@@ -19,8 +19,8 @@
 //
 // B200, one token / eight: gate+up 16,384 x 2,048 with its norm 13.9 / 14.9 us (the weight streamer and the norm kernel 13.4 + 3 / 13.9 +
 // 3.3), 2,048 x 8,192 7.8 / 8.7, 2,048 x 2,048 2.5 / 3.1.  Whole decode steps, before / after: 350M one row 456 / 362 us, eight rows
-// 505 / 439; 1.2B one row 722 / 647, four rows 783 / 703, eight rows 770 / 771 (from five rows on the norm in every CTA costs what its
-// kernel did).
+// 505 / 439; 1.2B one row 722 / 647, four rows 783 / 703, eight rows 770 / 771: there every SM's reading of the whole input costs what
+// was saved, and most of that step's products go elsewhere (FEW_ROWS_STREAM and _rows_pay in kernels/ops.py).
 //
 // Every wait on an mbarrier is bounded: when one runs out the kernel records IMPARO_ST_WAIT_LIMIT in the status word, stops waiting,
 // lets its copies land (again with a limit) and returns.

@@ -79,6 +79,7 @@ class LaunchState:
         self.pending_mean = {}       # data_ptr -> arguments of a norm_mean_add the next reader of the stream carries out
         self.pending_mix = {}        # data_ptr -> arguments of a streams_mix_add the next reader of the stream carries out
         self.pending_gnorm = {}      # data_ptr -> arguments of a group_norm_add the next reader of the stream carries out
+        self.rows_width = 0          # width of a stream whose norms are made inside products in this step (0: none so far)
         self.waiting_norms = {}      # data_ptr of a norm's output -> (stream, weight, eps): not made, the products that read it norm themselves
         self.unfinished = {}         # data_ptr of an output buffer whose reader finishes it -> [partials or None, bias or None]
         self.partials = {}           # device index -> scratch of products into the stream
@@ -179,6 +180,7 @@ def embed_gather(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, stat
     _S.pending_gnorm.pop(out.data_ptr(), None)
     _S.unfinished.clear()
     _S.waiting_norms.clear()
+    _S.rows_width = 0
     n, width = out.shape
     _need(ids.dtype == torch.int32 and ids.numel() >= n, "ids must be int32, one per output row")
     _need(out.dtype == torch.float32 and table.shape[1] == width, "embedding output is float32 [tokens, width]")
@@ -397,6 +399,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor,
             and x.data_ptr() not in _S.pending_gnorm and x.data_ptr() not in _S.pending_mix and out.dtype == torch.bfloat16
             and x.dtype == torch.float32 and w.dtype == torch.float32 and out.shape == x.shape and w.numel() == x.shape[1]
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and _few_rows(x.shape[0], x.shape[1], True)):
+        _S.rows_width = x.shape[1]
         _S.waiting_norms[out.data_ptr()] = (x, w, float(eps), out)          # (out: its address stays its own while the entry is there)
         return
     pm = _S.pending_mean.get(x.data_ptr())
@@ -668,9 +671,23 @@ ROWS_BF16, ROWS_F32, ROWS_ADD, ROWS_GATED = 0, 1, 2, 3
 _rows_plans = {}
 
 
+# Entries of a stream (rows x width) up to which its products go to the few-rows kernel.  Every SM reads all of a product's input, and
+# norms all of the stream: decode of 4 rows of 2,048 took 693 us that way and 745 with the weight streamer, of 8 rows of 1,024 442 and
+# 484, but of 8 rows of 1,536 612 and 609, and of 8 rows of 2,048 761 and 750 (350M, 700M and 1.2B, 700 keys, B200).
+FEW_ROWS_STREAM = 8192
+
+
+def _rows_pay(T: int, width: int) -> bool:
+    """Whether a product of T rows into (width: the stream's) or beside a stream gains by the few-rows kernel: up to four rows always,
+    above that where the stream's norms are inside products.  (Eight rows through routed experts, whose norms stand alone: 493 us with
+    it and 514 without, but another order of the sums, and a choice between two experts of nearly equal score may go by that.)"""
+    return T * width <= FEW_ROWS_STREAM and (T <= 4 or _S.rows_width == width)
+
+
 def _few_rows(T: int, K: int, norm: bool) -> bool:
     """Whether the few-rows product takes rows of K entries (of the stream, if norm) from T tokens."""
-    return T <= 8 and K % 64 == 0 and (not norm or K <= 2048) and _S.switches.few_rows and gemm_backend() == "tcgen05" and tc_max_tokens() >= T
+    return (T <= 8 and K % 64 == 0 and (not norm or (K <= 2048 and T * K <= FEW_ROWS_STREAM)) and _S.switches.few_rows
+            and gemm_backend() == "tcgen05" and tc_max_tokens() >= T)
 
 
 def _rows_take(x: torch.Tensor, w: torch.Tensor, parts: int = 1) -> bool:
@@ -698,7 +715,7 @@ def _rows_input(x: torch.Tensor):
 def combine_apart(T: int, w_out: torch.Tensor) -> bool:
     """Whether the attention's output product of T decode rows is faster with the combine of the key chunks as a kernel of its own:
     where the few-rows product takes it, which leaves the stream whole, so that the norm behind it need not be a kernel."""
-    return w_out.dtype == torch.bfloat16 and _few_rows(T, w_out.shape[1], False)
+    return w_out.dtype == torch.bfloat16 and _rows_pay(T, w_out.shape[0]) and _few_rows(T, w_out.shape[1], False)
 
 
 def forget_waiting(x: torch.Tensor) -> None:
@@ -833,7 +850,8 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
                                               _ptr(_status_word(x.device, status)), _stream()), "sgemm_nt")
     elif x.dtype == torch.bfloat16:
         _need(not accumulate or out.dtype == torch.float32, "linear: accumulate needs a float32 output")
-        if out.dtype in _DT and _rows_take(x, w):
+        if (out.dtype in _DT and (_rows_pay(M, N) if accumulate else M <= 4 or x.data_ptr() in _S.waiting_norms)
+                and _rows_take(x, w)):
             if accumulate:
                 settle(out)
             _gemm_rows(x, w, out, ROWS_ADD if accumulate else ROWS_F32 if out.dtype == torch.float32 else ROWS_BF16, status=status)
