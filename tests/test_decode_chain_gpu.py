@@ -1,4 +1,4 @@
-"""The small kernels of a decode step at the edges of their forms: routed experts of few rows (rounds of four and of six stretches, a
+"""The small kernels of a decode step at the edges of their forms: routed experts of few rows (one round of stretches and several, a
 round that is partly empty, experts nobody names, a shared expert), the combine of an attention's key chunks (a warp's form up to 32
 chunks and the block's beyond), products per head and the choice of experts, against 64 bits."""
 import pytest
