@@ -478,11 +478,9 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
 // ahead wherever it can know them: a shared expert's always, and all of the down launch's.  That launch's choices were made two
 // kernels ahead, and the up launch lets it start only once its own wait is over (pdl_trigger after pdl_wait, in every block), so
 // when a block of it runs, the kernel that chose is complete.  The blocks without an expert come last in the grid.
-// B200, eight rows, ten experts of 1,536 x 1,024 named (36 MB a launch): up 11.4 -> 10.3 us, down 13.4 -> 11.5.  Blocks that stay and
-// walk over units, the next unit's rows asked for while the sums meet, took as long together (up 12.0, down 9.0): what one launch no
-// longer waits for, the other does.
-// Rounds of six for rows of 1,536 (one turn of the warps, not one and a half) gained 0.8 us of the down launch, but another order of
-// the sums for it.
+// B200, eight rows, ten experts of 1,536 x 1,024 named (36 MB a launch): up 11.4 -> 8.8 us, down 13.4 -> 9.2.  Blocks that stay and
+// walk over units, the next unit's rows asked for while the sums meet, took longer together (up 12.0, down 9.0).  So did rounds of six
+// for rows of 1,536 (one turn of the warps, not one and a half, but three blocks on an SM: 10.3 and 10.7), with another order of the sums.
 template <bool UP, int NB>
 __global__ void __launch_bounds__(MM_WARPS * 32, NB == 1 ? 4 : 2)
 moe_few_mma_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w, const int* __restrict__ ids,
