@@ -394,11 +394,9 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor,
     linear_unfolded, linear_swiglu, linear_gated and linear_conv_rows only, before x changes: with few rows nothing is launched
     then, and those products norm the stream themselves."""
     _cuda(x, w, out, rows)
-    _S.waiting_norms.pop(out.data_ptr(), None)
-    if (may_wait and rows is None and x.data_ptr() not in _S.pending and x.data_ptr() not in _S.pending_mean
-            and x.data_ptr() not in _S.pending_gnorm and x.data_ptr() not in _S.pending_mix and out.dtype == torch.bfloat16
-            and x.dtype == torch.float32 and w.dtype == torch.float32 and out.shape == x.shape and w.numel() == x.shape[1]
-            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and _few_rows(x.shape[0], x.shape[1], True)):
+    if _S.waiting_norms:
+        _S.waiting_norms.pop(out.data_ptr(), None)
+    if may_wait and rows is None and x.shape[0] <= FEW_ROWS and _norm_may_wait(x, w, out):
         _S.rows_width = x.shape[1]
         _S.waiting_norms[out.data_ptr()] = (x, w, float(eps), out)          # (out: its address stays its own while the entry is there)
         return
@@ -443,6 +441,14 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor,
         _need(rows.dtype == torch.int32 and rows.numel() >= n, "rmsnorm: rows must be int32, one per output row")
     _check(_lib.kernels().imparo_rmsnorm(_ptr(x), _ptr(rows), _ptr(w), float(eps), _ptr(out), _code(out), n, width,
                                          _stream()), "rmsnorm")
+
+
+def _norm_may_wait(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether the products that read the norm of the whole stream x can make it themselves."""
+    at = x.data_ptr()
+    return (_few_rows(x.shape[0], x.shape[1], True) and at not in _S.pending and at not in _S.pending_mean and at not in _S.pending_gnorm
+            and at not in _S.pending_mix and out.dtype == torch.bfloat16 and x.dtype == torch.float32 and w.dtype == torch.float32
+            and out.shape == x.shape and w.numel() == x.shape[1] and at % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def swiglu_act(gu: torch.Tensor, out: torch.Tensor) -> None:
@@ -667,6 +673,10 @@ def gemm_prefill(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
 
 
 # ---- products of at most eight rows (csrc/kernels/gemm_rows.cu) -----------------------------------
+# Every step that is not replayed pays for the questions here in host time, and most products have more rows: the number of rows is
+# asked first, and nothing else of a tensor while no norm waits.  (One forward issued from Python, launches left out, us on one core:
+# 131 tokens of 1.2B 1,040 -> 850, a mixed step of 700M 1,280 -> 1,140, 64 decode rows of 1.2B 1,370 -> 1,280.)
+FEW_ROWS = 8
 ROWS_BF16, ROWS_F32, ROWS_ADD, ROWS_GATED = 0, 1, 2, 3
 _rows_plans = {}
 
@@ -686,14 +696,17 @@ def _rows_pay(T: int, width: int) -> bool:
 
 def _few_rows(T: int, K: int, norm: bool) -> bool:
     """Whether the few-rows product takes rows of K entries (of the stream, if norm) from T tokens."""
-    return (T <= 8 and K % 64 == 0 and (not norm or (K <= 2048 and T * K <= FEW_ROWS_STREAM)) and _S.switches.few_rows
-            and gemm_backend() == "tcgen05" and tc_max_tokens() >= T)
+    s = _S.switches
+    return (T <= FEW_ROWS and K % 64 == 0 and (not norm or (K <= 2048 and T * K <= FEW_ROWS_STREAM)) and s.few_rows
+            and s.gemm == "tcgen05" and s.tc_max_tokens >= T)
 
 
 def _rows_take(x: torch.Tensor, w: torch.Tensor, parts: int = 1) -> bool:
     """Whether the few-rows product takes x w^T, w [parts * F, K]: a question of shape and alignment only."""
     T, K = x.shape
-    wait = x.data_ptr() in _S.waiting_norms
+    if T > FEW_ROWS:
+        return False
+    wait = bool(_S.waiting_norms) and x.data_ptr() in _S.waiting_norms
     if not (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and _few_rows(T, K, wait) and w.is_contiguous()
             and w.data_ptr() % 16 == 0 and (wait or (x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and x.stride(1) == 1))):
         return False
@@ -702,6 +715,11 @@ def _rows_take(x: torch.Tensor, w: torch.Tensor, parts: int = 1) -> bool:
     if takes is None:
         takes = _rows_plans[key] = bool(_lib.kernels().imparo_gemm_rows_takes(T, w.shape[0] // parts, K, parts, int(wait), sm_count()))
     return takes
+
+
+def _waits(x: torch.Tensor) -> bool:
+    """Whether x is a norm that was left to the products that read it."""
+    return bool(_S.waiting_norms) and x.data_ptr() in _S.waiting_norms
 
 
 def _rows_input(x: torch.Tensor):
@@ -720,7 +738,8 @@ def combine_apart(T: int, w_out: torch.Tensor) -> bool:
 
 def forget_waiting(x: torch.Tensor) -> None:
     """x's readers are done: a norm that waited for them is not made any more."""
-    _S.waiting_norms.pop(x.data_ptr(), None)
+    if _S.waiting_norms:
+        _S.waiting_norms.pop(x.data_ptr(), None)
 
 
 def make_waiting(x: torch.Tensor) -> None:
@@ -766,11 +785,12 @@ def linear_swiglu(x, w_gu: torch.Tensor, out: torch.Tensor, status: Optional[tor
     bfloat16 on the tensor-core kernels (the weight streamer for few tokens, the persistent tile kernel for
     many): one launch, the activation in the epilogue.  Otherwise: the product into tmp [T, 2F] (a tensor,
     or a function that makes it, called only on this path), then the activation kernel."""
-    if out.dtype == torch.bfloat16 and _rows_take(x, w_gu, parts=2):
+    if x.shape[0] <= FEW_ROWS and out.dtype == torch.bfloat16 and _rows_take(x, w_gu, parts=2):
         _need(out.shape == (x.shape[0], w_gu.shape[0] // 2) and w_gu.shape[1] == x.shape[1] and out.stride(1) == 1, "linear_swiglu: shapes")
         _gemm_rows(x, w_gu, out, ROWS_GATED, parts=2, status=status)
         return
-    make_waiting(x)
+    if _S.waiting_norms:
+        make_waiting(x)
     if x.dtype == torch.bfloat16 and gemm_backend() == "tcgen05" and tc_usable(x, w_gu):
         gemm_tc(x, w_gu, out, EPI_SWIGLU, status)
         return
@@ -791,14 +811,15 @@ def linear_gated(x, w_gu: torch.Tensor, out: torch.Tensor, kind: str, limit: flo
     that adds the biases and applies the activation.  For many bfloat16 tokens: the persistent tensor-core product with the
     biases and the activation in its epilogue (one launch, no [T, 2F] tensor); for few: the weight-streaming tensor-core
     product with the same epilogue."""
-    if out.dtype == torch.bfloat16 and _rows_take(x, w_gu, parts=2):
+    if x.shape[0] <= FEW_ROWS and out.dtype == torch.bfloat16 and _rows_take(x, w_gu, parts=2):
         _need(out.shape == (x.shape[0], w_gu.shape[0] // 2) and w_gu.shape[1] == x.shape[1] and out.stride(1) == 1, "linear_gated: shapes")
         if bias is not None:
             _cuda(bias)
             _need(bias.dtype == torch.float32 and bias.numel() == w_gu.shape[0], "linear_gated: bias float32 [2F]")
         _gemm_rows(x, w_gu, out, ROWS_GATED, parts=2, act=kind, limit=limit, bias=bias, status=status)
         return
-    make_waiting(x)
+    if _S.waiting_norms:
+        make_waiting(x)
     if x.dtype == torch.bfloat16 and gemm_backend() == "tcgen05" and tc_usable(x, w_gu):
         gemm_tc(x, w_gu, out, EPI_SWIGLU, status, act=kind, limit=limit, bias=bias)
         return
@@ -850,13 +871,13 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
                                               _ptr(_status_word(x.device, status)), _stream()), "sgemm_nt")
     elif x.dtype == torch.bfloat16:
         _need(not accumulate or out.dtype == torch.float32, "linear: accumulate needs a float32 output")
-        if (out.dtype in _DT and (_rows_pay(M, N) if accumulate else M <= 4 or x.data_ptr() in _S.waiting_norms)
-                and _rows_take(x, w)):
+        if M <= FEW_ROWS and out.dtype in _DT and (_rows_pay(M, N) if accumulate else M <= 4 or _waits(x)) and _rows_take(x, w):
             if accumulate:
                 settle(out)
             _gemm_rows(x, w, out, ROWS_ADD if accumulate else ROWS_F32 if out.dtype == torch.float32 else ROWS_BF16, status=status)
             return
-        make_waiting(x)
+        if _S.waiting_norms:
+            make_waiting(x)
         if gemm_backend() == "tcgen05" and tc_usable(x, w):
             epi = EPI_ADD_F32 if accumulate else (EPI_STORE_F32 if out.dtype == torch.float32 else EPI_STORE_BF16)
             u = _S.unfinished.get(out.data_ptr()) if not accumulate else None
@@ -935,10 +956,10 @@ def linear_unfolded(x, w: torch.Tensor, out: torch.Tensor, status: Optional[torc
     PartialProduct: each split's CTAs store their tile and are done, with no fold across CTAs inside
     the product, and the consumer adds the splits while it reads."""
     if unfolded_products() and x.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32) and out.is_contiguous() \
-            and gemm_backend() == "tcgen05" and (tc_usable(x, w) or x.data_ptr() in _S.waiting_norms):
+            and gemm_backend() == "tcgen05" and (tc_usable(x, w) or _waits(x)):
         M, K = x.shape
         N = w.shape[0]
-        whole = x.data_ptr() in _S.waiting_norms and w.shape[1] == K and _rows_take(x, w)    # K is not cut: one part, the product
+        whole = _waits(x) and w.shape[1] == K and _rows_take(x, w)           # K is not cut: one part, the product
         splits, floats = (1, M * N) if whole else _tc_plan(M, N, K, EPI_PARTIAL)[1:3]
         if splits > 1 or whole:
             key = torch.device(x.device).index or 0
@@ -951,7 +972,8 @@ def linear_unfolded(x, w: torch.Tensor, out: torch.Tensor, status: Optional[torc
                 _need(out.shape == (M, N), "linear_unfolded: out must be [tokens, N]")
                 _gemm_rows(x, w, buf[:M * N].view(M, N), ROWS_F32, status=status)
             else:
-                make_waiting(x)
+                if _S.waiting_norms:
+                    make_waiting(x)
                 gemm_tc(x, w, out, EPI_PARTIAL, status, scratch=buf)
             return PartialProduct(buf, splits, (M, N), out)
     linear(x, w, out, status=status)

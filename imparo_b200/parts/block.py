@@ -28,6 +28,9 @@ class PreNormResidualBlock(Block):
         self._copies = (self.after is not None and getattr(self.after, "reads_copy", False) and getattr(self.ff, "leaves_copy", False))
         self.graph_safe = all(p.graph_safe for p in self.parts)
         self.picks_rows = True         # forward(only_rows=...) is implemented
+        # which of the two norms may be left to the products that read it (ops.rmsnorm): asked once, here
+        self._mixer_waits = {"may_wait": True} if self.mixer.input_by_products else {}
+        self._ff_waits = {"may_wait": True} if self.ff is not None and self.ff.input_by_products else {}
 
     def weight_specs(self):
         return [w for p in self.parts for w in p.weight_specs()]
@@ -49,9 +52,10 @@ class PreNormResidualBlock(Block):
         from ..kernels import ops
         if self.rt.probe_now:
             return self._forward_probed(x, batch, caches, only_rows)
-        h = self.mixer_norm.forward(x, tag="normed_mixer", **({"may_wait": True} if self.mixer.input_by_products else {}))
+        h = self.mixer_norm.forward(x, tag="normed_mixer", **self._mixer_waits)
         self._run(self.mixer, x, lambda: self.mixer.forward(h, batch, caches, x))
-        ops.forget_waiting(h)
+        if self._mixer_waits:
+            ops.forget_waiting(h)
         if only_rows is not None:
             rows, n = only_rows
             if n == 0:
@@ -69,7 +73,7 @@ class PreNormResidualBlock(Block):
         from ..kernels import ops
         copy = None
         if self.ff is not None:
-            ff_in = self.ff_norm.forward(x, tag="normed_ff", **({"may_wait": True} if self.ff.input_by_products and not probe else {}))
+            ff_in = self.ff_norm.forward(x, tag="normed_ff", **({} if probe else self._ff_waits))
             if probe:
                 probe("ff_norm", ff_in)
             kw = {"accumulate": True} if self._ff_accumulates else {}
@@ -81,7 +85,8 @@ class PreNormResidualBlock(Block):
                 ops.settle(x)
             else:
                 self._run(self.ff, x, lambda: self.ff.forward(ff_in, batch, x, **kw))
-                ops.forget_waiting(ff_in)
+                if self._ff_waits:
+                    ops.forget_waiting(ff_in)
         if self.after is not None:
             self.after.forward(x, batch, rows=rows, **({"copy": copy} if copy is not None else {}))
 

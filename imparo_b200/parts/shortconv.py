@@ -56,8 +56,9 @@ class ShortConvMixer(Part):
         st = caches[0]
         rt, T, H = self.rt, x.shape[0], self.hidden
         y = rt.workspace.get("conv_y", (T, H), rt.act_dtype, first="tokens")
-        if batch.decode_only and self.b_in is None and ops.linear_conv_rows(x, self.w_in, self.w_conv, self.b_conv, st.state, batch.item_of_token,
-                                                                            batch.item_slot, y, self.taps, rt.status):
+        if (T <= ops.FEW_ROWS and batch.decode_only and self.b_in is None
+                and ops.linear_conv_rows(x, self.w_in, self.w_conv, self.b_conv, st.state, batch.item_of_token, batch.item_slot, y,
+                                         self.taps, rt.status)):
             ops.linear(y, self.w_out, residual, accumulate=True, status=rt.status)
             if self.b_out is not None:
                 ops.add_bias(residual, self.b_out)

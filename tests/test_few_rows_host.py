@@ -1,0 +1,68 @@
+"""The rules around products of few rows on the host (no GPU; the launches are left out): what a step of more rows asks, which norms
+may be left to the products that read them, and what becomes of such a norm."""
+import pytest
+import torch
+
+from imparo_b200.kernels import lib, ops
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """The launchers on CPU tensors: entry points are noted by name and do nothing (a plan cuts K in two)."""
+    noted = []
+
+    class Entries:
+        def __getattr__(self, name):
+            def entry(*args):
+                if name == "imparo_gemm_tc_plan":
+                    T, N, _, _, nt, splits, floats, counters = args
+                    nt._obj.value, splits._obj.value, floats._obj.value, counters._obj.value = 16, 2, 2 * T * N, 128
+                    return 0
+                if name == "imparo_gemm_rows_takes":
+                    return 1
+                noted.append(name[len("imparo_"):])
+                return 0
+            return entry
+
+    entries = Entries()
+    monkeypatch.setattr(lib, "kernels", lambda: entries)
+    monkeypatch.setattr(ops, "_cuda", lambda *tensors: None)
+    monkeypatch.setattr(ops, "_need", lambda cond, text: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "_sm_count", {0: 148})
+    monkeypatch.setattr(ops, "_tc_plans", {})
+    monkeypatch.setattr(ops, "_rows_plans", {})
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    state = ops.LaunchState()
+    previous = ops.use_state(state)
+    yield noted
+    ops.use_state(previous)
+
+
+def _sizes(T, K=256, F=128):
+    half = dict(dtype=torch.bfloat16)
+    return {"x": torch.zeros(T, K), "norm": torch.ones(K), "h": torch.zeros(T, K, **half), "w": torch.zeros(2 * F, K, **half),
+            "product": torch.zeros(T, 2 * F, **half), "gated": torch.zeros(T, F, **half)}
+
+
+class _Asked(dict):
+    def _ask(self, *args):
+        raise AssertionError("a step of more rows asks for norms that wait")
+    __contains__ = get = pop = _ask
+
+
+@pytest.mark.parametrize("T", [9, 64, 131])
+def test_more_rows_ask_nothing_of_the_rule_for_few(launches, monkeypatch, T):
+    """Their launches are issued from Python whenever a step is not replayed, and each question costs host time."""
+    monkeypatch.setattr(ops._S, "waiting_norms", _Asked())
+    monkeypatch.setattr(ops, "_few_rows", lambda *args: pytest.fail("asked"))
+    t = _sizes(T)
+    ops.rmsnorm(t["x"], t["norm"], 1e-5, t["h"], may_wait=True)
+    ops.linear_swiglu(t["h"], t["w"], t["gated"], tmp=t["product"])
+    ops.linear_gated(t["h"], t["w"], t["gated"], "gelu_tanh", tmp=t["product"])
+    ops.linear_unfolded(t["h"], t["w"], t["product"])
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True)
+    ops.linear(t["h"], t["w"], t["product"])
+    ops.forget_waiting(t["h"])
+    assert launches[0] == "rmsnorm" and len(launches) >= 5
