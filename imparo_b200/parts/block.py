@@ -3,7 +3,17 @@ x += mixer(norm(x)); x += feed_forward(norm(x)), pre-norms only
 (imparo-model/src/lfm2/workflow_cpu.rs:8-18,172-319)."""
 from __future__ import annotations
 
+import inspect
+
 from .base import Block, make_part
+
+
+def norm_waits(norm, reader) -> dict:
+    """The keyword that leaves the norm before `reader` to the products that read it (ops.rmsnorm(may_wait=True)), where both know of
+    it: the norm's forward has the keyword, the reader declares input_by_products."""
+    if reader is None or not reader.input_by_products or "may_wait" not in inspect.signature(norm.forward).parameters:
+        return {}
+    return {"may_wait": True}
 
 
 class PreNormResidualBlock(Block):
@@ -23,14 +33,12 @@ class PreNormResidualBlock(Block):
             self.ff = make_part("feed_forward", spec.feed_forward, prefix, rt)
         self.after = make_part("stream_op", spec.params["after"], prefix, rt) if spec.params.get("after") else None
         self.parts = tuple(p for p in (self.mixer_norm, self.mixer, self.ff_norm, self.ff, self.after) if p is not None)
-        import inspect
         self._ff_accumulates = self.ff is not None and "accumulate" in inspect.signature(self.ff.forward).parameters
         self._copies = (self.after is not None and getattr(self.after, "reads_copy", False) and getattr(self.ff, "leaves_copy", False))
         self.graph_safe = all(p.graph_safe for p in self.parts)
         self.picks_rows = True         # forward(only_rows=...) is implemented
-        # which of the two norms may be left to the products that read it (ops.rmsnorm): asked once, here
-        self._mixer_waits = {"may_wait": True} if self.mixer.input_by_products else {}
-        self._ff_waits = {"may_wait": True} if self.ff is not None and self.ff.input_by_products else {}
+        self._mixer_waits = norm_waits(self.mixer_norm, self.mixer)              # asked once, here
+        self._ff_waits = norm_waits(self.ff_norm, self.ff)
 
     def weight_specs(self):
         return [w for p in self.parts for w in p.weight_specs()]
@@ -155,7 +163,6 @@ class ParallelResidualBlock(Block):
                 raise ValueError(f"parallel block: {type(p).__name__} cannot scale its output (residual_scale {self.scale})")
         self.graph_safe = all(p.graph_safe for p in self.parts)
         self.picks_rows = False
-        import inspect
         self._one_pass = (self.ff is not None and hasattr(self.ff, "forward_into")
                           and "extra" in inspect.signature(self.mixer.forward).parameters)
         # a feed-forward whose forward() has an `accumulate` keyword may default to overwriting: here it adds, or (beside
@@ -168,7 +175,6 @@ class ParallelResidualBlock(Block):
         return [w for p in self.parts for w in p.weight_specs()]
 
     def bind(self, tensors):
-        import inspect
         import torch
         for p in self.parts:
             p.bind(tensors)

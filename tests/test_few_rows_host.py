@@ -66,3 +66,51 @@ def test_more_rows_ask_nothing_of_the_rule_for_few(launches, monkeypatch, T):
     ops.linear(t["h"], t["w"], t["product"])
     ops.forget_waiting(t["h"])
     assert launches[0] == "rmsnorm" and len(launches) >= 5
+
+
+# ---- which norms may wait ------------------------------------------------------------------------------------------------------
+
+def _block(norm_cls, mixer_cls):
+    from imparo_b200.parts.base import Runtime, Workspace, register_part
+    from imparo_b200.parts.block import PreNormResidualBlock
+    from imparo_b200.parts.spec import LayerSpec, PartSpec
+    register_part("norm", "few_rows_test", norm_cls, replace=True)
+    register_part("mixer", "few_rows_test", mixer_cls, replace=True)
+    cpu = torch.device("cpu")
+    rt = Runtime(precision="bfloat16", device=cpu, workspace=Workspace(cpu))
+    norm = PartSpec("few_rows_test", {"width": 64, "eps": 1e-5, "name": "n"})
+    layer = LayerSpec(prefix="", mixer=PartSpec("few_rows_test", {}), mixer_norm=norm, feed_forward=None, feed_forward_norm=None)
+    return PreNormResidualBlock({"layer": layer}, "", rt)
+
+
+def _noting_parts():
+    from imparo_b200.parts.base import Part
+    noted = []
+
+    class DocumentedNorm(Part):
+        def forward(self, x32, rows=None, n_rows=None, tag="normed"):
+            noted.append("documented")
+            return x32.to(torch.bfloat16)
+
+    class WaitingNorm(Part):
+        def forward(self, x32, rows=None, n_rows=None, tag="normed", may_wait=False):
+            noted.append(may_wait)
+            return x32.to(torch.bfloat16)
+
+    class Reader(Part):
+        input_by_products = True
+
+        def forward(self, x, batch, caches, residual):
+            noted.append(tuple(x.shape))
+
+    return noted, DocumentedNorm, WaitingNorm, Reader
+
+
+def test_a_norm_with_the_documented_signature_runs(launches):
+    noted, documented, waiting, reader = _noting_parts()
+    x = torch.zeros(3, 64)
+    _block(documented, reader).forward(x, None, ())
+    assert noted == ["documented", (3, 64)]
+    noted.clear()
+    _block(waiting, reader).forward(x, None, ())
+    assert noted == [True, (3, 64)]
