@@ -127,8 +127,10 @@ class Part:
     # (ops.add_bias after it is fine): that add may then stay split partials that the next norm folds in
     # (ops.allow_deferred_add).  A part that writes the residual any other way keeps False.
     adds_with_linear = False
-    # Its input is read by products of ops (linear, linear_unfolded, linear_swiglu, linear_gated, linear_conv_rows) and nothing else:
-    # the norm before it may then be left to them (ops.rmsnorm(may_wait=True)).
+    # Its input is read by products of ops (linear, linear_unfolded, linear_swiglu, linear_gated, linear_conv_rows), each given the
+    # whole of it and no rows of it, and by nothing else: the norm before it may then be left to them (ops.rmsnorm(may_wait=True)).
+    # It holds for the class that says it alone: a subclass may read its input in another way, so it says it for itself or not at all
+    # (reads_by_products).
     input_by_products = False
 
     def __init__(self, params: dict, prefix: str, rt: Runtime):
@@ -154,6 +156,11 @@ class Part:
     # its columns p [tokens, input_rows()] (rows dense, a column range of the shared product) instead of computing them.
     def input_rows(self) -> int:
         return 0
+
+
+def reads_by_products(part) -> bool:
+    """input_by_products as the part's own class declares it (not a base class, and not with another forward put into the object)."""
+    return bool(vars(type(part)).get("input_by_products", False)) and "forward" not in getattr(part, "__dict__", {})
 
 
 class Block(Part):

@@ -5,13 +5,13 @@ from __future__ import annotations
 
 import inspect
 
-from .base import Block, make_part
+from .base import Block, make_part, reads_by_products
 
 
 def norm_waits(norm, reader) -> dict:
     """The keyword that leaves the norm before `reader` to the products that read it (ops.rmsnorm(may_wait=True)), where both know of
-    it: the norm's forward has the keyword, the reader declares input_by_products."""
-    if reader is None or not reader.input_by_products or "may_wait" not in inspect.signature(norm.forward).parameters:
+    it: the norm's forward has the keyword, the reader's own class declares input_by_products."""
+    if reader is None or not reads_by_products(reader) or "may_wait" not in inspect.signature(norm.forward).parameters:
         return {}
     return {"may_wait": True}
 

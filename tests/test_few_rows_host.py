@@ -114,3 +114,33 @@ def test_a_norm_with_the_documented_signature_runs(launches):
     noted.clear()
     _block(waiting, reader).forward(x, None, ())
     assert noted == [True, (3, 64)]
+
+
+def test_a_subclass_does_not_inherit_how_its_input_is_read(launches):
+    noted, _, waiting, reader = _noting_parts()
+
+    class ReadsItself(reader):
+        def forward(self, x, batch, caches, residual):
+            residual += x.float()
+
+    class ReadsInAHelper(reader):
+        pass
+
+    class SaysSo(reader):
+        input_by_products = True
+
+    x = torch.zeros(3, 64)
+    for cls, waits in ((ReadsItself, False), (ReadsInAHelper, False), (SaysSo, True), (reader, True)):
+        noted.clear()
+        block = _block(waiting, cls)
+        block.forward(x, None, ())
+        assert noted[0] is waits, cls
+    from imparo_b200.parts.attention import AttentionMixer
+    from imparo_b200.parts.base import reads_by_products
+    from imparo_b200.parts.feedforward import SwiGLU
+    from imparo_b200.parts.shortconv import ShortConvMixer
+    for cls in (AttentionMixer, SwiGLU, ShortConvMixer):
+        part = cls.__new__(cls)
+        assert reads_by_products(part)
+        part.forward = lambda *args: None
+        assert not reads_by_products(part)
