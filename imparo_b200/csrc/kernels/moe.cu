@@ -309,7 +309,8 @@ struct SharedRows {
 
 // The launch's pairs as a block sees them: the k-th of the experts they name (-1: there are fewer), its pairs (in order) in list,
 // and how many.  Up to 32 pairs every warp finds the answer by itself; with more the block first marks the experts in a bit set.
-// (All warps write the same list.)  Every thread of the block calls it.
+// (All warps write the same list.)  Every thread of the block calls it.  The down launch calls it before its wait, and the buffer is
+// every layer's: all reads go to the L2, where the kernel that chose has left them, never to an SM's L1, which may hold the last layer's.
 constexpr int FEW_EXPERTS = 2048;
 __device__ __forceinline__ int few_pairs_of(const int* __restrict__ ids, int n_pairs, int experts, int k, int* list, int& count) {
     const int lane = threadIdx.x & 31;
@@ -360,7 +361,7 @@ __device__ __forceinline__ int few_pairs_of(const int* __restrict__ ids, int n_p
     e = __shfl_sync(0xffffffffu, e, __ffs(hit) - 1);
     int n = 0;
     for (int p0 = 0; p0 < n_pairs; p0 += 32) {
-        const bool member = p0 + lane < n_pairs && ids[p0 + lane] == e;
+        const bool member = p0 + lane < n_pairs && __ldcg(ids + p0 + lane) == e;
         const unsigned m = __ballot_sync(0xffffffffu, member);
         if (member) list[n + __popc(m & below)] = p0 + lane;
         n += __popc(m);

@@ -68,6 +68,38 @@ def test_routed_experts(rows, width, ff, s_ff):
         near(y, s @ sd.double().T, s.abs() @ sd.double().abs().T)
 
 
+@pytest.mark.parametrize("rows,top", [(4, 8), (17, 2), (16, 8), (32, 8)])
+@pytest.mark.parametrize("width,ff", [(1024, 1536), (264, 72)])
+def test_layers_in_a_row_share_the_choices_buffer(rows, top, width, ff):
+    """Every layer's choice goes into the same buffer and the down launch reads it before its wait (32 pairs and more): a chain of
+    layers without anything between gives bit for bit what each layer gives alone, from a buffer of its own."""
+    o = ops()
+    g = torch.Generator().manual_seed(rows * top + ff)
+    E, layers = 40, 6
+    h = torch.randn(rows, width, generator=g).to(torch.bfloat16).to(DEV)
+    up = (torch.randn(E, ff, width, generator=g) * width ** -0.5).to(torch.bfloat16).to(DEV)
+    down = (torch.randn(E, width, ff, generator=g) * ff ** -0.5).to(torch.bfloat16).to(DEV)
+    logits = torch.randn(layers, rows, E, generator=g).to(DEV)
+    mid = torch.empty(rows * top, ff, dtype=torch.bfloat16, device=DEV)
+    pair_out = torch.empty(rows * top, width, device=DEV)
+    ids, wts = torch.empty(rows, top, dtype=torch.int32, device=DEV), torch.empty(rows, top, device=DEV)
+
+    def layer(i, ids, wts, out):
+        o.moe_pick(logits[i], E, 1, top, ids, wts, renormalise=True)
+        o.moe_experts(h, up, down, ids, wts, top, False, mid, out, act="plain:relu2", pair_out=pair_out)
+
+    want = torch.full((layers, rows, width), float("nan"), device=DEV)
+    for i in range(layers):
+        layer(i, torch.empty_like(ids), torch.empty_like(wts), want[i])
+        torch.cuda.synchronize()
+    for _ in range(3):
+        got = torch.full_like(want, float("nan"))
+        torch.cuda.synchronize()
+        for i in range(layers):
+            layer(i, ids, wts, got[i])
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("sink", [False, True])
 @pytest.mark.parametrize("hd", [32, 96, 128, 200])
 @pytest.mark.parametrize("splits", [1, 8, 16, 17, 32, 33])
