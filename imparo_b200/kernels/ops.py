@@ -956,11 +956,14 @@ def linear_unfolded(x, w: torch.Tensor, out: torch.Tensor, status: Optional[torc
     PartialProduct: each split's CTAs store their tile and are done, with no fold across CTAs inside
     the product, and the consumer adds the splits while it reads."""
     if unfolded_products() and x.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32) and out.is_contiguous() \
-            and gemm_backend() == "tcgen05" and (tc_usable(x, w) or _waits(x)):
+            and gemm_backend() == "tcgen05":
         M, K = x.shape
         N = w.shape[0]
         whole = _waits(x) and w.shape[1] == K and _rows_take(x, w)           # K is not cut: one part, the product
-        splits, floats = (1, M * N) if whole else _tc_plan(M, N, K, EPI_PARTIAL)[1:3]
+        if whole:
+            splits, floats = 1, M * N
+        else:
+            splits, floats = _tc_plan(M, N, K, EPI_PARTIAL)[1:3] if tc_usable(x, w) else (1, 0)
         if splits > 1 or whole:
             key = torch.device(x.device).index or 0
             buf = _S.consumer_parts.get(key)

@@ -144,3 +144,33 @@ def test_a_subclass_does_not_inherit_how_its_input_is_read(launches):
         assert reads_by_products(part)
         part.forward = lambda *args: None
         assert not reads_by_products(part)
+
+
+# ---- what becomes of a norm that waits -------------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("product", ["linear", "linear_unfolded", "linear_swiglu", "linear_gated"])
+def test_a_matrix_off_its_alignment_gets_the_norm_made(launches, monkeypatch, product):
+    """A matrix that no own product takes goes to the library's, as for any other input; the norm is made first."""
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True)
+    monkeypatch.setattr(ops, "_gemm_ws", {0: None})
+
+    def need(cond, text):
+        if not cond:
+            raise ops.KernelError(text)
+    monkeypatch.setattr(ops, "_need", need)
+    t = _sizes(4)
+    w = torch.zeros(t["w"].numel() + 4, dtype=torch.bfloat16)[4:].view(t["w"].shape)      # 8 bytes off
+    assert w.data_ptr() % 16 == 8
+    ops.rmsnorm(t["x"], t["norm"], 1e-5, t["h"], may_wait=True)
+    assert launches == [] and t["h"].data_ptr() in ops._S.waiting_norms
+    if product in ("linear", "linear_unfolded"):
+        out = getattr(ops, product)(t["h"], w, t["product"])
+        assert out is None or out is t["product"]
+        tail = []
+    elif product == "linear_swiglu":
+        ops.linear_swiglu(t["h"], w, t["gated"], tmp=t["product"])
+        tail = ["swiglu_act"]
+    else:
+        ops.linear_gated(t["h"], w, t["gated"], "gelu_tanh", tmp=t["product"])
+        tail = ["gated_act"]
+    assert launches == ["rmsnorm", "gemm_bf16_nt"] + tail and not ops._S.waiting_norms
