@@ -172,15 +172,24 @@ def selftest_wait_limit(status: torch.Tensor, limit: int = 1000) -> int:
     return int(outcome.item())
 
 
-def embed_gather(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, status: torch.Tensor) -> None:
-    _cuda(table, ids, out, status)
-    _S.pending.pop(out.data_ptr(), None)       # the stream starts afresh: partials of an unfinished step are void
-    _S.pending_mean.pop(out.data_ptr(), None)
-    _S.pending_mix.pop(out.data_ptr(), None)
-    _S.pending_gnorm.pop(out.data_ptr(), None)
+def step_starts() -> None:
+    """What the state holds for the length of a step, a step that raised has left there: it is void."""
     _S.unfinished.clear()
     _S.waiting_norms.clear()
     _S.rows_width = 0
+
+
+def _stream_starts(out: torch.Tensor) -> None:
+    """A step's stream starts afresh in `out`."""
+    at = out.data_ptr()
+    for left in (_S.pending, _S.pending_mean, _S.pending_mix, _S.pending_gnorm):
+        left.pop(at, None)
+    step_starts()
+
+
+def embed_gather(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, status: torch.Tensor) -> None:
+    _cuda(table, ids, out, status)
+    _stream_starts(out)
     n, width = out.shape
     _need(ids.dtype == torch.int32 and ids.numel() >= n, "ids must be int32, one per output row")
     _need(out.dtype == torch.float32 and table.shape[1] == width, "embedding output is float32 [tokens, width]")
@@ -349,6 +358,7 @@ def group_rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, groups: int, out
     """out[r] = x[rows[r]] (or x[r]) cut into `groups` equal stretches, each divided by its own root mean square, times w.
     A group_norm_add left pending on x is carried out by the same kernel when the norm reads every row in place."""
     _cuda(x, w, out, rows)
+    forget_waiting(out)
     n, width = out.shape
     _need(x.dtype == torch.float32 and w.dtype == torch.float32, "group_rmsnorm reads a float32 stream and float32 weights")
     _need(x.shape[1] == width and w.numel() == width and width % groups == 0, "group_rmsnorm: widths and groups")
@@ -394,8 +404,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor,
     linear_unfolded, linear_swiglu, linear_gated and linear_conv_rows only, before x changes: with few rows nothing is launched
     then, and those products norm the stream themselves."""
     _cuda(x, w, out, rows)
-    if _S.waiting_norms:
-        _S.waiting_norms.pop(out.data_ptr(), None)
+    forget_waiting(out)
     if may_wait and rows is None and x.shape[0] <= FEW_ROWS and _norm_may_wait(x, w, out):
         _S.rows_width = x.shape[1]
         _S.waiting_norms[out.data_ptr()] = (x, w, float(eps), out)          # (out: its address stays its own while the entry is there)
@@ -737,7 +746,7 @@ def combine_apart(T: int, w_out: torch.Tensor) -> bool:
 
 
 def forget_waiting(x: torch.Tensor) -> None:
-    """x's readers are done: a norm that waited for them is not made any more."""
+    """x's readers are done, or x is written anew: a norm that waited for them is not made any more."""
     if _S.waiting_norms:
         _S.waiting_norms.pop(x.data_ptr(), None)
 
@@ -2161,9 +2170,7 @@ def embed_copies(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, stat
         _need(pos_table.dtype == table.dtype and pos_table.is_contiguous() and pos_table.shape[1] == table.shape[1],
               "position table: the embedding table's dtype and width")
         _need(positions.dtype == torch.int32 and positions.numel() >= out.shape[0], "positions must be int32, one per output row")
-    for d in (_S.pending, _S.pending_mean, _S.pending_mix, _S.pending_gnorm):      # the stream starts afresh
-        d.pop(out.data_ptr(), None)
-    _S.unfinished.clear()
+    _stream_starts(out)
     n = out.shape[0]
     width = table.shape[1]
     _need(ids.dtype == torch.int32 and ids.numel() >= n, "ids must be int32, one per output row")
@@ -2180,6 +2187,7 @@ def streams_norm(x: torch.Tensor, n: int, coef: Optional[torch.Tensor], w: torch
     x: float32 [*, n * width]; rows (int32) picks input rows.  A streams_mix_add left pending on x is carried out
     by the same kernel when the norm reads every row in place."""
     _cuda(x, coef, w, out, rows)
+    forget_waiting(out)
     n_rows, width = out.shape
     _need(x.dtype == torch.float32 and x.is_contiguous() and x.shape[1] == n * width, "streams_norm: x float32 [rows, n * width]")
     _need(w.dtype == torch.float32 and w.numel() == width, "streams_norm: weight float32 [width]")

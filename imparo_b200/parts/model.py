@@ -76,6 +76,8 @@ class Model:
         they are fewer than the batch's tokens and the last entry is a block that can run its
         feed-forward on picked rows, the result is (stream of the picked rows [n, width] or None
         for n = 0, True); else (the whole stream, False)."""
+        from ..kernels import ops
+        ops.step_starts()                # (an embedding of another kind may not go through the launchers that say it)
         x = self.embedding.forward(batch)
         last = len(self.schedule) - 1
         for i, e in enumerate(self.schedule):

@@ -174,3 +174,44 @@ def test_a_matrix_off_its_alignment_gets_the_norm_made(launches, monkeypatch, pr
         ops.linear_gated(t["h"], w, t["gated"], "gelu_tanh", tmp=t["product"])
         tail = ["gated_act"]
     assert launches == ["rmsnorm", "gemm_bf16_nt"] + tail and not ops._S.waiting_norms
+
+
+@pytest.mark.parametrize("start", ["embed_gather", "embed_copies"])
+def test_a_stream_that_starts_voids_what_a_step_left(launches, start):
+    """A step that raised may leave a norm waiting; the next step's choice of kernels follows nothing of it, however the stream starts."""
+    t = _sizes(4)
+    ops.rmsnorm(t["x"], t["norm"], 1e-5, t["h"], may_wait=True)
+    assert ops._S.waiting_norms and ops._S.rows_width == 256
+    ids, table, status = torch.zeros(4, dtype=torch.int32), torch.zeros(9, 256, dtype=torch.bfloat16), torch.zeros(4, dtype=torch.int32)
+    getattr(ops, start)(table, ids, t["x"], status)
+    assert not ops._S.waiting_norms and ops._S.rows_width == 0
+
+
+def test_another_norm_of_the_same_buffer_takes_the_place_of_one_that_waits(launches):
+    t = _sizes(4)
+    for again in (lambda: ops.group_rmsnorm(t["x"], t["norm"], 1e-5, 4, t["h"]),
+                  lambda: ops.streams_norm(t["x"], 1, None, t["norm"], 1e-5, t["h"]),
+                  lambda: ops.rmsnorm(t["x"], t["norm"], 1e-5, t["h"])):
+        ops.rmsnorm(t["x"], t["norm"], 1e-5, t["h"], may_wait=True)
+        launches.clear()
+        again()
+        assert not ops._S.waiting_norms
+        ops.linear_swiglu(t["h"], t["w"], t["gated"])
+        assert launches[1:] == ["gemm_rows"] and len(launches) == 2
+
+
+def test_a_model_whose_embedding_is_its_own_starts_clean(launches):
+    """An embedding that does not go through the launchers leaves the state to Model.forward."""
+    from imparo_b200.parts.model import Model
+    t = _sizes(4)
+    ops.rmsnorm(t["x"], t["norm"], 1e-5, t["h"], may_wait=True)
+    seen = []
+
+    class Embedding:
+        def forward(self, batch):
+            seen.append((dict(ops._S.waiting_norms), ops._S.rows_width))
+            return t["x"]
+    model = Model.__new__(Model)
+    model.embedding, model.schedule, model.rt = Embedding(), [], type("Rt", (), {"probe": None, "probe_now": False})()
+    model.forward(None, None)
+    assert seen == [({}, 0)]
