@@ -54,6 +54,7 @@ class KernelSwitches:
     prefill_tc_min_tokens: int = 256      # IMPARO_PREFILL_TC_MIN_TOKENS: fewest tokens of the persistent tile product
     prefill_linear: bool = False          # IMPARO_PREFILL_LINEAR: the tile product also for plain products (not only SwiGLU)
     few_rows: bool = True                 # IMPARO_FEW_ROWS: products of at most eight rows on their own kernel, norms and convolution inside
+    cut_f32: bool = True                  # IMPARO_CUT_F32: operands of 32-bit products of many rows cut once, beforehand (off: inside the product)
     unfolded: bool = True                 # IMPARO_UNFOLDED: in_proj / qkv leave split partials to their consumer
     defer_adds: bool = True               # IMPARO_DEFER_ADDS: products into the stream leave partials to the next norm
     fuse_producers: bool = True           # IMPARO_FUSE_PRODUCERS: the attention combine inside the output product (decode rows)

@@ -104,7 +104,6 @@ class Engine:
             tensors = {w.name: drawn[w.name].to(target_dtype(w.role, self.precision)) for w in specs if w.name in drawn}
         self.weight_bytes = sum(t.numel() * t.element_size() for t in tensors.values())
         self.model.bind(tensors)
-        matrices = [tuple(t.shape) for t in tensors.values() if t.dim() == 2]
         del tensors
         self.ctx = min(int(ctx), self.model.spec.max_positions)
         self.parallel = int(parallel)
@@ -127,8 +126,8 @@ class Engine:
         self.rt.workspace.expect(tokens=min(self.max_step_tokens + rows, 8192), rows=min(rows, 512), context=self.ctx)
         previous = ops.use_state(self.rt.launch_state)
         try:
-            if self.rt.act_dtype == torch.float32:      # (parts stack up to three matrices of one input)
-                ops.prepare_cut(self.device, min(self.max_step_tokens + rows, 8192), [(c * n, k) for n, k in matrices for c in (1, 2, 3)])
+            if self.rt.act_dtype == torch.float32:
+                ops.prepare_cut(self.device, min(self.max_step_tokens + rows, 8192), self.model.product_matrices(min(rows, 512)))
             ops.prepare(self.device, rows=rows)         # nothing is left to be made at a first use, i.e. under capture
         finally:
             ops.use_state(previous)

@@ -88,7 +88,7 @@ class LaunchState:
         self.argmax_scratch = {}
         self.sample_scratch = {}
         self.status_fallback = {}
-        self.planes = {}             # device index -> scratch of cut operands (prepare_cut), or none
+        self.planes = {}             # device index -> scratch of cut operands (none: products cut their operands themselves)
         self.generation = 0          # bumped when a scratch buffer moves: captured graphs that used it are stale
 
 
@@ -243,19 +243,30 @@ def prepare(device, rows: int = 8) -> None:
 
 
 CUT_MOST_BYTES = 512 << 20       # of scratch for cut operands
+CUT_FEWEST_ROWS = 65
 
 
 def prepare_cut(device, most_rows: int, matrices) -> None:
     """Scratch for 32-bit products whose operands are cut beforehand (csrc/kernels/gemm_f32.cu), for the launch state that is current:
-    made once, for the largest of the (N, K) in `matrices` that fits CUT_MOST_BYTES beside most_rows rows.  Without it, or where a
-    product needs more, linear() cuts inside the product."""
+    made once, for the largest of `matrices` ((N, K) each, or (N, K, most rows) where an input has other rows than most_rows) at
+    the most rows with which cutting pays, as long as that fits CUT_MOST_BYTES.  Without it (the switch cut_f32, or a device that
+    has no room left), or where a product needs more, linear() cuts inside the product."""
+    if not _S.switches.cut_f32:
+        return
     device = torch.device(device)
-    need = [_lib.kernels().imparo_sgemm_cut_bytes(int(most_rows), int(n), int(k)) for n, k in matrices]
-    need = max((b for b in need if b <= CUT_MOST_BYTES), default=0)
+    need = 0
+    for n, k, *most in matrices:
+        rows = next((m for m in range(int(most[0] if most else most_rows), CUT_FEWEST_ROWS - 1, -1) if _cut_pays(m, n, k)), 0)
+        size = _lib.kernels().imparo_sgemm_cut_bytes(rows, int(n), int(k)) if rows else 0
+        need = max(need, size if size <= CUT_MOST_BYTES else 0)
     key = device.index or 0
     if need and (key not in _S.planes or _S.planes[key].numel() < need):
+        try:
+            scratch = torch.empty(need, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            return
         _S.generation += 1 if key in _S.planes else 0
-        _S.planes[key] = torch.empty(need, dtype=torch.uint8, device=device)
+        _S.planes[key] = scratch
 
 
 def _cut_scratch(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
@@ -278,7 +289,7 @@ def _cut_scratch(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
 def _cut_pays(M: int, N: int, K: int) -> bool:
     rows, wide = -(-M // 128), -(-N // 128)
     tiles = rows * wide if rows * wide * 2 > 148 else rows * -(-N // 64)          # (the product's own choice of tile)
-    return M >= 65 and 0.42 * -(-tiles // 148) * -(-K // 64) > 1.5 + 1.6e-6 * (M + N) * K
+    return M >= CUT_FEWEST_ROWS and 0.42 * -(-tiles // 148) * -(-K // 64) > 1.5 + 1.6e-6 * (M + N) * K
 
 
 def defer_adds() -> bool:

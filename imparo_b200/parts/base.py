@@ -158,6 +158,30 @@ class Part:
         return 0
 
 
+def product_matrices(part, seen=None) -> set:
+    """(rows, inputs) of the matrices that the part, and the parts it is made of, hold after bind (attributes named w_..., two
+    dimensions): as they were stacked, not as the file has them."""
+    seen = set() if seen is None else seen
+    if id(part) in seen:
+        return set()
+    seen.add(id(part))
+    found = set()
+
+    def look(name, value):
+        if isinstance(value, torch.Tensor):
+            if name.startswith("w_") and value.dim() == 2:
+                found.add(tuple(value.shape))
+        elif isinstance(value, Part):
+            found.update(product_matrices(value, seen))
+        elif isinstance(value, (list, tuple)):
+            for v in value:
+                look(name, v)
+
+    for name, value in vars(part).items():
+        look(name, value)
+    return found
+
+
 def reads_by_products(part) -> bool:
     """input_by_products as the part's own class declares it (not a base class, and not with another forward put into the object)."""
     return bool(vars(type(part)).get("input_by_products", False)) and "forward" not in getattr(part, "__dict__", {})

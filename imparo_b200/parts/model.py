@@ -6,7 +6,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
-from .base import Part, Runtime, make_part
+from .base import Part, Runtime, make_part, product_matrices
 from .spec import ModelSpec, PartSpec, WeightSpec, keeping_for, reads_as
 
 
@@ -51,6 +51,13 @@ class Model:
     def bind(self, tensors: Dict[str, torch.Tensor]) -> None:
         for p in self.parts():
             p.bind(tensors)
+
+    def product_matrices(self, wanted: int) -> List[Tuple[int, ...]]:
+        """(N, K) of the matrices the layers multiply the step's tokens with, (N, K, wanted) of the head's, which only sees the
+        wanted rows."""
+        body = set().union(*(product_matrices(p) for p in (*self.layers, *self.before.values())))
+        head = getattr(self.head, "table", None)
+        return sorted(body) + ([(*head.shape, int(wanted))] if head is not None else [])
 
     # -- cache needs -------------------------------------------------------------------
     def cache_requirements(self) -> List[Tuple[int, Tuple]]:

@@ -79,3 +79,28 @@ def test_the_rule_and_the_room(monkeypatch):
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     finally:
         o.use_state(old)
+
+
+def test_a_model_with_cut_operands_and_without():
+    """The engine's switch: a 32-bit prompt and a mixed step give the same bits either way, through other launches."""
+    from imparo_b200.engine import Engine, StepItem
+    from imparo_b200.kernels import ops as o
+    cfg = {"architectures": ["Lfm2ForCausalLM"], "vocab_size": 512, "hidden_size": 512, "num_hidden_layers": 2,
+           "layer_types": ["conv", "full_attention"], "num_attention_heads": 8, "num_key_value_heads": 4, "block_ff_dim": 2048,
+           "block_auto_adjust_ff_dim": False, "conv_L_cache": 3, "conv_bias": False, "rope_theta": 1000000.0, "norm_eps": 1e-5,
+           "tie_embedding": True, "max_position_embeddings": 2048}
+    tokens = torch.arange(700).remainder(509).tolist()
+    outs, launched = [], []
+    for on in (True, False):
+        eng = Engine(config=cfg, seed=3, dtype="float32", ctx=1024, parallel=3, page_size=16, max_step_tokens=1024, switches={"cut_f32": on})
+        assert bool(eng.rt.launch_state.planes) == on
+        before = o.COUNTS["own"]
+        eng.add_request(1)
+        eng.add_request(2)
+        rows = [eng.step([StepItem(1, tokens[:600], list(range(600)))]),
+                eng.step([StepItem(1, tokens[600:601], [0]), StepItem(2, tokens[:300], [0, 299])])]
+        eng.check_device_status()
+        outs.append(torch.cat(rows).cpu())
+        launched.append(o.COUNTS["own"] - before)
+        del eng
+    assert same(*outs) and launched[0] > launched[1]
