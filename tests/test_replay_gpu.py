@@ -39,7 +39,7 @@ def test_family(name, dtype, family):
         assert traces.max_live_tokens(steps) < total
 
 
-SWITCHED = [{"decode_from_qkv": False}, {"fuse_producers": False}, {"unfolded": False}, {"defer_adds": False},
+SWITCHED = [{"few_rows": False}, {"decode_from_qkv": False}, {"fuse_producers": False}, {"unfolded": False}, {"defer_adds": False},
             {"gemm": "library"}, {"prefill_gemm": "library"}, {"prefill_linear": True}, {"attn_prefill": "mma"},
             {"attn_prefill": "tcgen05_one_tile"}, {"attn_side_by_side": False}, {"pad_rows": False}, {"capture_first": False},
             {"use_graphs": False}]
@@ -67,9 +67,36 @@ def test_every_switch_leaves_a_path_that_gives_the_same_logits(name, switched):
 _WIDE = {}
 
 
+class _Noted:
+    """The launches that are issued while this is entered (a captured step's once), by the launchers' names; the weight streamer's with
+    the epilogue, which tells a product that leaves split partials from one that adds them up itself."""
+
+    def __init__(self):
+        self.names = []
+
+    def __enter__(self):
+        from imparo_b200.kernels import ops
+        self.check, self.gemm_tc = ops._check, ops.gemm_tc
+
+        def check(rc, what, *kind):
+            self.names.append(what)
+            return self.check(rc, what, *kind)
+
+        def gemm_tc(x, w, out, epilogue, *args, **kw):
+            self.names.append(f"epilogue {epilogue}")
+            return self.gemm_tc(x, w, out, epilogue, *args, **kw)
+        ops._check, ops.gemm_tc = check, gemm_tc
+        return self
+
+    def __exit__(self, *exc):
+        from imparo_b200.kernels import ops
+        ops._check, ops.gemm_tc = self.check, self.gemm_tc
+
+
 def _wide_run(switched):
     """Two layers at LFM2-1.2B width: a prompt of 1,100 tokens, a second request's portion of 270 beside the first's
-    decode row, then both decoding; every wanted row's logits."""
+    decode row, both decoding, then ten more requests with short prompts and all twelve decoding (sixteen rows with the padding:
+    beyond the few-rows products); every wanted row's logits, and what the decode steps of two and of twelve rows launch."""
     import torch
     from imparo_b200.engine import Engine, StepItem
     cfg = {"architectures": ["Lfm2ForCausalLM"], "vocab_size": 8192, "hidden_size": 2048, "num_hidden_layers": 2,
@@ -77,7 +104,7 @@ def _wide_run(switched):
            "block_ff_dim": 12288, "block_auto_adjust_ff_dim": True, "block_multiple_of": 256, "conv_L_cache": 3,
            "conv_bias": False, "rope_theta": 1000000.0, "norm_eps": 1e-5, "tie_embedding": True}
     top = {k: v for k, v in switched.items() if k in ("pad_rows", "capture_first", "use_graphs")}
-    eng = Engine(config=cfg, seed=11, dtype="bfloat16", ctx=2048, parallel=3, page_size=16, max_step_tokens=2048,
+    eng = Engine(config=cfg, seed=11, dtype="bfloat16", ctx=2048, parallel=12, page_size=16, max_step_tokens=2048,
                  random_init={"norm_jitter": 0.1, "matrix_std": 0.02},
                  switches={k: v for k, v in switched.items() if k not in top}, **top)
     rng = np.random.default_rng(23)
@@ -86,15 +113,30 @@ def _wide_run(switched):
     eng.add_request(2)
     rows = [eng.step([StepItem(1, a[:1100], [0, 500, 1099])])]
     rows.append(eng.step([StepItem(1, [a[1100]], [0]), StepItem(2, b[:270], [0, 269])]))
-    for i in range(1, 8):
-        rows.append(eng.step([StepItem(1, [a[1100 + i]], [0]), StepItem(2, [b[269 + i]], [0])]))
+    with _Noted() as two:
+        for i in range(1, 8):
+            rows.append(eng.step([StepItem(1, [a[1100 + i]], [0]), StepItem(2, [b[269 + i]], [0])]))
+    more = {r: rng.integers(0, 8192, 9 + r + 4).tolist() for r in range(3, 13)}
+    for r, t in more.items():
+        eng.add_request(r)
+        rows.append(eng.step([StepItem(r, t[:-4], [len(t) - 5])]))
+    with _Noted() as twelve:
+        for i in range(4):
+            rows.append(eng.step([StepItem(r, [int(rng.integers(0, 8192))], [0]) for r in (1, 2)]
+                                 + [StepItem(r, [t[len(t) - 4 + i]], [0]) for r, t in more.items()]))
     eng.check_device_status()
-    eng.end_request(1); eng.end_request(2)
+    for r in range(1, 13):
+        eng.end_request(r)
     eng.cache.check()
     out = np.concatenate([r.cpu().numpy() for r in rows])
     del eng
     torch.cuda.empty_cache()
-    return out
+    return out, {"two rows": two.names, "twelve rows": twelve.names}
+
+
+# where a switch has to show in the launches, so that the comparison is one of two paths
+SHOWS = {"few_rows": "two rows", "decode_from_qkv": "twelve rows", "fuse_producers": "twelve rows", "unfolded": "twelve rows",
+         "defer_adds": "twelve rows", "gemm": "twelve rows"}
 
 
 @pytest.mark.parametrize("switched", SWITCHED, ids=lambda d: "-".join(f"{k}={v}" for k, v in d.items()))
@@ -103,13 +145,16 @@ def test_every_switch_at_full_width(switched):
     switch's other setting against the defaults, in bfloat16."""
     if "default" not in _WIDE:
         _WIDE["default"] = _wide_run({})
-    ref = _WIDE["default"]
-    got = _wide_run(switched)
+    ref, launched = _WIDE["default"]
+    got, other = _wide_run(switched)
     assert np.isfinite(ref).all() and np.isfinite(got).all()
     scale = float(np.abs(ref).max())
     assert scale > 0.1 and np.abs(ref[0] - ref[-1]).max() > 0.2 * scale
     err = float(np.abs(got - ref).max())
     assert err <= 2.5e-2 * scale, (switched, err, scale)
+    for name in switched:
+        if name in SHOWS:
+            assert other[SHOWS[name]] != launched[SHOWS[name]], f"{name} changes nothing in the steps it is compared in"
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
@@ -245,8 +290,9 @@ def test_full_width_layers_against_the_plain_implementation(dtype, tmp_path_fact
     """One conv layer and one attention layer at LFM2-1.2B width (hidden 2048, 32 heads in 8 groups, head 64,
     ff 8192, vocabulary 65536) from a model folder, against the plain implementation in float64 on the same
     folder: a mistake that the bfloat16 and the 32-bit path share at width (a descriptor, a table stride) cannot
-    pass here.  Three ways of cutting: the prompt whole and then single tokens; portions of 64 tokens (the
-    tensor-core product at its widest token tile); a stretch of single tokens from the start."""
+    pass here.  Four ways of cutting: the prompt whole and then single tokens; portions of 64 tokens (the
+    tensor-core product at its widest token tile); a stretch of single tokens from the start; decode steps of twelve and of
+    eight requests."""
     import torch
     from imparo_b200.engine import Engine, StepItem
     from imparo_b200.weights import write_random_model
@@ -263,7 +309,7 @@ def test_full_width_layers_against_the_plain_implementation(dtype, tmp_path_fact
     ref = _full_width_reference(d, tuple(toks))
     scale = float(np.abs(ref).max())
     tol = (2.5e-2 if dtype == "bfloat16" else 2e-5) * scale
-    eng = Engine(d, dtype=dtype, ctx=512, parallel=3, page_size=16, max_step_tokens=512)
+    eng = Engine(d, dtype=dtype, ctx=512, parallel=12, page_size=16, max_step_tokens=512)
 
     def check(got, places, what):
         for row, p in zip(got, places):
@@ -296,8 +342,20 @@ def test_full_width_layers_against_the_plain_implementation(dtype, tmp_path_fact
         check(out[:1], [i], "single tokens from the start")
         if i % 8 == 0:
             check(out[1:], [i * 4 + 31], "a portion beside a single token")
-    eng.check_device_status()
     eng.end_request(3); eng.end_request(4)
+    # 4. decode steps of twelve requests (the weight streamer with deferred adds, the combine inside the output product), then of eight
+    for live in (12, 8):
+        at = {}
+        for r in range(10, 10 + live):
+            eng.add_request(r)
+            at[r] = 9 + 23 * (r - 10)
+            eng.step([StepItem(r, toks[:at[r]], [])])
+        for i in range(3):
+            out = eng.step([StepItem(r, [toks[a + i]], [0]) for r, a in at.items()]).cpu().numpy()
+            check(out, [a + i for a in at.values()], f"{live} decode rows")
+        for r in at:
+            eng.end_request(r)
+    eng.check_device_status()
     eng.cache.check()
     del eng
     torch.cuda.empty_cache()
