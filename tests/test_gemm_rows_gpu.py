@@ -54,6 +54,30 @@ def test_most_rows_of_w():
     assert not o._rows_take(torch.zeros(9, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(64, 64, dtype=torch.bfloat16, device=DEV))
 
 
+def normed(x, nw, eps):
+    """The RMS norm of 32-bit rows in bfloat16, and how far an entry may be off.  The kernel's 32-bit value is within 2^-18 of the exact
+    one (a lane's sum of up to 64 squares, half of whose error the root leaves, and four more roundings: under 40 times 2^-24), so an
+    entry is the rounding of the exact value unless a boundary lies that near; then it may be the neighbour."""
+    h = x.double() / torch.sqrt(x.double().pow(2).mean(1, keepdim=True) + eps) * nw.double()
+    low, high = ((h * (1 + s * 2 ** -18)).to(torch.bfloat16).double() for s in (-1, 1))
+    return h.to(torch.bfloat16).double(), (high - low).abs()
+
+
+def product_of_normed(h, off, w):
+    """The product and the bound of its error: at most seventeen cuts at 2^-24 of the terms' magnitudes (a matrix instruction's, and the
+    warps' sums), and the entries of h that may be the neighbour."""
+    wa = w.double().abs()
+    return h @ w.double().T, 17 * 2 ** -24 * (h.abs() @ wa.T) + off @ wa.T
+
+
+def waiting_norm(o, x, nw, eps=1e-5):
+    T, K = x.shape
+    h = torch.full((T, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    o.rmsnorm(x.to(DEV), nw.to(DEV), eps, h, may_wait=True)
+    assert h.data_ptr() in o._S.waiting_norms and bool(h.isnan().all())
+    return h
+
+
 @pytest.mark.parametrize("F,K", [(1, 64), (9, 832), (4608, 1024), (8192, 2048), (148 * 64, 128)])
 @pytest.mark.parametrize("act,bias", [("silu", False), ("clamped_swish", True)])
 def test_gated_of_a_waiting_norm(F, K, act, bias):
@@ -63,24 +87,52 @@ def test_gated_of_a_waiting_norm(F, K, act, bias):
         x, nw = torch.randn(T, K, generator=g) * 3, 1 + 0.1 * torch.randn(K, generator=g)
         b = torch.randn(2 * F, generator=g) if bias else None
         xd, nd, wd = x.to(DEV), nw.to(DEV), w.to(DEV)
-        h, h2 = (torch.full((T, K), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        h2 = torch.full((T, K), float("nan"), dtype=torch.bfloat16, device=DEV)
         o.rmsnorm(xd, nd, 1e-5, h2)
-        o.rmsnorm(xd, nd, 1e-5, h, may_wait=True)
-        assert h.data_ptr() in o._S.waiting_norms and bool(h.isnan().all())
+        h = waiting_norm(o, x, nw)
         out = torch.full((T, F), float("nan"), dtype=torch.bfloat16, device=DEV)
         o.linear_gated(h, wd, out, act, limit=7.0, bias=b.to(DEV) if bias else None)
-        gu = h2.cpu().double() @ w.double().T + (b.double() if bias else 0.0)
-        gate, up = gu[:, :F], gu[:, F:]
+        z, d = product_of_normed(*normed(x, nw, 1e-5), w)
+        if bias:
+            z = z + b.double()
+            d = d + 2 ** -24 * z.abs()
+        gate, up, dg, du = z[:, :F], z[:, F:], d[:, :F], d[:, F:]
         if act == "silu":
             want = gate * torch.sigmoid(gate) * up
         else:
             gate, up = gate.clamp(max=7.0), up.clamp(-7.0, 7.0)
             want = gate * torch.sigmoid(1.702 * gate) * (up + 1.0)
-        # the result's own rounding (2^-8 of itself), and normed entries that fall to the other side of theirs: one unit (2^-7 of
-        # itself) of a few of the K terms
-        assert (out.double().cpu() - want).abs().max() <= 2 ** -6 * want.abs().max()
+        # an activation's slope is at most 1.2 and its value at most its argument's; the fast exponential and division: 2^-18; bfloat16: 2^-8
+        tol = 1.2 * dg * (up.abs() + 1 + du) + gate.abs() * du + 2 ** -18 * gate.abs() * (up.abs() + 1) + (2 ** -8 + 2 ** -18) * want.abs()
+        assert bool(((out.double().cpu() - want).abs() <= tol).all())
         o.make_waiting(h)
         assert torch.equal(h, h2)                                # the norm itself, when somebody else reads it
+
+
+@pytest.mark.parametrize("N,K", [(1, 64), (72, 832), (1536, 1024), (3072, 2048), (6144, 1024)])
+def test_plain_products_of_a_waiting_norm(N, K):
+    """linear into both types, and the one-part product that linear_unfolded leaves to its reader."""
+    o = ops()
+    for T in (1, 4, min(8, o.FEW_ROWS_STREAM // K)):
+        _, w, g = case(T, N, K, N + K + T)
+        x, nw = torch.randn(T, K, generator=g) * 3, 1 + 0.1 * torch.randn(K, generator=g)
+        want, d = product_of_normed(*normed(x, nw, 1e-5), w)
+        wd, h = w.to(DEV), waiting_norm(o, x, nw)
+
+        def near(got, half):
+            assert bool(((got.double().cpu() - want).abs() <= d + (2 ** -8 * (want.abs() + d) if half else 0)).all())
+        for dtype in (torch.float32, torch.bfloat16):
+            out = torch.full((T, N), float("nan"), dtype=dtype, device=DEV)
+            o.linear(h, wd, out)
+            near(out, dtype == torch.bfloat16)
+            out = torch.full((T, N), float("nan"), dtype=dtype, device=DEV)
+            made = o.linear_unfolded(h, wd, out)
+            assert isinstance(made, o.PartialProduct) and made.splits == 1 and made.shape == (T, N) and bool(out.isnan().all())
+            near(made.parts[:T * N].view(T, N), False)
+            whole = made.parts[:T * N].view(T, N).to(dtype)
+            assert made.tensor() is out and torch.equal(out, whole)
+        assert h.data_ptr() in o._S.waiting_norms and bool(h.isnan().all())
+        o.forget_waiting(h)
 
 
 @pytest.mark.parametrize("taps", [2, 3, 4])
