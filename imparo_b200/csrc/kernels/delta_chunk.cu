@@ -18,10 +18,13 @@
 // scan 82, out 16); error against 64 bits 1.1e-7 and 1.4e-7.  Which portions come here: parts/delta_rule.py.
 //
 // A request's rows are cut into chunks from its portion's first row on, so the cut depends on the portion alone.
-#include "common.cuh"
+#include "chunk_products.cuh"
 
 namespace imparo {
 namespace dc {
+
+using chunks::chunk_rows;
+using chunks::cp16;
 
 constexpr int C = 64;               // rows per chunk
 constexpr int PC = C + 4;           // row of a staged matrix with 64 columns: four floats more, so that eight lanes' 16-byte
@@ -52,25 +55,6 @@ struct Layout {
     }
 };
 
-__device__ __forceinline__ void cp16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-
-// chunk number -> request, first row, rows (0: no such chunk)
-__device__ __forceinline__ int chunk_rows(const Rows& p, int chunk, int& item, int& first) {
-    for (item = 0; item < p.n_items; ++item) {
-        const int r0 = p.item_row_start[item], n = p.item_row_start[item + 1] - r0;
-        const int chunks = (n + C - 1) / C;
-        if (chunk < chunks) {
-            first = r0 + chunk * C;
-            return min(C, n - chunk * C);
-        }
-        chunk -= chunks;
-    }
-    first = 0;
-    return 0;
-}
-
 // ---- (1) -------------------------------------------------------------------------------------------------------------
 // Bound by the issue of 32-bit arithmetic and the latency of its reads of shared memory: 3 operations per pair of rows and
 // channel for the two matrices (eight lanes share a column j of them, each with an eighth of the channels and its running
@@ -99,7 +83,7 @@ delta_local_kernel(const Rows p, float* __restrict__ scratch) {
     pdl_trigger();
     const int chunk = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     int item, first;
-    const int n = chunk_rows(p, chunk, item, first);
+    const int n = chunk_rows<C>(p, chunk, item, first);
     pdl_wait();
     if (n == 0) return;
     const int dim = p.dim, vdim = p.vdim, kvh = h / (p.heads / p.kv_heads);
@@ -403,7 +387,7 @@ delta_out_kernel(const Rows p, const float* __restrict__ scratch, float* __restr
     pdl_trigger();
     const int chunk = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * 64, tid = threadIdx.x;
     int item, first;
-    const int n = chunk_rows(p, chunk, item, first);
+    const int n = chunk_rows<C>(p, chunk, item, first);
     pdl_wait();
     if (n == 0) return;
     const int slot = p.item_slot[item];

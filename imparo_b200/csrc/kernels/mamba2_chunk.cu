@@ -15,94 +15,19 @@
 // values, state size 64 and 1,999 rows 47 + 20 + 68 us (state, scan, out), here 18 + 7 + 42 (B200; bound by the latency of the
 // products' reads at 8 warps per SM).  Error against 64 bits 1.4e-7 and 1.7e-7.  Which portions come here: parts/mamba2.py and
 // mamba2_products_pay in kernels/ops.py.
-#include "common.cuh"
+#include "chunk_products.cuh"
 
 namespace imparo {
 namespace mc {
 
+using namespace chunks;             // (a CTA has VB value columns and THREADS threads)
 constexpr int C = 64;               // rows per chunk
-constexpr int VB = 64;              // value columns of a CTA
-constexpr int THREADS = 128;        // a patch of 8 x 4 of a 64 x 64 product each
 
 struct Rows {
     const float* xbc; const float* dt; const float* A_log; const float* D;
     const int* item_row_start; const int* item_slot;
     int n_items, n_slots, heads, vdim, N, groups;
 };
-
-// chunk number -> request, first row, rows (0: no such chunk)
-__device__ __forceinline__ int chunk_rows(const Rows& p, int chunk, int& item, int& first) {
-    for (item = 0; item < p.n_items; ++item) {
-        const int r0 = p.item_row_start[item], n = p.item_row_start[item + 1] - r0;
-        const int chunks = (n + C - 1) / C;
-        if (chunk < chunks) {
-            first = r0 + chunk * C;
-            return min(C, n - chunk * C);
-        }
-        chunk -= chunks;
-    }
-    first = 0;
-    return 0;
-}
-
-__device__ __forceinline__ void cp16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-// acc[8][4] += left[k][l0 ..] x right[k][r0 ..] over k in [0, to): three 16-byte reads of shared memory per 32 operations.
-// Every 32 terms are summed by themselves: a third less rounding than one chain of 64 (3% more operations).
-// CAUSAL (to = l0 + 8): row l0 + i has the terms up to its own.  Those beyond are left out and not multiplied by zero, so that a
-// row that is not finite reaches no earlier one.
-template <int LD, bool CAUSAL = false>
-__device__ __forceinline__ void product(float2 (&acc)[8][2], const float* left, int l0, const float* right, int r0, int to) {
-#pragma unroll 1
-    for (int k0 = 0; k0 < to; k0 += 32) {
-        float2 part[8][2] = {};
-        const int end = min(k0 + 32, CAUSAL ? l0 : to);
-#pragma unroll 4
-        for (int k = k0; k < end; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(left + k * LD + l0), b = *reinterpret_cast<const float4*>(left + k * LD + l0 + 4);
-            const float4 r = *reinterpret_cast<const float4*>(right + k * VB + r0);
-            const float2 r01 = make_float2(r.x, r.y), r23 = make_float2(r.z, r.w);
-            const float av[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 a2 = make_float2(av[i], av[i]);
-                part[i][0] = __ffma2_rn(a2, r01, part[i][0]);
-                part[i][1] = __ffma2_rn(a2, r23, part[i][1]);
-            }
-        }
-        if (CAUSAL && k0 + 32 > l0) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float4 a = *reinterpret_cast<const float4*>(left + (l0 + u) * LD + l0), b = *reinterpret_cast<const float4*>(left + (l0 + u) * LD + l0 + 4);
-                const float4 r = *reinterpret_cast<const float4*>(right + (l0 + u) * VB + r0);
-                const float2 r01 = make_float2(r.x, r.y), r23 = make_float2(r.z, r.w);
-                const float av[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-                for (int i = u; i < 8; ++i) {
-                    const float2 a2 = make_float2(av[i], av[i]);
-                    part[i][0] = __ffma2_rn(a2, r01, part[i][0]);
-                    part[i][1] = __ffma2_rn(a2, r23, part[i][1]);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int v = 0; v < 2; ++v) acc[i][v] = make_float2(acc[i][v].x + part[i][v].x, acc[i][v].y + part[i][v].y);
-    }
-}
-
-// 64 rows of `cols` columns (dst rows of VB floats): zeros beyond n rows and beyond the columns there are
-__device__ __forceinline__ void fetch_rows(float* dst, const float* src, size_t stride, int n, int cols) {
-    for (int e = threadIdx.x; e < C * (VB / 4); e += THREADS) {
-        const int r = e / (VB / 4), v = (e % (VB / 4)) * 4;
-        if (r < n && v < cols) cp16(dst + r * VB + v, src + (size_t)r * stride + v);
-        else *reinterpret_cast<float4*>(dst + r * VB + v) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-}
 
 // ---- (1) -------------------------------------------------------------------------------------------------------------
 template <int NM, int HG>
@@ -119,7 +44,7 @@ state_kernel(const Rows p, float* __restrict__ chunk_state, float* __restrict__ 
     pdl_trigger();
     const int h0 = blockIdx.x * HG, chunk = blockIdx.y, v0 = blockIdx.z * VB, tid = threadIdx.x;
     int item, first;
-    const int n = chunk_rows(p, chunk, item, first);
+    const int n = chunk_rows<C>(p, chunk, item, first);
     const int inner = p.heads * p.vdim, g = h0 / (p.heads / p.groups);
     const size_t channels = (size_t)inner + 2 * p.groups * p.N;
     pdl_wait();
@@ -131,7 +56,7 @@ state_kernel(const Rows p, float* __restrict__ chunk_state, float* __restrict__ 
         if (r < n && s < p.N) cp16(bs + r * NM + s, rows + (size_t)r * channels + inner + g * p.N + s);
         else *reinterpret_cast<float4*>(bs + r * NM + s) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    fetch_rows(xs, rows + (size_t)h0 * p.vdim + v0, channels, n, cols);
+    fetch_rows<C>(xs, rows + (size_t)h0 * p.vdim + v0, channels, n, cols);
     cp_commit();
     for (int e = tid; e < HG * C; e += THREADS) {
         const int hh = e / C, r = e % C;
@@ -156,7 +81,7 @@ state_kernel(const Rows p, float* __restrict__ chunk_state, float* __restrict__ 
     }
     const int nq = (tid >> 4) * 8, vq = (tid & 15) * 4;
     for (int hh = 0; hh < HG; ++hh) {
-        if (hh + 1 < HG) fetch_rows(xs + ((hh + 1) & 1) * C * VB, rows + (size_t)(h0 + hh + 1) * p.vdim + v0, channels, n, cols);
+        if (hh + 1 < HG) fetch_rows<C>(xs + ((hh + 1) & 1) * C * VB, rows + (size_t)(h0 + hh + 1) * p.vdim + v0, channels, n, cols);
         cp_commit();
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
@@ -247,7 +172,7 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
     pdl_trigger();
     const int h0 = blockIdx.x * HG, chunk = blockIdx.y, v0 = blockIdx.z * VB, tid = threadIdx.x;
     int item, first;
-    const int n = chunk_rows(p, chunk, item, first);
+    const int n = chunk_rows<C>(p, chunk, item, first);
     const int inner = p.heads * p.vdim, g = h0 / (p.heads / p.groups);
     const size_t channels = (size_t)inner + 2 * p.groups * p.N;
     pdl_wait();
@@ -264,7 +189,7 @@ out_kernel(const Rows p, const float* __restrict__ chunk_state, float* __restric
             if (k < p.N && v < cols) cp16(s + k * VB + v, from + (size_t)k * p.vdim + v);
             else *reinterpret_cast<float4*>(s + k * VB + v) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        fetch_rows(s + NM * VB, rows + (size_t)(h0 + hh) * p.vdim + v0, channels, n, cols);
+        fetch_rows<C>(s + NM * VB, rows + (size_t)(h0 + hh) * p.vdim + v0, channels, n, cols);
     };
     for (int e = tid; e < C * (NM / 4); e += THREADS) {    // a lane a row: its four entries go to four rows of the transposed tile
         const int r = e % C, s = (e / C) * 4;

@@ -15,34 +15,13 @@
 // values and 2,048 rows 37 + 9 + 81 us (local, scan, out), here 15 + 9 + 28 (B200).  Against 64 bits the states are as exact as the row
 // walk's, the outputs in the median too (2e-7; a row whose n . q nearly cancels is off by more either way).
 #include "mlstm_chunk.cuh"
+#include "chunk_products.cuh"
 
 namespace imparo {
 namespace mx {
 
+using namespace chunks;             // (a block has VB value columns and THREADS threads)
 constexpr int C = MLSTM_PRODUCTS_CHUNK;
-constexpr int VB = 64;              // value columns of a block
-constexpr int THREADS = 128;        // a patch of 8 x 4 of a 64 x 64 product each
-
-// chunk number -> request, first row, rows (0: no such chunk)
-__device__ __forceinline__ int chunk_rows(const MlstmProducts& p, int chunk, int& item, int& first) {
-    for (item = 0; item < p.n_items; ++item) {
-        const int r0 = p.item_row_start[item], n = p.item_row_start[item + 1] - r0;
-        const int chunks = (n + C - 1) / C;
-        if (chunk < chunks) {
-            first = r0 + chunk * C;
-            return min(C, n - chunk * C);
-        }
-        chunk -= chunks;
-    }
-    first = 0;
-    return 0;
-}
-
-__device__ __forceinline__ void cp16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ float log_sigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
@@ -73,60 +52,6 @@ __device__ __forceinline__ void factors(float m, int n, float* as, float* fs, co
     }
 }
 
-// acc[8][4] += left[k][l0 ..] x right[k][r0 ..] over k in [0, to): three 16-byte reads of shared memory per 32 operations.
-// Every 32 terms are summed by themselves: a third less rounding than one chain of 64 (3% more operations).
-// CAUSAL (to = l0 + 8): row l0 + i has the terms up to its own.  Those beyond are left out and not multiplied by zero, so that a
-// row that is not finite reaches no earlier one.
-template <int LD, bool CAUSAL = false>
-__device__ __forceinline__ void product(float2 (&acc)[8][2], const float* left, int l0, const float* right, int r0, int to) {
-#pragma unroll 1
-    for (int k0 = 0; k0 < to; k0 += 32) {
-        float2 part[8][2] = {};
-        const int end = min(k0 + 32, CAUSAL ? l0 : to);
-#pragma unroll 4
-        for (int k = k0; k < end; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(left + k * LD + l0), b = *reinterpret_cast<const float4*>(left + k * LD + l0 + 4);
-            const float4 r = *reinterpret_cast<const float4*>(right + k * VB + r0);
-            const float2 r01 = make_float2(r.x, r.y), r23 = make_float2(r.z, r.w);
-            const float av[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 a2 = make_float2(av[i], av[i]);
-                part[i][0] = __ffma2_rn(a2, r01, part[i][0]);
-                part[i][1] = __ffma2_rn(a2, r23, part[i][1]);
-            }
-        }
-        if (CAUSAL && k0 + 32 > l0) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float4 a = *reinterpret_cast<const float4*>(left + (l0 + u) * LD + l0), b = *reinterpret_cast<const float4*>(left + (l0 + u) * LD + l0 + 4);
-                const float4 r = *reinterpret_cast<const float4*>(right + (l0 + u) * VB + r0);
-                const float2 r01 = make_float2(r.x, r.y), r23 = make_float2(r.z, r.w);
-                const float av[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-                for (int i = u; i < 8; ++i) {
-                    const float2 a2 = make_float2(av[i], av[i]);
-                    part[i][0] = __ffma2_rn(a2, r01, part[i][0]);
-                    part[i][1] = __ffma2_rn(a2, r23, part[i][1]);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int v = 0; v < 2; ++v) acc[i][v] = make_float2(acc[i][v].x + part[i][v].x, acc[i][v].y + part[i][v].y);
-    }
-}
-
-// 64 rows of `cols` columns (dst rows of VB floats): zeros beyond n rows and beyond the columns there are
-__device__ __forceinline__ void fetch_rows(float* dst, const float* src, size_t stride, int n, int cols) {
-    for (int e = threadIdx.x; e < C * (VB / 4); e += THREADS) {
-        const int r = e / (VB / 4), v = (e % (VB / 4)) * 4;
-        if (r < n && v < cols) cp16(dst + r * VB + v, src + (size_t)r * stride + v);
-        else *reinterpret_cast<float4*>(dst + r * VB + v) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-}
-
 // ---- (1) -------------------------------------------------------------------------------------------------------------
 template <int NM> struct LocalSmem { static constexpr size_t FLOATS = (size_t)C * NM + C * VB + 3 * C; };
 
@@ -142,7 +67,7 @@ mlstm_local_kernel(const MlstmProducts p) {
     pdl_trigger();
     const int chunk = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * VB, tid = threadIdx.x;
     int item, first;
-    const int n = chunk_rows(p, chunk, item, first);
+    const int n = chunk_rows<C>(p, chunk, item, first);
     pdl_wait();
     if (n == 0) return;
     const float* rows = p.proj + (size_t)first * p.stride;
@@ -152,7 +77,7 @@ mlstm_local_kernel(const MlstmProducts p) {
         if (r < n && d < p.dim) cp16(ks + r * NM + d, rows + (size_t)r * p.stride + p.k_off + h * p.dim + d);
         else *reinterpret_cast<float4*>(ks + r * NM + d) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    fetch_rows(xs, rows + p.v_off + (size_t)h * p.vdim + v0, p.stride, n, cols);
+    fetch_rows<C>(xs, rows + p.v_off + (size_t)h * p.vdim + v0, p.stride, n, cols);
     cp_commit();
     gates(p, first, n, h, as, fs);
     __syncthreads();
@@ -231,7 +156,7 @@ mlstm_out_kernel(const MlstmProducts p) {
     pdl_trigger();
     const int chunk = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     int item, first;
-    const int n = chunk_rows(p, chunk, item, first);
+    const int n = chunk_rows<C>(p, chunk, item, first);
     pdl_wait();
     if (n == 0) return;
     const float* rows = p.proj + (size_t)first * p.stride;
@@ -244,7 +169,7 @@ mlstm_out_kernel(const MlstmProducts p) {
             if (k < p.dim && v < cols) cp16(right + k * VB + v, from + (size_t)k * p.vdim + v);
             else *reinterpret_cast<float4*>(right + k * VB + v) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        fetch_rows(right + NM * VB, rows + p.v_off + (size_t)h * p.vdim + v0, p.stride, n, cols);
+        fetch_rows<C>(right + NM * VB, rows + p.v_off + (size_t)h * p.vdim + v0, p.stride, n, cols);
         cp_commit();
     };
     fetch(0);
