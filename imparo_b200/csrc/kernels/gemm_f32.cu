@@ -225,11 +225,10 @@ sgemm_split_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, co
         if (lane == 0) {
             pdl_wait();                                       // the planes were written by the kernel before
             int kb = 0;
-            bool ok = true;
             // (the first stretch's MMAs also wait for the workers to have cleared the accumulators: acc_empty, below)
             for (; kb < p.kblocks; ++kb) {
                 const int s = kb % STAGES;
-                if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 93, blockIdx.x, kb); ok = false; break; }
+                if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 93, blockIdx.x, kb); break; }
                 uint8_t* base = smem + s * STAGE;
                 mbar_expect_tx(&full[s], STAGE);
 #pragma unroll
@@ -238,7 +237,8 @@ sgemm_split_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, co
                     tma_load_2d(base + 3 * A_PLANE + u * B_PLANE, &map_w, &full[s], kb * 64, u * p.N + n0);
                 }
             }
-            if (!ok) for (int u = max(0, kb - STAGES); u < kb; ++u) mbar_wait(&full[u % STAGES], (u / STAGES) & 1);      // the copies land
+            // the last copies land before the warp leaves, also where the MMAs gave up on them
+            for (int u = max(0, kb - STAGES); u < kb; ++u) mbar_wait(&full[u % STAGES], (u / STAGES) & 1);
         }
     } else {
         // a thread's piece of a stretch: 8 neighbours of k (chunk `c`) of the rows r0, r0 + ROUND, ...

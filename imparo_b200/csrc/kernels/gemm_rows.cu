@@ -169,8 +169,9 @@ __device__ __forceinline__ void rows_product(const CUtensorMap& map_w, const Par
                 }
             }
         }
-        if (lane == 0 && !ok) {
-            report(p.status, IMPARO_ST_WAIT_LIMIT, 50, blockIdx.x, i);
+        if (lane == 0) {
+            if (!ok) report(p.status, IMPARO_ST_WAIT_LIMIT, 50, blockIdx.x, i);
+            // the last copies land before the warp leaves, also where the multiplying warps gave up on them
             for (int u = max(0, i - STAGES); u < i; ++u) wait_for(&full[u % STAGES], (u / STAGES) & 1);
         }
         __syncwarp();
