@@ -199,7 +199,10 @@ sgemm_split_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, co
             for (int kb = 0; kb < p.kblocks; ++kb) {
                 const int s = kb % STAGES, b = kb & 1;
                 // CUT: the workers arrive once more, when they have cleared all accumulators
-                if ((CUT || kb >= 2) && !mbar_wait(&acc_empty[b], ((kb >> 1) - (CUT ? 0 : 1)) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 90, blockIdx.x, kb); break; }
+                if ((CUT || kb >= 2) && !mbar_wait(&acc_empty[b], ((kb >> 1) - (CUT ? 0 : 1)) & 1)) {
+                    report(p.status, IMPARO_ST_WAIT_LIMIT, 90, blockIdx.x, kb);
+                    break;
+                }
                 if (!mbar_wait(&full[s], (kb / STAGES) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 91, blockIdx.x, kb); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t a0 = smem_desc(smem_u32(smem) + s * STAGE), b0 = smem_desc(smem_u32(smem) + s * STAGE + 3 * A_PLANE);
@@ -228,7 +231,10 @@ sgemm_split_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, co
             // (the first stretch's MMAs also wait for the workers to have cleared the accumulators: acc_empty, below)
             for (; kb < p.kblocks; ++kb) {
                 const int s = kb % STAGES;
-                if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) { report(p.status, IMPARO_ST_WAIT_LIMIT, 93, blockIdx.x, kb); break; }
+                if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) {
+                    report(p.status, IMPARO_ST_WAIT_LIMIT, 93, blockIdx.x, kb);
+                    break;
+                }
                 uint8_t* base = smem + s * STAGE;
                 mbar_expect_tx(&full[s], STAGE);
 #pragma unroll
@@ -381,7 +387,8 @@ sgemm_split_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, co
 // The planes of a matrix of `rows` rows of K (row stride ld): [3][rows][Kp] bfloat16, Kp = K rounded up to 8, zeros beyond K.  A thread
 // cuts eight neighbours.  Bound by memory: 4 bytes in, 6 out.  Both operands in one launch: the first a_rows rows are A's.
 __global__ void __launch_bounds__(256)
-cut_planes_kernel(const float* __restrict__ a, int lda, int a_rows, const float* __restrict__ w, int w_rows, int K, uint4* __restrict__ pa, uint4* __restrict__ pw) {
+cut_planes_kernel(const float* __restrict__ a, int lda, int a_rows, const float* __restrict__ w, int w_rows, int K, uint4* __restrict__ pa,
+                  uint4* __restrict__ pw) {
     pdl_trigger();
     const int per_row = (K + 7) / 8;
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -473,7 +480,8 @@ extern "C" int imparo_sgemm_cut(const float* A, const float* W, float* C, int M,
     int rc = tc::get_map(pa, 3 * (uint64_t)M, Kp, Kp, 128u, &ma);
     if (!rc) rc = tc::get_map(pw, 3 * (uint64_t)N, Kp, Kp, thin ? 64u : 128u, &mw);
     if (rc) return rc;
-    launch(sp::cut_planes_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, A, lda, M, W, N, K, reinterpret_cast<uint4*>(pa), reinterpret_cast<uint4*>(pw));
+    launch(sp::cut_planes_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, A, lda, M, W, N, K, reinterpret_cast<uint4*>(pa),
+           reinterpret_cast<uint4*>(pw));
     IMPARO_CHECK_LAUNCH();
     const sp::Params p{A, W, C, M, N, K, lda, ldc, accumulate, (K + 63) / 64, status};
     return thin ? sp::launch_split<64, true>(p, ma, mw, stream) : sp::launch_split<128, true>(p, ma, mw, stream);

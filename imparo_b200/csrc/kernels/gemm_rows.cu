@@ -6,13 +6,13 @@
 // What bounds it: W streams from HBM once, and a step is a chain of some hundred such products, so what the kernels cost beside
 // their bytes counts as much.  So K stays whole inside a CTA (no split partials to fold by a later kernel, no cluster), every SM
 // gets the same number of output features to within one (F / 148, any number: no tile of 128 rows that leaves SMs idle), and
-// all weights a CTA can hold ahead (96 KB) are requested before the wait on the kernel ahead.
+// all weights that the ring holds (64 KB) are requested before the wait on the kernel ahead.
 //
 // A ninth warp copies W into a ring of stages, two tiles of 8 rows by 512 k each: W is seen as [k / 64][row][64 k], so that one tensor
-// copy brings a tile of any first row, 8 KB, in 128-byte lines swizzled by row.  The eight others share a stage's k: a warp owns two groups of 32.  Sixteen rows of W are the M of
-// mma.sync.m16n8k16 and the T tokens its N; k is permuted inside a group of 32 the same way for both operands (lane c of a row holds
-// k = 8c .. 8c+7), so a 16-byte load is two fragments.  The tokens of a stretch of 2,048 k stay in registers.  At the end the eight
-// warps' sums meet in shared memory and are added in warp order.
+// copy brings a tile of any first row, 8 KB, in 128-byte lines swizzled by row.  The eight others share a stage's k: a warp owns two
+// groups of 32.  Sixteen rows of W are the M of mma.sync.m16n8k16 and the T tokens its N; k is permuted inside a group of 32 the
+// same way for both operands (lane c of a row holds k = 8c .. 8c+7), so a 16-byte load is two fragments.  The tokens of a stretch of
+// 2,048 k stay in registers.  At the end the eight warps' sums meet in shared memory and are added in warp order.
 // (The tensor cores run at a few percent of their rate here, so tcgen05 would gain nothing: eight tokens fill a sixteenth of its
 // smallest tile, and its accumulator would have to come back through tensor memory.  W by untiled copies of 1 KB, or by 16-byte
 // cp.async of every thread, streamed at 3.4 TB/s with as many bytes in flight, this way at 5.5.)
@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(THREADS + 32, 2) rows_kernel(const __grid_cons
 
 // (a name of its own in profiles and timelines)
 template <int IN>
-__global__ void __launch_bounds__(nr::THREADS + 32, 2) gated_conv_product_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ nr::Params p) {
+__global__ void __launch_bounds__(nr::THREADS + 32, 2)
+gated_conv_product_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ nr::Params p) {
     nr::rows_product<IN, nr::OUT_CONV>(map_w, p);
 }
 

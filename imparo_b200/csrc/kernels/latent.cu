@@ -177,7 +177,8 @@ heads_linear_kernel(const T* __restrict__ x, size_t x_stride, const T* __restric
     const int t0 = blockIdx.z * HL_ROWS;
     const T* wr = w + ((size_t)h * n_out + o) * n_in;
     // A step of few rows waits for each trip to memory and for little else: the matrix row's first entries are read before the wait
-    // (no kernel writes them), all rows' inputs of a turn together, and a row's gate by the lane that will write the row (eight rows, 16 heads of 64: 3.9 -> 3.5 us).
+    // (no kernel writes them), all rows' inputs of a turn together, and a row's gate by the lane that will write the row (eight
+    // rows, 16 heads of 64: 3.9 -> 3.5 us).
     T w0[HL_EARLY];
 #pragma unroll
     for (int k = 0; k < HL_EARLY; ++k) w0[k] = o < n_out && lane + 32 * k < n_in ? wr[lane + 32 * k] : from_f32<T>(0.f);

@@ -128,8 +128,9 @@ moe_pick_kernel(const float* __restrict__ logits, int n_rows, int experts, int c
     pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r = blockIdx.x * 4 + warp;
-    // For the few rows of a decode step this is one warp's chain (5.0 -> 3.5 us for eight rows).  So it has one trip to memory: a logit's pieces together, the first
-    // experts' corrections before the wait (no kernel writes them), and nothing that was written is read back.
+    // For the few rows of a decode step this is one warp's chain (5.0 -> 3.5 us for eight rows).  So it has one trip to memory: a
+    // logit's pieces together, the first experts' corrections before the wait (no kernel writes them), and nothing that was written
+    // is read back.
     const float early = correction && lane < experts ? correction[lane] : 0.f;
     pdl_wait();
     if (r >= n_rows) return;

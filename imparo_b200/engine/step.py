@@ -155,8 +155,9 @@ class StepFunction:
         With pad_rows the one-token rows are filled up to padded_rows(their number) with rows that belong to no
         request: token 0 at position 0 of the cache's spare page and slot, logits wanted (their rows come after
         every real wanted row; host["n_want_real"] says how many are real).  A row reads only its own token,
-        cache and state, so the real rows' results do not change; the step's shape does: it no longer follows
-        every change of the number of decoding requests."""
+        cache and state, so what the padding rows hold reaches no real row.  The step's shape does change: it no longer follows
+        every change of the number of decoding requests, and the number of rows may choose another kernel, whose sums are in
+        another order (five to eight rows of 1,536 or 2,048, for instance): the same results to rounding, not bit for bit."""
         cache = self.cache
         n_single = 0
         lens = [len(it.tokens) for it in items]

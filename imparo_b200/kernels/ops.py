@@ -708,9 +708,10 @@ FEW_ROWS_STREAM = 8192
 
 
 def _rows_pay(T: int, width: int) -> bool:
-    """Whether a product of T rows into (width: the stream's) or beside a stream gains by the few-rows kernel: up to four rows always,
-    above that where the stream's norms are inside products.  (Eight rows through routed experts, whose norms stand alone: 493 us with
-    it and 514 without, but another order of the sums, and a choice between two experts of nearly equal score may go by that.)"""
+    """Whether a product of T rows into (width: the stream's) or beside a stream gains by the few-rows kernel: streams of at most
+    FEW_ROWS_STREAM entries; of these up to four rows always, above that where the stream's norms are inside products.  (Eight rows
+    through routed experts, whose norms stand alone: 493 us with it and 514 without, but another order of the sums than they had,
+    and a choice between two experts of nearly equal score may go by that.  It is no promise: one to four rows are ordered otherwise.)"""
     return T * width <= FEW_ROWS_STREAM and (T <= 4 or _S.rows_width == width)
 
 
