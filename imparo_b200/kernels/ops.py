@@ -369,7 +369,8 @@ def group_rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, groups: int, out
     """out[r] = x[rows[r]] (or x[r]) cut into `groups` equal stretches, each divided by its own root mean square, times w.
     A group_norm_add left pending on x is carried out by the same kernel when the norm reads every row in place."""
     _cuda(x, w, out, rows)
-    forget_waiting(out)
+    if _S.waiting_norms:
+        forget_waiting(out)
     n, width = out.shape
     _need(x.dtype == torch.float32 and w.dtype == torch.float32, "group_rmsnorm reads a float32 stream and float32 weights")
     _need(x.shape[1] == width and w.numel() == width and width % groups == 0, "group_rmsnorm: widths and groups")
@@ -415,7 +416,8 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor,
     linear_unfolded, linear_swiglu, linear_gated and linear_conv_rows only, before x changes: with few rows nothing is launched
     then, and those products norm the stream themselves."""
     _cuda(x, w, out, rows)
-    forget_waiting(out)
+    if _S.waiting_norms:
+        forget_waiting(out)
     if may_wait and rows is None and x.shape[0] <= FEW_ROWS and _norm_may_wait(x, w, out):
         _S.rows_width = x.shape[1]
         _S.waiting_norms[out.data_ptr()] = (x, w, float(eps), out)          # (out: its address stays its own while the entry is there)
@@ -2199,7 +2201,8 @@ def streams_norm(x: torch.Tensor, n: int, coef: Optional[torch.Tensor], w: torch
     x: float32 [*, n * width]; rows (int32) picks input rows.  A streams_mix_add left pending on x is carried out
     by the same kernel when the norm reads every row in place."""
     _cuda(x, coef, w, out, rows)
-    forget_waiting(out)
+    if _S.waiting_norms:
+        forget_waiting(out)
     n_rows, width = out.shape
     _need(x.dtype == torch.float32 and x.is_contiguous() and x.shape[1] == n * width, "streams_norm: x float32 [rows, n * width]")
     _need(w.dtype == torch.float32 and w.numel() == width, "streams_norm: weight float32 [width]")
