@@ -10,7 +10,8 @@
 // Everything is 32-bit; maxima are walked row by row, and a weight between two rows is the product of the rows' factors between
 // them, as the row walk would have it (never the exponential of a difference of long sums).
 //
-// Bound by the issue of 32-bit products and the latency of their reads of shared memory (8 warps per SM).  In mlstm.cu a chunk's CTA
+// Bound by the latency of the products' own operations and of their reads of shared memory at 7 to 8 warps per SM (the output launch
+// issues in 31% of the cycles, its 32-bit units work in 17%).  In mlstm.cu a chunk's CTA
 // walks its rows one after the other with a state column per lane: with 8 heads of 64 keys and 128
 // values and 2,048 rows 37 + 9 + 81 us (local, scan, out), here 15 + 9 + 28 (B200).  Against 64 bits the states are as exact as the row
 // walk's, the outputs in the median too (2e-7; a row whose n . q nearly cancels is off by more either way).
